@@ -180,6 +180,25 @@ def test_embedding_backward_matches_oracle_bit_for_bit_and_aten_closely(backend,
         ops.check_device_status()
 
 
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 33), (torch.float32, 264), (torch.bfloat16, 1), (torch.bfloat16, 67), (torch.float16, 66), (torch.bfloat16, 264), (torch.float16, 4104)])
+def test_embedding_backward_at_the_edges_of_its_batches_and_windows(backend, dtype, D):
+    """Rows with counts on both sides of the long-row limit (32), of the batch of loads and of the
+    CTA's width, and positions on both sides of a sorting window (2^17), bit for bit."""
+    from conftest import bits_equal
+
+    g = torch.Generator().manual_seed(D)
+    counts = [0, 1, 2, 3, 4, 5, 15, 16, 17, 31, 32, 33, 34, 47, 48, 49, 63, 64, 65, 96, 97, 255, 257, 1000]
+    idx = torch.repeat_interleave(torch.arange(len(counts)) * 7, torch.tensor(counts))
+    if D == 33:  # long rows that cross from one window of positions into the next
+        idx = torch.cat([idx, torch.full((2**17,), 3), idx[-1300:], torch.full((2,), 3)])
+    else:
+        idx = idx[torch.randperm(idx.numel(), generator=g)]
+    grad = torch.randn((idx.numel(), D), generator=g).to(dtype)
+    V = 7 * len(counts) + 5
+    got = backend[get_operator(EMB)](grad.to(DEV), idx.to(DEV), V, 7, False)
+    assert bits_equal(oracle.embedding_backward(grad, idx, V, 7, False), got.cpu())
+
+
 def test_full_size_embedding_backward(backend):
     c = named_case("embedding_backward_bf16_128256x4096_16384")
     op = get_operator(c.op)
