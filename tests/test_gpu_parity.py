@@ -290,6 +290,30 @@ def test_argmax_rows_where_whole_vectors_are_skipped(backend, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [33, 257, 4095, 4097, 8209, 50257])
+def test_row_reductions_of_rows_off_the_16_byte_grid(backend, dtype, cols):
+    """Every phase of a row's start against the 16-byte grid, the largest element (and a NaN) in
+    the first elements, the last ones and at the edges of the vectors; split and unsplit rows."""
+    g = torch.Generator().manual_seed(cols)
+    argmax, total = backend[torch.ops.aten.argmax.default], backend[torch.ops.aten.sum.dim_IntList]
+    for rows in (17, 300):
+        base = torch.randn(rows * cols + 1, generator=g).to(dtype).to(DEV)[1:]  # the base is off the grid too
+        x = base.view(rows, cols)
+        for r in range(rows):
+            x[r, (0, 1, 7, 8, cols - 1, cols - 2, cols // 2)[r % 7]] = 9.0
+        assert torch.equal(torch.argmax(x, -1), argmax(x, -1))
+        exact = x.double().sum(-1)
+        # an fp32 sum of n terms in any order is within n 2^-24 sum|x| of the exact one; the result is rounded once
+        bound = cols * 2.0**-24 * x.double().abs().sum(-1) + exact.abs() * {torch.float32: 2.0**-24, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype]
+        assert bool(((total(x, [-1]).double() - exact).abs() <= bound).all())
+        x[3, cols - 1] = x[5, 2] = float("nan")
+        x[7] = float("-inf")
+        x[8] = -0.0
+        x[8, cols // 2 :] = 0.0  # equal to the elements before it: the first one counts
+        assert torch.equal(torch.argmax(x.cpu().float(), -1), argmax(x, -1).cpu())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_gather_along_the_last_dim(backend, dtype):
     """2-D gather along the last dim: 16 bytes of adjacent outputs per thread; fewer index rows
     than source rows, a pitched source, an index width that is not a multiple of the vector
