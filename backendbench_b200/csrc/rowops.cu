@@ -171,6 +171,80 @@ softmax_bwd_resident(const T* __restrict__ g, const T* __restrict__ y, void* __r
   }
 }
 
+// Rows too long for the registers of a CTA, or off the 16-byte grid (a vocabulary of 50,257):
+// one CTA per row, single elements up to the row's first 16-byte boundary and behind its
+// last one, 16-byte accesses in between, four of each operand in flight per thread. The first
+// pass needs grad alone for log_softmax (and both operands for softmax); the second reads it
+// again from L2. All three rows have to lie at the same offset from the grid. Bound by HBM:
+// log_softmax, bf16 4096 x 50257, 205 us (6.0 TB/s; a warp per row with element-wise accesses,
+// the kernel below, 468 us).
+template <typename T, bool IS_LOG>
+__global__ void __launch_bounds__(512) softmax_bwd_stream(const T* __restrict__ g, const T* __restrict__ y, T* __restrict__ out, int cols) {
+  constexpr int VE = Vec<T>::N;
+  __shared__ float red[64];
+  const int64_t row = blockIdx.x;
+  const T* gr = g + row * cols;
+  const T* yr = y + row * cols;
+  T* orow = out + row * cols;
+  const int t = threadIdx.x, nth = blockDim.x;
+  const int to_grid = static_cast<int>((16u - (reinterpret_cast<uintptr_t>(gr) & 15u)) & 15u) / static_cast<int>(sizeof(T));
+  const int lead = to_grid < cols ? to_grid : cols;
+  const int nv = (cols - lead) / VE, tail = lead + nv * VE;
+  const int single = t < lead ? t : (tail + t - lead < cols ? tail + t - lead : -1);  // one of the at most 2 (VE - 1) elements off the vectors
+  const T* gv = gr + lead;
+  const T* yv = yr + lead;
+  float s = 0.f;
+  if (single >= 0) s = IS_LOG ? to_f32(gr[single]) : to_f32(gr[single]) * to_f32(yr[single]);
+  auto take = [&](const uint4& rg, const uint4& ry) {
+    if (IS_LOG) {
+      vec_accumulate<T>(s, rg);
+    } else {
+      float fg[VE], fy[VE];
+      widen<T>(rg, fg);
+      widen<T>(ry, fy);
+#pragma unroll
+      for (int e = 0; e < VE; ++e) s += fg[e] * fy[e];
+    }
+  };
+  int j = t;
+  for (; j + 3 * nth < nv; j += 4 * nth) {
+    uint4 rg[4], ry[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      rg[u] = ld_keep(gv + (j + u * nth) * VE);
+      ry[u] = IS_LOG ? rg[u] : ld_keep(yv + (j + u * nth) * VE);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) take(rg[u], ry[u]);
+  }
+  for (; j < nv; j += nth) {
+    const uint4 rg = ld_keep(gv + j * VE);
+    take(rg, IS_LOG ? rg : ld_keep(yv + j * VE));
+  }
+  s = block_reduce_once(s, SumF{}, 0.f, red, 0);
+  auto gradient = [&](float fg, float fy) { return IS_LOG ? fg - ex2_approx(fy * kLog2e) * s : (fg - s) * fy; };
+  if (single >= 0) orow[single] = from_f32<T>(gradient(to_f32(gr[single]), to_f32(yr[single])));
+  auto give = [&](int jj, const uint4& rg, const uint4& ry) {
+    float fg[VE], fy[VE];
+    widen<T>(rg, fg);
+    widen<T>(ry, fy);
+#pragma unroll
+    for (int e = 0; e < VE; ++e) fg[e] = gradient(fg[e], fy[e]);
+    st_stream(orow + lead + jj * VE, narrow<T>(fg));
+  };
+  for (j = t; j + 3 * nth < nv; j += 4 * nth) {
+    uint4 rg[4], ry[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      ry[u] = ld_stream(yv + (j + u * nth) * VE);
+      rg[u] = ld_stream(gv + (j + u * nth) * VE);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) give(j + u * nth, rg[u], ry[u]);
+  }
+  for (; j < nv; j += nth) give(j, ld_stream(gv + j * VE), ld_stream(yv + j * VE));
+}
+
 // Any geometry and alignment: one warp per (outer, inner) line, elements `inner` apart,
 // two passes over the line (the second from cache).
 template <typename T, bool IS_LOG>
@@ -1491,6 +1565,15 @@ static int softmax_bwd_T(const void* g, const void* y, void* out, int64_t outer,
       }
       return check_launch();
     }
+  }
+  const bool same_phase = (((reinterpret_cast<uintptr_t>(g) ^ reinterpret_cast<uintptr_t>(y)) | (reinterpret_cast<uintptr_t>(g) ^ reinterpret_cast<uintptr_t>(out))) & 15u) == 0;
+  // shorter rows are a warp's work (the kernel below); a CTA for each would idle most of its threads
+  if (inner == 1 && dto == dti && same_phase && dim > kRaggedMaxCols && dim < (1LL << 30) && outer <= 0x7fffffffLL) {
+    int64_t th = (dim / VE + 31) / 32 * 32;
+    th = th < 128 ? 128 : (th > 512 ? 512 : th);
+    if (is_log) softmax_bwd_stream<T, true><<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(pg, py, static_cast<T*>(out), static_cast<int>(dim));
+    else softmax_bwd_stream<T, false><<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(pg, py, static_cast<T*>(out), static_cast<int>(dim));
+    return check_launch();
   }
   const int64_t lines = outer * inner;
   if ((lines + 3) / 4 > 0x7fffffffLL) return B200_EINVAL;

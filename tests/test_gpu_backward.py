@@ -67,6 +67,27 @@ def test_ragged_non_last_dim_and_strided_inputs(backend, dtype):
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [1025, 2048 + 1, 8199, 33000, 50257, 65536])
+def test_long_rows_off_the_grid_or_past_the_registers(backend, dtype, cols):
+    """Rows that start at every offset from the 16-byte grid, bases on and off it (grad, output and
+    result alike, or the base of one of them differently), against the fp64 formulas."""
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    for rows, shift_g, shift_y in ((9, 0, 0), (5, 1, 1), (3, 0, 1)):
+        grad = torch.randn(rows * cols + 1, device=DEV, generator=g).to(dtype)[shift_g : shift_g + rows * cols].view(rows, cols)
+        x = torch.randn(rows, cols, device=DEV, generator=g)
+        for spec, fwd in ((SOFT, torch.softmax), (LOGSOFT, torch.log_softmax)):
+            y = torch.empty(rows * cols + 1, device=DEV, dtype=dtype)[shift_y : shift_y + rows * cols].view(rows, cols).copy_(fwd(x, -1))
+            got = backend[get_operator(spec)](grad, y, -1, dtype)
+            gd, yd = grad.double(), y.double()
+            want = gd - yd.exp() * gd.sum(-1, keepdim=True) if spec == LOGSOFT else (gd - (gd * yd).sum(-1, keepdim=True)) * yd
+            # an fp32 sum of n terms is off by n 2^-24 sum|terms| at most; ex2 by 2^-21 of its value (argument and unit); one rounding of the result
+            terms = gd if spec == LOGSOFT else gd * yd
+            off = (cols * 2.0**-24 * terms.abs().sum(-1, keepdim=True) + (2.0**-20 * terms.sum(-1, keepdim=True).abs() if spec == LOGSOFT else 0)) * (yd.exp() if spec == LOGSOFT else yd)
+            bound = off + want.abs() * {torch.float32: 2.0**-21, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype] + gd.abs() * 2.0**-22 * (1 if spec == LOGSOFT else yd) + (2.0**-24 if dtype == torch.float16 else 0)
+            assert bool(((got.double() - want).abs() <= bound).all()), (spec, rows, float(((got.double() - want).abs() - bound).max()))
+
+
 def test_float_gradients_for_a_half_input(backend):
     """The half_to_float form: fp32 grad_output / output, 16-bit grad_input."""
     g = torch.Generator(device=DEV).manual_seed(7)
