@@ -291,10 +291,12 @@ __global__ void __launch_bounds__(256) softmax_stream(const T* __restrict__ x, v
 // the row. Pass 1 keeps a running (max, sum of exponentials relative to it) per thread and
 // merges them over the CTA; pass 2 re-reads the row (from L2 for rows up to some hundreds
 // of KB), writes whole 16-byte vectors inside the row and single elements in the first and
-// last block. Measured on vocabulary-size bf16 rows: 4.4-4.6 TB/s of 1 read + 1 write;
-// prefetching through a cp.async ring gave the same, and holding the row in shared memory
-// between the passes (one 1024-thread CTA per SM) was slower, 3.9 TB/s. The output row must sit at the same offset inside its 16-byte block as the
-// input row and have the input's type. max.NaN makes a NaN element the maximum, hence the
+// last block. Four vectors are in flight per thread, and one look
+// at the maximum (packed max.NaN) serves all four. bf16 4096 x 50257, log: 146 us (5.6 TB/s of
+// 1 read + 1 write); one vector at a time in CTAs of 1024 threads took 188. Prefetching through a
+// cp.async ring gained nothing, holding the row in shared memory between the passes lost. The
+// output row must sit at the same offset inside its 16-byte block as the input row and have the
+// input's type. max.NaN makes a NaN element the maximum, hence the
 // whole row NaN, as the three-pass kernel above does through its sum.
 __device__ __forceinline__ float max_nan(float a, float b) {
   float r;
@@ -325,34 +327,64 @@ __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float
   m = mn;
   s = a + b;
 }
-// one 16-byte vector into a thread's running (m, s); `masked`: the vector reaches outside the row
-template <typename T, bool MASKED>
-__device__ __forceinline__ void online_take(uint4 v, int j, int head, int cols, float& m, float& s) {
-  constexpr int VE = Vec<T>::N;
-  float f[VE];
-  widen<T>(v, f);
-  if (MASKED) {
-    const int c0 = j * VE - head;
+template <typename T, int NV> __device__ __forceinline__ float vecs_max_nan(const uint4* v) {
+  if constexpr (sizeof(T) == 4) {
+    float m = vec_max_nan<T>(v[0]);
 #pragma unroll
-    for (int e = 0; e < VE; ++e)
-      if (c0 + e < 0 || c0 + e >= cols) f[e] = -CUDART_INF_F;
+    for (int u = 1; u < NV; ++u) m = max_nan(m, vec_max_nan<T>(v[u]));
+    return m;
+  } else {
+    uint32_t w = vec_max_word<T>(v[0]);
+#pragma unroll
+    for (int u = 1; u < NV; ++u) w = max_nan_pair<T>(w, vec_max_word<T>(v[u]));
+    return pair_max_nan<T>(w);
   }
-  float lm = f[0];
+}
+// elements f[0, N), none of them above m, into a thread's running sum
+template <int N>
+__device__ __forceinline__ void online_add(const float* f, float m, float& s) {
+  if (fabsf(m) < 1e37f) {  // 2^(x log2e - m log2e) in one fused multiply-add per element
+    const float c = m * kLog2e;
 #pragma unroll
-  for (int e = 1; e < VE; ++e) lm = max_nan(lm, f[e]);
+    for (int e = 0; e < N; ++e) s += ex2_approx(fmaf(f[e], kLog2e, -c));
+  } else if (m != -CUDART_INF_F) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) s += ex2_approx((f[e] - m) * kLog2e);
+  }
+}
+__device__ __forceinline__ void online_raise(float lm, float& m, float& s) {
   const float mn = max_nan(m, lm);
   if (mn != m) {  // a new maximum (or a NaN): bring the sum so far onto it; 0 * 2^-inf when there was none
     s *= ex2_approx((m - mn) * kLog2e);
     m = mn;
   }
-  if (fabsf(m) < 1e37f) {  // 2^(x log2e - m log2e) in one fused multiply-add per element
-    const float c = m * kLog2e;
+}
+// NV whole vectors at once: one look at the maximum for all of them
+template <typename T, int NV>
+__device__ __forceinline__ void online_take(const uint4* v, float& m, float& s) {
+  online_raise(vecs_max_nan<T, NV>(v), m, s);
 #pragma unroll
-    for (int e = 0; e < VE; ++e) s += ex2_approx(fmaf(f[e], kLog2e, -c));
-  } else if (m != -CUDART_INF_F) {
-#pragma unroll
-    for (int e = 0; e < VE; ++e) s += ex2_approx((f[e] - m) * kLog2e);
+  for (int u = 0; u < NV; ++u) {
+    float f[Vec<T>::N];
+    widen<T>(v[u], f);
+    online_add<Vec<T>::N>(f, m, s);
   }
+}
+// a vector that reaches outside the row
+template <typename T>
+__device__ __forceinline__ void online_take_edge(uint4 v, int j, int head, int cols, float& m, float& s) {
+  constexpr int VE = Vec<T>::N;
+  float f[VE];
+  widen<T>(v, f);
+  const int c0 = j * VE - head;
+#pragma unroll
+  for (int e = 0; e < VE; ++e)
+    if (c0 + e < 0 || c0 + e >= cols) f[e] = -CUDART_INF_F;
+  float lm = f[0];
+#pragma unroll
+  for (int e = 1; e < VE; ++e) lm = max_nan(lm, f[e]);
+  online_raise(lm, m, s);
+  online_add<VE>(f, m, s);
 }
 template <typename T, bool IS_LOG, bool MASKED>
 __device__ __forceinline__ void online_write(uint4 v, T* __restrict__ orow, int j, int head, int cols, float m, float k, bool fused) {
@@ -380,7 +412,7 @@ __device__ __forceinline__ void online_write(uint4 v, T* __restrict__ orow, int 
   }
 }
 template <typename T, bool IS_LOG>
-__global__ void __launch_bounds__(1024) softmax_stream_vec(const T* __restrict__ x, T* __restrict__ out, int cols) {
+__global__ void __launch_bounds__(512, 3) softmax_stream_vec(const T* __restrict__ x, T* __restrict__ out, int cols) {
   constexpr int VE = Vec<T>::N;
   __shared__ float red_m[32], red_s[32];
   const int64_t row = blockIdx.x;
@@ -391,9 +423,19 @@ __global__ void __launch_bounds__(1024) softmax_stream_vec(const T* __restrict__
   const int tid = threadIdx.x, nth = blockDim.x;
   const int last = nvec - 1;  // interior vectors are 1 .. last - 1: they never reach outside the row
   float m = -CUDART_INF_F, s = 0.f;
-  if (tid == 0) online_take<T, true>(ld_keep(xa), 0, head, cols, m, s);
-  if (tid == 32 && nvec > 1) online_take<T, true>(ld_keep(xa + static_cast<int64_t>(last) * VE), last, head, cols, m, s);
-  for (int j = 1 + tid; j < last; j += nth) online_take<T, false>(ld_keep(xa + static_cast<int64_t>(j) * VE), j, head, cols, m, s);
+  if (tid == 0) online_take_edge<T>(ld_keep(xa), 0, head, cols, m, s);
+  if (tid == 32 && nvec > 1) online_take_edge<T>(ld_keep(xa + static_cast<int64_t>(last) * VE), last, head, cols, m, s);
+  int j = 1 + tid;
+  for (; j + 3 * nth < last; j += 4 * nth) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = ld_keep(xa + static_cast<int64_t>(j + u * nth) * VE);
+    online_take<T, 4>(v, m, s);
+  }
+  for (; j < last; j += nth) {
+    const uint4 v = ld_keep(xa + static_cast<int64_t>(j) * VE);
+    online_take<T, 1>(&v, m, s);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) online_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
   const int lane = tid & 31, warp = tid >> 5, nwarps = nth >> 5;
@@ -408,7 +450,14 @@ __global__ void __launch_bounds__(1024) softmax_stream_vec(const T* __restrict__
   T* orow = out + row * cols;
   if (tid == 0) online_write<T, IS_LOG, true>(ld_stream(xa), orow, 0, head, cols, m, k, fused);
   if (tid == 32 && nvec > 1) online_write<T, IS_LOG, true>(ld_stream(xa + static_cast<int64_t>(last) * VE), orow, last, head, cols, m, k, fused);
-  for (int j = 1 + tid; j < last; j += nth) online_write<T, IS_LOG, false>(ld_stream(xa + static_cast<int64_t>(j) * VE), orow, j, head, cols, m, k, fused);
+  for (j = 1 + tid; j + 3 * nth < last; j += 4 * nth) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = ld_stream(xa + static_cast<int64_t>(j + u * nth) * VE);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) online_write<T, IS_LOG, false>(v[u], orow, j + u * nth, head, cols, m, k, fused);
+  }
+  for (; j < last; j += nth) online_write<T, IS_LOG, false>(ld_stream(xa + static_cast<int64_t>(j) * VE), orow, j, head, cols, m, k, fused);
 }
 
 // ------------------------------------------------------------------ ragged rows, one warp each
@@ -1524,7 +1573,7 @@ static int softmax_T(const void* x, void* out, int64_t outer, int64_t dim, int64
       if (outer > 0x7fffffffLL) return B200_EINVAL;
       if (same_phase && dim < (1LL << 30)) {  // same type out, and rows of x and out at the same offset inside their 16-byte blocks
         int64_t th = (dim / VE + 31) / 32 * 32;
-        th = th < 128 ? 128 : (th > 1024 ? 1024 : th);
+        th = th < 128 ? 128 : (th > 512 ? 512 : th);
         auto go = [&](auto kernel) { kernel<<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(px, static_cast<T*>(out), static_cast<int>(dim)); };
         if (is_log) go(softmax_stream_vec<T, true>);
         else go(softmax_stream_vec<T, false>);
