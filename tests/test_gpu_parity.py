@@ -266,6 +266,31 @@ def test_gather_rows_of_self_held_in_shared_memory(backend):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(16, 16), (63, 65), (64, 64), (66, 130), (129, 62), (200, 127), (1000, 258)])
+def test_transposed_tiles_at_their_edges_in_words_and_elements(backend, dtype, rows, cols):
+    """Even and odd extents, pitches and bases (16-bit elements move in pairs only where all of them
+    allow it), one or both operands transposed, every kind of partner, one batch dim, bit copies."""
+    g = torch.Generator(device=DEV).manual_seed(rows * cols)
+    add, mul, relu = (backend[o] for o in (torch.ops.aten.add.Tensor, torch.ops.aten.mul.Tensor, torch.ops.aten.relu.default))
+    rnd = lambda *shape: torch.randn(shape, device=DEV, generator=g).to(dtype)
+    for batch, pad, shift in ((1, 0, 0), (1, 1, 0), (1, 2, 0), (3, 0, 0), (2, 1, 1)):
+        flat = rnd(batch * cols * (rows + pad) + 1)[shift:]
+        a = flat[: batch * cols * (rows + pad)].view(batch, cols, rows + pad)[:, :, :rows].transpose(1, 2)
+        if batch == 1:
+            a = a[0]
+        lead = a.shape[:-2]
+        partners = [rnd(*lead, cols, rows).transpose(-1, -2), rnd(*a.shape), rnd(cols)] + ([rnd(rows, 1), rnd(rows, cols + 1)[:, 1:]] if batch == 1 else [])
+        for b in partners:
+            # fp32 products and sums are rounded once (add of 0.5 b as one fused multiply-add)
+            want = (a.double() + 0.5 * b.double()).to(torch.float32).to(dtype) if dtype != torch.float32 else (a.double() + 0.5 * b.double()).to(dtype)
+            assert bits_equal(want, add(a, b, alpha=0.5))
+            assert bits_equal((a.float() * b.float()).to(dtype), mul(b, a))
+        assert bits_equal(torch.relu(a).contiguous(), relu(a)) and bits_equal((a.float() * 3.0).to(dtype), mul(a, 3.0))
+        raw = a.contiguous()
+        assert bits_equal(raw, ops._contig(a))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_argmax_rows_where_whole_vectors_are_skipped(backend, dtype):
     """The row kernel screens 16-byte vectors (largest element and a NaN guard) before it looks
     at elements: ties must still go to the first index, NaN to the first NaN, and vectors
