@@ -541,8 +541,10 @@ static void launch_binary_T(const void* a, const void* b, void* out, int64_t n, 
 // either contiguous along c (column stride 1, any row stride, 0 included: a bias vector) or
 // constant along c (column stride 0: one value per row). The bias add and the per-row scale
 // of ordinary model code; the generic strided kernel would pay an index decomposition per
-// element. A thread produces 16 bytes of a row (VEC: rows, bases and C on the 16-byte grid)
-// or one element; one 32-bit division per thread and trip finds its row.
+// element. A thread produces four times 16 bytes (VEC: rows, bases and C on the 16-byte grid) or
+// four elements, with every load of the four in flight at once, and finds its rows with one
+// 32-bit division where a row is at least a CTA wide. A partner that every row shares is kept in
+// L2. Bound by HBM: bf16 32 x 2048 x 2048 plus a mask of 2048 x 2048 (537 MB) 123 -> 102 us (5.3 TB/s).
 struct Rows2dArgs {
   int64_t R, C;
   int64_t ar, br;  // row strides, elements
@@ -550,42 +552,63 @@ struct Rows2dArgs {
 };
 template <typename T, int OP, bool VEC>
 __global__ void __launch_bounds__(256) ew_rows2d(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, Rows2dArgs A, float alpha) {
-  constexpr int VE = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;
+  constexpr int VE = VEC ? 16 / static_cast<int>(sizeof(T)) : 1, U = 4;
+  typedef typename std::conditional<VEC, uint4, T>::type Word;
   const int64_t per_row = A.C / VE, total = A.R * per_row;
-  const bool small = total <= 0x7fffffffLL;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int64_t r, g;
-    if (small) {
-      const uint32_t q = static_cast<uint32_t>(i) / static_cast<uint32_t>(per_row);
-      r = q;
-      g = static_cast<uint32_t>(i) - q * static_cast<uint32_t>(per_row);
-    } else {
-      r = i / per_row;
-      g = i - r * per_row;
-    }
-    const int64_t c = g * VE;
-    float x[VE], y[VE], res[VE];
-    if (VEC) {
-      if (A.a_c) widen<T>(ld_stream(a + r * A.ar + c), x);
-      if (A.b_c) widen<T>(ld_stream(b + r * A.br + c), y);
-    } else {
-      if (A.a_c) x[0] = to_f32(a[r * A.ar + c]);
-      if (A.b_c) y[0] = to_f32(b[r * A.br + c]);
-    }
-    if (!A.a_c) {
-      const float v = to_f32(a[r * A.ar]);
+  const bool small = total <= 0x7fffffffLL - 256 * U, wide = per_row >= 256;
+  auto load = [](const T* p, int64_t o, int64_t row_stride) {
+    if constexpr (VEC) return row_stride ? ld_stream(p + o) : ld_keep(p + o);
+    else return p[o];
+  };
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; base < total; base += static_cast<int64_t>(gridDim.x) * (256 * U)) {
+    Word wa[U], wb[U];
+    int64_t oo[U];
+    int64_t r = 0, g = 0;
 #pragma unroll
-      for (int e = 0; e < VE; ++e) x[e] = v;
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = base + u * 256;
+      if (u > 0 && wide) {  // the next element of this thread is in the same row or the next one
+        g += 256;
+        if (g >= per_row) { g -= per_row; ++r; }
+      } else if (small) {
+        const uint32_t q = static_cast<uint32_t>(i) / static_cast<uint32_t>(per_row);
+        r = q;
+        g = static_cast<uint32_t>(i) - q * static_cast<uint32_t>(per_row);
+      } else {
+        r = i / per_row;
+        g = i - r * per_row;
+      }
+      const int64_t c = g * VE;
+      oo[u] = r * A.C + c;
+      wa[u] = wb[u] = Word{};
+      if (i < total) {
+        if (A.a_c) wa[u] = load(a, r * A.ar + c, A.ar);
+        else *reinterpret_cast<T*>(&wa[u]) = a[r * A.ar];
+        if (A.b_c) wb[u] = load(b, r * A.br + c, A.br);
+        else *reinterpret_cast<T*>(&wb[u]) = b[r * A.br];
+      }
     }
-    if (!A.b_c) {
-      const float v = to_f32(b[r * A.br]);
 #pragma unroll
-      for (int e = 0; e < VE; ++e) y[e] = v;
+    for (int u = 0; u < U; ++u) {
+      if (base + u * 256 >= total) break;
+      float x[VE], y[VE], res[VE];
+      if constexpr (VEC) {
+        widen<T>(wa[u], x);
+        widen<T>(wb[u], y);
+      } else {
+        x[0] = to_f32(wa[u]);
+        y[0] = to_f32(wb[u]);
+      }
+#pragma unroll
+      for (int e = 1; e < VE; ++e) {
+        if (!A.a_c) x[e] = x[0];
+        if (!A.b_c) y[e] = y[0];
+      }
+#pragma unroll
+      for (int e = 0; e < VE; ++e) res[e] = OP == OP_ADD ? fmaf(alpha, y[e], x[e]) : x[e] * y[e];
+      if constexpr (VEC) st_stream(out + oo[u], narrow<T>(res));
+      else out[oo[u]] = from_f32<T>(res[0]);
     }
-#pragma unroll
-    for (int e = 0; e < VE; ++e) res[e] = OP == OP_ADD ? fmaf(alpha, y[e], x[e]) : x[e] * y[e];
-    if (VEC) st_stream(out + r * A.C + c, narrow<T>(res));
-    else out[r * A.C + c] = from_f32<T>(res[0]);
   }
 }
 
@@ -607,7 +630,7 @@ static void launch_rows2d_T(const void* a, const void* b, void* out, const Rows2
   const bool a_ok = !A.a_c || (aligned16(a) && A.ar % VE == 0), b_ok = !A.b_c || (aligned16(b) && A.br % VE == 0);
   const bool vec = A.C % VE == 0 && aligned16(out) && a_ok && b_ok;
   const int64_t work = A.R * (vec ? A.C / VE : A.C);
-  const int g = strided_grid(work);
+  const int g = grid_for(work, 256 * 4);
   if (vec) ew_rows2d<T, OP, true><<<g, 256, 0, st>>>(static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), A, alpha);
   else ew_rows2d<T, OP, false><<<g, 256, 0, st>>>(static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), A, alpha);
 }
