@@ -1078,48 +1078,80 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
   }
 }
 
-// Column reduction (inner > 1): thread per inner element, grid = (inner tiles, outer, splits).
-template <typename T, bool ARG>
-__global__ void __launch_bounds__(256) reduce_cols(const T* __restrict__ x, void* __restrict__ out, float* __restrict__ part_v, int64_t* __restrict__ part_i,
-                                                   int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int dto) {
+// argmax over columns (inner > 1): thread per inner element, grid = (inner tiles, outer, splits).
+template <typename T>
+__global__ void __launch_bounds__(256) argmax_cols(const T* __restrict__ x, int64_t* __restrict__ out, float* __restrict__ part_v, int64_t* __restrict__ part_i,
+                                                   int64_t outer, int64_t dim, int64_t inner, int64_t chunk) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= inner) return;
   const int64_t o = blockIdx.y;
   const int64_t k0 = static_cast<int64_t>(blockIdx.z) * chunk;
   const int64_t k1 = k0 + chunk < dim ? k0 + chunk : dim;
   const T* p = x + o * dim * inner + i;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   ArgPair a{0.f, -1};
   int64_t k = k0;
-  if (!ARG) {
-    for (; k + 3 < k1; k += 4) {
-      s0 += to_f32(p[k * inner]);
-      s1 += to_f32(p[(k + 1) * inner]);
-      s2 += to_f32(p[(k + 2) * inner]);
-      s3 += to_f32(p[(k + 3) * inner]);
-    }
-  } else {
-    for (; k + 7 < k1; k += 8) {  // eight rows requested before the first comparison
-      T f[8];
+  for (; k + 7 < k1; k += 8) {  // eight rows requested before the first comparison
+    T f[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) f[u] = p[(k + u) * inner];
+    for (int u = 0; u < 8; ++u) f[u] = p[(k + u) * inner];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) arg_take(a, to_f32(f[u]), k + u);
-    }
+    for (int u = 0; u < 8; ++u) arg_take(a, to_f32(f[u]), k + u);
   }
-  for (; k < k1; ++k) {
-    const float fv = to_f32(p[k * inner]);
-    if (ARG) arg_take(a, fv, k);
-    else s0 += fv;
-  }
-  const float s = (s0 + s1) + (s2 + s3);
+  for (; k < k1; ++k) arg_take(a, to_f32(p[k * inner]), k);
   const int64_t oi = o * inner + i;
   if (gridDim.z > 1) {
     const int64_t slot = static_cast<int64_t>(blockIdx.z) * outer * inner + oi;
-    if (ARG) { part_v[slot] = a.v; part_i[slot] = a.i; }
-    else part_v[slot] = s;
+    part_v[slot] = a.v;
+    part_i[slot] = a.i;
   } else {
-    if (ARG) static_cast<int64_t*>(out)[oi] = a.i;
+    out[oi] = a.i;
+  }
+}
+
+// Sum over columns (inner > 1; the bias gradient of a linear layer). grid = (inner tiles, outer,
+// splits). A lane owns the columns of one WORD (as wide as the rows' length and base allow), a
+// warp 32 such words of every blockDim / 32 -th row of the slice, eight rows in flight; the
+// warps' sums are added in warp order. A thread per column with four 2-byte loads in flight
+// left the memory idle: bf16 8192 x 11008 (180 MB) 93 us, so %T%.
+template <typename T, typename WORD>
+__global__ void __launch_bounds__(512, 2) sum_cols(const T* __restrict__ x, void* __restrict__ out, float* __restrict__ part_v, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int dto) {
+  constexpr int E = sizeof(WORD) / sizeof(T), U = 8;
+  __shared__ float red[16][32 * E];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int64_t o = blockIdx.y;
+  const int64_t col = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * E;
+  const int64_t k0 = static_cast<int64_t>(blockIdx.z) * chunk;
+  const int64_t k1 = k0 + chunk < dim ? k0 + chunk : dim;
+  float acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
+  if (col < inner) {
+    const T* p = x + o * dim * inner + col;
+    for (int64_t k = k0 + warp; k < k1; k += U * warps) {
+      WORD v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        v[u] = WORD{};
+        if (k + u * warps < k1) v[u] = __ldcs(reinterpret_cast<const WORD*>(p + (k + u * warps) * inner));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const T* f = reinterpret_cast<const T*>(&v[u]);
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] += to_f32(f[e]);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) red[warp][e * 32 + lane] = acc[e];
+  __syncthreads();
+  for (int c = threadIdx.x; c < 32 * E; c += blockDim.x) {
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * 32 + (c & 31)) * E + (c >> 5);
+    if (i >= inner) continue;
+    float s = red[0][c];
+    for (int w = 1; w < warps; ++w) s += red[w][c];
+    const int64_t oi = o * inner + i;
+    if (gridDim.z > 1) part_v[static_cast<int64_t>(blockIdx.z) * outer * inner + oi] = s;
     else store_from_f32(out, oi, dto, s);
   }
 }
@@ -1459,9 +1491,36 @@ static ReducePlan plan_reduce(int64_t outer, int64_t dim, int64_t inner) {
   return p;
 }
 
+template <typename T, typename WORD>
+static void launch_sum_cols_word(const T* x, void* out, float* pv, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int splits, int dto, cudaStream_t st) {
+  constexpr int E = sizeof(WORD) / sizeof(T);
+  int warps = 1;  // eight rows to a warp: more warps than that would find no rows in a short slice
+  while (warps < 16 && warps * 8 < chunk) warps <<= 1;
+  const dim3 g(grid_for(inner, 32 * E), static_cast<unsigned>(outer), static_cast<unsigned>(splits));
+  sum_cols<T, WORD><<<g, 32 * warps, 0, st>>>(x, out, pv, outer, dim, inner, chunk, dto);
+}
+// Bytes of the words `sum_cols` reads: the widest that every row starts on and ends with, and
+// that still gives 32 lanes columns.
+static int sum_cols_word(const void* x, int64_t inner, int esize) {
+  int bytes = 16;
+  while (bytes > esize && (((inner * esize) | static_cast<int64_t>(reinterpret_cast<uintptr_t>(x))) % bytes || inner * esize < 32 * bytes)) bytes >>= 1;
+  return bytes;
+}
+template <typename T>
+static void launch_sum_cols(const T* x, void* out, float* pv, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int splits, int dto, cudaStream_t st) {
+  switch (sum_cols_word(x, inner, sizeof(T))) {
+    case 16: launch_sum_cols_word<T, uint4>(x, out, pv, outer, dim, inner, chunk, splits, dto, st); break;
+    case 8: launch_sum_cols_word<T, uint2>(x, out, pv, outer, dim, inner, chunk, splits, dto, st); break;
+    case 4: launch_sum_cols_word<T, uint32_t>(x, out, pv, outer, dim, inner, chunk, splits, dto, st); break;
+    default:
+      if constexpr (sizeof(T) == 2) launch_sum_cols_word<T, uint16_t>(x, out, pv, outer, dim, inner, chunk, splits, dto, st);
+      break;
+  }
+}
+
 template <typename T, bool ARG>
 static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim, int64_t inner, int dto, void* scratch, int64_t scratch_bytes, cudaStream_t st) {
-  const ReducePlan p = plan_reduce(outer, dim, inner);
+  ReducePlan p = plan_reduce(outer, dim, inner);
   const int64_t nout = outer * inner;
   float* pv = nullptr;
   int64_t* pi = nullptr;
@@ -1487,9 +1546,8 @@ static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim,
       // grid.y limit: fold by launching per slab of 65535 outer rows
       for (int64_t o0 = 0; o0 < outer; o0 += 65535) {
         const int64_t on = outer - o0 < 65535 ? outer - o0 : 65535;
-        dim3 g(grid_for(inner, 256), static_cast<unsigned>(on), 1);
-        void* o_ptr = ARG ? static_cast<void*>(static_cast<int64_t*>(out) + o0 * inner) : static_cast<void*>(static_cast<char*>(out) + o0 * inner * dtype_size(dto));
-        reduce_cols<T, ARG><<<g, 256, 0, st>>>(px + o0 * dim * inner, o_ptr, nullptr, nullptr, on, dim, inner, dim, dto);
+        if (ARG) argmax_cols<T><<<dim3(grid_for(inner, 256), static_cast<unsigned>(on), 1), 256, 0, st>>>(px + o0 * dim * inner, static_cast<int64_t*>(out) + o0 * inner, nullptr, nullptr, on, dim, inner, dim);
+        else launch_sum_cols<T>(px + o0 * dim * inner, static_cast<char*>(out) + o0 * inner * dtype_size(dto), nullptr, on, dim, inner, dim, 1, dto, st);
       }
       return check_launch();
     }
@@ -1498,9 +1556,21 @@ static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim,
       while (W < inner) W <<= 1;
       dim3 g(1, static_cast<unsigned>(outer), p.splits);
       reduce_cols_narrow<T, ARG><<<g, 256, 0, st>>>(px, out, pv, pi, outer, dim, static_cast<int>(inner), W, p.chunk, dto);
-    } else {
+    } else if (ARG) {
       dim3 g(grid_for(inner, 256), static_cast<unsigned>(outer), p.splits);
-      reduce_cols<T, ARG><<<g, 256, 0, st>>>(px, out, pv, pi, outer, dim, inner, p.chunk, dto);
+      argmax_cols<T><<<g, 256, 0, st>>>(px, static_cast<int64_t*>(out), pv, pi, outer, dim, inner, p.chunk);
+    } else {
+      if (p.splits > 1) {
+        // no more slices than fit the SMs at once, two CTAs to each: a CTA more is a round more
+        const int64_t tile = 32 * sum_cols_word(x, inner, sizeof(T));
+        int64_t fit = 2 * kNumSMs / (outer * ((inner * static_cast<int64_t>(sizeof(T)) + tile - 1) / tile));
+        if (fit < 1) fit = 1;
+        if (p.splits > fit) {
+          p.chunk = (dim + fit - 1) / fit;
+          p.splits = static_cast<int>((dim + p.chunk - 1) / p.chunk);
+        }
+      }
+      launch_sum_cols<T>(px, out, pv, outer, dim, inner, p.chunk, p.splits, dto, st);
     }
   }
   if (p.splits >= 64 && nout <= 8LL * kNumSMs * 8) reduce_finalize_warp<ARG><<<grid_for(nout, 8), 256, 0, st>>>(pv, pi, out, nout, p.splits, dto);

@@ -339,6 +339,22 @@ def test_row_reductions_of_rows_off_the_16_byte_grid(backend, dtype, cols):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("outer,dim,inner", [(1, 1, 33), (1, 7, 4096), (1, 8, 65), (2, 9, 66), (1, 65, 254), (1, 1000, 2050), (1, 8192, 1028), (3, 130, 256), (2, 513, 127), (66000, 2, 40)])
+def test_column_sums_in_every_word_width(backend, dtype, outer, dim, inner):
+    """Column counts and bases that allow 16-, 8-, 4- and 2-byte words, slices of one row up to
+    many per warp, split and unsplit, and more outer slabs than a grid dimension."""
+    impl = backend[torch.ops.aten.sum.dim_IntList]
+    g = torch.Generator(device=DEV).manual_seed(dim * inner)
+    n = outer * dim * inner
+    for shift in (0, 1, 2):
+        x = torch.randn(n + 2, device=DEV, generator=g).to(dtype)[shift : shift + n].view(outer, dim, inner)
+        got, exact = impl(x, [1]).double(), x.double().sum(1)
+        # fp32 additions of dim terms in any order, one rounding of the result
+        bound = dim * 2.0**-24 * x.double().abs().sum(1) + exact.abs() * {torch.float32: 2.0**-24, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype] + 2.0**-24
+        assert got.shape == exact.shape and bool(((got - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_gather_along_the_last_dim(backend, dtype):
     """2-D gather along the last dim: 16 bytes of adjacent outputs per thread; fewer index rows
     than source rows, a pitched source, an index width that is not a multiple of the vector
