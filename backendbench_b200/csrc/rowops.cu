@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(256) argmax_cols(const T* __restrict__ x, int6
 // splits). A lane owns the columns of one WORD (as wide as the rows' length and base allow), a
 // warp 32 such words of every blockDim / 32 -th row of the slice, eight rows in flight; the
 // warps' sums are added in warp order. A thread per column with four 2-byte loads in flight
-// left the memory idle: bf16 8192 x 11008 (180 MB) 93 us, so %T%.
+// left the memory idle: bf16 8192 x 11008 (180 MB) 93 us, so 34 us (5.3 TB/s).
 template <typename T, typename WORD>
 __global__ void __launch_bounds__(512, 2) sum_cols(const T* __restrict__ x, void* __restrict__ out, float* __restrict__ part_v, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int dto) {
   constexpr int E = sizeof(WORD) / sizeof(T), U = 8;
@@ -1562,6 +1562,7 @@ static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim,
     } else {
       if (p.splits > 1) {
         // no more slices than fit the SMs at once, two CTAs to each: a CTA more is a round more
+        // (bf16 8192 x 11008: 49 us in the 7 slices of the plan at one CTA per SM, 34 us in 6 at two)
         const int64_t tile = 32 * sum_cols_word(x, inner, sizeof(T));
         int64_t fit = 2 * kNumSMs / (outer * ((inner * static_cast<int64_t>(sizeof(T)) + tile - 1) / tile));
         if (fit < 1) fit = 1;
