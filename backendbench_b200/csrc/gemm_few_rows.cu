@@ -1,0 +1,132 @@
+// 16-bit mm / addmm with at most 16 rows of A against a large B whose rows lie along K (the weight
+// matrix of a linear layer, [out, in], while a model decodes a few tokens): bound by reading B
+// once. The tcgen05 kernel gives such a product 128-row tiles of which 16 are used, N / 256
+// CTAs, and a handful of stages in flight in each: 16 x 4096 x 11008 ran on 43 SMs (44 us,
+// 2.1 TB/s), 16 x 11008 x 4096 in 16 CTAs split over K with a second pass (29 us).
+//
+// Here a CTA owns 8 * NT columns of C and its eight warps share K. A warp streams B from global
+// memory straight into mma.sync operands, with no shared memory in between: in
+// mma.m16n8k16 lane (q, c) holds elements 2c, 2c + 1, 2c + 8, 2c + 9 of row q of B (and of rows
+// q, q + 8 of A). The order of the products in a sum over k is free, so the 32 k of
+// two such steps are dealt out as the 16-byte pieces 8c .. 8c + 7 of a row: one load
+// each. Four steps of both operands are in flight per lane; A comes from L2, where every CTA
+// reads it. The warps' sums are added in warp order in fp32, then alpha, beta, the bias and
+// one rounding.
+#include <type_traits>
+
+#include "b200_common.cuh"
+
+namespace b200 {
+
+namespace {
+
+constexpr int kFewRows = 16;
+constexpr int kFewWarps = 8;
+constexpr int kFewSteps = 4;              // 32-k steps in flight per lane
+constexpr int64_t kFewMaxK = 16384;       // a CTA walks all of K: beyond, ranges of K on several CTAs win
+
+struct FewRowsArgs {
+  int64_t M, N, K, sAm, sBn, sbm, sbn;
+  float alpha, beta;
+};
+
+template <typename T>
+__device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if (std::is_same<T, __nv_bfloat16>::value) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  } else {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ bias, T* __restrict__ C, FewRowsArgs p) {
+  constexpr int kCols = 8 * NT, kPitch = kCols + 1;
+  __shared__ float red[kFewWarps][kFewRows][kPitch];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane >> 2, c = lane & 3;
+  const int64_t n0 = static_cast<int64_t>(blockIdx.x) * kCols;
+  const bool row0 = q < p.M, row1 = q + 8 < p.M;
+  const T* a0 = A + (row0 ? q : 0) * p.sAm + 8 * c;
+  const T* a1 = A + (row1 ? q + 8 : 0) * p.sAm + 8 * c;
+  const T* b[NT];
+  bool col[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    col[t] = n0 + 8 * t + q < p.N;
+    b[t] = B + (col[t] ? n0 + 8 * t + q : 0) * p.sBn + 8 * c;
+  }
+  float acc[NT][4];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+  const int K = static_cast<int>(p.K);  // a multiple of 8: a piece is inside the row or outside it
+  for (int k0 = warp * 32 * kFewSteps; k0 < K; k0 += kFewWarps * 32 * kFewSteps) {
+    uint4 ra[kFewSteps], rA[kFewSteps], rb[NT][kFewSteps];
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < kFewSteps; ++u) {
+      const int k = k0 + 32 * u;
+      const bool in = k + 8 * c < K;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) rb[t][u] = in && col[t] ? ld_stream(b[t] + k) : zero;
+      ra[u] = in && row0 ? ld_keep(a0 + k) : zero;
+      rA[u] = in && row1 ? ld_keep(a1 + k) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < kFewSteps; ++u) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        mma_step<T>(acc[t], ra[u].x, rA[u].x, ra[u].y, rA[u].y, rb[t][u].x, rb[t][u].y);
+        mma_step<T>(acc[t], ra[u].z, rA[u].z, ra[u].w, rA[u].w, rb[t][u].z, rb[t][u].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    red[warp][q][8 * t + 2 * c] = acc[t][0];
+    red[warp][q][8 * t + 2 * c + 1] = acc[t][1];
+    red[warp][q + 8][8 * t + 2 * c] = acc[t][2];
+    red[warp][q + 8][8 * t + 2 * c + 1] = acc[t][3];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kFewRows * kCols; i += 32 * kFewWarps) {
+    const int m = i / kCols, j = i - m * kCols;
+    const int64_t n = n0 + j;
+    if (m >= p.M || n >= p.N) continue;
+    float s = red[0][m][j];
+#pragma unroll
+    for (int w = 1; w < kFewWarps; ++w) s += red[w][m][j];
+    float r = p.alpha * s;
+    if (bias) r = fmaf(p.beta, to_f32(bias[m * p.sbm + n * p.sbn]), r);
+    C[m * p.N + n] = from_f32<T>(r);
+  }
+}
+
+}  // namespace
+
+bool gemm_few_rows_preferred(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sAk, int64_t sBk, int64_t sBn, int dtype) {
+  if (dtype != B200_BF16 && dtype != B200_F16) return false;
+  if (batch != 1 || M < 1 || M > kFewRows || N < 1 || N > 0x7fffffffLL || K < 64 || K > kFewMaxK || K % 8 != 0) return false;
+  if (sAk != 1 || sBk != 1 || !aligned16(A) || !aligned16(B)) return false;
+  return (M == 1 || (sAm % 8 == 0 && sAm >= 0)) && (N == 1 || (sBn % 8 == 0 && sBn >= 0));
+}
+
+template <typename T>
+static void launch_few_rows(const void* A, const void* B, const void* bias, void* C, const FewRowsArgs& p, cudaStream_t st) {
+  // 16 columns to a CTA: enough CTAs for two on every SM from N = 4736 on
+  gemm_few_rows<T, 2><<<grid_for(p.N, 16), 32 * kFewWarps, 0, st>>>(static_cast<const T*>(A), static_cast<const T*>(B), static_cast<const T*>(bias), static_cast<T*>(C), p);
+}
+
+int gemm_few_rows_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sBn, int64_t sbm, int64_t sbn, double alpha,
+                           double beta, int dtype, cudaStream_t st) {
+  const FewRowsArgs p{M, N, K, sAm, sBn, sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta)};
+  const void* bs = static_cast<float>(beta) != 0.f ? bias : nullptr;  // beta = 0 ignores the bias, NaN included
+  if (dtype == B200_BF16) launch_few_rows<__nv_bfloat16>(A, B, bs, C, p, st);
+  else launch_few_rows<__half>(A, B, bs, C, p, st);
+  return check_launch();
+}
+
+}  // namespace b200

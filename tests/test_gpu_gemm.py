@@ -404,3 +404,27 @@ def test_small_products_on_the_mma_kernel(dtype):
             assert prefers(a3, b2, 1, M, N, K) == 0
             _check(ops.mm_default(a3, b2), a3.double() @ b2.double(), dtype)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 15, 16, 17])
+def test_few_rows_against_weights_along_k(dtype, M):
+    """Row counts on both sides of 8 and 16, N and K at the edges of a CTA's columns, a step, a
+    batch of steps and the warps' shares, row pitches, every form of bias, poison outside the rows."""
+    from backendbench_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *shape: torch.randn(shape, device="cuda", generator=g).to(dtype)
+    eps = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
+    for N, K, pad in [(1, 64, 0), (7, 72, 0), (16, 128, 8), (17, 136, 0), (250, 1024, 0), (33, 1032, 16), (4099, 2056, 0), (130, 16384, 0), (64, 16392, 0), (9600, 256, 0)]:
+        x, w = rnd(M, K + pad)[:, :K], rnd(N, K + pad)[:, :K]
+        if pad:  # what lies between the rows must not be read as part of them
+            x._base[:, K:] = float("nan")
+            w._base[:, K:] = float("nan")
+        prod, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+        for bias, alpha, beta in [(None, 1, 1), (rnd(N), 1, 1), (rnd(M, 1), 0.5, 2), (rnd(M, N), 1, 1), (torch.full((N,), float("nan"), device="cuda", dtype=dtype), 1, 0)]:
+            got = ops.mm_default(x, w.t()) if bias is None else ops.addmm_default(bias, x, w.t(), beta=beta, alpha=alpha)
+            want = alpha * prod + (beta * bias.double() if bias is not None and beta else 0)
+            # fp32 accumulation (truncating adds: 2^-23 of the running sum each) and one rounding
+            bound = want.abs() * eps + (K + 8) * 2.0**-23 * size + 1e-7
+            assert got.shape == (M, N) and bool(((got.double() - want).abs() <= bound).all()), (M, N, K)
