@@ -467,6 +467,41 @@ def test_scatter_add_grouped_by_destination_path_bit_exact(backend, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [1, 3, 63])
+def test_scatter_add_chains_of_every_depth_bit_exact(backend, dtype, cols):
+    """Destinations with 0 .. 5, 31 .. 34 and hundreds of contributions among many with none (chains
+    of up to three in registers, up to 32 in an array, longer ones grouped), on both sides of
+    one contribution per destination, with strided index and values, and an index out of range."""
+    impl = backend[torch.ops.aten.scatter_add.default]
+    g = torch.Generator().manual_seed(cols)
+    rows = 9001
+    counts = [1, 2, 3, 4, 5, 31, 32, 33, 34, 700]
+    fixed = torch.repeat_interleave(torch.arange(len(counts)) * 13, torch.tensor(counts))
+    for n in (65, 1000, rows, rows + 1):
+        idx = torch.randint(0, rows, (n, cols), generator=g)
+        k = min(n, fixed.numel())
+        for c in range(cols):
+            idx[torch.randperm(n, generator=g)[:k], c] = fixed[torch.randperm(fixed.numel(), generator=g)[:k]]
+        x, src = torch.randn(rows, cols, generator=g).to(dtype), torch.randn(n, cols, generator=g).to(dtype)
+        x[26] = -0.0
+        want = oracle.scatter_add(x, 0, idx, src)
+        assert bits_equal(want, impl(x.to(DEV), 0, idx.to(DEV), src.to(DEV))), n
+        wide = torch.empty(n, cols + 5, dtype=dtype, device=DEV)[:, 2 : 2 + cols].copy_(src)
+        idx_t = torch.empty(cols, n, dtype=torch.int64, device=DEV).t().copy_(idx)
+        assert bits_equal(want, impl(x.to(DEV), 0, idx_t, wide)), n
+        # the same along the last dim of the transposed problem
+        assert bits_equal(want.t().contiguous(), impl(x.t().contiguous().to(DEV), 1, idx.t().contiguous().to(DEV), src.t().contiguous().to(DEV)).cpu()), n
+    ops.check_device_status()
+    idx[17, 0] = rows
+    got = impl(x.to(DEV), 0, idx.to(DEV), src.to(DEV))
+    with pytest.raises(IndexError):
+        ops.check_device_status()
+    src[17, 0] = 0.0
+    idx[17, 0] = 8999
+    assert torch.equal(oracle.scatter_add(x, 0, idx, src).float(), got.cpu().float())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_scatter_add_with_an_empty_index_copies_self(backend, dtype):
     """No contributions at all (an index with a zero extent): the result is self, for every
     dtype and geometry, and no scratch is asked for."""
