@@ -931,20 +931,25 @@ static int launch_bucket(const void* self, const void* index, const void* src, v
 // The same geometries with no more contributions than destinations (features of graph nodes, a
 // random half of the rows): most destinations get none or one, so grouping costs more than
 // the sums. One pass hangs every contribution into its destination's chain (`head[d]`, then
-// `next[p]`; any order), one pass over the destinations walks the chains and adds in ascending
+// `link[p]`; any order), one pass over the destinations walks the chains and adds in ascending
 // position -- for one destination the linear position p orders like the position along the
 // dim. Four destinations per thread advance together, three links deep with the entries in
 // registers; deeper chains collect their positions in an array. What bounds it: the random
-// 4-byte exchanges, and per contribution one random look into `next` and one into `src`. f16
-// 150134 x 63, half as many rows picked: %T%.
+// 4-byte exchanges, and one random 8-byte look per contribution (the value lies beside the
+// link: a second look, into `src`, made the second pass 91 us instead of %R%). f16
+// 150134 x 63, half as many rows picked: 251 us in segments -> %T%.
 // A chain of more than kLightMax entries is not walked to its end (a dependent chain of loads):
 // its destination goes on a list, and four kernels that end at once when the list is empty
 // group just those contributions the way the bucket path does.
 constexpr int kChainUnroll = 4;
 
-__global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ index, int* __restrict__ head, int* __restrict__ next, BucketArgs A, uint32_t* status) {
+// link[p] = {the entry hung before p, or -1; the value's bits as fp32}
+template <typename T>
+__global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ index, const T* __restrict__ src, int* __restrict__ head, int2* __restrict__ link,
+                                                  const __grid_constant__ BucketArgs A, uint32_t* status) {
   for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * kChainUnroll) + threadIdx.x; p0 < A.n_idx; p0 += static_cast<int64_t>(gridDim.x) * (256 * kChainUnroll)) {
     int64_t dest[kChainUnroll];
+    T v[kChainUnroll];
     int before[kChainUnroll];
 #pragma unroll
     for (int u = 0; u < kChainUnroll; ++u) {
@@ -952,91 +957,81 @@ __global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ in
       int64_t so;
       int pos;
       if (p >= A.n_idx || !bucket_decode(A, p, index, dest[u], so, pos, status)) dest[u] = -1;
+      else v[u] = src[so];
     }
 #pragma unroll
     for (int u = 0; u < kChainUnroll; ++u)
       if (dest[u] >= 0) before[u] = atomicExch(&head[dest[u]], static_cast<int>(p0 + u * 256));
 #pragma unroll
     for (int u = 0; u < kChainUnroll; ++u)
-      if (dest[u] >= 0) next[p0 + u * 256] = before[u];
+      if (dest[u] >= 0) link[p0 + u * 256] = make_int2(before[u], __float_as_int(to_f32(v[u])));
   }
-}
-
-// element offset in `src` of linear position p of the index
-__device__ __forceinline__ int64_t chain_src(const BucketArgs& A, int p, int direct) {
-  if (direct) return p;
-  uint32_t lin = static_cast<uint32_t>(p);
-  int64_t so = 0;
-  for (int d = A.ndim - 1; d >= 0; --d) {
-    const uint32_t ext = static_cast<uint32_t>(A.shape[d]);
-    const uint32_t q = lin / ext;
-    so += static_cast<int64_t>(lin - q * ext) * A.src_stride[d];
-    lin = q;
-  }
-  return so;
 }
 
 // A chain of four entries or more. False: too long to walk.
-template <typename T>
-__device__ __noinline__ bool chain_deep(const T* __restrict__ src, const int* __restrict__ next, const BucketArgs& A, int direct, int p, float& acc) {
+__device__ __noinline__ bool chain_deep(const int2* __restrict__ link, int p, float& acc) {
   int pos[kLightMax];
+  float val[kLightMax];
   int c = 0;
-  for (; p >= 0; p = next[p], ++c) {
+  while (p >= 0) {
     if (c == kLightMax) return false;
-    int k = c;
-    for (; k > 0 && pos[k - 1] > p; --k) pos[k] = pos[k - 1];
+    const int2 e = link[p];
+    int k = c++;
+    for (; k > 0 && pos[k - 1] > p; --k) {
+      pos[k] = pos[k - 1];
+      val[k] = val[k - 1];
+    }
     pos[k] = p;
+    val[k] = __int_as_float(e.y);
+    p = e.x;
   }
-  for (int k = 0; k < c; ++k) acc += to_f32(src[chain_src(A, pos[k], direct)]);
+  for (int k = 0; k < c; ++k) acc += val[k];
   return true;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, T* __restrict__ out, const T* __restrict__ src, int* __restrict__ head, const int* __restrict__ next,
-                                                    const __grid_constant__ BucketArgs A, int direct, int* __restrict__ heavy_count, int* __restrict__ heavy_list) {
+__global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, T* __restrict__ out, int* __restrict__ head, const int2* __restrict__ link, int64_t n_self,
+                                                    int* __restrict__ heavy_count, int* __restrict__ heavy_list) {
   constexpr int U = kChainUnroll;
-  for (int64_t d0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; d0 < A.n_self; d0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
-    int k[3][U];  // the first three entries of each chain, -1 past its end
-    T s[U], v[3][U];
-    int rest[U];
+  for (int64_t d0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; d0 < n_self; d0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
+    int k[4][U];  // the first three entries of each chain and what follows them, -1 past its end
+    T s[U];
+    float v[3][U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t d = d0 + u * 256;
-      k[0][u] = d < A.n_self ? head[d] : -1;
-      if (d < A.n_self) s[u] = self[d];
+      k[0][u] = d < n_self ? head[d] : -1;
+      if (d < n_self) s[u] = self[d];
     }
 #pragma unroll
     for (int l = 0; l < 3; ++l) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        int n = -1;
-        if (k[l][u] >= 0) {
-          n = next[k[l][u]];
-          v[l][u] = src[chain_src(A, k[l][u], direct)];
-        }
-        if (l < 2) k[l < 2 ? l + 1 : 0][u] = n;
-        else rest[u] = n;
+        int2 e = make_int2(-1, 0);
+        if (k[l][u] >= 0) e = link[k[l][u]];
+        k[l + 1][u] = e.x;
+        v[l][u] = __int_as_float(e.y);
       }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t d = d0 + u * 256;
-      if (d >= A.n_self) break;
+      if (d >= n_self) break;
       if (k[0][u] < 0) {
         out[d] = s[u];
         continue;
       }
       float acc = to_f32(s[u]);
-      if (rest[u] < 0) {
+      if (k[3][u] < 0) {
         int a = k[0][u], b = k[1][u] < 0 ? 0x7fffffff : k[1][u], c = k[2][u] < 0 ? 0x7fffffff : k[2][u];
-        T va = v[0][u], vb = v[1][u], vc = v[2][u];
-        if (b < a) { int t = a; a = b; b = t; T x = va; va = vb; vb = x; }
-        if (c < b) { int t = b; b = c; c = t; T x = vb; vb = vc; vc = x; }
-        if (b < a) { int t = a; a = b; b = t; T x = va; va = vb; vb = x; }
-        acc += to_f32(va);
-        if (b != 0x7fffffff) acc += to_f32(vb);
-        if (c != 0x7fffffff) acc += to_f32(vc);
-      } else if (!chain_deep<T>(src, next, A, direct, k[0][u], acc)) {
+        float va = v[0][u], vb = v[1][u], vc = v[2][u];
+        if (b < a) { int t = a; a = b; b = t; float x = va; va = vb; vb = x; }
+        if (c < b) { int t = b; b = c; c = t; float x = vb; vb = vc; vc = x; }
+        if (b < a) { int t = a; a = b; b = t; float x = va; va = vb; vb = x; }
+        acc += va;
+        if (b != 0x7fffffff) acc += vb;
+        if (c != 0x7fffffff) acc += vc;
+      } else if (!chain_deep(link, k[0][u], acc)) {
         const int h = atomicAdd(heavy_count, 1);
         heavy_list[h] = static_cast<int>(d);
         head[d] = -2 - h;
@@ -1073,15 +1068,15 @@ __global__ void __launch_bounds__(256) chain_heavy_fill(const int64_t* __restric
 }
 
 struct ChainScratch {
-  int64_t head_bytes, next_bytes, list_bytes, seg_bytes, total;
+  int64_t head_bytes, link_bytes, list_bytes, seg_bytes, total;
 };
 static ChainScratch chain_scratch(int64_t n_self, int64_t n_idx) {
   ChainScratch s;
   s.head_bytes = up256(4 * n_self);
-  s.next_bytes = up256(4 * n_idx);
+  s.link_bytes = up256(8 * n_idx);
   s.list_bytes = up256(4 * (n_idx / (kLightMax + 1) + 1));
   s.seg_bytes = up256(8 * n_idx);
-  s.total = s.head_bytes + 256 + 3 * s.list_bytes + s.next_bytes + s.seg_bytes;
+  s.total = s.head_bytes + 256 + 3 * s.list_bytes + s.link_bytes + s.seg_bytes;
   return s;
 }
 
@@ -1094,28 +1089,23 @@ static int launch_chain(const void* self, const void* index, const void* src, vo
   int* cnt = reinterpret_cast<int*>(base + S.head_bytes + 256);
   int* cursor = reinterpret_cast<int*>(base + S.head_bytes + 256 + S.list_bytes);
   int* list = reinterpret_cast<int*>(base + S.head_bytes + 256 + 2 * S.list_bytes);
-  int* next = reinterpret_cast<int*>(base + S.head_bytes + 256 + 3 * S.list_bytes);
-  int2* seg = reinterpret_cast<int2*>(base + S.head_bytes + 256 + 3 * S.list_bytes + S.next_bytes);
+  int2* link = reinterpret_cast<int2*>(base + S.head_bytes + 256 + 3 * S.list_bytes);
+  int2* seg = reinterpret_cast<int2*>(base + S.head_bytes + 256 + 3 * S.list_bytes + S.link_bytes);
   cudaError_t e = cudaMemsetAsync(head, 0xff, static_cast<size_t>(S.head_bytes), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(heads, 0, static_cast<size_t>(256 + S.list_bytes), st);
   if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
-  int direct = 1;  // src is laid out as the index's positions count
-  int64_t expect = 1;
-  for (int d = A.ndim - 1; d >= 0; --d) {
-    if (A.shape[d] != 1 && A.src_stride[d] != expect) direct = 0;
-    expect *= A.shape[d];
-  }
   const int64_t* pi = static_cast<const int64_t*>(index);
   const T* ps = static_cast<const T*>(src);
   const T* px = static_cast<const T*>(self);
   T* po = static_cast<T*>(out);
   const int64_t listed = A.n_idx / (kLightMax + 1);  // no more long chains than this
-  chain_link<<<items_grid(A.n_idx, 256 * kChainUnroll), 256, 0, st>>>(pi, head, next, A, status);
-  chain_replay<T><<<grid_for(A.n_self, 256 * kChainUnroll), 256, 0, st>>>(px, po, ps, head, next, A, direct, heads + 1, list);
+  chain_link<T><<<items_grid(A.n_idx, 256 * kChainUnroll), 256, 0, st>>>(pi, ps, head, link, A, status);
+  chain_replay<T><<<grid_for(A.n_self, 256 * kChainUnroll), 256, 0, st>>>(px, po, head, link, A.n_self, heads + 1, list);
   if (listed == 0) return check_launch(2);
-  chain_heavy_count<<<items_grid(A.n_idx, 256), 256, 0, st>>>(pi, head, cnt, A, heads + 1);
+  const int walk = items_grid(A.n_idx, 256) < 8 * kNumSMs ? items_grid(A.n_idx, 256) : 8 * kNumSMs;  // as a rule they have nothing to do
+  chain_heavy_count<<<walk, 256, 0, st>>>(pi, head, cnt, A, heads + 1);
   assign_segments<16><<<grid_for(listed, 4096), 256, 0, st>>>(cnt, cursor, listed, heads, 0x7fffffff, nullptr, nullptr);
-  chain_heavy_fill<T><<<items_grid(A.n_idx, 256), 256, 0, st>>>(pi, ps, head, cursor, seg, A, heads + 1);
+  chain_heavy_fill<T><<<walk, 256, 0, st>>>(pi, ps, head, cursor, seg, A, heads + 1);
   bucket_replay_heavy<T><<<2 * kNumSMs, 256, 0, st>>>(px, po, cnt, cursor, 1, seg, A.dim_len, heads + 1, list);
   return check_launch(6);
 }
