@@ -936,8 +936,8 @@ static int launch_bucket(const void* self, const void* index, const void* src, v
 // dim. Four destinations per thread advance together, three links deep with the entries in
 // registers; deeper chains collect their positions in an array. What bounds it: the random
 // 4-byte exchanges, and one random 8-byte look per contribution (the value lies beside the
-// link: a second look, into `src`, made the second pass 91 us instead of %R%). f16
-// 150134 x 63, half as many rows picked: 251 us in segments -> %T%.
+// link: a second look, into `src`, made the second pass 91 us instead of 61). f16
+// 150134 x 63, half as many rows picked: 251 us in segments -> 133 us.
 // A chain of more than kLightMax entries is not walked to its end (a dependent chain of loads):
 // its destination goes on a list, and four kernels that end at once when the list is empty
 // group just those contributions the way the bucket path does.
