@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(1024)
 layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW* __restrict__ w, const void* __restrict__ mean, const void* __restrict__ rstd, T* __restrict__ dx,
                     float* __restrict__ part_w, float* __restrict__ part_b, int64_t rows, int cols, int dt_stat) {
   constexpr int VE = Vec<T>::N;
-  __shared__ float red[64];
+  __shared__ float2 red[2][32];
   const int t = threadIdx.x, tpr = blockDim.x;
   const int nvec = cols / VE;
   const float inv_cols = 1.f / static_cast<float>(cols);
@@ -773,7 +773,10 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
   }
   // the vectors of the next row are requested before this row is worked on: twice the bytes in flight per thread
   uint4 ndy[VPT], nx[VPT];
+  float nmu = 0.f, nrs = 0.f;
   if (static_cast<int64_t>(blockIdx.x) < rows) {
+    nmu = load_as_f32(mean, blockIdx.x, dt_stat);
+    nrs = load_as_f32(rstd, blockIdx.x, dt_stat);
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
       const int j = t + u * tpr;
@@ -783,8 +786,9 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
       }
     }
   }
-  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    const float mu = load_as_f32(mean, row, dt_stat), rs = load_as_f32(rstd, row, dt_stat);
+  int phase = 0;
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, phase ^= 1) {
+    const float mu = nmu, rs = nrs;
     float g[VPT][VE], h[VPT][VE];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
@@ -794,6 +798,8 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
     }
     const int64_t next = row + gridDim.x;
     if (next < rows) {
+      nmu = load_as_f32(mean, next, dt_stat);
+      nrs = load_as_f32(rstd, next, dt_stat);
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
         const int j = t + u * tpr;
@@ -820,8 +826,14 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         }
       }
     }
-    s1 = block_reduce_once(s1, SumF{}, 0.f, red, 0);
-    s2 = block_reduce_once(s2, SumF{}, 0.f, red, 1);
+    // both sums behind one barrier; the row after next is the first to write these slots again
+    s1 = warp_reduce(s1, SumF{});
+    s2 = warp_reduce(s2, SumF{});
+    if ((t & 31) == 0) red[phase][t >> 5] = make_float2(s1, s2);
+    __syncthreads();
+    const float2 part = (t & 31) < (tpr >> 5) ? red[phase][t & 31] : make_float2(0.f, 0.f);
+    s1 = warp_reduce(part.x, SumF{});
+    s2 = warp_reduce(part.y, SumF{});
     const float c1 = s1 * inv_cols, c2 = s2 * inv_cols;
     if (dx) {
 #pragma unroll
