@@ -794,7 +794,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
       widen<T>(ndy[u], g[u]);
-      widen<T>(nx[u], h[u]);
+      vec_minus<T>(nx[u], mu, h[u]);  // 16-bit elements are widened inside the subtraction
     }
     const int64_t next = row + gridDim.x;
     if (next < rows) {
@@ -815,7 +815,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
       if (j < nvec) {
 #pragma unroll
         for (int e = 0; e < VE; ++e) {
-          const float xhat = (h[u][e] - mu) * rs;
+          const float xhat = h[u][e] * rs;
           ab[u][e] += g[u][e];
           aw[u][e] = fmaf(g[u][e], xhat, aw[u][e]);
           const float gy = g[u][e] * wv[u][e];
@@ -834,7 +834,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
     const float2 part = (t & 31) < (tpr >> 5) ? red[phase][t & 31] : make_float2(0.f, 0.f);
     s1 = warp_reduce(part.x, SumF{});
     s2 = warp_reduce(part.y, SumF{});
-    const float c1 = s1 * inv_cols, c2 = s2 * inv_cols;
+    const float k1 = -rs * (s1 * inv_cols), k2 = -rs * (s2 * inv_cols);
     if (dx) {
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
@@ -842,7 +842,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         if (j < nvec) {
           float o[VE];
 #pragma unroll
-          for (int e = 0; e < VE; ++e) o[e] = rs * (g[u][e] - c1 - h[u][e] * c2);
+          for (int e = 0; e < VE; ++e) o[e] = fmaf(g[u][e], rs, fmaf(h[u][e], k2, k1));
           st_stream(dx + row * cols + j * VE, narrow<T>(o));
         }
       }
