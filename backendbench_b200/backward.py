@@ -25,7 +25,7 @@ def _softmax_backward(grad_output: torch.Tensor, output: torch.Tensor, dim: int,
     if grad_output.dtype not in ops._FLOATS or input_dtype not in ops._FLOATS:
         raise ops.UnsupportedByB200(f"softmax backward: dtypes {grad_output.dtype} -> {input_dtype}")
     dim = ops._norm_dim(dim, grad_output.dim())
-    out = ops._new(grad_output.shape, input_dtype, grad_output.device)
+    out = ops._new_like(grad_output) if input_dtype == grad_output.dtype else ops._new(grad_output.shape, input_dtype, grad_output.device)
     if out.numel():
         outer, d, inner = ops._split_at(list(grad_output.shape) or [1], dim)
         g, y = ops._contig(grad_output), ops._contig(output)
@@ -67,7 +67,7 @@ def native_layer_norm_backward_default(grad_out, input, normalized_shape, mean, 
     rows = input.numel() // cols if cols else 0
     param = weight if weight is not None else bias
     wb_dtype = param.dtype if param is not None else input.dtype
-    dx = ops._new(input.shape, input.dtype, input.device) if want_dx else None
+    dx = ops._new_like(input) if want_dx else None
     dw = ops._new(normalized_shape, wb_dtype, input.device) if want_dw else None
     db = ops._new(normalized_shape, wb_dtype, input.device) if want_db else None
     if cols and (rows or want_dw or want_db):

@@ -155,11 +155,12 @@ class _Compare:
             return
         from . import ops  # strided copies go through our own kernel
 
-        rc, sc = ops._contig(r.detach()), ops._contig(s.detach())
+        rc = r if r.is_contiguous() else ops._contig(r.detach())
+        sc = s if s.is_contiguous() else ops._contig(s.detach())
         if self.rec is None:
             self.rec = _record(r.device)
         _abi.check(
-            _abi.lib().b200_allclose(rc.data_ptr(), sc.data_ptr(), rc.numel(), code, self.rtol, self.atol, self.rec.data_ptr(), 0 if self.rec_used else 1, torch.cuda.current_stream().cuda_stream),
+            _abi.lib().b200_allclose(rc.data_ptr(), sc.data_ptr(), rc.numel(), code, self.rtol, self.atol, self.rec.data_ptr(), 0 if self.rec_used else 1, ops._stream_handle()),
             "b200_allclose",
         )
         self.rec_used = True
