@@ -428,3 +428,23 @@ def test_few_rows_against_weights_along_k(dtype, M):
             # fp32 accumulation (truncating adds: 2^-23 of the running sum each) and one rounding
             bound = want.abs() * eps + (K + 8) * 2.0**-23 * size + 1e-7
             assert got.shape == (M, N) and bool(((got.double() - want).abs() <= bound).all()), (M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 129, 4100), (257, 260, 1027), (300, 515, 1027), (1531, 2050, 1027), (130, 1024, 1030), (513, 1027, 2050)])
+def test_fp32_rows_of_c_on_and_off_the_16_byte_grid(M, N, K):
+    """The fp32 epilogue writes C row by row from its staging buffer: N odd, even, a multiple of 4 and of
+    the tile, ragged M, a bias of each form, batches, transposed operands."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    for batch in (1, 2):
+        a, b = torch.randn(batch, M, K, device=DEV, generator=g), torch.randn(batch, N, K, device=DEV, generator=g).transpose(1, 2)
+        exact, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+        # accumulation adds truncate: at most K / 16 + 8 of them carry the full running sum
+        bound = (K / 16 + 32) * 2.0**-23 * size
+        if batch == 2:
+            assert bool(((ops.bmm_default(a, b).double() - exact).abs() <= bound).all())
+            continue
+        assert bool(((ops.mm_default(a[0], b[0]).double() - exact[0]).abs() <= bound[0]).all())
+        for bias in (torch.randn(N, device=DEV, generator=g), torch.randn(M, 1, device=DEV, generator=g), torch.randn(M, N, device=DEV, generator=g)):
+            got = ops.addmm_default(bias, a[0], b[0], beta=0.5, alpha=2.0)
+            assert bool(((got.double() - (2 * exact[0] + 0.5 * bias.double())).abs() <= 2 * bound[0] + 2.0**-20 * (1 + bias.double().abs())).all())
+    ops.check_device_status()
