@@ -467,24 +467,44 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int cc = lane; cc < ncols; cc += 32)
               crow[cc] = *reinterpret_cast<const TO*>(mine + rr * 128 + (((cc >> 3) ^ (rr & 7)) << 4) + (cc & 7) * 2);
           }
-        } else if (m < p.M && nb < p.N) {
-          TO* crow = C + (b * p.M + m) * p.N;
+        } else {
+          // fp32 C: the same parking, 32 columns at a time, written out row by row: 128 contiguous
+          // bytes per store, 16 per lane where rows and base allow it. Stores straight from the
+          // registers put every lane in another row, a sector per 4-byte element where N is not a
+          // multiple of 4 (1531 x 2050 x 1027 with six plane pairs: 65 us, so %EP%).
+          unsigned char* mine = epi_stage + (warp - 2) * kEpiStageBytes;
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            const int64_t n = nb + g * 8;
-            float v[8];
+          for (int h = 0; h < 2; ++h) {
+            const int64_t nh = nb + h * 32;
+            __syncwarp();  // the columns before have been read out of the buffer
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              v[e] = p.alpha * __uint_as_float(rc[g * 8 + e]);
-              if (p.has_bias && n + e < p.N) v[e] = fmaf(p.beta, to_f32(bias[m * p.sbm + (n + e) * p.sbn]), v[e]);
+            for (int g = 0; g < 8; ++g) {
+              float v[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int64_t n = nh + g * 4 + e;
+                v[e] = p.alpha * __uint_as_float(rc[h * 32 + g * 4 + e]);
+                if (p.has_bias && m < p.M && n < p.N) v[e] = fmaf(p.beta, to_f32(bias[m * p.sbm + n * p.sbn]), v[e]);
+              }
+              *reinterpret_cast<uint4*>(mine + lane * 128 + ((g ^ (lane & 7)) << 4)) = narrow<float>(v);
             }
-            if (vec_ok && n + 8 <= p.N) {
+            __syncwarp();
+            const int64_t mr0 = m0 + q * 32;
+            if (vec_ok) {
+              const int piece = lane & 7;
+              const int64_t n = nh + piece * 4;
 #pragma unroll
-              for (int h = 0; h < 8 / kOutVec; ++h) *reinterpret_cast<uint4*>(crow + n + h * kOutVec) = narrow<TO>(v + h * kOutVec);
+              for (int r4 = 0; r4 < 32; r4 += 4) {
+                const int rr = r4 + (lane >> 3);
+                if (mr0 + rr < p.M && n < p.N)
+                  *reinterpret_cast<uint4*>(C + (b * p.M + mr0 + rr) * p.N + n) = *reinterpret_cast<const uint4*>(mine + rr * 128 + ((piece ^ (rr & 7)) << 4));
+              }
             } else {
-#pragma unroll
-              for (int e = 0; e < 8; ++e)
-                if (n + e < p.N) crow[n + e] = from_f32<TO>(v[e]);
+              const int64_t n = nh + lane;
+              for (int rr = 0; rr < 32; ++rr) {
+                if (mr0 + rr >= p.M) break;
+                if (n < p.N) C[(b * p.M + mr0 + rr) * p.N + n] = *reinterpret_cast<const TO*>(mine + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+              }
             }
           }
         }
