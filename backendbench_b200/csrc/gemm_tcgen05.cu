@@ -471,7 +471,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           // fp32 C: the same parking, 32 columns at a time, written out row by row: 128 contiguous
           // bytes per store, 16 per lane where rows and base allow it. Stores straight from the
           // registers put every lane in another row, a sector per 4-byte element where N is not a
-          // multiple of 4 (1531 x 2050 x 1027 with six plane pairs: 65 us, so %EP%).
+          // multiple of 4 (1531 x 2050 x 1027 in fp32: 65.6 -> 59.6 us).
           unsigned char* mine = epi_stage + (warp - 2) * kEpiStageBytes;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
