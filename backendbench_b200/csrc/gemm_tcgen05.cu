@@ -132,6 +132,7 @@ struct GemmTcParams {
   int tma_store;    // 1 = C goes out through TMA tile stores (N % 8 == 0, aligned), 0 = plain stores
   int col_fastest;  // tile order: 1 = column-block fastest (write-bound shapes), 0 = grouped row-block fastest
   int split_slabs;  // 0, or K slabs per plane of fp32 operands split into three bf16 planes (see gemm_f32_split_dispatch)
+  int range_slabs;  // with split_slabs: 0, or slabs per range of K; the ranges are what the kernel sees as batch entries
   const uint32_t* skip_if_set;  // when not NULL: the kernel returns at once if this device word is non-zero
   uint64_t wait_limit_ns;       // every mbarrier wait gives up after this long (kWaitLimitNs in ordinary calls)
   int withhold_first_slab;      // wait probe only: the producer never loads the first K slab of a CTA's first tile
@@ -224,7 +225,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // tensor map, Kp = 64 * split_slabs. One slab of the product needs the six plane pairs
   // whose product is not below fp32 resolution: (0,0) (0,1) (1,0) (0,2) (1,1) (2,0).
   // They are walked pair by pair over all slabs (see the producer).
-  const int num_kb = p.split_slabs ? 6 * p.split_slabs : static_cast<int>((p.K + kBK - 1) / kBK);
+  const int num_kb_all = p.split_slabs ? 6 * p.split_slabs : static_cast<int>((p.K + kBK - 1) / kBK);
+  // a range of K has the slabs [b * range_slabs, (b + 1) * range_slabs), the last one what is left
+  auto slabs_of = [&](int64_t b) {
+    const int left = p.split_slabs - static_cast<int>(b) * p.range_slabs;
+    return left < p.range_slabs ? left : p.range_slabs;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -238,6 +244,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tile_coords(rem, mt, nt, mb, nb, p.col_fastest, p.group_m);
         // pair: this CTA's 128 rows of A and its half of the B slab's 256 rows
         const int m0 = mb * kTileM + static_cast<int>(cta_rank) * kBM, n0 = nb * kBN + static_cast<int>(cta_rank) * (kPair ? kBRows : 0);
+        const int tile_slabs = p.range_slabs ? slabs_of(b) : p.split_slabs, slab0 = p.range_slabs ? static_cast<int>(b) * p.range_slabs : 0;
+        const int num_kb = p.range_slabs ? 6 * tile_slabs : num_kb_all;
+        const int entry = p.range_slabs ? 0 : static_cast<int>(b);  // the planes are one batch entry whatever range is walked
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
           const uint32_t a_dst = smem_base + stage * kStageBytes, b_dst = a_dst + kABytes;
@@ -262,21 +271,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             // core truncates when it adds into the accumulator, by half a unit in the last
             // place of the running sum on average, so the small products go in while the sum
             // is still small and only the K/16 steps of the leading product pay full price
-            const int pair = kb / p.split_slabs, slab = kb - pair * p.split_slabs;
+            const int pair = kb / tile_slabs, slab = slab0 + kb - pair * tile_slabs;
             ka = (((0x001012 >> (4 * pair)) & 0xf) * p.split_slabs + slab) * kBK;
             kbb = (((0x010210 >> (4 * pair)) & 0xf) * p.split_slabs + slab) * kBK;
           }
           if (!p.a_mn_major) {
-            load(a_dst, &map_a, ka, m0, static_cast<int>(b));  // box [128 rows][64 k]
+            load(a_dst, &map_a, ka, m0, entry);  // box [128 rows][64 k]
           } else {
 #pragma unroll
-            for (int c = 0; c < kBM / 64; ++c) load(a_dst + c * 8192, &map_a, m0 + c * 64, ka, static_cast<int>(b));  // box [64 k][64 m]
+            for (int c = 0; c < kBM / 64; ++c) load(a_dst + c * 8192, &map_a, m0 + c * 64, ka, entry);  // box [64 k][64 m]
           }
           if (!p.b_mn_major) {
-            load(b_dst, &map_b, kbb, n0, static_cast<int>(b));  // box [kBRows rows][64 k]
+            load(b_dst, &map_b, kbb, n0, entry);  // box [kBRows rows][64 k]
           } else {
 #pragma unroll
-            for (int c = 0; c < kBRows / 64; ++c) load(b_dst + c * 8192, &map_b, n0 + c * 64, kbb, static_cast<int>(b));  // box [64 k][64 n]
+            for (int c = 0; c < kBRows / 64; ++c) load(b_dst + c * 8192, &map_b, n0 + c * 64, kbb, entry);  // box [64 k][64 n]
           }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
@@ -312,6 +321,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kBN);
+        const int num_kb = p.range_slabs ? 6 * slabs_of(t / (mt * nt)) : num_kb_all;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
           tc_fence_after();
@@ -680,6 +690,7 @@ int gemm_tc_dispatch(const void* A, const void* B, const void* bias, void* C, in
   // tiles for operand reuse in L2
   p.col_fastest = (K + kBK - 1) / kBK <= 4 ? 1 : 0;
   p.split_slabs = 0;
+  p.range_slabs = 0;
   p.skip_if_set = nullptr;
   p.wait_limit_ns = wait_probe_limit_ns ? wait_probe_limit_ns : kWaitLimitNs;
   p.withhold_first_slab = wait_probe_limit_ns ? 1 : 0;
@@ -753,7 +764,8 @@ int64_t gemm_tc_splitk_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_
 
 template <typename T>
 __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ part, int splits, int64_t M, int64_t N, const T* __restrict__ bias, int64_t sbm, int64_t sbn, float alpha, float beta,
-                                                     T* __restrict__ C) {
+                                                     T* __restrict__ C, const uint32_t* __restrict__ skip_if_set) {
+  if (skip_if_set && *skip_if_set != 0u) return;  // the partial products were not computed either
   const int64_t total = M * N;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     float sum = 0.f;
@@ -794,6 +806,7 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   p.has_bias = 0;
   p.col_fastest = 1;
   p.split_slabs = 0;
+  p.range_slabs = 0;
   p.skip_if_set = nullptr;
   p.wait_limit_ns = kWaitLimitNs;
   p.withhold_first_slab = 0;
@@ -809,9 +822,9 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   if (blocks > kNumSMs * 8) blocks = kNumSMs * 8;
   const float al = static_cast<float>(alpha), be = static_cast<float>(beta);
   if (dtype == B200_BF16)
-    splitk_reduce<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, st>>>(part, static_cast<int>(S), M, N, static_cast<const __nv_bfloat16*>(bias), sbm, sbn, al, be, static_cast<__nv_bfloat16*>(C));
+    splitk_reduce<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, st>>>(part, static_cast<int>(S), M, N, static_cast<const __nv_bfloat16*>(bias), sbm, sbn, al, be, static_cast<__nv_bfloat16*>(C), nullptr);
   else
-    splitk_reduce<__half><<<static_cast<int>(blocks), 256, 0, st>>>(part, static_cast<int>(S), M, N, static_cast<const __half*>(bias), sbm, sbn, al, be, static_cast<__half*>(C));
+    splitk_reduce<__half><<<static_cast<int>(blocks), 256, 0, st>>>(part, static_cast<int>(S), M, N, static_cast<const __half*>(bias), sbm, sbn, al, be, static_cast<__half*>(C), nullptr);
   return check_launch(2);
 }
 
@@ -903,9 +916,31 @@ __global__ void __launch_bounds__(256) split_f32_planes(const float* __restrict_
 
 static inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
+// Ranges of K for a product with fewer tiles than CTA pairs. What the product takes is the rounds of
+// tiles a pair walks times the slabs of a range (a slab, six plane pairs, takes about
+// 2.8 us), and writing and adding up the ranges' fp32 sums, 8 bytes per range and element of C at
+// about 5 TB/s; the cut that makes the sum least is taken where it saves an eighth or more. fp32
+// 1531 x 1027 x 2050 (30 tiles on 74 pairs) %SK1%, 2050 x 1027 x 1531 (45 tiles) %SK2%.
+// Shorter chains of truncating additions make the result more exact, not less.
+static int plan_f32_ranges(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  if (batch != 1 || M <= kBM || N <= 128 || !pair_launch_ok()) return 1;
+  const int64_t tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + 255) / 256), slots = kNumSMs / 2, slabs = (K + kBK - 1) / kBK;
+  if (tiles >= slots) return 1;
+  const double sums = static_cast<double>(M) * static_cast<double>(N) * 8 / 14e6;  // slabs' worth of time per range
+  double best = static_cast<double>(slabs);
+  int64_t ranges = 1;
+  for (int64_t s = 2; s <= 8 && slabs / s >= 4; ++s) {
+    const int64_t per = (slabs + s - 1) / s, n = (slabs + per - 1) / per;
+    const double cost = static_cast<double>((tiles * n + slots - 1) / slots * per) + sums * static_cast<double>(n);
+    if (cost < best) { best = cost; ranges = n; }
+  }
+  return best <= 0.875 * static_cast<double>(slabs) ? static_cast<int>(ranges) : 1;
+}
+
 int64_t gemm_f32_split_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   const int64_t kp = round_up(K, kBK);
-  return batch * 3 * kp * (round_up(M, 8) + round_up(N, 8)) * 2 + 256 + 512;
+  const int ranges = plan_f32_ranges(batch, M, N, K);
+  return batch * 3 * kp * (round_up(M, 8) + round_up(N, 8)) * 2 + 256 + 512 + (ranges > 1 ? ranges * M * N * 4 : 0);
 }
 
 bool gemm_f32_split_eligible(int64_t batch, int64_t M, int64_t N, int64_t K) {
@@ -955,23 +990,34 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   p.is_bf16 = 1;
   p.has_bias = (bias != nullptr && p.beta != 0.f) ? 1 : 0;
   p.split_slabs = static_cast<int>(kp / kBK);
+  // fp32 partial products [ranges][M][N] behind the planes, added in the order of the ranges
+  const int ranges = plan_f32_ranges(batch, M, N, K);
+  float* part = reinterpret_cast<float*>(pb + batch * b_rows * b_row);
+  p.range_slabs = ranges > 1 ? (p.split_slabs + ranges - 1) / ranges : 0;
+  if (ranges > 1) {
+    p.batch = ranges;
+    p.alpha = 1.f;
+    p.has_bias = 0;
+  }
   p.skip_if_set = any_flag;
   p.wait_limit_ns = kWaitLimitNs;
   p.withhold_first_slab = 0;
   p.col_fastest = 6 * p.split_slabs <= 4 ? 1 : 0;
   p.group_m = group_rows_for(3 * kp) / (pair ? 2 * kBM : kBM);
   const int tile_m = pair ? 2 * kBM : kBM;
-  const int64_t tiles = batch * ((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn);
+  const int64_t tiles = p.batch * ((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn);
   const int64_t slots = pair ? kNumSMs / 2 : kNumSMs;
   const int grid = static_cast<int>(tiles < slots ? tiles : slots) * (pair ? 2 : 1);
-  auto launch = [&](auto kernel) -> int { return launch_tc(kernel, pair, grid, st, map_a, map_b, map_a, static_cast<const float*>(bias), static_cast<float*>(C), p, status); };
+  auto launch = [&](auto kernel) -> int { return launch_tc(kernel, pair, grid, st, map_a, map_b, map_a, static_cast<const float*>(bias), ranges > 1 ? part : static_cast<float*>(C), p, status); };
   const int rc = pair ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float, true>)
                       : bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float>);
   if (rc) return rc;
+  if (ranges > 1)
+    splitk_reduce<float><<<blocks(M * N), 256, 0, st>>>(part, ranges, M, N, static_cast<const float*>(bias), sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), static_cast<float*>(C), any_flag);
   // the same product on the CUDA cores, run only when the split met an infinity or a NaN
   const int rs = gemm_simt_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, B200_F32, st, any_flag);
   if (rs) return rs;
-  return check_launch(3);
+  return check_launch(ranges > 1 ? 4 : 3);
 }
 
 }  // namespace b200

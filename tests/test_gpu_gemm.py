@@ -448,3 +448,25 @@ def test_fp32_rows_of_c_on_and_off_the_16_byte_grid(M, N, K):
             got = ops.addmm_default(bias, a[0], b[0], beta=0.5, alpha=2.0)
             assert bool(((got.double() - (2 * exact[0] + 0.5 * bias.double())).abs() <= 2 * bound[0] + 2.0**-20 * (1 + bias.double().abs())).all())
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 300, 2100), (1531, 1027, 2050), (2050, 1027, 1531), (256, 256, 20000), (257, 1000, 513), (1000, 1000, 4096)])
+def test_fp32_products_cut_into_ranges_of_k(M, N, K):
+    """Few tiles and a long K: fp32 partial products over ranges of K (the last one short), added in
+    order; the operands in both layouts, a bias, and an infinity, which sends the product to the
+    CUDA-core kernel and must leave nothing of the partial products behind."""
+    g = torch.Generator(device=DEV).manual_seed(K)
+    for ta, tb in ((False, False), (True, True)):
+        a = torch.randn(K, M, device=DEV, generator=g).t() if ta else torch.randn(M, K, device=DEV, generator=g)
+        b = torch.randn(K, N, device=DEV, generator=g) if tb else torch.randn(N, K, device=DEV, generator=g).t()
+        bias = torch.randn(N, device=DEV, generator=g)
+        exact, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+        bound = (K / 16 + 32) * 2.0**-23 * size + 1e-6
+        got = ops.mm_default(a, b)
+        assert bool(((got.double() - exact).abs() <= bound).all()) and torch.equal(got, ops.mm_default(a, b))
+        assert bool(((ops.addmm_default(bias, a, b, beta=2.0, alpha=0.5).double() - (0.5 * exact + 2.0 * bias.double())).abs() <= bound + 1e-5).all())
+    b = b.contiguous()
+    b[K // 2, 7] = float("inf")
+    got = ops.mm_default(a, b)
+    assert bool(torch.isinf(got[:, 7]).all()) and bool((torch.isfinite(got).sum(1) == N - 1).all())
+    ops.check_device_status()
