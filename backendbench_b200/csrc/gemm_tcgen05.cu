@@ -766,16 +766,30 @@ template <typename T>
 __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ part, int splits, int64_t M, int64_t N, const T* __restrict__ bias, int64_t sbm, int64_t sbn, float alpha, float beta,
                                                      T* __restrict__ C, const uint32_t* __restrict__ skip_if_set) {
   if (skip_if_set && *skip_if_set != 0u) return;  // the partial products were not computed either
+  // four elements per thread, the partial sums of all of them in flight together
+  constexpr int U = 4;
   const int64_t total = M * N;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    float sum = 0.f;
-    for (int s = 0; s < splits; ++s) sum += part[s * total + i];
-    float r = alpha * sum;
-    if (bias && beta != 0.f) {
-      const int64_t m = i / N, n = i - m * N;
-      r = fmaf(beta, to_f32(bias[m * sbm + n * sbn]), r);
+  for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; i0 < total; i0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
+    float sum[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) sum[u] = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * 256 < total) sum[u] += __ldcs(part + s * total + i0 + u * 256);
     }
-    C[i] = from_f32<T>(r);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * 256;
+      if (i >= total) break;
+      float r = alpha * sum[u];
+      if (bias && beta != 0.f) {
+        const int64_t m = i / N, n = i - m * N;
+        r = fmaf(beta, to_f32(bias[m * sbm + n * sbn]), r);
+      }
+      C[i] = from_f32<T>(r);
+    }
   }
 }
 
@@ -818,7 +832,7 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   if (dtype == B200_BF16) rc = bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float>);
   else rc = bn == 128 ? launch(gemm_tcgen05_kernel<__half, 128, float>) : launch(gemm_tcgen05_kernel<__half, 256, float>);
   if (rc) return rc;
-  int64_t blocks = (M * N + 255) / 256;
+  int64_t blocks = (M * N + 1023) / 1024;
   if (blocks > kNumSMs * 8) blocks = kNumSMs * 8;
   const float al = static_cast<float>(alpha), be = static_cast<float>(beta);
   if (dtype == B200_BF16)
@@ -1013,7 +1027,7 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
                       : bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float>);
   if (rc) return rc;
   if (ranges > 1)
-    splitk_reduce<float><<<blocks(M * N), 256, 0, st>>>(part, ranges, M, N, static_cast<const float*>(bias), sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), static_cast<float*>(C), any_flag);
+    splitk_reduce<float><<<blocks((M * N + 3) / 4), 256, 0, st>>>(part, ranges, M, N, static_cast<const float*>(bias), sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), static_cast<float*>(C), any_flag);
   // the same product on the CUDA cores, run only when the split met an infinity or a NaN
   const int rs = gemm_simt_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, B200_F32, st, any_flag);
   if (rs) return rs;
