@@ -548,86 +548,16 @@ __global__ void __launch_bounds__(128) layernorm_warp_ragged(const T* __restrict
   else { constexpr int NPL = 32; BODY; }
 constexpr int kRaggedMaxCols = 1024;
 
-// ------------------------------------------------------------------ softmax along a non-last dim, tiles of columns
-// [outer, dim, inner], `inner` not too small: a CTA owns 32 words of columns (a word is one element,
-// or two 16-bit ones where rows and bases allow it), its warps share `dim`, four rows in
-// flight per thread. Pass 1 keeps a running (max, sum) per thread and column (backward: the
-// sum), merged over the warps; pass 2 reads again (from L2 where it fits) and writes. One
-// element per lane of consecutive columns at a time, where a thread per column (forward) read with
-// dim / 1 dependent trips and a warp per line (backward) a sector per element:
-// bf16 4096 x 4096 along dim 0: %CF% / backward %CB%.
+// ------------------------------------------------------------------ softmax backward along a non-last dim
+// [outer, dim, inner] with many columns: a CTA owns 32 words of columns (a word is one element, or
+// two 16-bit ones where rows and bases allow it), its warps share `dim`, four rows in flight per
+// thread; the warps' sums are added in order, and the second pass reads again (from L2 where it
+// fits). A warp per line touches a sector per element and lane: bf16 4096 x 4096 along dim 0 327 us,
+// so 44 us; fp32 1000 x 50257 890 us, so 158 us.
 template <typename T, typename WORD, bool IS_LOG>
-__global__ void __launch_bounds__(512) softmax_cols_tile(const T* __restrict__ x, T* __restrict__ out, int64_t dim, int64_t inner) {
+__global__ void __launch_bounds__(1024) softmax_bwd_cols_tile(const T* __restrict__ g, const T* __restrict__ y, T* __restrict__ out, int64_t dim, int64_t inner) {
   constexpr int E = sizeof(WORD) / sizeof(T), U = 4;
-  __shared__ float red_m[16][32 * E], red_s[16][32 * E];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int64_t col = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * E;
-  const bool in = col < inner;
-  const T* p = x + static_cast<int64_t>(blockIdx.y) * dim * inner + col;
-  T* o = out + static_cast<int64_t>(blockIdx.y) * dim * inner + col;
-  float m[E], s[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) { m[e] = -CUDART_INF_F; s[e] = 0.f; }
-  if (in) {
-    for (int64_t k = warp; k < dim; k += U * warps) {
-      WORD v[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u * warps < dim) v[u] = *reinterpret_cast<const WORD*>(p + (k + u * warps) * inner);
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        float f[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) f[u] = k + u * warps < dim ? to_f32(reinterpret_cast<const T*>(&v[u])[e]) : -CUDART_INF_F;
-        online_raise(max_nan(max_nan(f[0], f[1]), max_nan(f[2], f[3])), m[e], s[e]);
-        online_add<U>(f, m[e], s[e]);
-      }
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < E; ++e) { red_m[warp][e * 32 + lane] = m[e]; red_s[warp][e * 32 + lane] = s[e]; }
-  __syncthreads();
-  if (!in) return;
-  float k_[E];
-  bool fused = true;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    m[e] = red_m[0][e * 32 + lane];
-    s[e] = red_s[0][e * 32 + lane];
-    for (int w = 1; w < warps; ++w) online_merge(m[e], s[e], red_m[w][e * 32 + lane], red_s[w][e * 32 + lane]);
-    k_[e] = IS_LOG ? logf(s[e]) : 1.f / s[e];
-    fused = fused && fabsf(m[e]) < 1e37f && (!IS_LOG || fabsf(k_[e]) < 1e37f);
-  }
-  for (int64_t k = warp; k < dim; k += U * warps) {
-    WORD v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (k + u * warps < dim) v[u] = __ldcs(reinterpret_cast<const WORD*>(p + (k + u * warps) * inner));
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (k + u * warps >= dim) break;
-      WORD r;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const float f = to_f32(reinterpret_cast<const T*>(&v[u])[e]);
-        float y;
-        if (fused) {
-          const float c = IS_LOG ? m[e] + k_[e] : m[e] * kLog2e;
-          y = IS_LOG ? f - c : ex2_approx(fmaf(f, kLog2e, -c)) * k_[e];
-        } else {
-          const float d = f - m[e];
-          y = IS_LOG ? d - k_[e] : ex2_approx(d * kLog2e) * k_[e];
-        }
-        reinterpret_cast<T*>(&r)[e] = from_f32<T>(y);
-      }
-      __stcs(reinterpret_cast<WORD*>(o + (k + u * warps) * inner), r);
-    }
-  }
-}
-template <typename T, typename WORD, bool IS_LOG>
-__global__ void __launch_bounds__(512) softmax_bwd_cols_tile(const T* __restrict__ g, const T* __restrict__ y, T* __restrict__ out, int64_t dim, int64_t inner) {
-  constexpr int E = sizeof(WORD) / sizeof(T), U = 4;
-  __shared__ float red[16][32 * E];
+  __shared__ float red[32][32 * E];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int64_t col = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * E;
   const bool in = col < inner;
@@ -689,9 +619,11 @@ template <typename T>
 static bool cols_in_pairs(int64_t inner, const void* a, const void* b, const void* c) {
   return sizeof(T) == 2 && inner % 2 == 0 && inner >= 64 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 3u) == 0;
 }
-static int cols_tile_threads(int64_t dim) {
+static int cols_tile_threads(int64_t dim, int64_t ctas) {
+  // four rows to a warp; with two CTAs for every SM sixteen warps to each, else all a CTA can have
+  const int most = ctas >= 2 * kNumSMs ? 16 : 32;
   int warps = 1;
-  while (warps < 16 && warps * 4 < dim) warps <<= 1;
+  while (warps < most && warps * 4 < dim) warps <<= 1;
   return 32 * warps;
 }
 
@@ -1818,20 +1750,6 @@ static int softmax_T(const void* x, void* out, int64_t outer, int64_t dim, int64
   } else {
     for (int64_t o0 = 0; o0 < outer; o0 += 65535) {
       const int64_t on = outer - o0 < 65535 ? outer - o0 : 65535;
-      if (inner >= 16 && dto == dtype_of<T>()) {
-        // (fewer columns than half a warp has lanes: a thread per column, below)
-        const T* xs = px + o0 * dim * inner;
-        T* os = static_cast<T*>(out) + o0 * dim * inner;
-        auto go = [&](auto word) {
-          typedef decltype(word) W;
-          const dim3 g(grid_for(inner, 32 * (sizeof(W) / sizeof(T))), static_cast<unsigned>(on));
-          if (is_log) softmax_cols_tile<T, W, true><<<g, cols_tile_threads(dim), 0, st>>>(xs, os, dim, inner);
-          else softmax_cols_tile<T, W, false><<<g, cols_tile_threads(dim), 0, st>>>(xs, os, dim, inner);
-        };
-        if (cols_in_pairs<T>(inner, xs, os, os)) go(uint32_t{});
-        else go(typename std::conditional<sizeof(T) == 2, uint16_t, uint32_t>::type{});
-        continue;
-      }
       dim3 g(grid_for(inner, 128), static_cast<unsigned>(on));
       softmax_cols<T><<<g, 128, 0, st>>>(px + o0 * dim * inner, static_cast<char*>(out) + o0 * dim * inner * dtype_size(dto), dim, inner, dto, is_log);
     }
@@ -1872,13 +1790,16 @@ static int softmax_bwd_T(const void* g, const void* y, void* out, int64_t outer,
     else softmax_bwd_stream<T, false><<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(pg, py, static_cast<T*>(out), static_cast<int>(dim));
     return check_launch();
   }
-  if (inner >= 16 && dto == dti && outer <= 65535) {
+  // (fewer columns: 32 of them to a CTA leave too few CTAs -- fp32 2000 x 333 took 23 us so, 15 us with
+  // a warp per line)
+  if (inner >= 64 && outer * inner >= 1024 && dto == dti && outer <= 65535) {
     T* po = static_cast<T*>(out);
     auto go = [&](auto word) {
       typedef decltype(word) W;
       const dim3 gr(grid_for(inner, 32 * (sizeof(W) / sizeof(T))), static_cast<unsigned>(outer));
-      if (is_log) softmax_bwd_cols_tile<T, W, true><<<gr, cols_tile_threads(dim), 0, st>>>(pg, py, po, dim, inner);
-      else softmax_bwd_cols_tile<T, W, false><<<gr, cols_tile_threads(dim), 0, st>>>(pg, py, po, dim, inner);
+      const int threads = cols_tile_threads(dim, static_cast<int64_t>(gr.x) * gr.y);
+      if (is_log) softmax_bwd_cols_tile<T, W, true><<<gr, threads, 0, st>>>(pg, py, po, dim, inner);
+      else softmax_bwd_cols_tile<T, W, false><<<gr, threads, 0, st>>>(pg, py, po, dim, inner);
     };
     if (cols_in_pairs<T>(inner, g, y, out)) go(uint32_t{});
     else go(typename std::conditional<sizeof(T) == 2, uint16_t, uint32_t>::type{});

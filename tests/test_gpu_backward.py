@@ -88,6 +88,30 @@ def test_long_rows_off_the_grid_or_past_the_registers(backend, dtype, cols):
             assert bool(((got.double() - want).abs() <= bound).all()), (spec, rows, float(((got.double() - want).abs() - bound).max()))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("outer,dim,inner", [(1, 1, 1024), (1, 3, 1025), (1, 65, 4096), (1, 700, 1023), (1, 130, 2050), (3, 129, 700), (40, 33, 64), (1, 4100, 2111)])
+def test_softmax_backward_along_a_leading_dim(backend, dtype, outer, dim, inner):
+    """Columns in pairs and singly, rows that fill some, all and many trips of the warps, tiles that
+    reach past the last column, a base off the word grid; against the fp64 formulas."""
+    g = torch.Generator(device=DEV).manual_seed(dim * inner)
+    for shift in (0, 1):
+        n = outer * dim * inner
+        grad = torch.randn(n + 1, device=DEV, generator=g).to(dtype)[shift : shift + n].view(outer, dim, inner)
+        x = torch.randn(outer, dim, inner, device=DEV, generator=g)
+        for spec, fwd in ((SOFT, torch.softmax), (LOGSOFT, torch.log_softmax)):
+            y = fwd(x, 1).to(dtype)
+            got = backend[get_operator(spec)](grad, y, 1, dtype).double()
+            gd, yd = grad.double(), y.double()
+            terms = gd if spec == LOGSOFT else gd * yd
+            total = terms.sum(1, keepdim=True)
+            want = gd - yd.exp() * total if spec == LOGSOFT else (gd - total) * yd
+            # fp32 sums of dim terms in any order, ex2 to 2^-20 of its value, one rounding of the result
+            scale = yd.exp() if spec == LOGSOFT else yd
+            bound = (dim * 2.0**-24 * terms.abs().sum(1, keepdim=True) + 2.0**-20 * total.abs()) * scale + gd.abs() * 2.0**-22 * (1 if spec == LOGSOFT else yd)
+            bound = bound + want.abs() * {torch.float32: 2.0**-21, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype] + (2.0**-24 if dtype == torch.float16 else 0)
+            assert bool(((got - want).abs() <= bound).all()), (spec, shift, float(((got - want).abs() - bound).max()))
+
+
 def test_float_gradients_for_a_half_input(backend):
     """The half_to_float form: fp32 grad_output / output, 16-bit grad_input."""
     g = torch.Generator(device=DEV).manual_seed(7)
