@@ -1108,7 +1108,7 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
   const T* xa = xr + a0;
   const int nv = static_cast<int>((c1 - a0) / VE);
   // argmax keeps the largest element of whole vectors and the first vector that holds it (a
-  // NaN beats everything, the first one stays); which element it was is asked once at the end
+  // NaN beats everything, the first one stays); which element it was is asked once per row
   float best = -CUDART_INF_F;
   int best_j = -1;
   auto take = [&](const uint4& raw, int j) {
@@ -1133,13 +1133,7 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
   for (; j < nv; j += tpr) take(ld_stream(xa + static_cast<int64_t>(j) * VE), j);
   if (ARG && t < nv) {
     if (best_j < 0) best_j = t;  // nothing but -inf so far: the first element is the answer
-    float f[VE];
-    widen<T>(ld_stream(xa + static_cast<int64_t>(best_j) * VE), f);
-    int first = 0;
-#pragma unroll
-    for (int e = VE - 1; e >= 0; --e)
-      if (best == best ? f[e] == best : f[e] != f[e]) first = e;
-    arg_take(a, best, a0 + static_cast<int64_t>(best_j) * VE + first);
+    arg_take(a, best, a0 + static_cast<int64_t>(best_j) * VE);  // the vector's place stands for its element's until the row is decided
   }
   if (const int64_t c = a0 + static_cast<int64_t>(nv) * VE + t; c < c1) {
     const float fv = to_f32(xr[c]);
@@ -1167,6 +1161,15 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
       }
     }
     if (threadIdx.x == 0 || (WARP && t == 0)) {
+      if (a.i >= a0 && a.i < a0 + static_cast<int64_t>(nv) * VE) {  // a vector won: its first element of that value
+        float f[VE];
+        widen<T>(ld_stream(xr + a.i), f);
+        int first = 0;
+#pragma unroll
+        for (int e = VE - 1; e >= 0; --e)
+          if (a.v == a.v ? f[e] == a.v : f[e] != f[e]) first = e;
+        a.i += first;
+      }
       if (split) { part_v[slot] = a.v; part_i[slot] = a.i; }
       else static_cast<int64_t*>(out)[row] = a.i;
     }
