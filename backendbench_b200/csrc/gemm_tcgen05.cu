@@ -225,6 +225,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // tensor map, Kp = 64 * split_slabs. One slab of the product needs the six plane pairs
   // whose product is not below fp32 resolution: (0,0) (0,1) (1,0) (0,2) (1,1) (2,0).
   // They are walked pair by pair over all slabs (see the producer).
+  const bool ranged = kPair && sizeof(TO) == 4 && p.range_slabs != 0;  // only fp32 results on pairs are cut into ranges
   const int num_kb_all = p.split_slabs ? 6 * p.split_slabs : static_cast<int>((p.K + kBK - 1) / kBK);
   // a range of K has the slabs [b * range_slabs, (b + 1) * range_slabs), the last one what is left
   auto slabs_of = [&](int64_t b) {
@@ -244,9 +245,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tile_coords(rem, mt, nt, mb, nb, p.col_fastest, p.group_m);
         // pair: this CTA's 128 rows of A and its half of the B slab's 256 rows
         const int m0 = mb * kTileM + static_cast<int>(cta_rank) * kBM, n0 = nb * kBN + static_cast<int>(cta_rank) * (kPair ? kBRows : 0);
-        const int tile_slabs = p.range_slabs ? slabs_of(b) : p.split_slabs, slab0 = p.range_slabs ? static_cast<int>(b) * p.range_slabs : 0;
-        const int num_kb = p.range_slabs ? 6 * tile_slabs : num_kb_all;
-        const int entry = p.range_slabs ? 0 : static_cast<int>(b);  // the planes are one batch entry whatever range is walked
+        const int tile_slabs = ranged ? slabs_of(b) : p.split_slabs, slab0 = ranged ? static_cast<int>(b) * p.range_slabs : 0;
+        const int num_kb = ranged ? 6 * tile_slabs : num_kb_all;
+        const int entry = ranged ? 0 : static_cast<int>(b);  // the planes are one batch entry whatever range is walked
         int slab = 0, pair4 = 0;  // split operands: slab of the range, plane pair (times 4)
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
@@ -267,7 +268,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             else tma_load_3d(dst, map, fbar, c0, c1, c2);
           };
           int ka = kb * kBK, kbb = kb * kBK;
-          if (p.split_slabs) {
+          if (sizeof(TO) == 4 && p.split_slabs) {
             // pairs (2,0) (1,1) (0,2) (1,0) (0,1) over all slabs first, then (0,0): the tensor
             // core truncates when it adds into the accumulator, by half a unit in the last
             // place of the running sum on average, so the small products go in while the sum
@@ -322,7 +323,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kBN);
-        const int num_kb = p.range_slabs ? 6 * slabs_of(t / (mt * nt)) : num_kb_all;
+        const int num_kb = ranged ? 6 * slabs_of(t / (mt * nt)) : num_kb_all;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
           tc_fence_after();

@@ -856,10 +856,13 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
   }
   // the vectors of the next row are requested before this row is worked on: twice the bytes in flight per thread
   uint4 ndy[VPT], nx[VPT];
+  constexpr bool kAhead = sizeof(T) == 2;
   float nmu = 0.f, nrs = 0.f;
   if (static_cast<int64_t>(blockIdx.x) < rows) {
-    nmu = load_as_f32(mean, blockIdx.x, dt_stat);
-    nrs = load_as_f32(rstd, blockIdx.x, dt_stat);
+    if (kAhead) {
+      nmu = load_as_f32(mean, blockIdx.x, dt_stat);
+      nrs = load_as_f32(rstd, blockIdx.x, dt_stat);
+    }
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
       const int j = t + u * tpr;
@@ -871,18 +874,22 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
   }
   int phase = 0;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, phase ^= 1) {
-    const float mu = nmu, rs = nrs;
+    // (fp32: eight small CTAs per SM hide these loads by themselves, and the registers are short)
+    const float mu = kAhead ? nmu : load_as_f32(mean, row, dt_stat), rs = kAhead ? nrs : load_as_f32(rstd, row, dt_stat);
     float g[VPT][VE], h[VPT][VE];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
       widen<T>(ndy[u], g[u]);
-      vec_minus<T>(nx[u], mu, h[u]);  // 16-bit elements are widened inside the subtraction
+      if (sizeof(T) == 2) vec_minus<T>(nx[u], mu, h[u]);  // widened inside the subtraction
+      else widen<T>(nx[u], h[u]);
     }
     const int64_t next = row + gridDim.x;
     if (next < rows) {
-      nmu = load_as_f32(mean, next, dt_stat);
-      nrs = load_as_f32(rstd, next, dt_stat);
+      if (kAhead) {
+        nmu = load_as_f32(mean, next, dt_stat);
+        nrs = load_as_f32(rstd, next, dt_stat);
+      }
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
         const int j = t + u * tpr;
@@ -898,7 +905,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
       if (j < nvec) {
 #pragma unroll
         for (int e = 0; e < VE; ++e) {
-          const float xhat = h[u][e] * rs;
+          const float xhat = (sizeof(T) == 2 ? h[u][e] : h[u][e] - mu) * rs;
           ab[u][e] += g[u][e];
           aw[u][e] = fmaf(g[u][e], xhat, aw[u][e]);
           const float gy = g[u][e] * wv[u][e];
@@ -909,15 +916,20 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         }
       }
     }
-    // both sums behind one barrier; the row after next is the first to write these slots again
-    s1 = warp_reduce(s1, SumF{});
-    s2 = warp_reduce(s2, SumF{});
-    if ((t & 31) == 0) red[phase][t >> 5] = make_float2(s1, s2);
-    __syncthreads();
-    const float2 part = (t & 31) < (tpr >> 5) ? red[phase][t & 31] : make_float2(0.f, 0.f);
-    s1 = warp_reduce(part.x, SumF{});
-    s2 = warp_reduce(part.y, SumF{});
-    const float k1 = -rs * (s1 * inv_cols), k2 = -rs * (s2 * inv_cols);
+    if constexpr (kAhead) {
+      // both sums behind one barrier; the row after next is the first to write these slots again
+      s1 = warp_reduce(s1, SumF{});
+      s2 = warp_reduce(s2, SumF{});
+      if ((t & 31) == 0) red[phase][t >> 5] = make_float2(s1, s2);
+      __syncthreads();
+      const float2 part = (t & 31) < (tpr >> 5) ? red[phase][t & 31] : make_float2(0.f, 0.f);
+      s1 = warp_reduce(part.x, SumF{});
+      s2 = warp_reduce(part.y, SumF{});
+    } else {  // (one after the other where the CTAs are small and many: fp32 65536 x 1024 144 us, 153 us behind one barrier)
+      s1 = block_reduce_once(s1, SumF{}, 0.f, &red[0][0].x, 0);
+      s2 = block_reduce_once(s2, SumF{}, 0.f, &red[0][0].x, 1);
+    }
+    const float c1 = s1 * inv_cols, c2 = s2 * inv_cols, k1 = -rs * c1, k2 = -rs * c2;
     if (dx) {
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
@@ -925,7 +937,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         if (j < nvec) {
           float o[VE];
 #pragma unroll
-          for (int e = 0; e < VE; ++e) o[e] = fmaf(g[u][e], rs, fmaf(h[u][e], k2, k1));
+          for (int e = 0; e < VE; ++e) o[e] = kAhead ? fmaf(g[u][e], rs, fmaf(h[u][e], k2, k1)) : rs * (g[u][e] - c1 - h[u][e] * c2);
           st_stream(dx + row * cols + j * VE, narrow<T>(o));
         }
       }
