@@ -465,6 +465,12 @@ def test_fp32_products_cut_into_ranges_of_k(M, N, K):
         got = ops.mm_default(a, b)
         assert bool(((got.double() - exact).abs() <= bound).all()) and torch.equal(got, ops.mm_default(a, b))
         assert bool(((ops.addmm_default(bias, a, b, beta=2.0, alpha=0.5).double() - (0.5 * exact + 2.0 * bias.double())).abs() <= bound + 1e-5).all())
+    # integers of nine bits take two planes each; with 24 terms every sum is exact, so a slab walked twice or left out shows
+    ai, bi = torch.zeros(M, K, device=DEV), torch.zeros(K, N, device=DEV)
+    ks = torch.cat([torch.arange(8, device=DEV), torch.arange(K - 8, K, device=DEV), torch.arange(K // 2 - 4, K // 2 + 4, device=DEV)])
+    ai[:, ks] = torch.randint(257, 512, (M, 24), device=DEV, generator=g).float()
+    bi[ks] = torch.randint(257, 512, (24, N), device=DEV, generator=g).float()
+    assert torch.equal(ops.mm_default(ai, bi).double(), ai.double() @ bi.double())
     b = b.contiguous()
     b[K // 2, 7] = float("inf")
     got = ops.mm_default(a, b)
