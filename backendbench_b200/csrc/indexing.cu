@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(128) gather_rows_wide(const uint4* __restrict_
 // Flattened index_select: x is [outer, dim_size, inner] in units of U, out is
 // [outer, n_idx, inner]. A thread has four units in flight, the index of each before any of
 // the units, and 32-bit coordinates wherever they suffice (two 64-bit divisions per unit were most
-// of the time: f16 150134 x 63, 75067 rows picked, %IS%).
+// of the time: f16 150134 x 63, 75067 rows picked, 22.7 -> 17.5 us).
 constexpr int kFlatUnroll = 4;
 template <typename U>
 __global__ void __launch_bounds__(256) index_select_flat(const U* __restrict__ x, const void* __restrict__ idx, U* __restrict__ out, int64_t outer, int64_t dim_size,
