@@ -18,6 +18,7 @@ bool gemm_mma_small_preferred(const void* A, const void* B, int64_t batch, int64
 int gemm_mma_small_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb,
                             int64_t sBk, int64_t sBn, int64_t sbm, int64_t sbn, double alpha, double beta, int dtype, cudaStream_t st);
 bool gemm_few_rows_preferred(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sAk, int64_t sBk, int64_t sBn, int dtype);
+bool gemm_few_rows_leaves_to_ranges(int64_t N, int64_t K);
 int gemm_few_rows_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sBn, int64_t sbm, int64_t sbn, double alpha,
                            double beta, int dtype, cudaStream_t st);
 int64_t gemm_tc_splitk_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K);
@@ -100,7 +101,7 @@ extern "C" int b200_gemm_f32(const void* A, const void* B, const void* bias, voi
 extern "C" int64_t b200_gemm_splitk_scratch_bytes(const void* A, const void* B, const void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk,
                                                   int64_t sBb, int64_t sBk, int64_t sBn, int dtype) {
   if (batch != 1 || M < 1 || N < 1 || K < 1) return 0;
-  if (g_small_path.load(std::memory_order_relaxed) && gemm_few_rows_preferred(A, B, batch, M, N, K, sAm, sAk, sBk, sBn, dtype)) return 0;
+  if (g_small_path.load(std::memory_order_relaxed) && gemm_few_rows_preferred(A, B, batch, M, N, K, sAm, sAk, sBk, sBn, dtype) && !gemm_few_rows_leaves_to_ranges(N, K)) return 0;
   if (!gemm_tc_eligible(batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype, A, B, C)) return 0;
   return gemm_tc_splitk_scratch_bytes(batch, M, N, K);
 }

@@ -24,7 +24,18 @@ namespace {
 constexpr int kFewRows = 16;
 constexpr int kFewWarps = 8;
 constexpr int kFewSteps = 4;              // 32-k steps in flight per lane
-constexpr int64_t kFewMaxK = 16384;       // a CTA walks all of K: beyond, ranges of K on several CTAs win
+// Where the kernel is the faster one; bf16 with B out of HBM, us here / the tcgen05 kernel or its ranges of K.
+// The tcgen05 kernel has a CTA to 256 columns: up to 96 of them leave it SMs idle (N 20000, K 4096: 8 rows 33 /
+// 44, 16 rows 43.5 / 44). Beyond, this one wins by what it does not read twice, as long as the rows of A, which
+// every CTA reads from L2, are few (N 32000, K 4096: 8 rows 48 / 52, 16 rows 51 / 48; K 2048: 16 rows 28 / 31) and K
+// is long enough to pay for the many CTAs (N 32000, K 264: 10 / 9; N 128256, K 1024: 4 rows 52 / 65, 16 rows 58 / 52).
+constexpr int64_t kFewMaxK = 16384;
+constexpr int64_t kFewMaxN = 96 * 256;  // with any number of rows
+constexpr int64_t kFewShortK = 256, kFewShortMaxN = 16384;  // (N 20000, K 64: 10-15 % slower here)
+static bool few_rows_pay(int64_t M, int64_t N, int64_t K) {
+  if (N > kFewShortMaxN && K < kFewShortK) return false;
+  return N <= kFewMaxN || (K >= (N > 65536 && M > 4 ? 2048 : 1024) && (M <= 8 || K <= 2048));
+}
 
 struct FewRowsArgs {
   int64_t M, N, K, sAm, sBn, sbm, sbn;
@@ -111,8 +122,17 @@ __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __re
 bool gemm_few_rows_preferred(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sAk, int64_t sBk, int64_t sBn, int dtype) {
   if (dtype != B200_BF16 && dtype != B200_F16) return false;
   if (batch != 1 || M < 1 || M > kFewRows || N < 1 || N > 0x7fffffffLL || K < 64 || K > kFewMaxK || K % 8 != 0) return false;
+  if (!few_rows_pay(M, N, K)) return false;
   if (sAk != 1 || sBk != 1 || !aligned16(A) || !aligned16(B)) return false;
   return (M == 1 || (sAm % 8 == 0 && sAm >= 0)) && (N == 1 || (sBn % 8 == 0 && sBn >= 0));
+}
+
+// A CTA walks all of K. With few columns, so few CTAs, a long K is better cut into ranges, where the K-split
+// can take the product: 4 rows, N 512: K 8192 10.4 / 10.5, K 12288 14.7 / 10.3; N 128: K 8192 10.3 / 8.7; N 64: K
+// 8192 8.1 / 8.5, K 11008 11.0 / 9.0; N 1024: K 11008 12.1 / 13.5, K 16384 19.5 / 15.6; N 1536: K 12288 15.9 / 17.9, K 16384 19.7 /
+// 18.7; N 2048: K 16384 20.7 / 21.8; N 1: K 8192 6.1 / 8.0, K 11008 7.0 / 8.2.
+bool gemm_few_rows_leaves_to_ranges(int64_t N, int64_t K) {
+  return N < 2048 && (K > (N <= 1024 ? 11264 : 14336) || (K > 8448 && N >= 16 && N <= 512) || (K > 7168 && N > 64 && N <= 128));
 }
 
 template <typename T>

@@ -410,17 +410,19 @@ def test_small_products_on_the_mma_kernel(dtype):
 @pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 15, 16, 17])
 def test_few_rows_against_weights_along_k(dtype, M):
     """Row counts on both sides of 8 and 16, N and K at the edges of a CTA's columns, a step, a
-    batch of steps and the warps' shares, row pitches, every form of bias, poison outside the rows."""
+    batch of steps and the warps' shares, row pitches, every form of bias, poison outside the rows. Small N with
+    K > 256 and short K with many columns: the other small products are a different kernel's."""
     from backendbench_b200 import ops
 
     g = torch.Generator(device="cuda").manual_seed(M)
     rnd = lambda *shape: torch.randn(shape, device="cuda", generator=g).to(dtype)
     eps = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
-    for N, K, pad in [(1, 64, 0), (7, 72, 0), (16, 128, 8), (17, 136, 0), (250, 1024, 0), (33, 1032, 16), (4099, 2056, 0), (130, 16384, 0), (64, 16392, 0), (9600, 256, 0)]:
+    for N, K, pad in [(1, 264, 0), (7, 520, 0), (16, 264, 8), (17, 1032, 0), (9601, 64, 0), (9601, 136, 8), (250, 1024, 0), (33, 1032, 16), (4099, 2056, 0), (130, 7168, 0), (130, 16384, 0), (64, 16392, 0), (9600, 256, 0)]:
         x, w = rnd(M, K + pad)[:, :K], rnd(N, K + pad)[:, :K]
         if pad:  # what lies between the rows must not be read as part of them
             x._base[:, K:] = float("nan")
             w._base[:, K:] = float("nan")
+        assert _abi.lib().b200_gemm_prefers_small(x.data_ptr(), w.data_ptr(), 1, M, N, K, 0, K + pad, 1, 0, 1, K + pad, _abi.BF16 if dtype == torch.bfloat16 else _abi.F16) == 0
         prod, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
         for bias, alpha, beta in [(None, 1, 1), (rnd(N), 1, 1), (rnd(M, 1), 0.5, 2), (rnd(M, N), 1, 1), (torch.full((N,), float("nan"), device="cuda", dtype=dtype), 1, 0)]:
             got = ops.mm_default(x, w.t()) if bias is None else ops.addmm_default(bias, x, w.t(), beta=beta, alpha=alpha)
@@ -428,6 +430,31 @@ def test_few_rows_against_weights_along_k(dtype, M):
             # fp32 accumulation (truncating adds: 2^-23 of the running sum each) and one rounding
             bound = want.abs() * eps + (K + 8) * 2.0**-23 * size + 1e-7
             assert got.shape == (M, N) and bool(((got.double() - want).abs() <= bound).all()), (M, N, K)
+
+
+def test_products_of_few_rows_and_columns_leave_a_long_k_to_ranges():
+    """Which of two kernels takes a 16-bit product of at most 16 rows: the one that walks all of K in a CTA asks for no
+    scratch, the K-split for 256 bytes and one fp32 copy of the result per range. Where few columns leave the first only a
+    handful of CTAs, a long K is cut into ranges (nothing is launched here, the pointers are never followed)."""
+    lib = _abi.lib()
+    a, b, c = 1 << 20, 1 << 21, 1 << 22
+    need = lambda M, N, K: lib.b200_gemm_splitk_scratch_bytes(a, b, c, 1, M, N, K, 0, K, 1, 0, 1, K, _abi.BF16)
+    for M, N, K in [(16, 64, 16384), (4, 512, 12288), (2, 128, 8192), (16, 1024, 16384), (8, 1536, 16384), (16, 256, 9216)]:
+        ranges, left = divmod(need(M, N, K) - 256, M * N * 4)
+        assert ranges >= 2 and left == 0, (M, N, K)
+    for M, N, K in [(16, 4096, 11008), (1, 2048, 16384), (16, 64, 4096), (4, 512, 8192), (8, 1536, 12288), (16, 1024, 11008), (16, 8, 11008)]:
+        assert need(M, N, K) == 0, (M, N, K)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_few_rows_carry_infinities_and_nan_to_their_own_results(dtype):
+    """An infinity or a NaN in one row of x or of the weights reaches that row or column of the result, as in aten, and no other."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x, w = torch.randn(5, 1032, device=DEV, generator=g).to(dtype), torch.randn(300, 1032, device=DEV, generator=g).to(dtype)
+    x[1, 1031], x[3, 0], w[7, 515], w[299, 5] = float("inf"), float("nan"), float("-inf"), float("nan")
+    got, want = ops.mm_default(x, w.t()).float(), x.double() @ w.double().t()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[torch.isinf(want)].double(), want[torch.isinf(want)])
+    assert int(torch.isfinite(got).sum()) == 3 * 298
 
 
 @pytest.mark.parametrize("M,N,K", [(129, 129, 4100), (257, 260, 1027), (300, 515, 1027), (1531, 2050, 1027), (130, 1024, 1030), (513, 1027, 2050)])
