@@ -156,7 +156,7 @@ __device__ __forceinline__ void tile_coords(int64_t rem, int64_t mt, int64_t nt,
 
 // T: operand type in shared memory (bf16 / f16). TO: type of C and of the bias -- T itself,
 // or float when the operands are the bf16 planes of split fp32 matrices.
-template <typename T, int kBN, typename TO, bool kPair = false>
+template <typename T, int kBN, typename TO, bool kPair = false, bool kRows = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c, const TO* __restrict__ bias, TO* __restrict__ C, GemmTcParams p,
                     uint32_t* __restrict__ status) {
@@ -479,43 +479,56 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int cc = lane; cc < ncols; cc += 32)
               crow[cc] = *reinterpret_cast<const TO*>(mine + rr * 128 + (((cc >> 3) ^ (rr & 7)) << 4) + (cc & 7) * 2);
           }
+        } else if constexpr (!kRows) {
+          // fp32 C, a lane to a row: 16 bytes at a time where the rows are on the grid. (Going through the
+          // buffer as below costs more than the wider stores give back: 8192 x 256 x 2048 91 us against 72.)
+          if (m < p.M && nb < p.N) {
+            TO* crow = C + (b * p.M + m) * p.N;
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+              const int64_t n = nb + g * 8;
+              float v[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                v[e] = p.alpha * __uint_as_float(rc[g * 8 + e]);
+                if (p.has_bias && n + e < p.N) v[e] = fmaf(p.beta, to_f32(bias[m * p.sbm + (n + e) * p.sbn]), v[e]);
+              }
+              if (vec_ok && n + 8 <= p.N) {
+#pragma unroll
+                for (int h = 0; h < 8 / kOutVec; ++h) *reinterpret_cast<uint4*>(crow + n + h * kOutVec) = narrow<TO>(v + h * kOutVec);
+              } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                  if (n + e < p.N) crow[n + e] = from_f32<TO>(v[e]);
+              }
+            }
+          }
         } else {
-          // fp32 C: the same parking, 32 columns at a time, written out row by row: 128 contiguous
-          // bytes per store, 16 per lane where rows and base allow it. Stores straight from the
-          // registers put every lane in another row, a sector per 4-byte element where N is not a
-          // multiple of 4 (1531 x 2050 x 1027 in fp32: 65.6 -> 59.6 us).
+          // fp32 C off the grid (kRows): the same parking, 32 columns at a time, written out row by row, 128
+          // contiguous bytes per store; the bias is looked up there, where a row and a column are all
+          // that is live. Stores straight from the registers put every lane in another row, a
+          // sector per 4-byte element (1531 x 2050 x 1027 in fp32: 65.6 -> 59.6 us).
           unsigned char* mine = epi_stage + (warp - 2) * kEpiStageBytes;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const int64_t nh = nb + h * 32;
+            const int64_t n = nb + h * 32 + lane;
             __syncwarp();  // the columns before have been read out of the buffer
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
               float v[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int64_t n = nh + g * 4 + e;
-                v[e] = p.alpha * __uint_as_float(rc[h * 32 + g * 4 + e]);
-                if (p.has_bias && m < p.M && n < p.N) v[e] = fmaf(p.beta, to_f32(bias[m * p.sbm + n * p.sbn]), v[e]);
-              }
+              for (int e = 0; e < 4; ++e) v[e] = p.alpha * __uint_as_float(rc[h * 32 + g * 4 + e]);
               *reinterpret_cast<uint4*>(mine + lane * 128 + ((g ^ (lane & 7)) << 4)) = narrow<float>(v);
             }
             __syncwarp();
             const int64_t mr0 = m0 + q * 32;
-            if (vec_ok) {
-              const int piece = lane & 7;
-              const int64_t n = nh + piece * 4;
-#pragma unroll
-              for (int r4 = 0; r4 < 32; r4 += 4) {
-                const int rr = r4 + (lane >> 3);
-                if (mr0 + rr < p.M && n < p.N)
-                  *reinterpret_cast<uint4*>(C + (b * p.M + mr0 + rr) * p.N + n) = *reinterpret_cast<const uint4*>(mine + rr * 128 + ((piece ^ (rr & 7)) << 4));
-              }
-            } else {
-              const int64_t n = nh + lane;
-              for (int rr = 0; rr < 32; ++rr) {
-                if (mr0 + rr >= p.M) break;
-                if (n < p.N) C[(b * p.M + mr0 + rr) * p.N + n] = *reinterpret_cast<const TO*>(mine + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+            for (int rr = 0; rr < 32; ++rr) {
+              const int64_t mr = mr0 + rr;
+              if (mr >= p.M) break;
+              if (n < p.N) {
+                float v = *reinterpret_cast<const float*>(mine + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+                if (p.has_bias) v = fmaf(p.beta, to_f32(bias[mr * p.sbm + n * p.sbn]), v);
+                C[(b * p.M + mr) * p.N + n] = from_f32<TO>(v);
               }
             }
           }
@@ -1025,8 +1038,14 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   const int64_t slots = pair ? kNumSMs / 2 : kNumSMs;
   const int grid = static_cast<int>(tiles < slots ? tiles : slots) * (pair ? 2 : 1);
   auto launch = [&](auto kernel) -> int { return launch_tc(kernel, pair, grid, st, map_a, map_b, map_a, static_cast<const float*>(bias), ranges > 1 ? part : static_cast<float*>(C), p, status); };
-  const int rc = pair ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float, true>)
-                      : bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float>);
+  // rows of C off the 16-byte grid go out through the staging buffer (a handful of columns does not pay for it)
+  const bool rows = N >= 32 && (N % 4 != 0 || (ranges == 1 && !aligned16(C)));
+  auto launch_as = [&](auto as_rows) -> int {
+    constexpr bool kRows = decltype(as_rows)::value;
+    return pair ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float, true, kRows>)
+                : bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float, false, kRows>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float, false, kRows>);
+  };
+  const int rc = rows ? launch_as(std::true_type{}) : launch_as(std::false_type{});
   if (rc) return rc;
   if (ranges > 1)
     splitk_reduce<float><<<blocks((M * N + 3) / 4), 256, 0, st>>>(part, ranges, M, N, static_cast<const float*>(bias), sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), static_cast<float*>(C), any_flag);

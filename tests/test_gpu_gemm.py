@@ -457,10 +457,10 @@ def test_few_rows_carry_infinities_and_nan_to_their_own_results(dtype):
     assert int(torch.isfinite(got).sum()) == 3 * 298
 
 
-@pytest.mark.parametrize("M,N,K", [(129, 129, 4100), (257, 260, 1027), (300, 515, 1027), (1531, 2050, 1027), (130, 1024, 1030), (513, 1027, 2050)])
+@pytest.mark.parametrize("M,N,K", [(129, 129, 4100), (129, 1029, 4100), (700, 33, 4100), (257, 260, 1027), (300, 515, 1027), (1531, 2050, 1027), (130, 1024, 1030), (513, 1027, 2050)])
 def test_fp32_rows_of_c_on_and_off_the_16_byte_grid(M, N, K):
-    """The fp32 epilogue writes C row by row from its staging buffer: N odd, even, a multiple of 4 and of
-    the tile, ragged M, a bias of each form, batches, transposed operands."""
+    """The fp32 epilogue writes C row by row from its staging buffer where rows are off the 16-byte grid, straight from registers
+    where they are on it: N odd, even, a multiple of 4 and of the tile, at most 32 columns past a multiple of it, ragged M, a bias of each form, batches, transposed operands."""
     g = torch.Generator(device=DEV).manual_seed(M + N)
     for batch in (1, 2):
         a, b = torch.randn(batch, M, K, device=DEV, generator=g), torch.randn(batch, N, K, device=DEV, generator=g).transpose(1, 2)
