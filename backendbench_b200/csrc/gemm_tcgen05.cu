@@ -777,22 +777,36 @@ int64_t gemm_tc_splitk_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_
   return pl.splits < 2 ? 0 : static_cast<int64_t>(pl.splits) * M * N * 4 + 256;
 }
 
-template <typename T>
+// The sum over the ranges. U elements per thread, the partial sums of all of them in flight
+// together: four where that leaves every SM eight CTAs' worth of elements (1531 x 1027 in 3 ranges
+// 12.3 -> 4.7 us), one below, where fewer and busier threads only wait longer, and of a small result B
+// ranges at a time (20000 deep, 40 x 128 outputs: the call 12.7 us, 16 with eight in flight).
+template <typename T, int U, int B>
 __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ part, int splits, int64_t M, int64_t N, const T* __restrict__ bias, int64_t sbm, int64_t sbn, float alpha, float beta,
                                                      T* __restrict__ C, const uint32_t* __restrict__ skip_if_set) {
   if (skip_if_set && *skip_if_set != 0u) return;  // the partial products were not computed either
-  // four elements per thread, the partial sums of all of them in flight together
-  constexpr int U = 4;
   const int64_t total = M * N;
   for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; i0 < total; i0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
     float sum[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) sum[u] = 0.f;
-#pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
+    if constexpr (B > 1) {
+      for (int s = 0; s < splits; s += B) {  // past the last one nothing is added
+        float v[B];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (i0 + u * 256 < total) sum[u] += __ldcs(part + s * total + i0 + u * 256);
+        for (int k = 0; k < B; ++k) v[k] = s + k < splits ? part[(s + k) * total + i0] : 0.f;
+#pragma unroll
+        for (int k = 0; k < B; ++k) sum[0] += v[k];
+      }
+    } else if constexpr (U == 1) {
+      for (int s = 0; s < splits; ++s) sum[0] += part[s * total + i0];
+    } else {
+#pragma unroll 4
+      for (int s = 0; s < splits; ++s) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u * 256 < total) sum[u] += __ldcs(part + s * total + i0 + u * 256);
+      }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -806,6 +820,19 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
       C[i] = from_f32<T>(r);
     }
   }
+}
+
+template <typename T>
+static void launch_splitk_reduce(const float* part, int splits, int64_t M, int64_t N, const void* bias, int64_t sbm, int64_t sbn, float alpha, float beta, void* C, const uint32_t* skip_if_set,
+                                 cudaStream_t st) {
+  const int64_t total = M * N, cap = kNumSMs * 8;
+  const bool wide = total >= cap * 1024;
+  int64_t blocks = wide ? (total + 1023) / 1024 : (total + 255) / 256;
+  if (blocks > cap) blocks = cap;
+  auto go = [&](auto kernel) { kernel<<<static_cast<int>(blocks), 256, 0, st>>>(part, splits, M, N, static_cast<const T*>(bias), sbm, sbn, alpha, beta, static_cast<T*>(C), skip_if_set); };
+  if (wide) go(splitk_reduce<T, 4, 1>);
+  else if (total >= 1 << 16) go(splitk_reduce<T, 1, 1>);
+  else go(splitk_reduce<T, 1, 16>);
 }
 
 int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sAk, int64_t sBk, int64_t sBn, int64_t sbm,
@@ -847,13 +874,9 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   if (dtype == B200_BF16) rc = bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float>);
   else rc = bn == 128 ? launch(gemm_tcgen05_kernel<__half, 128, float>) : launch(gemm_tcgen05_kernel<__half, 256, float>);
   if (rc) return rc;
-  int64_t blocks = (M * N + 1023) / 1024;
-  if (blocks > kNumSMs * 8) blocks = kNumSMs * 8;
   const float al = static_cast<float>(alpha), be = static_cast<float>(beta);
-  if (dtype == B200_BF16)
-    splitk_reduce<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, st>>>(part, static_cast<int>(S), M, N, static_cast<const __nv_bfloat16*>(bias), sbm, sbn, al, be, static_cast<__nv_bfloat16*>(C), nullptr);
-  else
-    splitk_reduce<__half><<<static_cast<int>(blocks), 256, 0, st>>>(part, static_cast<int>(S), M, N, static_cast<const __half*>(bias), sbm, sbn, al, be, static_cast<__half*>(C), nullptr);
+  if (dtype == B200_BF16) launch_splitk_reduce<__nv_bfloat16>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st);
+  else launch_splitk_reduce<__half>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st);
   return check_launch(2);
 }
 
@@ -1048,7 +1071,7 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   const int rc = rows ? launch_as(std::true_type{}) : launch_as(std::false_type{});
   if (rc) return rc;
   if (ranges > 1)
-    splitk_reduce<float><<<blocks((M * N + 3) / 4), 256, 0, st>>>(part, ranges, M, N, static_cast<const float*>(bias), sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), static_cast<float*>(C), any_flag);
+    launch_splitk_reduce<float>(part, ranges, M, N, bias, sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), C, any_flag, st);
   // the same product on the CUDA cores, run only when the split met an infinity or a NaN
   const int rs = gemm_simt_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, B200_F32, st, any_flag);
   if (rs) return rs;

@@ -457,6 +457,21 @@ def test_few_rows_carry_infinities_and_nan_to_their_own_results(dtype):
     assert int(torch.isfinite(got).sum()) == 3 * 298
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 64, 16384), (40, 129, 20000), (45, 2048, 4096), (256, 1030, 4096), (100, 1000, 3000)])
+def test_sums_over_ranges_of_k_are_complete(M, N, K):
+    """Few and many outputs, few and many ranges of K: with integers whose sums are exact in fp32 a range left out, added twice
+    or read past the last one shows in the result."""
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, w = (torch.randint(-3, 4, (n, K), device=DEV, generator=g).to(torch.bfloat16) for n in (M, N))
+    need = _abi.lib().b200_gemm_splitk_scratch_bytes(x.data_ptr(), w.data_ptr(), x.data_ptr(), 1, M, N, K, 0, K, 1, 0, 1, K, _abi.BF16)
+    assert need >= 2 * M * N * 4  # the K-split is what runs
+    bias = torch.randint(-3, 4, (N,), device=DEV, generator=g).to(torch.bfloat16)
+    exact = x.double() @ w.double().t()  # at most 9 K in size, below 2^24
+    assert torch.equal(ops.mm_default(x, w.t()), exact.to(torch.bfloat16))
+    assert torch.equal(ops.addmm_default(bias, x, w.t(), beta=2), (exact + 2 * bias.double()).to(torch.bfloat16))
+
+
+
 @pytest.mark.parametrize("M,N,K", [(129, 129, 4100), (129, 1029, 4100), (700, 33, 4100), (257, 260, 1027), (300, 515, 1027), (1531, 2050, 1027), (130, 1024, 1030), (513, 1027, 2050)])
 def test_fp32_rows_of_c_on_and_off_the_16_byte_grid(M, N, K):
     """The fp32 epilogue writes C row by row from its staging buffer where rows are off the 16-byte grid, straight from registers
@@ -477,7 +492,7 @@ def test_fp32_rows_of_c_on_and_off_the_16_byte_grid(M, N, K):
     ops.check_device_status()
 
 
-@pytest.mark.parametrize("M,N,K", [(129, 300, 2100), (1531, 1027, 2050), (2050, 1027, 1531), (256, 256, 20000), (257, 1000, 513), (1000, 1000, 4096)])
+@pytest.mark.parametrize("M,N,K", [(129, 300, 28000), (1531, 1027, 2050), (2050, 1027, 1531), (256, 256, 20000), (257, 1000, 513), (1000, 1000, 4096)])
 def test_fp32_products_cut_into_ranges_of_k(M, N, K):
     """Few tiles and a long K: fp32 partial products over ranges of K (the last one short), added in
     order; the operands in both layouts, a bias, and an infinity, which sends the product to the
