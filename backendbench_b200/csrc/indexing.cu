@@ -62,20 +62,24 @@ __global__ void __launch_bounds__(128) gather_rows_wide(const uint4* __restrict_
 }
 
 // Flattened index_select: x is [outer, dim_size, inner] in units of U, out is
-// [outer, n_idx, inner]. A thread has four units in flight, the index of each before any of
+// [outer, n_idx, inner]. A thread has W units in flight, the index of each before any of
 // the units, and 32-bit coordinates wherever they suffice (two 64-bit divisions per unit were most
 // of the time: f16 150134 x 63, 75067 rows picked, 22.7 -> 17.5 us).
+// W = 4 from 2^18 units on; with fewer, the SMs are not full and a thread's four units only take
+// longer than four threads' (fp32 5000 x 16, 5000 rows: 2.3 us with one, 3.2 with four; 64 x 300 x 33,
+// 150 picked, 4.1 with one, 3.6 with four).
 constexpr int kFlatUnroll = 4;
-template <typename U>
+constexpr int64_t kFlatUnrollMin = 1 << 18;
+template <typename U, int W>
 __global__ void __launch_bounds__(256) index_select_flat(const U* __restrict__ x, const void* __restrict__ idx, U* __restrict__ out, int64_t outer, int64_t dim_size,
                                                          int64_t inner, int64_t n_idx, int idx_i32, uint32_t* status) {
   const int64_t total = outer * n_idx * inner;
   const bool small = total <= 0x7fffffffLL;
-  for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * kFlatUnroll) + threadIdx.x; p0 < total; p0 += static_cast<int64_t>(gridDim.x) * (256 * kFlatUnroll)) {
-    int64_t src[kFlatUnroll], at[kFlatUnroll];
-    U v[kFlatUnroll];
+  for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * W) + threadIdx.x; p0 < total; p0 += static_cast<int64_t>(gridDim.x) * (256 * W)) {
+    int64_t src[W], at[W];
+    U v[W];
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u) {
+    for (int u = 0; u < W; ++u) {
       const int64_t p = p0 + u * 256;
       src[u] = -2;  // past the end
       if (p < total) {
@@ -101,9 +105,9 @@ __global__ void __launch_bounds__(256) index_select_flat(const U* __restrict__ x
       }
     }
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u) v[u] = src[u] >= 0 ? x[at[u] + src[u] * inner] : zero_of<U>();
+    for (int u = 0; u < W; ++u) v[u] = src[u] >= 0 ? x[at[u] + src[u] * inner] : zero_of<U>();
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u)
+    for (int u = 0; u < W; ++u)
       if (src[u] > -2) out[p0 + u * 256] = v[u];
   }
 }
@@ -115,15 +119,18 @@ struct GatherArgs {
   int64_t self_dim_size;
 };
 
-// Any layout: a thread has four elements in flight (four indices, then four elements of self).
-// f16 150134 x 63 along dim 0, 75067 rows of indices, 38.1 -> 32.9 us (one in flight, four).
-template <typename U>
+// Any layout: a thread has W elements in flight (W indices, then W elements of self). Four where
+// there are enough of them (as above; 300 x 333 2.7 us with one, 3.7 with four): f16 150134 x 63 along dim
+// 0, 75067 rows of indices, 38.1 -> 32.9 us. Where the index is not read along its rows,
+// threads of different CTAs share its sectors and four at a time make them meet later: only for results of 16 MB or
+// more (transposed views in fp32: 40000 x 100, 20000 rows, 22 us with one, 25 with four; 150134 x 63, 75067 rows, 57 / 52).
+template <typename U, int W>
 __global__ void __launch_bounds__(256) gather_generic(const U* __restrict__ self, const int64_t* __restrict__ index, U* __restrict__ out, const __grid_constant__ GatherArgs A, uint32_t* status) {
-  for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * kFlatUnroll) + threadIdx.x; p0 < A.n; p0 += static_cast<int64_t>(gridDim.x) * (256 * kFlatUnroll)) {
-    int64_t io[kFlatUnroll], so[kFlatUnroll], k[kFlatUnroll];
-    U v[kFlatUnroll];
+  for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * W) + threadIdx.x; p0 < A.n; p0 += static_cast<int64_t>(gridDim.x) * (256 * W)) {
+    int64_t io[W], so[W], k[W];
+    U v[W];
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u) {
+    for (int u = 0; u < W; ++u) {
       const int64_t p = p0 + u * 256;
       io[u] = so[u] = 0;
       if (A.n <= 0x7fffffffLL) {  // coordinates by 32-bit division (a 64-bit one costs ~5x the instructions)
@@ -146,9 +153,9 @@ __global__ void __launch_bounds__(256) gather_generic(const U* __restrict__ self
       }
     }
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u) k[u] = p0 + u * 256 < A.n ? index[io[u]] : 0;
+    for (int u = 0; u < W; ++u) k[u] = p0 + u * 256 < A.n ? index[io[u]] : 0;
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u) {
+    for (int u = 0; u < W; ++u) {
       v[u] = zero_of<U>();
       if (p0 + u * 256 < A.n) {
         if (k[u] < 0 || k[u] >= A.self_dim_size) flag_oob(status);
@@ -156,7 +163,7 @@ __global__ void __launch_bounds__(256) gather_generic(const U* __restrict__ self
       }
     }
 #pragma unroll
-    for (int u = 0; u < kFlatUnroll; ++u)
+    for (int u = 0; u < W; ++u)
       if (p0 + u * 256 < A.n) out[p0 + u * 256] = v[u];
   }
 }
@@ -372,7 +379,9 @@ static int common_unit(int64_t bytes, const void* a, const void* b) {
 template <typename U>
 static void launch_flat(const void* x, const void* idx, void* out, int64_t outer, int64_t dim_size, int64_t inner_units, int64_t n_idx, int idx_i32, uint32_t* status, cudaStream_t st) {
   const int64_t total = outer * n_idx * inner_units;
-  index_select_flat<U><<<capped_grid(total, 256 * kFlatUnroll, 16), 256, 0, st>>>(static_cast<const U*>(x), idx, static_cast<U*>(out), outer, dim_size, inner_units, n_idx, idx_i32, status);
+  auto go = [&](auto kernel, int w) { kernel<<<capped_grid(total, 256 * w, 16), 256, 0, st>>>(static_cast<const U*>(x), idx, static_cast<U*>(out), outer, dim_size, inner_units, n_idx, idx_i32, status); };
+  if (total >= kFlatUnrollMin) go(index_select_flat<U, kFlatUnroll>, kFlatUnroll);
+  else go(index_select_flat<U, 1>, 1);
 }
 
 // index_select along the LAST dim (inner == 1): every output row is a permutation-with-
@@ -562,13 +571,20 @@ extern "C" int b200_gather(const void* self, const void* index, void* out, int n
       gather_lastdim_vec<uint16_t><<<g2, 256, 0, st>>>(static_cast<const uint16_t*>(self), static_cast<const int64_t*>(index), static_cast<uint16_t*>(out), index_shape[0], index_shape[1], self_strides[0], self_dim_size, status);
     return check_launch();
   }
-  const int g = capped_grid(A.n, 256 * kFlatUnroll, 32);
-  const int64_t* pi = static_cast<const int64_t*>(index);
+  const bool along_rows = ndim == 0 || index_shape[ndim - 1] == 1 || index_strides[ndim - 1] == 1;
+  const int w = along_rows ? (A.n >= kFlatUnrollMin ? kFlatUnroll : 1) : (A.n * elem_size >= (16LL << 20) ? kFlatUnroll : 1);
+  const int g = capped_grid(A.n, 256 * w, 32);
+  auto go = [&](auto unit) {
+    typedef decltype(unit) U;
+    auto launch = [&](auto kernel) { kernel<<<g, 256, 0, st>>>(static_cast<const U*>(self), static_cast<const int64_t*>(index), static_cast<U*>(out), A, status); };
+    if (w == 1) launch(gather_generic<U, 1>);
+    else launch(gather_generic<U, kFlatUnroll>);
+  };
   switch (elem_size) {
-    case 1: gather_generic<uint8_t><<<g, 256, 0, st>>>(static_cast<const uint8_t*>(self), pi, static_cast<uint8_t*>(out), A, status); break;
-    case 2: gather_generic<uint16_t><<<g, 256, 0, st>>>(static_cast<const uint16_t*>(self), pi, static_cast<uint16_t*>(out), A, status); break;
-    case 4: gather_generic<uint32_t><<<g, 256, 0, st>>>(static_cast<const uint32_t*>(self), pi, static_cast<uint32_t*>(out), A, status); break;
-    case 8: gather_generic<uint64_t><<<g, 256, 0, st>>>(static_cast<const uint64_t*>(self), pi, static_cast<uint64_t*>(out), A, status); break;
+    case 1: go(uint8_t{}); break;
+    case 2: go(uint16_t{}); break;
+    case 4: go(uint32_t{}); break;
+    case 8: go(uint64_t{}); break;
     default: return B200_EDTYPE;
   }
   return check_launch();

@@ -355,6 +355,26 @@ def test_column_sums_in_every_word_width(backend, dtype, outer, dim, inner):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 3])
+def test_gather_and_index_select_from_one_element_per_thread_to_four(backend, dtype, n):
+    """Results just below and above the size from which a thread takes four, along rows and off them, an index out of range in the last one."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = torch.randn(41, 77, device=DEV, generator=g).to(dtype)
+    idx = torch.randint(0, 41, (n // 7, 7), device=DEV, generator=g)
+    assert bits_equal(torch.gather(x, 0, idx), backend[torch.ops.aten.gather.default](x, 0, idx))
+    assert bits_equal(torch.gather(x.t(), 1, idx.t()), backend[torch.ops.aten.gather.default](x.t(), 1, idx.t()))
+    pick = torch.randint(0, 41, (n // 77 + 1,), device=DEV, generator=g)
+    assert bits_equal(x.index_select(0, pick), backend[torch.ops.aten.index_select.default](x, 0, pick))
+    assert bits_equal(x.t().contiguous().index_select(1, pick), backend[torch.ops.aten.index_select.default](x.t().contiguous(), 1, pick))
+    ops.check_device_status()
+    idx[-1, 6] = 41
+    got = backend[torch.ops.aten.gather.default](x, 0, idx)
+    with pytest.raises(IndexError):
+        ops.check_device_status()
+    assert float(got[-1, 6]) == 0.0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_gather_along_the_last_dim(backend, dtype):
     """2-D gather along the last dim: 16 bytes of adjacent outputs per thread; fewer index rows
     than source rows, a pitched source, an index width that is not a multiple of the vector
