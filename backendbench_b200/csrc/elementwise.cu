@@ -299,12 +299,15 @@ __global__ void __launch_bounds__(256) ew_tiled(const void* a, const void* b, vo
   }
 }
 
-// The same walk for operands and result of one type T, on 64 x 64 tiles: a thread has its sixteen
-// elements of every operand in flight before it waits for any (with the four of a 32 x 32
-// tile the memory was idle most of the time), 16-bit elements move in pairs where the
+// The same walk for operands and result of one type T, on tiles of S x S. S = 64: a thread has its
+// sixteen elements of every operand in flight before it waits for any (with the four of a 32 x 32
+// tile the memory was idle most of the time), and 16-bit elements move in pairs where the
 // operands' rows, the result's rows and all bases allow it (PK = 2). Bound by HBM: add of a
-// transposed fp32 39934 x 1024 and a row vector (327 MB) 125 -> 68 us (4.8 TB/s).
-template <typename T> constexpr int kTilePitch = sizeof(T) == 2 ? 66 : 65;  // elements; rows of a column of lanes fall into different banks
+// transposed fp32 39934 x 1024 and a row vector (327 MB) 125 -> 68 us (4.8 TB/s). S = 32 where the
+// larger tiles would be few or mostly empty (see use_tiles64).
+// Pitch of a tile's rows in elements: read down a column, 4-byte elements fall into different banks, and
+// so do 16-bit ones taken singly; the pairs of PK = 2 read every second row, lanes l and l + 16 in one bank.
+template <typename T, int S> constexpr int kTilePitch = S + (sizeof(T) == 2 ? 2 : 1);
 template <typename T, int OP>
 __device__ __forceinline__ T tiled_result(T x, T y, float alpha) {
   if constexpr (OP == OP_COPY) {
@@ -318,42 +321,46 @@ __device__ __forceinline__ T tiled_result(T x, T y, float alpha) {
     else return from_f32<T>(f * to_f32(y));
   }
 }
-template <typename T, int OP, int PK>
+template <typename T, int OP, int PK, int S>
 __global__ void __launch_bounds__(256) ew_tiled_typed(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, TiledArgs A, float alpha) {
   constexpr bool kBinary = OP == OP_ADD || OP == OP_MUL;
-  constexpr int P = kTilePitch<T>, H = PK == 1 ? 2 : 1;
+  constexpr int P = kTilePitch<T, S>, J = S / 8, H = S / (32 * PK);  // a thread's rows of the tile, its words of a row
+  static_assert(PK == 1 || S == 64, "pairs need 64 columns for 32 lanes");
   typedef typename std::conditional<PK == 2, uint32_t, T>::type Word;
   extern __shared__ __align__(16) unsigned char tile_smem[];
   T* ta = reinterpret_cast<T*>(tile_smem);
-  T* tb = ta + (A.a_t ? 64 * P : 0);
+  T* tb = ta + (A.a_t ? S * P : 0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 64, c0 = static_cast<int64_t>(blockIdx.x) * 64, bz = blockIdx.z;
+  const int64_t r0 = static_cast<int64_t>(blockIdx.y) * S, c0 = static_cast<int64_t>(blockIdx.x) * S, bz = blockIdx.z;
   const T* ap = a + bz * A.ab;
   const T* bp = kBinary ? b + bz * A.bb : nullptr;
-  // transposed operands: lanes along their contiguous direction (r)
-  auto fetch = [&](const T* p, int64_t sc, T* t) {
-    Word v[8][H];
+  // transposed operands: lanes along their contiguous direction (r). Both operands are asked for before
+  // either is parked in shared memory
+  Word x[J][H], y[J][H];
+  auto fetch = [&](const T* p, int64_t sc, Word (&v)[J][H]) {
+    const T* q = p + r0 + PK * lane + (c0 + warp) * sc;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < J; ++j, q += 8 * sc) {
 #pragma unroll
       for (int h = 0; h < H; ++h) {
-        const int64_t r = r0 + PK * lane + 32 * h, c = c0 + warp + 8 * j;
         v[j][h] = Word{};
-        if (r < A.R && c < A.C) v[j][h] = *reinterpret_cast<const Word*>(p + r + c * sc);
+        if (r0 + PK * lane + 32 * h < A.R && c0 + warp + 8 * j < A.C) v[j][h] = *reinterpret_cast<const Word*>(q + 32 * h);
       }
     }
+  };
+  auto park = [&](const Word (&v)[J][H], T* t) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < J; ++j) {
 #pragma unroll
       for (int h = 0; h < H; ++h) *reinterpret_cast<Word*>(t + (warp + 8 * j) * P + PK * lane + 32 * h) = v[j][h];
     }
   };
   // the others: lanes along c, as the result is written. PK == 2: a thread's rows come in pairs
-  Word x[8][H], y[8][H];
   auto local_row = [&](int j) { return PK == 2 ? 2 * (warp + 8 * (j >> 1)) + (j & 1) : warp + 8 * j; };
-  auto direct = [&](const T* p, int64_t sr, int64_t sc, Word (&v)[8][H]) {
+  auto direct = [&](const T* p, int64_t sr, int64_t sc, Word (&v)[J][H]) {
+    const T* q = p + (r0 + warp) * sr + (c0 + lane) * sc;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < J; ++j) {
 #pragma unroll
       for (int h = 0; h < H; ++h) {
         const int64_t r = r0 + local_row(j), c = c0 + PK * lane + 32 * h;
@@ -367,23 +374,27 @@ __global__ void __launch_bounds__(256) ew_tiled_typed(const T* __restrict__ a, c
               v[j][h] = w | w << 16;
             }
           } else {
-            v[j][h] = p[r * sr + c * sc];
+            v[j][h] = q[8 * j * sr + 32 * h * sc];
           }
         }
       }
     }
   };
-  if (A.a_t) fetch(ap, A.ac, ta);
+  if (A.a_t) fetch(ap, A.ac, x);
   else direct(ap, A.ar, A.ac, x);
   if constexpr (kBinary) {
-    if (A.b_t) fetch(bp, A.bc, tb);
+    if (A.b_t) fetch(bp, A.bc, y);
     else direct(bp, A.br, A.bc, y);
   }
+  if (A.a_t) park(x, ta);
+  if constexpr (kBinary) {
+    if (A.b_t) park(y, tb);
+  }
   __syncthreads();
-  auto turned = [&](const T* t, Word (&v)[8][H]) {
+  auto turned = [&](const T* t, Word (&v)[J][H]) {
     if constexpr (PK == 2) {
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {  // a 2 x 2 block from the words of two columns
+      for (int j = 0; j < J; j += 2) {  // a 2 x 2 block from the words of two columns
         const int r = local_row(j);
         const uint32_t w0 = *reinterpret_cast<const uint32_t*>(t + 2 * lane * P + r), w1 = *reinterpret_cast<const uint32_t*>(t + (2 * lane + 1) * P + r);
         v[j][0] = __byte_perm(w0, w1, 0x5410);
@@ -391,7 +402,7 @@ __global__ void __launch_bounds__(256) ew_tiled_typed(const T* __restrict__ a, c
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < J; ++j) {
 #pragma unroll
         for (int h = 0; h < H; ++h) v[j][h] = t[(lane + 32 * h) * P + local_row(j)];
       }
@@ -401,8 +412,9 @@ __global__ void __launch_bounds__(256) ew_tiled_typed(const T* __restrict__ a, c
   if constexpr (kBinary) {
     if (A.b_t) turned(tb, y);
   }
+  T* q = out + (bz * A.R + r0 + warp) * A.C + c0 + lane;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < J; ++j) {
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const int64_t r = r0 + local_row(j), c = c0 + PK * lane + 32 * h;
@@ -417,40 +429,58 @@ __global__ void __launch_bounds__(256) ew_tiled_typed(const T* __restrict__ a, c
         } else {
           res = tiled_result<T, OP>(x[j][h], y[j][h], alpha);
         }
-        *reinterpret_cast<Word*>(out + (bz * A.R + r) * A.C + c) = res;
+        if constexpr (PK == 2) *reinterpret_cast<Word*>(out + (bz * A.R + r) * A.C + c) = res;
+        else q[8 * j * A.C + 32 * h] = res;
       }
     }
   }
 }
 
+// 64 x 64 tiles where there are enough of them for the SMs and they are not much emptier than tiles of
+// 32 x 32. Measured in fp32 (us, 32 / 64): relu of a transposed 256 x 256, 16 tiles, 1.8 / 2.2; copies of 60000
+// batches of 16 x 16, a sixteenth of each tile, 76 / 183, of 2000 batches of 33 x 129 28 / 22.
+static bool use_tiles64(const TiledArgs& T) {
+  const int64_t tr = (T.R + 63) / 64, tc = (T.C + 63) / 64, small = ((T.R + 31) / 32) * ((T.C + 31) / 32);
+  return T.B * tr * tc >= 128 && 4 * tr * tc * 5 <= small * 7;
+}
+
 template <typename T, int OP>
 static void launch_tiled_typed(const void* a, const void* b, void* out, const TiledArgs& A, float alpha, cudaStream_t st) {
   constexpr bool kBinary = OP == OP_ADD || OP == OP_MUL;
-  const dim3 g(static_cast<unsigned>((A.C + 63) / 64), static_cast<unsigned>((A.R + 63) / 64), static_cast<unsigned>(A.B));
-  const int smem = (A.a_t + (kBinary ? A.b_t : 0)) * 64 * kTilePitch<T> * static_cast<int>(sizeof(T));
   const T* pa = static_cast<const T*>(a);
   const T* pb = static_cast<const T*>(b);
+  auto go = [&](auto kernel, int side, int pitch) {
+    const dim3 g(static_cast<unsigned>((A.C + side - 1) / side), static_cast<unsigned>((A.R + side - 1) / side), static_cast<unsigned>(A.B));
+    const int smem = (A.a_t + (kBinary ? A.b_t : 0)) * side * pitch * static_cast<int>(sizeof(T));
+    kernel<<<g, 256, smem, st>>>(pa, pb, static_cast<T*>(out), A, alpha);
+  };
+  if (!use_tiles64(A)) {
+    go(ew_tiled_typed<T, OP, 1, 32>, 32, kTilePitch<T, 32>);
+    return;
+  }
   if constexpr (sizeof(T) == 2) {
     // pairs: every row that is read or written in words starts on one and has an even length
     auto even = [](const void* p, int64_t s0, int64_t s1) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0 && s0 % 2 == 0 && s1 % 2 == 0; };
     auto pairs = [&](const void* p, int t, int64_t sb, int64_t sr, int64_t sc) { return t ? A.R % 2 == 0 && even(p, sb, sc) : (sc == 0 || (sc == 1 && even(p, sb, sr))); };
     if (A.C % 2 == 0 && even(out, 0, 0) && pairs(a, A.a_t, A.ab, A.ar, A.ac) && (!kBinary || pairs(b, A.b_t, A.bb, A.br, A.bc))) {
-      ew_tiled_typed<T, OP, 2><<<g, 256, smem, st>>>(pa, pb, static_cast<T*>(out), A, alpha);
+      go(ew_tiled_typed<T, OP, 2, 64>, 64, kTilePitch<T, 64>);
       return;
     }
   }
-  ew_tiled_typed<T, OP, 1><<<g, 256, smem, st>>>(pa, pb, static_cast<T*>(out), A, alpha);
+  go(ew_tiled_typed<T, OP, 1, 64>, 64, kTilePitch<T, 64>);
 }
 
 template <int OP>
 static void launch_tiled(const void* a, const void* b, void* out, const TiledArgs& T, int dta, int dtb, int dto, float alpha, cudaStream_t st) {
   constexpr bool kBinary = OP == OP_ADD || OP == OP_MUL;
-  if (OP != OP_COPY && dta == dto && (!kBinary || dtb == dto)) {
-    switch (dto) {
-      case B200_F32: launch_tiled_typed<float, OP == OP_COPY ? OP_RELU : OP>(a, b, out, T, alpha, st); return;
-      case B200_BF16: launch_tiled_typed<__nv_bfloat16, OP == OP_COPY ? OP_RELU : OP>(a, b, out, T, alpha, st); return;
-      case B200_F16: launch_tiled_typed<__half, OP == OP_COPY ? OP_RELU : OP>(a, b, out, T, alpha, st); return;
-      default: break;
+  if constexpr (OP != OP_COPY) {  // (copies of one type move bits and do not come here)
+    if (dta == dto && (!kBinary || dtb == dto)) {
+      switch (dto) {
+        case B200_F32: launch_tiled_typed<float, OP>(a, b, out, T, alpha, st); return;
+        case B200_BF16: launch_tiled_typed<__nv_bfloat16, OP>(a, b, out, T, alpha, st); return;
+        case B200_F16: launch_tiled_typed<__half, OP>(a, b, out, T, alpha, st); return;
+        default: break;
+      }
     }
   }
   const dim3 g(static_cast<unsigned>((T.C + 31) / 32), static_cast<unsigned>((T.R + 31) / 32), static_cast<unsigned>(T.B));

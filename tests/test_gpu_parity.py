@@ -266,7 +266,7 @@ def test_gather_rows_of_self_held_in_shared_memory(backend):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("rows,cols", [(16, 16), (63, 65), (64, 64), (66, 130), (129, 62), (200, 127), (1000, 258)])
+@pytest.mark.parametrize("rows,cols", [(16, 16), (63, 65), (64, 64), (66, 130), (129, 62), (200, 127), (1000, 258), (520, 1030), (519, 1029)])
 def test_transposed_tiles_at_their_edges_in_words_and_elements(backend, dtype, rows, cols):
     """Even and odd extents, pitches and bases (16-bit elements move in pairs only where all of them
     allow it), one or both operands transposed, every kind of partner, one batch dim, bit copies."""
