@@ -571,18 +571,21 @@ static void launch_binary_T(const void* a, const void* b, void* out, int64_t n, 
 // either contiguous along c (column stride 1, any row stride, 0 included: a bias vector) or
 // constant along c (column stride 0: one value per row). The bias add and the per-row scale
 // of ordinary model code; the generic strided kernel would pay an index decomposition per
-// element. A thread produces four times 16 bytes (VEC: rows, bases and C on the 16-byte grid) or
-// four elements, with every load of the four in flight at once, and finds its rows with one
+// element. A thread produces U times 16 bytes (VEC: rows, bases and C on the 16-byte grid) or
+// U elements, with every load of the U in flight at once, and finds its rows with one
 // 32-bit division where a row is at least a CTA wide. A partner that every row shares is kept in
-// L2. Bound by HBM: bf16 32 x 2048 x 2048 plus a mask of 2048 x 2048 (537 MB) 123 -> 102 us (5.3 TB/s).
+// L2. Bound by HBM: bf16 32 x 2048 x 2048 plus a mask of 2048 x 2048 (537 MB) 123 -> 102 us (5.3 TB/s)
+// from one to four. One where four would leave threads without work, and in the long run also for single
+// elements (fp32 8191 x 4095 plus a row: 61 us with one, 82 with four; 7 x 100003, four times as many as there
+// are threads: 4.7 / 3.4) and for 16-bit operands with one value per row (8192 x 4096: 28.1 / 30.1; fp32 45 / 41.5).
 struct Rows2dArgs {
   int64_t R, C;
   int64_t ar, br;  // row strides, elements
   int a_c, b_c;    // column stride: 1 or 0
 };
-template <typename T, int OP, bool VEC>
+template <typename T, int OP, bool VEC, int U>
 __global__ void __launch_bounds__(256) ew_rows2d(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, Rows2dArgs A, float alpha) {
-  constexpr int VE = VEC ? 16 / static_cast<int>(sizeof(T)) : 1, U = 4;
+  constexpr int VE = VEC ? 16 / static_cast<int>(sizeof(T)) : 1;
   typedef typename std::conditional<VEC, uint4, T>::type Word;
   const int64_t per_row = A.C / VE, total = A.R * per_row;
   const bool small = total <= 0x7fffffffLL - 256 * U, wide = per_row >= 256;
@@ -660,9 +663,12 @@ static void launch_rows2d_T(const void* a, const void* b, void* out, const Rows2
   const bool a_ok = !A.a_c || (aligned16(a) && A.ar % VE == 0), b_ok = !A.b_c || (aligned16(b) && A.br % VE == 0);
   const bool vec = A.C % VE == 0 && aligned16(out) && a_ok && b_ok;
   const int64_t work = A.R * (vec ? A.C / VE : A.C);
-  const int g = grid_for(work, 256 * 4);
-  if (vec) ew_rows2d<T, OP, true><<<g, 256, 0, st>>>(static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), A, alpha);
-  else ew_rows2d<T, OP, false><<<g, 256, 0, st>>>(static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), A, alpha);
+  auto go = [&](auto kernel, int grid) { kernel<<<grid, 256, 0, st>>>(static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), A, alpha); };
+  constexpr int64_t kWave = 2048LL * kNumSMs;  // threads resident at once
+  if (!vec && (work <= kWave || work > 6 * kWave)) go(ew_rows2d<T, OP, false, 1>, strided_grid(work));
+  else if (!vec) go(ew_rows2d<T, OP, false, 4>, grid_for(work, 256 * 4));
+  else if (((A.a_c && A.b_c) || sizeof(T) == 4) && work > kWave) go(ew_rows2d<T, OP, true, 4>, grid_for(work, 256 * 4));
+  else go(ew_rows2d<T, OP, true, 1>, strided_grid(work));
 }
 
 template <typename Op, int OPCODE>

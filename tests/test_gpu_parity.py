@@ -375,6 +375,20 @@ def test_gather_and_index_select_from_one_element_per_thread_to_four(backend, dt
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(33, 40), (7, 100003), (40000, 9), (2000, 1001), (300, 1024), (700, 4096)])
+def test_broadcast_rows_from_one_element_per_thread_to_four(backend, dtype, rows, cols):
+    """Sizes on both sides of the lines between one and four elements (or vectors) per thread; one value per row, one row for all, a
+    row pitch."""
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    add, mul = backend[torch.ops.aten.add.Tensor], backend[torch.ops.aten.mul.Tensor]
+    a = torch.randn(rows, cols, device=DEV, generator=g).to(dtype)
+    for b in (torch.randn(cols, device=DEV, generator=g).to(dtype), torch.randn(rows, 1, device=DEV, generator=g).to(dtype), torch.randn(rows, cols + 8, device=DEV, generator=g).to(dtype)[:, :cols]):
+        # one fused multiply-add of two widened operands (in 64 bits the sum of two fp32 or 16-bit ones is exact or rounds the same), one rounding
+        assert bits_equal((a.double() + 0.5 * b.double()).to(torch.float32).to(dtype), add(a, b, alpha=0.5))
+        assert bits_equal((a.float() * b.float()).to(dtype), mul(b, a))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_gather_along_the_last_dim(backend, dtype):
     """2-D gather along the last dim: 16 bytes of adjacent outputs per thread; fewer index rows
     than source rows, a pitched source, an index width that is not a multiple of the vector
