@@ -244,6 +244,18 @@ def test_embedding_backward_at_the_edges_of_its_batches_and_windows(backend, dty
     assert bits_equal(oracle.embedding_backward(grad, idx, V, 7, False), got.cpu())
 
 
+@pytest.mark.parametrize("V,n,D", [(1, 5000, 9), (3, 40000, 64), (40, 3000, 192), (256, 20000, 63), (256, 20000, 200), (1000, 40000, 8)])
+def test_embedding_backward_of_short_tables_under_many_tokens(backend, V, n, D):
+    """More rows of many contributions than groups of 256 table rows: they are sorted by CTAs of their own."""
+    from conftest import bits_equal
+
+    g = torch.Generator().manual_seed(V)
+    for dtype in (torch.float32, torch.bfloat16):
+        idx, grad = torch.randint(0, V, (n,), generator=g), torch.randn(n, D, generator=g).to(dtype)
+        got = backend[get_operator(EMB)](grad.to(DEV), idx.to(DEV), V, -1, False)
+        assert bits_equal(oracle.embedding_backward(grad, idx, V, -1, False), got.cpu())
+
+
 def test_full_size_embedding_backward(backend):
     c = named_case("embedding_backward_bf16_128256x4096_16384")
     op = get_operator(c.op)
