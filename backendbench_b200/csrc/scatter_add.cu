@@ -729,10 +729,10 @@ __global__ void __launch_bounds__(256) bucket_count(const int64_t* __restrict__ 
 // Every counter gets a segment of its size: cursor[i] = first slot. Which part of the pool a
 // block of counters gets is decided by one atomic per block, since no result depends on
 // where a segment lies: one pass instead of an exclusive scan's three. Counters above `light`
-// are listed.
+// are listed. The counters start at `zero`.
 template <int ITEMS>
-__global__ void __launch_bounds__(256) assign_segments(const int* __restrict__ cnt, int* __restrict__ cursor, int64_t n, int* __restrict__ total, int light, int* __restrict__ heavy_count,
-                                                       int* __restrict__ heavy_list) {
+__device__ __forceinline__ void assign_segments_of(const int* __restrict__ cnt, int zero, int* __restrict__ cursor, int64_t n, int* __restrict__ total, int light, int* __restrict__ heavy_count,
+                                                   int* __restrict__ heavy_list) {
   __shared__ int warp_sums[8];
   __shared__ int block_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -747,10 +747,11 @@ __global__ void __launch_bounds__(256) assign_segments(const int* __restrict__ c
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) v[k] = base + k < n ? cnt[base + k] : 0;
+    for (int k = 0; k < ITEMS; ++k) v[k] = base + k < n ? cnt[base + k] : zero;
   }
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
+    v[k] -= zero;
     s += v[k];
     if (v[k] > light) heavy_list[atomicAdd(heavy_count, 1)] = static_cast<int>(base + k);
   }
@@ -788,6 +789,11 @@ __global__ void __launch_bounds__(256) assign_segments(const int* __restrict__ c
     prefix += v[k];
   }
 }
+template <int ITEMS>
+__global__ void __launch_bounds__(256) assign_segments(const int* __restrict__ cnt, int* __restrict__ cursor, int64_t n, int* __restrict__ total, int light, int* __restrict__ heavy_count,
+                                                       int* __restrict__ heavy_list) {
+  assign_segments_of<ITEMS>(cnt, 0, cursor, n, total, light, heavy_count, heavy_list);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) bucket_fill(const int64_t* __restrict__ index, const T* __restrict__ src, int* __restrict__ cursor, int2* __restrict__ seg,
@@ -802,12 +808,14 @@ __global__ void __launch_bounds__(256) bucket_fill(const int64_t* __restrict__ i
   }
 }
 
-// One thread per destination: replay its segment in ascending source position.
+// One thread per destination: replay its segment in ascending source position. The counters start at
+// `zero`; nothing is done where `only_if` points to a zero.
 template <typename T>
-__global__ void __launch_bounds__(256) bucket_replay(const T* __restrict__ self, T* __restrict__ out, const int* __restrict__ cnt, const int* __restrict__ cursor,
-                                                     const int2* __restrict__ seg, int64_t n_self) {
+__global__ void __launch_bounds__(256) bucket_replay(const T* __restrict__ self, T* __restrict__ out, const int* __restrict__ cnt, int zero, const int* __restrict__ cursor,
+                                                     const int2* __restrict__ seg, int64_t n_self, const int* __restrict__ only_if) {
+  if (only_if && *only_if == 0) return;
   for (int64_t d = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; d < n_self; d += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int c = cnt[d];
+    const int c = cnt[d] - zero;
     if (c == 0) {
       out[d] = self[d];
     } else if (c <= kLightMax) {
@@ -832,9 +840,19 @@ __global__ void __launch_bounds__(256) bucket_replay(const T* __restrict__ self,
 // Destinations with long segments: one CTA each. The segment is visited in windows of
 // kHeavyWindow source positions; inside a window every element is parked at its position,
 // the occupied slots are compacted in order with a block scan, and one thread adds them.
+// The counters belong to the destinations, starting at `zero`, or, unless *grouped is set, to the entries of the list
+// (`listed_cnt`, may be NULL).
+struct HeavyCounters {
+  const int* cnt;
+  const int* cursor;
+  int zero;
+  const int* listed_cnt;
+  const int* listed_cursor;
+  const int* grouped;
+};
 template <typename T>
-__global__ void __launch_bounds__(256) bucket_replay_heavy(const T* __restrict__ self, T* __restrict__ out, const int* __restrict__ cnt, const int* __restrict__ cursor, int by_list,
-                                                           const int2* __restrict__ seg, int64_t dim_len, const int* __restrict__ heavy_count, const int* __restrict__ heavy_list) {
+__global__ void __launch_bounds__(256) bucket_replay_heavy(const T* __restrict__ self, T* __restrict__ out, HeavyCounters H, const int2* __restrict__ seg, int64_t dim_len,
+                                                           const int* __restrict__ heavy_count, const int* __restrict__ heavy_list) {
   __shared__ float slot_val[kHeavyWindow];
   __shared__ unsigned char slot_set[kHeavyWindow];
   __shared__ float ordered[kHeavyWindow];
@@ -842,10 +860,11 @@ __global__ void __launch_bounds__(256) bucket_replay_heavy(const T* __restrict__
   __shared__ int window_count;
   __shared__ float acc_s;
   const int nheavy = *heavy_count;
+  const bool by_list = nheavy > 0 && H.listed_cnt && *H.grouped == 0;
   constexpr int kPer = kHeavyWindow / 256;
   for (int h = blockIdx.x; h < nheavy; h += gridDim.x) {
-    const int64_t d = heavy_list[h], i = by_list ? h : d;  // counters per entry of the list, or per destination
-    const int e = cursor[i], b = e - cnt[i];
+    const int64_t d = heavy_list[h];
+    const int e = by_list ? H.listed_cursor[h] : H.cursor[d], b = e - (by_list ? H.listed_cnt[h] : H.cnt[d] - H.zero);
     if (threadIdx.x == 0) acc_s = to_f32(self[d]);
     for (int64_t w0 = 0; w0 < dim_len; w0 += kHeavyWindow) {
       for (int i = threadIdx.x; i < kHeavyWindow; i += 256) slot_set[i] = 0;
@@ -922,13 +941,13 @@ static int launch_bucket(const void* self, const void* index, const void* src, v
   bucket_count<<<items_grid(A.n_idx, 256), 256, 0, st>>>(pi, cnt, A, status);
   assign_segments<16><<<grid_for(A.n_self, 4096), 256, 0, st>>>(cnt, cursor, A.n_self, head, kLightMax, head + 1, heavy);
   bucket_fill<T><<<items_grid(A.n_idx, 256), 256, 0, st>>>(pi, static_cast<const T*>(src), cursor, seg, A, status);
-  bucket_replay<T><<<items_grid(A.n_self, 256), 256, 0, st>>>(static_cast<const T*>(self), static_cast<T*>(out), cnt, cursor, seg, A.n_self);
-  bucket_replay_heavy<T><<<2 * kNumSMs, 256, 0, st>>>(static_cast<const T*>(self), static_cast<T*>(out), cnt, cursor, 0, seg, A.dim_len, head + 1, heavy);
+  bucket_replay<T><<<items_grid(A.n_self, 256), 256, 0, st>>>(static_cast<const T*>(self), static_cast<T*>(out), cnt, 0, cursor, seg, A.n_self, nullptr);
+  bucket_replay_heavy<T><<<2 * kNumSMs, 256, 0, st>>>(static_cast<const T*>(self), static_cast<T*>(out), HeavyCounters{cnt, cursor, 0, nullptr, nullptr, nullptr}, seg, A.dim_len, head + 1, heavy);
   return check_launch(5);
 }
 
 // ------------------------------------------------------------------ chain path
-// The same geometries with no more contributions than destinations (features of graph nodes, a
+// The same geometries with a scatter dimension no longer than self's (features of graph nodes, a
 // random half of the rows): most destinations get none or one, so grouping costs more than
 // the sums. One pass hangs every contribution into its destination's chain (`head[d]`, then
 // `link[p]`; any order), one pass over the destinations walks the chains and adds in ascending
@@ -939,14 +958,68 @@ static int launch_bucket(const void* self, const void* index, const void* src, v
 // link: a second look, into `src`, made the second pass 91 us instead of 61). f16
 // 150134 x 63, half as many rows picked: 251 us in segments -> 133 us.
 // A chain of more than kLightMax entries is not walked to its end (a dependent chain of loads):
-// its destination goes on a list, and four kernels that end at once when the list is empty
-// group just those contributions the way the bucket path does.
+// its destination goes on a list, and the kernels that follow group just those contributions the
+// way the bucket path does. Where the indices crowd on few destinations that is two passes more
+// than grouping everything at once (fp32 7000 x 333, 3500 rows into one: 224 us against 156;
+// Zipf-distributed 257 against 169), so a sample of the contributions is looked at first (`chain_begin`) and
+// where it is crowded the chains are left out and the same kernels group all of them.
 constexpr int kChainUnroll = 4;
+enum { kCtlSlots = 0, kCtlListed = 1, kCtlGrouped = 2 };  // words of the control block: slots handed out, long chains or segments, 1 = everything is grouped
+
+// Empties the chains, and the first CTA looks at up to 1024 contributions, one to a thread, spread over all of them. How
+// many pairs of them share a destination estimates how crowded the destinations are: evenly
+// spread indices give about s^2 / (2 destinations); four times that, and enough pairs for the estimate
+// to mean something, is crowded. Which way is taken changes no result.
+constexpr int kSample = 1024, kSampleSlotBits = 11;
+static_assert((1 << kSampleSlotBits) == 2 * kSample, "the table of samples");
+__global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict__ index, int* __restrict__ head, int64_t n_self, int* __restrict__ ctl, int* __restrict__ listed_cnt, int64_t listed,
+                                                   const __grid_constant__ BucketArgs A) {
+  __shared__ int key[2 * kSample], cnt[2 * kSample];
+  __shared__ int pairs;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kSample + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * kSample;
+  const int s = listed == 0 ? 0 : A.n_idx < kSample ? static_cast<int>(A.n_idx) : kSample;
+  int64_t dest = -1;
+  if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < s) {
+    const uint32_t every = static_cast<uint32_t>(A.n_idx / s);  // n_idx is below 2^31
+    // not an even spacing: it could keep to a few columns
+    const int64_t p = static_cast<int64_t>(threadIdx.x) * every + (threadIdx.x * 2654435761u >> 4) % every;
+    int64_t so;
+    int pos;
+    if (!bucket_decode(A, p, index, dest, so, pos, nullptr)) dest = -1;
+  }
+  for (int64_t i = first; i < listed; i += step) listed_cnt[i] = 0;
+  const int64_t words = (reinterpret_cast<uintptr_t>(head) & 15u) == 0 ? n_self / 4 : 0;
+  for (int64_t i = first; i < words; i += step) reinterpret_cast<int4*>(head)[i] = make_int4(-1, -1, -1, -1);
+  for (int64_t i = 4 * words + first; i < n_self; i += step) head[i] = -1;
+  if (blockIdx.x != 0) return;
+  for (int i = threadIdx.x; i < 2 * kSample; i += kSample) { key[i] = -1; cnt[i] = 0; }
+  if (threadIdx.x == 0) pairs = 0;
+  __syncthreads();
+  int mine = 0;
+  if (dest >= 0) {
+    uint32_t slot = static_cast<uint32_t>(dest) * 2654435761u >> (32 - kSampleSlotBits);
+    for (;;) {  // a free slot is found: there are twice as many as samples
+      const int was = atomicCAS(&key[slot], -1, static_cast<int>(dest));
+      if (was == -1 || was == static_cast<int>(dest)) break;
+      slot = (slot + 1) & (2 * kSample - 1);
+    }
+    mine = atomicAdd(&cnt[slot], 1);
+  }
+  if (mine) atomicAdd(&pairs, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double even = static_cast<double>(s) * s / (2.0 * static_cast<double>(A.n_idx / A.dim_len) * static_cast<double>(A.self_dim_size));
+    ctl[kCtlSlots] = 0;
+    ctl[kCtlListed] = 0;
+    ctl[kCtlGrouped] = pairs > 16.0 + 4.0 * even ? 1 : 0;
+  }
+}
 
 // link[p] = {the entry hung before p, or -1; the value's bits as fp32}
 template <typename T>
-__global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ index, const T* __restrict__ src, int* __restrict__ head, int2* __restrict__ link,
+__global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ index, const T* __restrict__ src, int* __restrict__ head, int2* __restrict__ link, const int* __restrict__ ctl,
                                                   const __grid_constant__ BucketArgs A, uint32_t* status) {
+  if (ctl[kCtlGrouped]) return;
   for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * kChainUnroll) + threadIdx.x; p0 < A.n_idx; p0 += static_cast<int64_t>(gridDim.x) * (256 * kChainUnroll)) {
     int64_t dest[kChainUnroll];
     T v[kChainUnroll];
@@ -991,8 +1064,9 @@ __device__ __noinline__ bool chain_deep(const int2* __restrict__ link, int p, fl
 
 template <typename T>
 __global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, T* __restrict__ out, int* __restrict__ head, const int2* __restrict__ link, int64_t n_self,
-                                                    int* __restrict__ heavy_count, int* __restrict__ heavy_list) {
+                                                    int* __restrict__ ctl, int* __restrict__ heavy_list) {
   constexpr int U = kChainUnroll;
+  if (ctl[kCtlGrouped]) return;
   for (int64_t d0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; d0 < n_self; d0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
     int k[4][U];  // the first three entries of each chain and what follows them, -1 past its end
     T s[U];
@@ -1032,7 +1106,7 @@ __global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, 
         if (b != 0x7fffffff) acc += vb;
         if (c != 0x7fffffff) acc += vc;
       } else if (!chain_deep(link, k[0][u], acc)) {
-        const int h = atomicAdd(heavy_count, 1);
+        const int h = atomicAdd(&ctl[kCtlListed], 1);
         heavy_list[h] = static_cast<int>(d);
         head[d] = -2 - h;
         continue;
@@ -1042,28 +1116,48 @@ __global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, 
   }
 }
 
-// the contributions of listed destinations: counted, then filled into the list's segments
-__global__ void __launch_bounds__(256) chain_heavy_count(const int64_t* __restrict__ index, const int* __restrict__ head, int* __restrict__ cnt, const __grid_constant__ BucketArgs A,
-                                                         const int* __restrict__ heavy_count) {
-  if (*heavy_count == 0) return;
+// The contributions of listed destinations, or all of them: counted (into the list's counters, or into
+// the heads, which stand at -1), given segments, filled in.
+__global__ void __launch_bounds__(256) chain_count(const int64_t* __restrict__ index, int* __restrict__ head, int* __restrict__ listed_cnt, const __grid_constant__ BucketArgs A,
+                                                   const int* __restrict__ ctl) {
+  const bool grouped = ctl[kCtlGrouped] != 0;
+  if (!grouped && ctl[kCtlListed] == 0) return;
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < A.n_idx; p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     int64_t dest, so;
     int pos;
     if (!bucket_decode(A, p, index, dest, so, pos, nullptr)) continue;
-    const int h = head[dest];
-    if (h <= -2) atomicAdd(&cnt[-2 - h], 1);
+    if (grouped) {
+      atomicAdd(&head[dest], 1);
+    } else {
+      const int h = head[dest];
+      if (h <= -2) atomicAdd(&listed_cnt[-2 - h], 1);
+    }
   }
 }
+__global__ void __launch_bounds__(256) chain_assign(const int* __restrict__ head, int* __restrict__ cursor, int64_t n_self, const int* __restrict__ listed_cnt, int* __restrict__ listed_cursor,
+                                                    int64_t listed, int* __restrict__ ctl, int* __restrict__ heavy_list) {
+  constexpr int ITEMS = 16;
+  const bool grouped = ctl[kCtlGrouped] != 0;
+  if (!grouped && (ctl[kCtlListed] == 0 || static_cast<int64_t>(blockIdx.x) * 256 * ITEMS >= listed)) return;
+  if (grouped) assign_segments_of<ITEMS>(head, -1, cursor, n_self, ctl + kCtlSlots, kLightMax, ctl + kCtlListed, heavy_list);
+  else assign_segments_of<ITEMS>(listed_cnt, 0, listed_cursor, listed, ctl + kCtlSlots, 0x7fffffff, nullptr, nullptr);
+}
 template <typename T>
-__global__ void __launch_bounds__(256) chain_heavy_fill(const int64_t* __restrict__ index, const T* __restrict__ src, const int* __restrict__ head, int* __restrict__ cursor, int2* __restrict__ seg,
-                                                        const __grid_constant__ BucketArgs A, const int* __restrict__ heavy_count) {
-  if (*heavy_count == 0) return;
+__global__ void __launch_bounds__(256) chain_fill(const int64_t* __restrict__ index, const T* __restrict__ src, const int* __restrict__ head, int* __restrict__ cursor, int* __restrict__ listed_cursor,
+                                                  int2* __restrict__ seg, const __grid_constant__ BucketArgs A, const int* __restrict__ ctl, uint32_t* status) {
+  const bool grouped = ctl[kCtlGrouped] != 0;
+  if (!grouped && ctl[kCtlListed] == 0) return;
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < A.n_idx; p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     int64_t dest, so;
     int pos;
-    if (!bucket_decode(A, p, index, dest, so, pos, nullptr)) continue;
-    const int h = head[dest];
-    if (h <= -2) seg[atomicAdd(&cursor[-2 - h], 1)] = make_int2(pos, __float_as_int(to_f32(src[so])));
+    if (!bucket_decode(A, p, index, dest, so, pos, grouped ? status : nullptr)) continue;  // (chains: chain_link has set it)
+    int* at = &cursor[dest];
+    if (!grouped) {
+      const int h = head[dest];
+      if (h > -2) continue;
+      at = &listed_cursor[-2 - h];
+    }
+    seg[atomicAdd(at, 1)] = make_int2(pos, __float_as_int(to_f32(src[so])));
   }
 }
 
@@ -1076,38 +1170,41 @@ static ChainScratch chain_scratch(int64_t n_self, int64_t n_idx) {
   s.link_bytes = up256(8 * n_idx);
   s.list_bytes = up256(4 * (n_idx / (kLightMax + 1) + 1));
   s.seg_bytes = up256(8 * n_idx);
-  s.total = s.head_bytes + 256 + 3 * s.list_bytes + s.link_bytes + s.seg_bytes;
+  s.total = 2 * s.head_bytes + 256 + 3 * s.list_bytes + s.link_bytes + s.seg_bytes;
   return s;
 }
 
 template <typename T>
 static int launch_chain(const void* self, const void* index, const void* src, void* out, const BucketArgs& A, void* scratch, uint32_t* status, cudaStream_t st) {
   const ChainScratch S = chain_scratch(A.n_self, A.n_idx);
-  char* base = static_cast<char*>(scratch);
-  int* head = reinterpret_cast<int*>(base);
-  int* heads = reinterpret_cast<int*>(base + S.head_bytes);  // [0] slots handed out, [1] long chains; the list's counters behind them
-  int* cnt = reinterpret_cast<int*>(base + S.head_bytes + 256);
-  int* cursor = reinterpret_cast<int*>(base + S.head_bytes + 256 + S.list_bytes);
-  int* list = reinterpret_cast<int*>(base + S.head_bytes + 256 + 2 * S.list_bytes);
-  int2* link = reinterpret_cast<int2*>(base + S.head_bytes + 256 + 3 * S.list_bytes);
-  int2* seg = reinterpret_cast<int2*>(base + S.head_bytes + 256 + 3 * S.list_bytes + S.link_bytes);
-  cudaError_t e = cudaMemsetAsync(head, 0xff, static_cast<size_t>(S.head_bytes), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(heads, 0, static_cast<size_t>(256 + S.list_bytes), st);
-  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+  char* at = static_cast<char*>(scratch);
+  auto take = [&](int64_t bytes) { char* p = at; at += bytes; return p; };
+  int* head = reinterpret_cast<int*>(take(S.head_bytes));
+  int* cursor = reinterpret_cast<int*>(take(S.head_bytes));
+  int* ctl = reinterpret_cast<int*>(take(256));
+  int* listed_cnt = reinterpret_cast<int*>(take(S.list_bytes));
+  int* listed_cursor = reinterpret_cast<int*>(take(S.list_bytes));
+  int* list = reinterpret_cast<int*>(take(S.list_bytes));
+  int2* link = reinterpret_cast<int2*>(take(S.link_bytes));
+  int2* seg = reinterpret_cast<int2*>(take(S.seg_bytes));
   const int64_t* pi = static_cast<const int64_t*>(index);
   const T* ps = static_cast<const T*>(src);
   const T* px = static_cast<const T*>(self);
   T* po = static_cast<T*>(out);
-  const int64_t listed = A.n_idx / (kLightMax + 1);  // no more long chains than this
-  chain_link<T><<<items_grid(A.n_idx, 256 * kChainUnroll), 256, 0, st>>>(pi, ps, head, link, A, status);
-  chain_replay<T><<<grid_for(A.n_self, 256 * kChainUnroll), 256, 0, st>>>(px, po, head, link, A.n_self, heads + 1, list);
-  if (listed == 0) return check_launch(2);
-  const int walk = items_grid(A.n_idx, 256) < 8 * kNumSMs ? items_grid(A.n_idx, 256) : 8 * kNumSMs;  // as a rule they have nothing to do
-  chain_heavy_count<<<walk, 256, 0, st>>>(pi, head, cnt, A, heads + 1);
-  assign_segments<16><<<grid_for(listed, 4096), 256, 0, st>>>(cnt, cursor, listed, heads, 0x7fffffff, nullptr, nullptr);
-  chain_heavy_fill<T><<<walk, 256, 0, st>>>(pi, ps, head, cursor, seg, A, heads + 1);
-  bucket_replay_heavy<T><<<2 * kNumSMs, 256, 0, st>>>(px, po, cnt, cursor, 1, seg, A.dim_len, heads + 1, list);
-  return check_launch(6);
+  const int64_t listed = A.n_idx / (kLightMax + 1);  // no more long chains (or segments) than this
+  auto capped = [](int64_t n, int per, int64_t cap) { const int64_t g = (n + per - 1) / per; return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g)); };
+  chain_begin<<<capped(A.n_self, 8 * kSample, 2 * kNumSMs), kSample, 0, st>>>(pi, head, A.n_self, ctl, listed_cnt, listed, A);
+  chain_link<T><<<items_grid(A.n_idx, 256 * kChainUnroll), 256, 0, st>>>(pi, ps, head, link, ctl, A, status);
+  chain_replay<T><<<grid_for(A.n_self, 256 * kChainUnroll), 256, 0, st>>>(px, po, head, link, A.n_self, ctl, list);
+  if (listed == 0) return check_launch(3);
+  // as a rule these five have nothing to do
+  const int walk = capped(A.n_idx, 256, 16 * kNumSMs);
+  chain_count<<<walk, 256, 0, st>>>(pi, head, listed_cnt, A, ctl);
+  chain_assign<<<grid_for(A.n_self, 4096), 256, 0, st>>>(head, cursor, A.n_self, listed_cnt, listed_cursor, listed, ctl, list);
+  chain_fill<T><<<walk, 256, 0, st>>>(pi, ps, head, cursor, listed_cursor, seg, A, ctl, status);
+  bucket_replay<T><<<capped(A.n_self, 256, 16 * kNumSMs), 256, 0, st>>>(px, po, head, -1, cursor, seg, A.n_self, ctl + kCtlGrouped);
+  bucket_replay_heavy<T><<<2 * kNumSMs, 256, 0, st>>>(px, po, HeavyCounters{head, cursor, -1, listed_cnt, listed_cursor, ctl + kCtlGrouped}, seg, A.dim_len, ctl + kCtlListed, list);
+  return check_launch(8);
 }
 
 // ------------------------------------------------------------------ embedding_dense_backward
@@ -1565,9 +1662,10 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
   }
   // short lines are cheapest walked by one thread each; anything longer is grouped by destination
   if (P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && index_shape[dim] < 0x7fffffffLL && index_shape[dim] > 64) {
-    // at most one contribution per destination on average: chains. More make chains long, and a
-    // segment's entries lie side by side where a chain's do not.
-    P.path = P.n_idx <= P.n_self ? kPathChain : kPathBucket;
+    // at most one contribution per reachable destination on average: chains (fp32 150134 x 63, as many
+    // rows: 245 us, segments 530). More make chains long, and a segment's entries lie side by side
+    // where a chain's do not.
+    P.path = index_shape[dim] <= self_shape[dim] ? kPathChain : kPathBucket;
     P.scratch_bytes = P.path == kPathChain ? chain_scratch(P.n_self, P.n_idx).total : bucket_scratch(P.n_self, P.n_idx).total;
     return P;
   }

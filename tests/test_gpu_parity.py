@@ -505,7 +505,7 @@ def test_scatter_add_grouped_by_destination_path_bit_exact(backend, dtype):
 def test_scatter_add_chains_of_every_depth_bit_exact(backend, dtype, cols):
     """Destinations with 0 .. 5, 31 .. 34 and hundreds of contributions among many with none (chains
     of up to three in registers, up to 32 in an array, longer ones grouped), on both sides of
-    one contribution per destination, with strided index and values, and an index out of range."""
+    one contribution per destination, with strided index and values."""
     impl = backend[torch.ops.aten.scatter_add.default]
     g = torch.Generator().manual_seed(cols)
     rows = 9001
@@ -526,13 +526,44 @@ def test_scatter_add_chains_of_every_depth_bit_exact(backend, dtype, cols):
         # the same along the last dim of the transposed problem
         assert bits_equal(want.t().contiguous(), impl(x.t().contiguous().to(DEV), 1, idx.t().contiguous().to(DEV), src.t().contiguous().to(DEV)).cpu()), n
     ops.check_device_status()
-    idx[17, 0] = rows
-    got = impl(x.to(DEV), 0, idx.to(DEV), src.to(DEV))
-    with pytest.raises(IndexError):
-        ops.check_device_status()
-    src[17, 0] = 0.0
-    idx[17, 0] = 8999
-    assert torch.equal(oracle.scatter_add(x, 0, idx, src).float(), got.cpu().float())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("spread", ["one", "zipf", "even", "some_hubs"])
+def test_scatter_add_crowded_or_not_bit_exact(backend, dtype, spread):
+    """No more contributions than destinations, on few of them or on many: crowded indices are grouped by destination, others
+    hang in chains, of which the long ones are grouped. The same bits on every way, along either dim, and an index out of range,
+    among long chains too, is reported and adds nothing."""
+    impl = backend[torch.ops.aten.scatter_add.default]
+    g = torch.Generator().manual_seed(7)
+    rows, cols, n = 4001, 7, 3500
+    if spread == "one":
+        idx = torch.full((n, cols), 4000)
+    elif spread == "zipf":
+        idx = (torch.exp(torch.rand(n, cols, generator=g, dtype=torch.float64) * math.log(rows + 1)).long() - 1).clamp_(0, rows - 1)
+    else:
+        idx = torch.randint(0, rows, (n, cols), generator=g)
+        if spread == "some_hubs":  # one long chain in 24,500 contributions: too few for the sample to call it crowded
+            idx[torch.randperm(n, generator=g)[:80], 3] = 11
+    for bad in (False, True):
+        if bad:
+            idx[17, 0], idx[18, 3], idx[3499, 6] = rows, -1, rows + 5
+        x, src = torch.randn(rows, cols, generator=g).to(dtype), torch.randn(n, cols, generator=g).to(dtype)
+        got = impl(x.to(DEV), 0, idx.to(DEV), src.to(DEV))
+        turned = impl(x.t().contiguous().to(DEV), 1, idx.t().contiguous().to(DEV), src.t().contiguous().to(DEV))
+        if not bad:
+            want = oracle.scatter_add(x, 0, idx, src)
+            assert bits_equal(want, got.cpu())
+            ops.check_device_status()
+        else:
+            with pytest.raises(IndexError):
+                ops.check_device_status()
+            out = (idx < 0) | (idx >= rows)
+            # what is out of range goes to an extra row that is cut off again
+            wide = torch.cat([x, torch.zeros(1, cols, dtype=dtype)])
+            want = oracle.scatter_add(wide, 0, torch.where(out, rows, idx), src)[:rows].contiguous()
+            assert bits_equal(want, got.cpu())
+        assert bits_equal(want.t().contiguous(), turned.cpu())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
