@@ -216,6 +216,16 @@ template <typename F> __device__ __forceinline__ float block_reduce_once(float v
   return warp_reduce(lane < nwarps ? part[lane] : identity, f);
 }
 
+// f[0] + ... + f[N - 1] as a tree (N a power of two): log2(N) roundings behind the result in place of N - 1
+template <int N> __device__ __forceinline__ float tree_sum(float* f) {
+#pragma unroll
+  for (int h = N / 2; h > 0; h /= 2) {
+#pragma unroll
+    for (int i = 0; i < h; ++i) f[i] += f[i + h];
+  }
+  return f[0];
+}
+
 // 2^x by the special-function unit alone (results below 2^-126 flush to zero).
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;

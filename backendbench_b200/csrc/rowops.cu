@@ -1219,51 +1219,91 @@ __global__ void __launch_bounds__(256) argmax_cols(const T* __restrict__ x, int6
 }
 
 // Sum over columns (inner > 1; the bias gradient of a linear layer). grid = (inner tiles, outer,
-// splits). A lane owns the columns of one WORD (as wide as the rows' length and base allow), a
-// warp 32 such words of every blockDim / 32 -th row of the slice, eight rows in flight; the
-// warps' sums are added in warp order. A thread per column with four 2-byte loads in flight
-// left the memory idle: bf16 8192 x 11008 (180 MB) 93 us, so 34 us (5.3 TB/s).
-template <typename T, typename WORD>
+// splits). A lane owns the columns of G WORDs that lie 32 words apart (a word as wide as the rows' length and
+// base allow), a warp 32 G such words of every blockDim / 32 -th row of the slice, eight rows in
+// flight; the eight are added as a tree before they go into the accumulator, and so are the warps'
+// sums: the chain of additions behind a result is a 128th of the slice long. Bound by HBM: bf16 8192 x 11008
+// (180 MB) 93 -> 32 us (5.6 TB/s) and fp32 8192 x 11007, off the grid, 94 -> 62 us against a thread
+// per column with four loads in flight (the kernel below); root mean square error there 3.2e-7 -> 1.2e-7.
+template <typename T, typename WORD, int G>
 __global__ void __launch_bounds__(512, 2) sum_cols(const T* __restrict__ x, void* __restrict__ out, float* __restrict__ part_v, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int dto) {
   constexpr int E = sizeof(WORD) / sizeof(T), U = 8;
-  __shared__ float red[16][32 * E];
+  __shared__ float red[16][32 * E * G];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int64_t o = blockIdx.y;
-  const int64_t col = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * E;
+  const int64_t o = blockIdx.y, first = static_cast<int64_t>(blockIdx.x) * (32 * E * G);
   const int64_t k0 = static_cast<int64_t>(blockIdx.z) * chunk;
   const int64_t k1 = k0 + chunk < dim ? k0 + chunk : dim;
-  float acc[E];
+  float acc[G][E];
+  bool in[G];
 #pragma unroll
-  for (int e = 0; e < E; ++e) acc[e] = 0.f;
-  if (col < inner) {
-    const T* p = x + o * dim * inner + col;
-    for (int64_t k = k0 + warp; k < k1; k += U * warps) {
-      WORD v[U];
+  for (int g = 0; g < G; ++g) {
+    in[g] = first + (g * 32 + lane) * E < inner;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        v[u] = WORD{};
-        if (k + u * warps < k1) v[u] = __ldcs(reinterpret_cast<const WORD*>(p + (k + u * warps) * inner));
+    for (int e = 0; e < E; ++e) acc[g][e] = 0.f;
+  }
+  const T* p = x + (o * dim + k0 + warp) * inner + first + lane * E;
+  for (int64_t k = k0 + warp; k < k1; k += U * warps, p += U * warps * inner) {
+    WORD v[U][G];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        v[u][g] = WORD{};
+        if (k + u * warps < k1 && in[g]) v[u][g] = __ldcs(reinterpret_cast<const WORD*>(p + u * warps * inner + g * 32 * E));
       }
+    }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const T* f = reinterpret_cast<const T*>(&v[u]);
+    for (int g = 0; g < G; ++g) {
 #pragma unroll
-        for (int e = 0; e < E; ++e) acc[e] += to_f32(f[e]);
+      for (int e = 0; e < E; ++e) {
+        float f[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) f[u] = to_f32(reinterpret_cast<const T*>(&v[u][g])[e]);
+        acc[g][e] += tree_sum<U>(f);
       }
     }
   }
 #pragma unroll
-  for (int e = 0; e < E; ++e) red[warp][e * 32 + lane] = acc[e];
-  __syncthreads();
-  for (int c = threadIdx.x; c < 32 * E; c += blockDim.x) {
-    const int64_t i = (static_cast<int64_t>(blockIdx.x) * 32 + (c & 31)) * E + (c >> 5);
-    if (i >= inner) continue;
-    float s = red[0][c];
-    for (int w = 1; w < warps; ++w) s += red[w][c];
-    const int64_t oi = o * inner + i;
-    if (gridDim.z > 1) part_v[static_cast<int64_t>(blockIdx.z) * outer * inner + oi] = s;
-    else store_from_f32(out, oi, dto, s);
+  for (int g = 0; g < G; ++g) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) red[warp][(g * E + e) * 32 + lane] = acc[g][e];
   }
+  __syncthreads();
+  for (int j = threadIdx.x; j < 32 * E * G; j += blockDim.x) {
+    const int64_t i = first + ((j / (32 * E)) * 32 + (j & 31)) * E + (j >> 5) % E;
+    if (i >= inner) continue;
+    float f[16];
+#pragma unroll
+    for (int w = 0; w < 16; ++w) f[w] = w < warps ? red[w][j] : 0.f;
+    const float sum = tree_sum<16>(f);
+    const int64_t oi = o * inner + i;
+    if (gridDim.z > 1) part_v[static_cast<int64_t>(blockIdx.z) * outer * inner + oi] = sum;
+    else store_from_f32(out, oi, dto, sum);
+  }
+}
+
+// The same with a thread to a column: few rows, or columns that would leave the tiles above mostly empty.
+template <typename T>
+__global__ void __launch_bounds__(256) sum_cols_thread(const T* __restrict__ x, void* __restrict__ out, float* __restrict__ part_v, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int dto) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= inner) return;
+  const int64_t o = blockIdx.y;
+  const int64_t k0 = static_cast<int64_t>(blockIdx.z) * chunk;
+  const int64_t k1 = k0 + chunk < dim ? k0 + chunk : dim;
+  const T* p = x + o * dim * inner + i;
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  int64_t k = k0;
+  for (; k + 3 < k1; k += 4) {
+    s0 += to_f32(p[k * inner]);
+    s1 += to_f32(p[(k + 1) * inner]);
+    s2 += to_f32(p[(k + 2) * inner]);
+    s3 += to_f32(p[(k + 3) * inner]);
+  }
+  for (; k < k1; ++k) s0 += to_f32(p[k * inner]);
+  const float s = (s0 + s1) + (s2 + s3);
+  const int64_t oi = o * inner + i;
+  if (gridDim.z > 1) part_v[static_cast<int64_t>(blockIdx.z) * outer * inner + oi] = s;
+  else store_from_f32(out, oi, dto, s);
 }
 
 // Column reduction with at most 32 columns (the bias-gradient shape: many rows, few columns):
@@ -1601,14 +1641,6 @@ static ReducePlan plan_reduce(int64_t outer, int64_t dim, int64_t inner) {
   return p;
 }
 
-template <typename T, typename WORD>
-static void launch_sum_cols_word(const T* x, void* out, float* pv, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int splits, int dto, cudaStream_t st) {
-  constexpr int E = sizeof(WORD) / sizeof(T);
-  int warps = 1;  // eight rows to a warp: more warps than that would find no rows in a short slice
-  while (warps < 16 && warps * 8 < chunk) warps <<= 1;
-  const dim3 g(grid_for(inner, 32 * E), static_cast<unsigned>(outer), static_cast<unsigned>(splits));
-  sum_cols<T, WORD><<<g, 32 * warps, 0, st>>>(x, out, pv, outer, dim, inner, chunk, dto);
-}
 // Bytes of the words `sum_cols` reads: the widest that every row starts on and ends with, and
 // that still gives 32 lanes columns.
 static int sum_cols_word(const void* x, int64_t inner, int esize) {
@@ -1616,15 +1648,73 @@ static int sum_cols_word(const void* x, int64_t inner, int esize) {
   while (bytes > esize && (((inner * esize) | static_cast<int64_t>(reinterpret_cast<uintptr_t>(x))) % bytes || inner * esize < 32 * bytes)) bytes >>= 1;
   return bytes;
 }
+struct SumColsPlan {
+  bool by_thread;  // sum_cols_thread, as `plan_reduce` cuts it
+  int word, groups, warps, splits;
+  int64_t chunk;
+};
+// How a column sum is cut up; `p`: what `plan_reduce` says (its scratch holds four fp32 partials per slice and output). All times in
+// us, fp32, with the other way behind the bar.
+static SumColsPlan plan_sum_cols(const void* x, int64_t outer, int64_t dim, int64_t inner, int esize, const ReducePlan& p) {
+  SumColsPlan s{false, sum_cols_word(x, inner, esize), 1, 16, 1, dim};
+  s.groups = s.word == esize ? 2 : 1;
+  auto tile = [&] { return static_cast<int64_t>(32) * (s.word / esize) * s.groups; };
+  auto tiles = [&] { return (inner + tile() - 1) / tile(); };
+  // 8 x 100 2.5 | 3.7; 7000 times 33 x 5 7.1 | 8.5; 16384 x 130 5.4 | 6.4, whose last tile is nearly empty
+  s.by_thread = dim < 16 || inner <= 16 || (tiles() > 1 && tiles() * tile() * 10 > inner * 13 && outer * dim * inner * esize <= (16LL << 20));
+  if (s.by_thread) {
+    s.splits = p.splits;
+    s.chunk = p.chunk;
+    return s;
+  }
+  constexpr int64_t kSlots = 2 * kNumSMs;  // CTAs of sixteen warps resident at once
+  if (dim <= 384 || (dim <= 512 && outer * tiles() >= kNumSMs)) {
+    // a CTA walks these rows in three or four trips, a second launch costs as much: no slices (100 x 4099 3.3 | 4.9),
+    // narrower tiles if that is what gives every SM one
+    while (outer * tiles() < kNumSMs && (s.groups > 1 || s.word > esize)) {
+      if (s.groups > 1) s.groups = 1;
+      else s.word >>= 1;
+    }
+  } else {
+    // the fewest slices that fill the rounds of CTAs to six sevenths (bf16 8192 x 11008, 43 tiles: 6 slices, one
+    // round, 32 us; 7, a round and a bit, 49), not below 32 rows each
+    const int64_t most = p.splits > 1 ? (4LL * p.splits < dim / 32 ? 4LL * p.splits : dim / 32) : 1;
+    int64_t best = 1;
+    double best_full = 0.;
+    for (int64_t n = 1; n <= most && best_full < 6. / 7; ++n) {
+      const int64_t ctas = outer * tiles() * n, rounds = (ctas + kSlots - 1) / kSlots;
+      const double full = static_cast<double>(ctas) / static_cast<double>(rounds * kSlots);
+      if (full > best_full) { best = n; best_full = full; }
+    }
+    s.chunk = (dim + best - 1) / best;
+    s.splits = static_cast<int>((dim + s.chunk - 1) / s.chunk);
+  }
+  // eight rows to a warp; more, smaller CTAs where sixteen warps each would make two rounds (64 x 50257 4.7 | 5.6)
+  while (s.warps > 1 && s.warps * 4 >= s.chunk) s.warps >>= 1;
+  while (s.warps > 4 && s.splits == 1 && outer * tiles() > kSlots * 16 / s.warps) s.warps >>= 1;
+  return s;
+}
+template <typename T, typename WORD, int G>
+static void launch_sum_cols_as(const T* x, void* out, float* pv, int64_t outer, int64_t dim, int64_t inner, const SumColsPlan& s, int dto, cudaStream_t st) {
+  const dim3 g(grid_for(inner, 32 * (sizeof(WORD) / sizeof(T)) * G), static_cast<unsigned>(outer), static_cast<unsigned>(s.splits));
+  sum_cols<T, WORD, G><<<g, 32 * s.warps, 0, st>>>(x, out, pv, outer, dim, inner, s.chunk, dto);
+}
 template <typename T>
-static void launch_sum_cols(const T* x, void* out, float* pv, int64_t outer, int64_t dim, int64_t inner, int64_t chunk, int splits, int dto, cudaStream_t st) {
-  switch (sum_cols_word(x, inner, sizeof(T))) {
-    case 16: launch_sum_cols_word<T, uint4>(x, out, pv, outer, dim, inner, chunk, splits, dto, st); break;
-    case 8: launch_sum_cols_word<T, uint2>(x, out, pv, outer, dim, inner, chunk, splits, dto, st); break;
-    case 4: launch_sum_cols_word<T, uint32_t>(x, out, pv, outer, dim, inner, chunk, splits, dto, st); break;
-    default:
-      if constexpr (sizeof(T) == 2) launch_sum_cols_word<T, uint16_t>(x, out, pv, outer, dim, inner, chunk, splits, dto, st);
-      break;
+static void launch_sum_cols(const T* x, void* out, float* pv, int64_t outer, int64_t dim, int64_t inner, const SumColsPlan& s, int dto, cudaStream_t st) {
+  typedef typename std::conditional<sizeof(T) == 2, uint16_t, uint32_t>::type One;
+  if (s.by_thread) {
+    const dim3 g(grid_for(inner, 256), static_cast<unsigned>(outer), static_cast<unsigned>(s.splits));
+    sum_cols_thread<T><<<g, 256, 0, st>>>(x, out, pv, outer, dim, inner, s.chunk, dto);
+  } else if (s.word == 16) {
+    launch_sum_cols_as<T, uint4, 1>(x, out, pv, outer, dim, inner, s, dto, st);
+  } else if (s.word == 8) {
+    launch_sum_cols_as<T, uint2, 1>(x, out, pv, outer, dim, inner, s, dto, st);
+  } else if (sizeof(T) == 2 && s.word == 4) {
+    launch_sum_cols_as<T, uint32_t, 1>(x, out, pv, outer, dim, inner, s, dto, st);
+  } else if (s.groups == 2) {
+    launch_sum_cols_as<T, One, 2>(x, out, pv, outer, dim, inner, s, dto, st);
+  } else {
+    launch_sum_cols_as<T, One, 1>(x, out, pv, outer, dim, inner, s, dto, st);
   }
 }
 
@@ -1657,7 +1747,7 @@ static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim,
       for (int64_t o0 = 0; o0 < outer; o0 += 65535) {
         const int64_t on = outer - o0 < 65535 ? outer - o0 : 65535;
         if (ARG) argmax_cols<T><<<dim3(grid_for(inner, 256), static_cast<unsigned>(on), 1), 256, 0, st>>>(px + o0 * dim * inner, static_cast<int64_t*>(out) + o0 * inner, nullptr, nullptr, on, dim, inner, dim);
-        else launch_sum_cols<T>(px + o0 * dim * inner, static_cast<char*>(out) + o0 * inner * dtype_size(dto), nullptr, on, dim, inner, dim, 1, dto, st);
+        else launch_sum_cols<T>(px + o0 * dim * inner, static_cast<char*>(out) + o0 * inner * dtype_size(dto), nullptr, on, dim, inner, plan_sum_cols(px + o0 * dim * inner, on, dim, inner, sizeof(T), ReducePlan{1, dim}), dto, st);
       }
       return check_launch();
     }
@@ -1670,21 +1760,14 @@ static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim,
       dim3 g(grid_for(inner, 256), static_cast<unsigned>(outer), p.splits);
       argmax_cols<T><<<g, 256, 0, st>>>(px, static_cast<int64_t*>(out), pv, pi, outer, dim, inner, p.chunk);
     } else {
-      if (p.splits > 1) {
-        // no more slices than fit the SMs at once, two CTAs to each: a CTA more is a round more
-        // (bf16 8192 x 11008: 49 us in the 7 slices of the plan at one CTA per SM, 34 us in 6 at two)
-        const int64_t tile = 32 * sum_cols_word(x, inner, sizeof(T));
-        int64_t fit = 2 * kNumSMs / (outer * ((inner * static_cast<int64_t>(sizeof(T)) + tile - 1) / tile));
-        if (fit < 1) fit = 1;
-        if (p.splits > fit) {
-          p.chunk = (dim + fit - 1) / fit;
-          p.splits = static_cast<int>((dim + p.chunk - 1) / p.chunk);
-        }
-      }
-      launch_sum_cols<T>(px, out, pv, outer, dim, inner, p.chunk, p.splits, dto, st);
+      const SumColsPlan sp = plan_sum_cols(px, outer, dim, inner, sizeof(T), p);
+      if (p.splits > 1) pv = static_cast<float*>(scratch);  // (no indices to keep: all of it is for sums)
+      launch_sum_cols<T>(px, out, pv, outer, dim, inner, sp, dto, st);
+      p.splits = sp.splits;
     }
   }
-  if (p.splits >= 64 && nout <= 8LL * kNumSMs * 8) reduce_finalize_warp<ARG><<<grid_for(nout, 8), 256, 0, st>>>(pv, pi, out, nout, p.splits, dto);
+  // few outputs of many slices: a warp to an output (2048 x 514 in 32 slices: 4.7 us the call, 6.0 with a thread to each)
+  if (p.splits >= (ARG ? 64 : 16) && nout <= 8LL * kNumSMs * 8) reduce_finalize_warp<ARG><<<grid_for(nout, 8), 256, 0, st>>>(pv, pi, out, nout, p.splits, dto);
   else if (p.splits > 1) reduce_finalize<ARG><<<grid_for(nout, 256), 256, 0, st>>>(pv, pi, out, nout, p.splits, dto);
   return check_launch(p.splits > 1 ? 2 : 1);
 }

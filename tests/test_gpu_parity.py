@@ -354,6 +354,19 @@ def test_column_sums_in_every_word_width(backend, dtype, outer, dim, inner):
         assert got.shape == exact.shape and bool(((got - exact).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("dim,inner", [(8192, 11007), (8192, 2051), (3000, 4099)])
+def test_column_sums_are_as_exact_as_short_chains_of_additions(backend, dim, inner):
+    """An fp32 sum of n terms of size 1 in chains of c, whose n / c results are added as a tree, is off by (root mean square)
+    at most 2^-24 / sqrt 3 of the sum per rounding, whose partial sums grow as their root: sqrt(c / 2 + log2(n / c) + 1) of them, taken
+    together. Widths off the 16-byte grid, with chains of an 128th of the rows."""
+    impl = backend[torch.ops.aten.sum.dim_IntList]
+    x = torch.randn(dim, inner, device=DEV, generator=torch.Generator(device=DEV).manual_seed(dim))
+    exact = x.double().sum(0)
+    chain = dim / 128
+    error = float((impl(x, [0]).double() - exact).norm() / exact.norm())
+    assert error < 2.0**-24 / 3**0.5 * (chain / 2 + math.log2(dim / chain) + 1) ** 0.5, error
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 3])
 def test_gather_and_index_select_from_one_element_per_thread_to_four(backend, dtype, n):
