@@ -1112,13 +1112,17 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
   // a0: the slice's first element on the grid
   const int64_t to_grid = static_cast<int64_t>((16u - (reinterpret_cast<uintptr_t>(xr + c0) & 15u)) & 15u) / static_cast<int64_t>(sizeof(T));
   const int64_t a0 = c0 + to_grid < c1 ? c0 + to_grid : c1;
-  if (c0 + t < a0) {  // (fewer elements than a warp has lanes)
-    const float fv = to_f32(xr[c0 + t]);
-    if (ARG) arg_take(a, fv, c0 + t);
-    else s += fv;
-  }
   const T* xa = xr + a0;
   const int nv = static_cast<int>((c1 - a0) / VE);
+  // the at most 2 (VE - 1) elements off the vectors, one to a thread: a sum asks for them before the first
+  // vector, argmax, which is short of registers, before and behind the vectors
+  float sv = 0.f;
+  if constexpr (ARG) {
+    if (c0 + t < a0) arg_take(a, to_f32(xr[c0 + t]), c0 + t);
+  } else {
+    const int64_t c = c0 + t < a0 ? c0 + t : a0 + static_cast<int64_t>(nv) * VE + t - (a0 - c0);
+    if (c < c1) sv = to_f32(xr[c]);
+  }
   // argmax keeps the largest element of whole vectors and the first vector that holds it (a
   // NaN beats everything, the first one stays); which element it was is asked once per row
   float best = -CUDART_INF_F;
@@ -1142,15 +1146,25 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
 #pragma unroll
     for (int u = 0; u < 4; ++u) take(v[u], j + u * tpr);
   }
-  for (; j < nv; j += tpr) take(ld_stream(xa + static_cast<int64_t>(j) * VE), j);
+  if constexpr (ARG) {
+    for (; j < nv; j += tpr) take(ld_stream(xa + static_cast<int64_t>(j) * VE), j);
+  } else if (j < nv) {  // up to three more
+    uint4 v[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (j + u * tpr < nv) v[u] = ld_stream(xa + static_cast<int64_t>(j + u * tpr) * VE);
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (j + u * tpr < nv) take(v[u], j + u * tpr);
+  }
   if (ARG && t < nv) {
     if (best_j < 0) best_j = t;  // nothing but -inf so far: the first element is the answer
     arg_take(a, best, a0 + static_cast<int64_t>(best_j) * VE);  // the vector's place stands for its element's until the row is decided
   }
-  if (const int64_t c = a0 + static_cast<int64_t>(nv) * VE + t; c < c1) {
-    const float fv = to_f32(xr[c]);
-    if (ARG) arg_take(a, fv, c);
-    else s += fv;
+  if constexpr (ARG) {
+    if (const int64_t c = a0 + static_cast<int64_t>(nv) * VE + t; c < c1) arg_take(a, to_f32(xr[c]), c);
+  } else {
+    s += sv;
   }
   const bool split = gridDim.y > 1;
   const int64_t slot = static_cast<int64_t>(blockIdx.y) * rows + row;
@@ -1185,6 +1199,29 @@ __global__ void __launch_bounds__(256) reduce_rows(const T* __restrict__ x, void
       if (split) { part_v[slot] = a.v; part_i[slot] = a.i; }
       else static_cast<int64_t*>(out)[row] = a.i;
     }
+  }
+}
+
+// The same for short rows, a warp to each and single elements throughout (see rows_one_by_one).
+template <typename T, bool ARG>
+__global__ void __launch_bounds__(256) reduce_rows_single(const T* __restrict__ x, void* __restrict__ out, int64_t rows, int64_t cols, int dto) {
+  const int lane = threadIdx.x & 31;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const T* xr = x + row * cols;
+  float s = 0.f;
+  ArgPair a{CUDART_NAN_F, -1};  // NaN start: the first element fails `v <= NaN` and is taken through a.i < 0
+  for (int64_t c = lane; c < cols; c += 32) {
+    const float v = to_f32(xr[c]);
+    if (ARG) arg_take_ascending(a, v, c);
+    else s += v;
+  }
+  if (ARG) {
+    a = arg_warp_reduce(a);
+    if (lane == 0) static_cast<int64_t*>(out)[row] = a.i;
+  } else {
+    s = warp_reduce(s, SumF{});
+    if (lane == 0) store_from_f32(out, row, dto, s);
   }
 }
 
@@ -1718,6 +1755,18 @@ static void launch_sum_cols(const T* x, void* out, float* pv, int64_t outer, int
   }
 }
 
+// Whether rows of a warp each go one element at a time. Off the 16-byte grid a vector costs the look at both ends of
+// the row, and argmax a second look at the vector that won. Measured with vectors / one by one, us: argmax f32
+// 65536 x 333 41 / 29, 16384 x 2047 32.8 / 29.2 (longer rows are a CTA's); bf16 65536 x 777 51 / 40, 32768 x 1001 26.6 / 29.4; on the grid f32
+// 65536 x 128 26 / 22, 65536 x 512 31 / 35; sum bf16 100000 x 131 22 / 18, 65536 x 333 16 / 18; f32 100000 x 33 18.4 / 16.9,
+// 100000 x 65 19 / 21.
+template <bool ARG>
+static bool rows_one_by_one(const void* x, int64_t dim, int esize) {
+  const bool on_grid = aligned16(x) && (dim * esize) % 16 == 0;
+  if (ARG) return on_grid ? dim * esize <= 512 : dim <= (esize == 4 ? 2048 : 896);
+  return !on_grid && dim <= (esize == 4 ? 48 : 160);
+}
+
 template <typename T, bool ARG>
 static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim, int64_t inner, int dto, void* scratch, int64_t scratch_bytes, cudaStream_t st) {
   ReducePlan p = plan_reduce(outer, dim, inner);
@@ -1732,11 +1781,14 @@ static int launch_reduce_T(const void* x, void* out, int64_t outer, int64_t dim,
   }
   const T* px = static_cast<const T*>(x);
   if (inner == 1) {
-    const bool warp = p.splits == 1 && dim * static_cast<int64_t>(sizeof(T)) <= 8192;
+    // a warp to a row; a few longer rows are sooner done by a CTA each (sum f32 300 x 2047: 6.3 us by warps)
+    const int64_t row_bytes = dim * static_cast<int64_t>(sizeof(T));
+    const bool warp = p.splits == 1 && row_bytes <= 8192 && (ARG || row_bytes <= 2048 || outer >= 4 * kNumSMs);
     if (!warp && outer > 0x7fffffffLL) return B200_EINVAL;
     if (warp) {
       dim3 g(grid_for(outer, 8), 1);
-      reduce_rows<T, true, ARG><<<g, 256, 0, st>>>(px, out, pv, pi, outer, dim, p.chunk, dto);
+      if (rows_one_by_one<ARG>(x, dim, sizeof(T))) reduce_rows_single<T, ARG><<<g, 256, 0, st>>>(px, out, outer, dim, dto);
+      else reduce_rows<T, true, ARG><<<g, 256, 0, st>>>(px, out, pv, pi, outer, dim, p.chunk, dto);
     } else {
       dim3 g(static_cast<unsigned>(outer), p.splits);
       reduce_rows<T, false, ARG><<<g, 256, 0, st>>>(px, out, pv, pi, outer, dim, p.chunk, dto);

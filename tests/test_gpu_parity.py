@@ -368,6 +368,24 @@ def test_column_sums_are_as_exact_as_short_chains_of_additions(backend, dim, inn
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(65, 48), (65, 49), (300, 128), (300, 132), (65, 160), (65, 161), (33, 256), (33, 264), (33, 896), (33, 897), (9, 2047), (600, 2047), (9, 2049), (300, 1030)])
+def test_row_reductions_at_the_edges_between_their_kernels(backend, dtype, rows, cols):
+    """Row lengths on both sides of every line between one element at a time and vectors, a warp and a CTA to a row, on and off the
+    16-byte grid: ties, NaN, -inf, exact sums of small integers."""
+    g = torch.Generator().manual_seed(cols)
+    argmax, total = backend[torch.ops.aten.argmax.default], backend[torch.ops.aten.sum.dim_IntList]
+    for shift in (0, 1):
+        x = torch.randint(-4, 5, (rows * cols + 1,), generator=g).to(dtype).to(DEV)[shift : shift + rows * cols].view(rows, cols)
+        assert torch.equal(total(x, [-1]), x.double().sum(-1).to(dtype))
+        x[1, cols - 1] = x[2, 0] = 9.0
+        x[3, 1] = x[3, cols - 2] = x[4, cols // 2] = float("nan")
+        x[5] = float("-inf")
+        x[6] = float("-inf")
+        x[6, cols - 1] = -3.0
+        assert torch.equal(torch.argmax(x.cpu().float(), -1), argmax(x, -1).cpu())  # (the CPU's argmax takes the first of equal ones)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 3])
 def test_gather_and_index_select_from_one_element_per_thread_to_four(backend, dtype, n):
     """Results just below and above the size from which a thread takes four, along rows and off them, an index out of range in the last one."""
