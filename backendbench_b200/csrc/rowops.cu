@@ -173,12 +173,13 @@ softmax_bwd_resident(const T* __restrict__ g, const T* __restrict__ y, void* __r
 
 // Rows too long for the registers of a CTA, or off the 16-byte grid (a vocabulary of 50,257):
 // one CTA per row, single elements up to the row's first 16-byte boundary and behind its
-// last one, 16-byte accesses in between, four of each operand in flight per thread. The first
+// last one, 16-byte accesses in between, four of each operand in flight per thread (ONE_TRIP: that is
+// all of the row). The first
 // pass needs grad alone for log_softmax (and both operands for softmax); the second reads it
 // again from L2. All three rows have to lie at the same offset from the grid. Bound by HBM:
 // log_softmax, bf16 4096 x 50257, 205 us (6.0 TB/s; a warp per row with element-wise accesses,
 // the kernel below, 468 us).
-template <typename T, bool IS_LOG>
+template <typename T, bool IS_LOG, bool ONE_TRIP>
 __global__ void __launch_bounds__(512) softmax_bwd_stream(const T* __restrict__ g, const T* __restrict__ y, T* __restrict__ out, int cols) {
   constexpr int VE = Vec<T>::N;
   __shared__ float red[64];
@@ -195,31 +196,47 @@ __global__ void __launch_bounds__(512) softmax_bwd_stream(const T* __restrict__ 
   const T* yv = yr + lead;
   float s = 0.f;
   if (single >= 0) s = IS_LOG ? to_f32(gr[single]) : to_f32(gr[single]) * to_f32(yr[single]);
-  auto take = [&](const uint4& rg, const uint4& ry) {
+  auto take = [&](const uint4& rg, const uint4& ry) {  // (one trip: a vector's own sum, then the thread's, a shorter chain of additions)
+    float own = ONE_TRIP ? 0.f : s;
     if (IS_LOG) {
-      vec_accumulate<T>(s, rg);
+      vec_accumulate<T>(own, rg);
     } else {
       float fg[VE], fy[VE];
       widen<T>(rg, fg);
       widen<T>(ry, fy);
 #pragma unroll
-      for (int e = 0; e < VE; ++e) s += fg[e] * fy[e];
+      for (int e = 0; e < VE; ++e) own += fg[e] * fy[e];
     }
+    s = ONE_TRIP ? s + own : own;
   };
   int j = t;
-  for (; j + 3 * nth < nv; j += 4 * nth) {
+  if constexpr (ONE_TRIP) {
     uint4 rg[4], ry[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      rg[u] = ld_keep(gv + (j + u * nth) * VE);
-      ry[u] = IS_LOG ? rg[u] : ld_keep(yv + (j + u * nth) * VE);
+      if (j + u * nth < nv) {
+        rg[u] = ld_keep(gv + (j + u * nth) * VE);
+        ry[u] = IS_LOG ? rg[u] : ld_keep(yv + (j + u * nth) * VE);
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) take(rg[u], ry[u]);
-  }
-  for (; j < nv; j += nth) {
-    const uint4 rg = ld_keep(gv + j * VE);
-    take(rg, IS_LOG ? rg : ld_keep(yv + j * VE));
+    for (int u = 0; u < 4; ++u)
+      if (j + u * nth < nv) take(rg[u], ry[u]);
+  } else {
+    for (; j + 3 * nth < nv; j += 4 * nth) {
+      uint4 rg[4], ry[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        rg[u] = ld_keep(gv + (j + u * nth) * VE);
+        ry[u] = IS_LOG ? rg[u] : ld_keep(yv + (j + u * nth) * VE);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) take(rg[u], ry[u]);
+    }
+    for (; j < nv; j += nth) {
+      const uint4 rg = ld_keep(gv + j * VE);
+      take(rg, IS_LOG ? rg : ld_keep(yv + j * VE));
+    }
   }
   s = block_reduce_once(s, SumF{}, 0.f, red, 0);
   auto gradient = [&](float fg, float fy) { return IS_LOG ? fg - ex2_approx(fy * kLog2e) * s : (fg - s) * fy; };
@@ -232,17 +249,32 @@ __global__ void __launch_bounds__(512) softmax_bwd_stream(const T* __restrict__ 
     for (int e = 0; e < VE; ++e) fg[e] = gradient(fg[e], fy[e]);
     st_stream(orow + lead + jj * VE, narrow<T>(fg));
   };
-  for (j = t; j + 3 * nth < nv; j += 4 * nth) {
+  j = t;
+  if constexpr (ONE_TRIP) {
     uint4 rg[4], ry[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      ry[u] = ld_stream(yv + (j + u * nth) * VE);
-      rg[u] = ld_stream(gv + (j + u * nth) * VE);
+      if (j + u * nth < nv) {
+        ry[u] = ld_stream(yv + (j + u * nth) * VE);
+        rg[u] = ld_stream(gv + (j + u * nth) * VE);
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) give(j + u * nth, rg[u], ry[u]);
+    for (int u = 0; u < 4; ++u)
+      if (j + u * nth < nv) give(j + u * nth, rg[u], ry[u]);
+  } else {
+    for (; j + 3 * nth < nv; j += 4 * nth) {
+      uint4 rg[4], ry[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        ry[u] = ld_stream(yv + (j + u * nth) * VE);
+        rg[u] = ld_stream(gv + (j + u * nth) * VE);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) give(j + u * nth, rg[u], ry[u]);
+    }
+    for (; j < nv; j += nth) give(j, ld_stream(gv + j * VE), ld_stream(yv + j * VE));
   }
-  for (; j < nv; j += nth) give(j, ld_stream(gv + j * VE), ld_stream(yv + j * VE));
 }
 
 // Any geometry and alignment: one warp per (outer, inner) line, elements `inner` apart,
@@ -326,6 +358,10 @@ __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float
   const float b = m2 == -CUDART_INF_F ? 0.f : s2 * ex2_approx((m2 - mn) * kLog2e);
   m = mn;
   s = a + b;
+}
+template <typename T> __device__ __forceinline__ uint4 vec_minus_inf() {
+  const uint32_t w = sizeof(T) == 4 ? 0xff800000u : std::is_same<T, __nv_bfloat16>::value ? 0xff80ff80u : 0xfc00fc00u;
+  return make_uint4(w, w, w, w);
 }
 template <typename T, int NV> __device__ __forceinline__ float vecs_max_nan(const uint4* v) {
   if constexpr (sizeof(T) == 4) {
@@ -411,7 +447,7 @@ __device__ __forceinline__ void online_write(uint4 v, T* __restrict__ orow, int 
       if (c0 + e >= 0 && c0 + e < cols) orow[c0 + e] = from_f32<T>(f[e]);
   }
 }
-template <typename T, bool IS_LOG>
+template <typename T, bool IS_LOG, bool ONE_TRIP>
 __global__ void __launch_bounds__(512, 3) softmax_stream_vec(const T* __restrict__ x, T* __restrict__ out, int cols) {
   constexpr int VE = Vec<T>::N;
   __shared__ float red_m[32], red_s[32];
@@ -426,15 +462,25 @@ __global__ void __launch_bounds__(512, 3) softmax_stream_vec(const T* __restrict
   if (tid == 0) online_take_edge<T>(ld_keep(xa), 0, head, cols, m, s);
   if (tid == 32 && nvec > 1) online_take_edge<T>(ld_keep(xa + static_cast<int64_t>(last) * VE), last, head, cols, m, s);
   int j = 1 + tid;
-  for (; j + 3 * nth < last; j += 4 * nth) {
-    uint4 v[4];
+  if constexpr (ONE_TRIP || sizeof(T) == 4) {  // what lies behind the last interior vector counts as -inf
+    for (; j < last; j += 4 * nth) {
+      uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = ld_keep(xa + static_cast<int64_t>(j + u * nth) * VE);
-    online_take<T, 4>(v, m, s);
-  }
-  for (; j < last; j += nth) {
-    const uint4 v = ld_keep(xa + static_cast<int64_t>(j) * VE);
-    online_take<T, 1>(&v, m, s);
+      for (int u = 0; u < 4; ++u) v[u] = j + u * nth < last ? ld_keep(xa + static_cast<int64_t>(j + u * nth) * VE) : vec_minus_inf<T>();
+      online_take<T, 4>(v, m, s);
+      if (ONE_TRIP) break;
+    }
+  } else {
+    for (; j + 3 * nth < last; j += 4 * nth) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = ld_keep(xa + static_cast<int64_t>(j + u * nth) * VE);
+      online_take<T, 4>(v, m, s);
+    }
+    for (; j < last; j += nth) {
+      const uint4 v = ld_keep(xa + static_cast<int64_t>(j) * VE);
+      online_take<T, 1>(&v, m, s);
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) online_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
@@ -450,14 +496,28 @@ __global__ void __launch_bounds__(512, 3) softmax_stream_vec(const T* __restrict
   T* orow = out + row * cols;
   if (tid == 0) online_write<T, IS_LOG, true>(ld_stream(xa), orow, 0, head, cols, m, k, fused);
   if (tid == 32 && nvec > 1) online_write<T, IS_LOG, true>(ld_stream(xa + static_cast<int64_t>(last) * VE), orow, last, head, cols, m, k, fused);
-  for (j = 1 + tid; j + 3 * nth < last; j += 4 * nth) {
-    uint4 v[4];
+  j = 1 + tid;
+  if constexpr (ONE_TRIP || sizeof(T) == 4) {
+    for (; j < last; j += 4 * nth) {
+      uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = ld_stream(xa + static_cast<int64_t>(j + u * nth) * VE);
+      for (int u = 0; u < 4; ++u)
+        if (j + u * nth < last) v[u] = ld_stream(xa + static_cast<int64_t>(j + u * nth) * VE);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) online_write<T, IS_LOG, false>(v[u], orow, j + u * nth, head, cols, m, k, fused);
+      for (int u = 0; u < 4; ++u)
+        if (j + u * nth < last) online_write<T, IS_LOG, false>(v[u], orow, j + u * nth, head, cols, m, k, fused);
+      if (ONE_TRIP) break;
+    }
+  } else {
+    for (; j + 3 * nth < last; j += 4 * nth) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = ld_stream(xa + static_cast<int64_t>(j + u * nth) * VE);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) online_write<T, IS_LOG, false>(v[u], orow, j + u * nth, head, cols, m, k, fused);
+    }
+    for (; j < last; j += nth) online_write<T, IS_LOG, false>(ld_stream(xa + static_cast<int64_t>(j) * VE), orow, j, head, cols, m, k, fused);
   }
-  for (; j < last; j += nth) online_write<T, IS_LOG, false>(ld_stream(xa + static_cast<int64_t>(j) * VE), orow, j, head, cols, m, k, fused);
 }
 
 // ------------------------------------------------------------------ ragged rows, one warp each
@@ -1862,6 +1922,14 @@ static void softmax_launch(unsigned grid, int threads, cudaStream_t st, int is_l
   if (is_log) softmax_resident<T, VPT, WARP, true><<<grid, threads, 0, st>>>(x, out, rows, cols, out_f32);
   else softmax_resident<T, VPT, WARP, false><<<grid, threads, 0, st>>>(x, out, rows, cols, out_f32);
 }
+// Threads of a CTA that streams a row of `nvec` vectors: four vectors to each, which is what a thread has in flight, so that rows
+// of up to 2048 vectors are one trip (ONE_TRIP; fp32 30000 x 1030: 46 us, with a vector to each of four times as many
+// threads 138; 8192 x 4097 49 / 90). Rows that do not give every SM one are done sooner by more threads.
+static int stream_threads(int64_t rows, int64_t nvec, int least) {
+  const int64_t th = (nvec / (rows >= kNumSMs ? 4 : 1) + 31) / 32 * 32;
+  return static_cast<int>(th < least ? least : (th > 512 ? 512 : th));
+}
+
 template <typename T>
 static int softmax_T(const void* x, void* out, int64_t outer, int64_t dim, int64_t inner, int dto, int is_log, cudaStream_t st) {
   constexpr int VE = Vec<T>::N;
@@ -1888,11 +1956,15 @@ static int softmax_T(const void* x, void* out, int64_t outer, int64_t dim, int64
     } else {
       if (outer > 0x7fffffffLL) return B200_EINVAL;
       if (same_phase && dim < (1LL << 30)) {  // same type out, and rows of x and out at the same offset inside their 16-byte blocks
-        int64_t th = (dim / VE + 31) / 32 * 32;
-        th = th < 128 ? 128 : (th > 512 ? 512 : th);
-        auto go = [&](auto kernel) { kernel<<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(px, static_cast<T*>(out), static_cast<int>(dim)); };
-        if (is_log) go(softmax_stream_vec<T, true>);
-        else go(softmax_stream_vec<T, false>);
+        const int th = stream_threads(outer, dim / VE, 64);  // (the second warp takes the last block)
+        auto go = [&](auto kernel) { kernel<<<static_cast<unsigned>(outer), th, 0, st>>>(px, static_cast<T*>(out), static_cast<int>(dim)); };
+        if (dim / VE <= 4 * th) {
+          if (is_log) go(softmax_stream_vec<T, true, true>);
+          else go(softmax_stream_vec<T, false, true>);
+        } else {
+          if (is_log) go(softmax_stream_vec<T, true, false>);
+          else go(softmax_stream_vec<T, false, false>);
+        }
       } else {
         softmax_stream<T><<<static_cast<unsigned>(outer), 256, 0, st>>>(px, out, dim, dto, is_log);
       }
@@ -1934,10 +2006,15 @@ static int softmax_bwd_T(const void* g, const void* y, void* out, int64_t outer,
   const bool same_phase = (((reinterpret_cast<uintptr_t>(g) ^ reinterpret_cast<uintptr_t>(y)) | (reinterpret_cast<uintptr_t>(g) ^ reinterpret_cast<uintptr_t>(out))) & 15u) == 0;
   // shorter rows are a warp's work (the kernel below); a CTA for each would idle most of its threads
   if (inner == 1 && dto == dti && same_phase && dim > kRaggedMaxCols && dim < (1LL << 30) && outer <= 0x7fffffffLL) {
-    int64_t th = (dim / VE + 31) / 32 * 32;
-    th = th < 128 ? 128 : (th > 512 ? 512 : th);
-    if (is_log) softmax_bwd_stream<T, true><<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(pg, py, static_cast<T*>(out), static_cast<int>(dim));
-    else softmax_bwd_stream<T, false><<<static_cast<unsigned>(outer), static_cast<unsigned>(th), 0, st>>>(pg, py, static_cast<T*>(out), static_cast<int>(dim));
+    const int th = stream_threads(outer, dim / VE, 32);
+    auto go = [&](auto kernel) { kernel<<<static_cast<unsigned>(outer), th, 0, st>>>(pg, py, static_cast<T*>(out), static_cast<int>(dim)); };
+    if (dim / VE <= 4 * th) {
+      if (is_log) go(softmax_bwd_stream<T, true, true>);
+      else go(softmax_bwd_stream<T, false, true>);
+    } else {
+      if (is_log) go(softmax_bwd_stream<T, true, false>);
+      else go(softmax_bwd_stream<T, false, false>);
+    }
     return check_launch();
   }
   // (fewer columns: 32 of them to a CTA leave too few CTAs -- fp32 2000 x 333 took 23 us so, 15 us with

@@ -256,6 +256,36 @@ def test_embedding_backward_of_short_tables_under_many_tokens(backend, V, n, D):
         assert bits_equal(oracle.embedding_backward(grad, idx, V, -1, False), got.cpu())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_softmax_backward_of_streamed_rows_and_columns_with_infinities_and_nan(backend, dtype):
+    """Rows off the 16-byte grid from one trip of a CTA to many, few and many of them, and columns by tiles of every size: a NaN or an infinity in
+    the gradient spoils its own row (column) and no other, as in aten."""
+    g = torch.Generator(device=DEV).manual_seed(8)
+    atol, rtol = _tol(dtype)
+    one_trip = 2048 * (16 // dtype.itemsize)
+    for shape, dim in [((160, 1025), -1), ((9, 1025), -1), ((150, one_trip + 1), -1), ((150, one_trip + 17), -1), ((5, 50257), -1), ((3, 2000), 0), ((8, 1030), 0), ((40, 1025), 0), ((300, 1100), 0), ((20, 70, 64), 1), ((130, 20000), 0)]:
+        x = torch.randn(shape, device=DEV, generator=g)
+        grad = torch.randn(shape, device=DEV, generator=g).to(dtype)
+        for spec, fwd in ((SOFT, torch.softmax), (LOGSOFT, torch.log_softmax)):
+            y = fwd(x, dim).to(dtype)
+            got = backend[get_operator(spec)](grad, y, dim, dtype)
+            ok, ea, er = compare(get_operator(spec)(grad, y, dim, dtype), got, atol, rtol)
+            assert ok, (spec, shape, dim, ea, er)
+            rows_got, rows_grad = got.movedim(dim, -1).reshape(-1, shape[dim]), grad.clone()
+            lines = rows_grad.movedim(dim, -1)
+            lines = lines.reshape(-1, shape[dim])  # (a copy where dim is not the last)
+            bad = {0: float("nan"), 2: float("inf"), lines.shape[0] - 1: float("-inf")}
+            for r, v in bad.items():
+                lines[r, (0, shape[dim] // 2, shape[dim] - 1)[r % 3]] = v
+            spoiled = lines.reshape(*[n for i, n in enumerate(shape) if i != dim % len(shape)], shape[dim]).movedim(-1, dim).contiguous()
+            again = backend[get_operator(spec)](spoiled, y, dim, dtype).movedim(dim, -1).reshape(-1, shape[dim])
+            clean = torch.ones(lines.shape[0], dtype=torch.bool, device=DEV)
+            for r in bad:
+                clean[r] = False
+                assert not bool(torch.isfinite(again[r].float()).all()), (spec, shape, r)
+            assert torch.equal(again[clean], rows_got[clean]), (spec, shape)
+
+
 def test_full_size_embedding_backward(backend):
     c = named_case("embedding_backward_bf16_128256x4096_16384")
     op = get_operator(c.op)

@@ -742,7 +742,7 @@ def test_long_and_misaligned_rows_take_the_vector_streaming_softmax(backend, dty
     rows that start off the 16-byte grid: two passes of 16-byte accesses over the aligned
     span around each row. Special rows: a NaN, all -inf, one +inf, -inf everywhere but one."""
     g = torch.Generator().manual_seed(34)
-    for rows, cols in ((9, 1025), (7, 4099), (6, 33000), (5, 50257), (5, 131072), (6, 70001)):
+    for rows, cols in ((9, 1025), (1200, 1025), (7, 4099), (150, 2049), (6, 33000), (5, 50257), (5, 131072), (6, 70001), (149, 8191 if dtype == torch.float32 else 16385), (149, 8209 if dtype == torch.float32 else 16411)):
         x = (torch.randn(rows + 1, cols, generator=g) * 3).to(dtype)
         x[1, cols // 3] = float("nan")
         x[2, :] = float("-inf")
