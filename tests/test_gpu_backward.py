@@ -286,6 +286,17 @@ def test_softmax_backward_of_streamed_rows_and_columns_with_infinities_and_nan(b
             assert torch.equal(again[clean], rows_got[clean]), (spec, shape)
 
 
+def test_log_softmax_backward_of_columns_is_as_exact_as_its_chains(backend):
+    """With y = 0 the result is grad minus the column's sum. In chains of c fp32 additions, of which n / c are added as a tree, that sum is off
+    (root mean square) by at most 2^-24 / sqrt 3 sqrt(c / 2 + log2(n / c) + 1) of its size, and the result is rounded once more; c = n / 32."""
+    n, cols = 4096, 9600
+    grad = torch.randn(n, cols, device=DEV, generator=torch.Generator(device=DEV).manual_seed(2))
+    got = backend[get_operator(LOGSOFT)](grad, torch.zeros_like(grad), 0, torch.float32)[:64].double()
+    exact = grad[:64].double() - grad.double().sum(0)
+    error = float((got - exact).norm() / exact.norm())
+    assert error < 2.0**-24 / 3**0.5 * (n / 32 / 2 + 5 + 1 + 1) ** 0.5, error
+
+
 def test_full_size_embedding_backward(backend):
     c = named_case("embedding_backward_bf16_128256x4096_16384")
     op = get_operator(c.op)
