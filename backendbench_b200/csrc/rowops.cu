@@ -997,7 +997,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
       s1 = block_reduce_once(s1, SumF{}, 0.f, &red[0][0].x, 0);
       s2 = block_reduce_once(s2, SumF{}, 0.f, &red[0][0].x, 1);
     }
-    const float c1 = s1 * inv_cols, c2 = s2 * inv_cols, k1 = -rs * c1, k2 = -rs * c2;
+    const float c1 = s1 * inv_cols, c2 = s2 * inv_cols;
     if (dx) {
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
@@ -1005,7 +1005,7 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         if (j < nvec) {
           float o[VE];
 #pragma unroll
-          for (int e = 0; e < VE; ++e) o[e] = kAhead ? fmaf(g[u][e], rs, fmaf(h[u][e], k2, k1)) : rs * (g[u][e] - c1 - h[u][e] * c2);
+          for (int e = 0; e < VE; ++e) o[e] = rs * (g[u][e] - c1 - h[u][e] * c2);
           st_stream(dx + row * cols + j * VE, narrow<T>(o));
         }
       }

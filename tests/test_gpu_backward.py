@@ -297,6 +297,23 @@ def test_log_softmax_backward_of_columns_is_as_exact_as_its_chains(backend):
     assert error < 2.0**-24 / 3**0.5 * (n / 32 / 2 + 5 + 1 + 1) ** 0.5, error
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [256, 512, 4096])
+def test_layer_norm_backward_of_a_constant_gradient(backend, dtype, cols):
+    """One value g everywhere under weights of one: what is left of rstd (g - mean g - xhat mean(g xhat)) is next to nothing. The sums of g are exact,
+    so the error is that of an fp32 mean of g xhat, about 2^-27 g rstd; rounding rstd mean g, 2^-24 / sqrt 12 of rstd g times the place of
+    rstd g in its binade, would show above 2^-26 (both as root mean squares)."""
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    x = (0.6 * torch.randn(500, cols, device=DEV, generator=g)).to(dtype)
+    mean, var = x.double().mean(1, keepdim=True), x.double().var(1, unbiased=False, keepdim=True)
+    mean, rstd = mean.float(), (var + 1e-5).rsqrt().float()
+    one = torch.ones(cols, device=DEV, dtype=dtype)
+    dx = backend[get_operator("native_layer_norm_backward.default")](torch.full_like(x, 0.703125), x, [cols], mean, rstd, one, one, [True, True, True])[0].double()
+    xhat = (x.double() - mean.double()) * rstd.double()
+    exact = rstd.double() * 0.703125 * (-xhat * xhat.mean(1, keepdim=True))
+    assert float(((dx - exact) / (0.703125 * rstd.double())).pow(2).mean().sqrt()) < 2.0**-26
+
+
 def test_full_size_embedding_backward(backend):
     c = named_case("embedding_backward_bf16_128256x4096_16384")
     op = get_operator(c.op)
