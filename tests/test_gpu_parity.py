@@ -419,6 +419,38 @@ def test_broadcast_rows_from_one_element_per_thread_to_four(backend, dtype, rows
         assert bits_equal((a.float() * b.float()).to(dtype), mul(b, a))
 
 
+def test_plain_operands_and_those_that_only_look_it(backend):
+    """add / mul / where take a short way for two contiguous operands of one shape and type. Next to it: a base off the 16-byte grid, a
+    0-dim operand (no promotion by it), one operand not contiguous, an empty one, alpha with an in-place target, operands that overlap."""
+    from backendbench_b200 import variants
+
+    add, mul, where = (backend[o] for o in (torch.ops.aten.add.Tensor, torch.ops.aten.mul.Tensor, torch.ops.aten.where.self))
+    g = torch.Generator(device=DEV).manual_seed(3)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    base = r(4097)
+    half = r(64, 64).to(torch.bfloat16)
+    pairs = [(base[1:].view(64, 64), base[:-1].view(64, 64)), (r(64, 64), torch.tensor(2.5, device=DEV)), (half, torch.tensor(2.5, device=DEV)), (torch.tensor(1.5, device=DEV), torch.tensor(2.5, device=DEV)),
+             (r(64, 64).t(), r(64, 64)), (r(64, 64), r(64, 128)[:, ::2]), (r(0, 5), r(0, 5)), (half, r(64, 64)), (r(64, 64), r(64))]
+    cond = r(64, 64) < 0
+    for a, b in pairs:
+        for got, want in ((add(a, b, alpha=2), torch.add(a, b, alpha=2)), (mul(a, b), a * b)):
+            assert got.dtype == want.dtype and got.shape == want.shape and got.is_contiguous()
+            torch.testing.assert_close(got, want, rtol=1e-2 if got.dtype == torch.bfloat16 else 1e-6, atol=1e-6)
+        if a.shape == (64, 64):
+            for c in (cond, cond.t(), cond[:1]):
+                got, want = where(c, a, b), torch.where(c, a, b)
+                assert got.dtype == want.dtype and torch.equal(got, want)
+    t = r(64, 64)
+    want = t + 3 * half.float()
+    assert variants.add__Tensor(t, half, alpha=3) is t and torch.allclose(t, want)
+    want = t + 0.5 * t.t()
+    assert variants.add__Tensor(t, t.t(), alpha=0.5) is t and torch.allclose(t, want)
+    flat = r(4097)
+    a, b = flat[:-1], flat[1:]
+    want = a.clone() + 0.5 * b
+    assert variants.add__Tensor(a, b, alpha=0.5) is a and torch.equal(a, want)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_gather_along_the_last_dim(backend, dtype):
     """2-D gather along the last dim: 16 bytes of adjacent outputs per thread; fewer index rows
