@@ -966,7 +966,7 @@ static int launch_bucket(const void* self, const void* index, const void* src, v
 constexpr int kChainUnroll = 4;
 enum { kCtlSlots = 0, kCtlListed = 1, kCtlGrouped = 2 };  // words of the control block: slots handed out, long chains or segments, 1 = everything is grouped
 
-// Empties the chains, and the first CTA looks at up to 1024 contributions, one to a thread, spread over all of them. How
+// Empties the chains, while the first CTA looks at up to 1024 contributions, one to a thread, spread over all of them. How
 // many pairs of them share a destination estimates how crowded the destinations are: evenly
 // spread indices give about s^2 / (2 destinations); four times that, and enough pairs for the estimate
 // to mean something, is crowded. Which way is taken changes no result.
@@ -976,10 +976,17 @@ __global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict
                                                    const __grid_constant__ BucketArgs A) {
   __shared__ int key[2 * kSample], cnt[2 * kSample];
   __shared__ int pairs;
-  const int64_t first = static_cast<int64_t>(blockIdx.x) * kSample + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * kSample;
+  if (blockIdx.x != 0) {
+    const int64_t first = static_cast<int64_t>(blockIdx.x - 1) * kSample + threadIdx.x, step = static_cast<int64_t>(gridDim.x - 1) * kSample;
+    for (int64_t i = first; i < listed; i += step) listed_cnt[i] = 0;
+    const int64_t words = (reinterpret_cast<uintptr_t>(head) & 15u) == 0 ? n_self / 4 : 0;
+    for (int64_t i = first; i < words; i += step) reinterpret_cast<int4*>(head)[i] = make_int4(-1, -1, -1, -1);
+    for (int64_t i = 4 * words + first; i < n_self; i += step) head[i] = -1;
+    return;
+  }
   const int s = listed == 0 ? 0 : A.n_idx < kSample ? static_cast<int>(A.n_idx) : kSample;
   int64_t dest = -1;
-  if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < s) {
+  if (static_cast<int>(threadIdx.x) < s) {
     const uint32_t every = static_cast<uint32_t>(A.n_idx / s);  // n_idx is below 2^31
     // not an even spacing: it could keep to a few columns
     const int64_t p = static_cast<int64_t>(threadIdx.x) * every + (threadIdx.x * 2654435761u >> 4) % every;
@@ -987,11 +994,6 @@ __global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict
     int pos;
     if (!bucket_decode(A, p, index, dest, so, pos, nullptr)) dest = -1;
   }
-  for (int64_t i = first; i < listed; i += step) listed_cnt[i] = 0;
-  const int64_t words = (reinterpret_cast<uintptr_t>(head) & 15u) == 0 ? n_self / 4 : 0;
-  for (int64_t i = first; i < words; i += step) reinterpret_cast<int4*>(head)[i] = make_int4(-1, -1, -1, -1);
-  for (int64_t i = 4 * words + first; i < n_self; i += step) head[i] = -1;
-  if (blockIdx.x != 0) return;
   for (int i = threadIdx.x; i < 2 * kSample; i += kSample) { key[i] = -1; cnt[i] = 0; }
   if (threadIdx.x == 0) pairs = 0;
   __syncthreads();
@@ -1193,7 +1195,7 @@ static int launch_chain(const void* self, const void* index, const void* src, vo
   T* po = static_cast<T*>(out);
   const int64_t listed = A.n_idx / (kLightMax + 1);  // no more long chains (or segments) than this
   auto capped = [](int64_t n, int per, int64_t cap) { const int64_t g = (n + per - 1) / per; return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g)); };
-  chain_begin<<<capped(A.n_self, 8 * kSample, 2 * kNumSMs), kSample, 0, st>>>(pi, head, A.n_self, ctl, listed_cnt, listed, A);
+  chain_begin<<<1 + capped(A.n_self, 8 * kSample, 2 * kNumSMs), kSample, 0, st>>>(pi, head, A.n_self, ctl, listed_cnt, listed, A);
   chain_link<T><<<items_grid(A.n_idx, 256 * kChainUnroll), 256, 0, st>>>(pi, ps, head, link, ctl, A, status);
   chain_replay<T><<<grid_for(A.n_self, 256 * kChainUnroll), 256, 0, st>>>(px, po, head, link, A.n_self, ctl, list);
   if (listed == 0) return check_launch(3);
