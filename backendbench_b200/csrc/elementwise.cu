@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(256) ew_tiled(const void* a, const void* b, vo
 // sixteen elements of every operand in flight before it waits for any (with the four of a 32 x 32
 // tile the memory was idle most of the time), and 16-bit elements move in pairs where the
 // operands' rows, the result's rows and all bases allow it (PK = 2). Bound by HBM: add of a
-// transposed fp32 39934 x 1024 and a row vector (327 MB) 125 -> 68 us (4.8 TB/s). S = 32 where the
+// transposed fp32 39934 x 1024 and a row vector (327 MB) 125 -> 57 us (5.7 TB/s). S = 32 where the
 // larger tiles would be few or mostly empty (see use_tiles64).
 // Pitch of a tile's rows in elements: read down a column, 4-byte elements fall into different banks, and
 // so do 16-bit ones taken singly; the pairs of PK = 2 read every second row, lanes l and l + 16 in one bank.

@@ -4,7 +4,7 @@
 // CTAs, and a handful of stages in flight in each: 16 x 4096 x 11008 ran on 43 SMs (44 us,
 // 2.1 TB/s), 16 x 11008 x 4096 in 16 CTAs split over K with a second pass (29 us).
 //
-// Here a CTA owns 8 * NT columns of C and its eight warps share K. A warp streams B from global
+// Here a CTA owns 16 columns of C and its eight warps share K. A warp streams B from global
 // memory straight into mma.sync operands, with no shared memory in between: in
 // mma.m16n8k16 lane (q, c) holds elements 2c, 2c + 1, 2c + 8, 2c + 9 of row q of B (and of rows
 // q, q + 8 of A). The order of the products in a sum over k is free, so the 32 k of
@@ -23,6 +23,7 @@ namespace {
 
 constexpr int kFewRows = 16;
 constexpr int kFewWarps = 8;
+constexpr int kFewFragments = 2;           // of eight columns each: 16 columns to a CTA, enough CTAs for two on every SM from N = 4736 on
 constexpr int kFewSteps = 4;              // 32-k steps in flight per lane
 // Where the kernel is the faster one; bf16 with B out of HBM, us here / the tcgen05 kernel or its ranges of K.
 // The tcgen05 kernel has a CTA to 256 columns: up to 96 of them leave it SMs idle (N 20000, K 4096: 8 rows 33 /
@@ -55,9 +56,9 @@ __device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1
   }
 }
 
-template <typename T, int NT>
+template <typename T>
 __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ bias, T* __restrict__ C, FewRowsArgs p) {
-  constexpr int kCols = 8 * NT, kPitch = kCols + 1;
+  constexpr int NT = kFewFragments, kCols = 8 * NT, kPitch = kCols + 1;
   __shared__ float red[kFewWarps][kFewRows][kPitch];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane >> 2, c = lane & 3;
   const int64_t n0 = static_cast<int64_t>(blockIdx.x) * kCols;
@@ -137,8 +138,7 @@ bool gemm_few_rows_leaves_to_ranges(int64_t N, int64_t K) {
 
 template <typename T>
 static void launch_few_rows(const void* A, const void* B, const void* bias, void* C, const FewRowsArgs& p, cudaStream_t st) {
-  // 16 columns to a CTA: enough CTAs for two on every SM from N = 4736 on
-  gemm_few_rows<T, 2><<<grid_for(p.N, 16), 32 * kFewWarps, 0, st>>>(static_cast<const T*>(A), static_cast<const T*>(B), static_cast<const T*>(bias), static_cast<T*>(C), p);
+  gemm_few_rows<T><<<grid_for(p.N, 8 * kFewFragments), 32 * kFewWarps, 0, st>>>(static_cast<const T*>(A), static_cast<const T*>(B), static_cast<const T*>(bias), static_cast<T*>(C), p);
 }
 
 int gemm_few_rows_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sBn, int64_t sbm, int64_t sbn, double alpha,

@@ -901,10 +901,10 @@ layernorm_persistent(const T* __restrict__ x, const TW* __restrict__ w, const TW
 // carries its share of dw / db in registers across rows and writes one partial per CTA at
 // the end (dy and x are read once for all three results). A small second kernel adds the
 // per-CTA partials in order. fp32 arithmetic throughout. bf16 8192 x 4096: 53.7 -> 51.3 us (3.9 TB/s of
-// two reads and a write) with both sums behind one barrier, the row statistics fetched ahead
-// and three instructions less per element; a ring of four rows in shared memory (`cp.async`)
-// in place of the one row in registers changed nothing (52.4 us): not the bytes in flight but
-// 16 warps' instructions and the one reduction per row are what it waits for.
+// two reads and a write) with both sums behind one barrier and the row statistics fetched ahead; a
+// ring of four rows in shared memory (`cp.async`) in place of the one row in registers changed
+// nothing (52.4 us). Two CTAs of 512 threads run on an SM, 29 of its warps active on average, half of the
+// issue slots busy; the stalls are waits for a row's loads and for the shuffles and shared memory of its sums.
 template <typename T, typename TW, int VPT, bool kAhead>
 __global__ void __launch_bounds__(1024)
 layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW* __restrict__ w, const void* __restrict__ mean, const void* __restrict__ rstd, T* __restrict__ dx,
