@@ -223,7 +223,9 @@ int b200_gather(const void* self, const void* index, void* out, int ndim,
  * results are bit-identical to it. self/out contiguous; index/src strided. bf16/f16
  * tensors accumulate in fp32 and round once (as aten CPU does). Wide matrices run on
  * shared-memory strip / row kernels without scratch; tall, narrow or strided geometries
- * are grouped by destination first and need scratch (counters, segment storage): ask
+ * chain or group the contributions by destination first and need scratch: counters and a
+ * segment of 8 bytes per contribution, and where the scatter dimension is no longer than
+ * self's also chain heads and links (8 n_self + 16.4 n_index bytes in all). Ask
  * b200_scatter_add_scratch_bytes with the same arguments and pass at least that much. */
 int64_t b200_scatter_add_scratch_bytes(const void* self, const void* index, const void* src,
                                        const void* out, int ndim, const int64_t* self_shape,
@@ -296,7 +298,10 @@ int b200_gemm_f32(const void* A, const void* B, const void* bias, void* C, int64
  * by a four-warp mma.sync kernel with cp.async staging instead of the tcgen05 kernel, whose
  * set-up alone takes about 5 us. b200_gemm_prefers_small tells a caller whether b200_gemm
  * will go that way.
- * b200_gemm_small_path(0) switches the path off process-wide (1 on again) and returns the
+ * Products of at most 16 rows against weights along K (64 <= K <= 16384, on the 16-byte grid)
+ * go to another mma.sync kernel that streams the weights once, unless they are so wide or so
+ * deep and narrow that the tcgen05 kernel or its K-split is faster.
+ * b200_gemm_small_path(0) switches both off process-wide (1 on again) and returns the
  * previous setting -- for comparisons and for testing the larger kernels on small shapes. */
 int b200_gemm_prefers_small(const void* A, const void* B, int64_t batch, int64_t M, int64_t N,
                             int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb, int64_t sBk,
