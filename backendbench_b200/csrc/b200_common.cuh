@@ -25,6 +25,27 @@ inline int check_launch(int launches = 1) {
   return B200_OK;
 }
 
+// A kernel that follows one of the same call: its CTAs may start before that one has ended (programmatic
+// dependent launch), which hides the launch, and begin with after_grids_before() or do first what does not depend on it. Every
+// kernel launched so calls after_grids_before(), whatever it then does: the next one relies on it for all that came earlier.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), int64_t grid, int block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+// (device) what the grids before have written is there; the next grid's CTAs may start where there is room
+__device__ __forceinline__ void after_grids_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 inline int dtype_size(int dt) {

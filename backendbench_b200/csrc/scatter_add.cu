@@ -812,7 +812,8 @@ __global__ void __launch_bounds__(256) bucket_fill(const int64_t* __restrict__ i
 // `zero`; nothing is done where `only_if` points to a zero.
 template <typename T>
 __global__ void __launch_bounds__(256) bucket_replay(const T* __restrict__ self, T* __restrict__ out, const int* __restrict__ cnt, int zero, const int* __restrict__ cursor,
-                                                     const int2* __restrict__ seg, int64_t n_self, const int* __restrict__ only_if) {
+                                                     const int2* __restrict__ seg, int64_t n_self, const int* only_if) {
+  after_grids_before();
   if (only_if && *only_if == 0) return;
   for (int64_t d = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; d < n_self; d += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int c = cnt[d] - zero;
@@ -852,13 +853,14 @@ struct HeavyCounters {
 };
 template <typename T>
 __global__ void __launch_bounds__(256) bucket_replay_heavy(const T* __restrict__ self, T* __restrict__ out, HeavyCounters H, const int2* __restrict__ seg, int64_t dim_len,
-                                                           const int* __restrict__ heavy_count, const int* __restrict__ heavy_list) {
+                                                           const int* heavy_count, const int* heavy_list) {
   __shared__ float slot_val[kHeavyWindow];
   __shared__ unsigned char slot_set[kHeavyWindow];
   __shared__ float ordered[kHeavyWindow];
   __shared__ int warp_sums[8];
   __shared__ int window_count;
   __shared__ float acc_s;
+  after_grids_before();
   const int nheavy = *heavy_count;
   const bool by_list = nheavy > 0 && H.listed_cnt && *H.grouped == 0;
   constexpr int kPer = kHeavyWindow / 256;
@@ -972,10 +974,53 @@ enum { kCtlSlots = 0, kCtlListed = 1, kCtlGrouped = 2 };  // words of the contro
 // to mean something, is crowded. Which way is taken changes no result.
 constexpr int kSample = 1024, kSampleSlotBits = 11;
 static_assert((1 << kSampleSlotBits) == 2 * kSample, "the table of samples");
+// Pairs among the samples `key` (one per thread and trip; negative: none) that agree. `table`: 4 * kSample words of shared memory.
+template <int THREADS>
+__device__ __forceinline__ int equal_pairs(const int (&key)[kSample / THREADS], int* table) {
+  __shared__ int pairs;
+  int* cnt = table + 2 * kSample;
+  for (int i = threadIdx.x; i < 2 * kSample; i += THREADS) { table[i] = -1; cnt[i] = 0; }
+  if (threadIdx.x == 0) pairs = 0;
+  __syncthreads();
+  int mine = 0;
+#pragma unroll
+  for (int t = 0; t < kSample / THREADS; ++t) {
+    if (key[t] < 0) continue;
+    uint32_t slot = static_cast<uint32_t>(key[t]) * 2654435761u >> (32 - kSampleSlotBits);
+    for (;;) {  // a free slot is found: there are twice as many as samples
+      const int was = atomicCAS(&table[slot], -1, key[t]);
+      if (was == -1 || was == key[t]) break;
+      slot = (slot + 1) & (2 * kSample - 1);
+    }
+    mine += atomicAdd(&cnt[slot], 1);
+  }
+  if (mine) atomicAdd(&pairs, mine);
+  __syncthreads();
+  const int all = pairs;
+  __syncthreads();
+  return all;
+}
+__device__ __forceinline__ bool crowded(int pairs, int s, double places) { return pairs > 16.0 + 4.0 * (static_cast<double>(s) * s / (2.0 * places)); }
+// This thread's samples: their destinations, -1 where there is none.
+template <int THREADS>
+__device__ __forceinline__ int sample_destinations(const int64_t* __restrict__ index, const BucketArgs& A, int (&dest)[kSample / THREADS]) {
+  const int s = A.n_idx < kSample ? static_cast<int>(A.n_idx) : kSample;
+  const uint32_t every = static_cast<uint32_t>(A.n_idx / s);  // n_idx is below 2^31
+#pragma unroll
+  for (int t = 0; t < kSample / THREADS; ++t) {
+    const uint32_t i = threadIdx.x + t * THREADS;
+    dest[t] = -1;
+    if (static_cast<int>(i) >= s) continue;
+    // not an even spacing: it could keep to a few columns
+    const int64_t p = static_cast<int64_t>(i) * every + (i * 2654435761u >> 4) % every;
+    int64_t d, so;
+    int pos;
+    if (bucket_decode(A, p, index, d, so, pos, nullptr)) dest[t] = static_cast<int>(d);
+  }
+  return s;
+}
 __global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict__ index, int* __restrict__ head, int64_t n_self, int* __restrict__ ctl, int* __restrict__ listed_cnt, int64_t listed,
                                                    const __grid_constant__ BucketArgs A) {
-  __shared__ int key[2 * kSample], cnt[2 * kSample];
-  __shared__ int pairs;
   if (blockIdx.x != 0) {
     const int64_t first = static_cast<int64_t>(blockIdx.x - 1) * kSample + threadIdx.x, step = static_cast<int64_t>(gridDim.x - 1) * kSample;
     for (int64_t i = first; i < listed; i += step) listed_cnt[i] = 0;
@@ -984,36 +1029,14 @@ __global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict
     for (int64_t i = 4 * words + first; i < n_self; i += step) head[i] = -1;
     return;
   }
-  const int s = listed == 0 ? 0 : A.n_idx < kSample ? static_cast<int>(A.n_idx) : kSample;
-  int64_t dest = -1;
-  if (static_cast<int>(threadIdx.x) < s) {
-    const uint32_t every = static_cast<uint32_t>(A.n_idx / s);  // n_idx is below 2^31
-    // not an even spacing: it could keep to a few columns
-    const int64_t p = static_cast<int64_t>(threadIdx.x) * every + (threadIdx.x * 2654435761u >> 4) % every;
-    int64_t so;
-    int pos;
-    if (!bucket_decode(A, p, index, dest, so, pos, nullptr)) dest = -1;
-  }
-  for (int i = threadIdx.x; i < 2 * kSample; i += kSample) { key[i] = -1; cnt[i] = 0; }
-  if (threadIdx.x == 0) pairs = 0;
-  __syncthreads();
-  int mine = 0;
-  if (dest >= 0) {
-    uint32_t slot = static_cast<uint32_t>(dest) * 2654435761u >> (32 - kSampleSlotBits);
-    for (;;) {  // a free slot is found: there are twice as many as samples
-      const int was = atomicCAS(&key[slot], -1, static_cast<int>(dest));
-      if (was == -1 || was == static_cast<int>(dest)) break;
-      slot = (slot + 1) & (2 * kSample - 1);
-    }
-    mine = atomicAdd(&cnt[slot], 1);
-  }
-  if (mine) atomicAdd(&pairs, mine);
-  __syncthreads();
+  __shared__ int table[4 * kSample];
+  int dest[1] = {-1};
+  const int s = listed == 0 ? 0 : sample_destinations<kSample>(index, A, dest);
+  const int pairs = equal_pairs<kSample>(dest, table);
   if (threadIdx.x == 0) {
-    const double even = static_cast<double>(s) * s / (2.0 * static_cast<double>(A.n_idx / A.dim_len) * static_cast<double>(A.self_dim_size));
     ctl[kCtlSlots] = 0;
     ctl[kCtlListed] = 0;
-    ctl[kCtlGrouped] = pairs > 16.0 + 4.0 * even ? 1 : 0;
+    ctl[kCtlGrouped] = crowded(pairs, s, static_cast<double>(A.n_idx / A.dim_len) * static_cast<double>(A.self_dim_size)) ? 1 : 0;
   }
 }
 
@@ -1121,7 +1144,8 @@ __global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, 
 // The contributions of listed destinations, or all of them: counted (into the list's counters, or into
 // the heads, which stand at -1), given segments, filled in.
 __global__ void __launch_bounds__(256) chain_count(const int64_t* __restrict__ index, int* __restrict__ head, int* __restrict__ listed_cnt, const __grid_constant__ BucketArgs A,
-                                                   const int* __restrict__ ctl) {
+                                                   const int* ctl) {
+  after_grids_before();
   const bool grouped = ctl[kCtlGrouped] != 0;
   if (!grouped && ctl[kCtlListed] == 0) return;
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < A.n_idx; p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -1139,6 +1163,7 @@ __global__ void __launch_bounds__(256) chain_count(const int64_t* __restrict__ i
 __global__ void __launch_bounds__(256) chain_assign(const int* __restrict__ head, int* __restrict__ cursor, int64_t n_self, const int* __restrict__ listed_cnt, int* __restrict__ listed_cursor,
                                                     int64_t listed, int* __restrict__ ctl, int* __restrict__ heavy_list) {
   constexpr int ITEMS = 16;
+  after_grids_before();
   const bool grouped = ctl[kCtlGrouped] != 0;
   if (!grouped && (ctl[kCtlListed] == 0 || static_cast<int64_t>(blockIdx.x) * 256 * ITEMS >= listed)) return;
   if (grouped) assign_segments_of<ITEMS>(head, -1, cursor, n_self, ctl + kCtlSlots, kLightMax, ctl + kCtlListed, heavy_list);
@@ -1146,7 +1171,8 @@ __global__ void __launch_bounds__(256) chain_assign(const int* __restrict__ head
 }
 template <typename T>
 __global__ void __launch_bounds__(256) chain_fill(const int64_t* __restrict__ index, const T* __restrict__ src, const int* __restrict__ head, int* __restrict__ cursor, int* __restrict__ listed_cursor,
-                                                  int2* __restrict__ seg, const __grid_constant__ BucketArgs A, const int* __restrict__ ctl, uint32_t* status) {
+                                                  int2* __restrict__ seg, const __grid_constant__ BucketArgs A, const int* ctl, uint32_t* status) {
+  after_grids_before();
   const bool grouped = ctl[kCtlGrouped] != 0;
   if (!grouped && ctl[kCtlListed] == 0) return;
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < A.n_idx; p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -1161,6 +1187,22 @@ __global__ void __launch_bounds__(256) chain_fill(const int64_t* __restrict__ in
     }
     seg[atomicAdd(at, 1)] = make_int2(pos, __float_as_int(to_f32(src[so])));
   }
+}
+
+// As a rule these five have nothing to do. listed_cnt: NULL where there are no chains
+template <typename T>
+static int launch_group(const int64_t* index, const T* src, const T* self, T* out, const BucketArgs& A, int* head, int* cursor, int* ctl, int* listed_cnt, int* listed_cursor, int* list, int2* seg,
+                        int64_t listed, uint32_t* status, cudaStream_t st) {
+  auto capped = [](int64_t n, int per, int64_t cap) { const int64_t g = (n + per - 1) / per; return g < 1 ? 1 : (g > cap ? cap : g); };
+  const int64_t walk = capped(A.n_idx, 256, 16 * kNumSMs);
+  cudaError_t e = launch_after(chain_count, walk, 256, 0, st, index, head, listed_cnt, A, ctl);
+  if (e == cudaSuccess) e = launch_after(chain_assign, grid_for(A.n_self, 4096), 256, 0, st, head, cursor, A.n_self, listed_cnt, listed_cursor, listed, ctl, list);
+  if (e == cudaSuccess) e = launch_after(chain_fill<T>, walk, 256, 0, st, index, src, head, cursor, listed_cursor, seg, A, ctl, status);
+  if (e == cudaSuccess) e = launch_after(bucket_replay<T>, capped(A.n_self, 256, 16 * kNumSMs), 256, 0, st, self, out, head, -1, cursor, seg, A.n_self, ctl + kCtlGrouped);
+  if (e == cudaSuccess)
+    e = launch_after(bucket_replay_heavy<T>, 2 * kNumSMs, 256, 0, st, self, out, HeavyCounters{head, cursor, -1, listed_cnt, listed_cursor, ctl + kCtlGrouped}, seg, A.dim_len, ctl + kCtlListed, list);
+  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+  return check_launch(5);
 }
 
 struct ChainScratch {
@@ -1198,15 +1240,411 @@ static int launch_chain(const void* self, const void* index, const void* src, vo
   chain_begin<<<1 + capped(A.n_self, 8 * kSample, 2 * kNumSMs), kSample, 0, st>>>(pi, head, A.n_self, ctl, listed_cnt, listed, A);
   chain_link<T><<<items_grid(A.n_idx, 256 * kChainUnroll), 256, 0, st>>>(pi, ps, head, link, ctl, A, status);
   chain_replay<T><<<grid_for(A.n_self, 256 * kChainUnroll), 256, 0, st>>>(px, po, head, link, A.n_self, ctl, list);
-  if (listed == 0) return check_launch(3);
-  // as a rule these five have nothing to do
-  const int walk = capped(A.n_idx, 256, 16 * kNumSMs);
-  chain_count<<<walk, 256, 0, st>>>(pi, head, listed_cnt, A, ctl);
-  chain_assign<<<grid_for(A.n_self, 4096), 256, 0, st>>>(head, cursor, A.n_self, listed_cnt, listed_cursor, listed, ctl, list);
-  chain_fill<T><<<walk, 256, 0, st>>>(pi, ps, head, cursor, listed_cursor, seg, A, ctl, status);
-  bucket_replay<T><<<capped(A.n_self, 256, 16 * kNumSMs), 256, 0, st>>>(px, po, head, -1, cursor, seg, A.n_self, ctl + kCtlGrouped);
-  bucket_replay_heavy<T><<<2 * kNumSMs, 256, 0, st>>>(px, po, HeavyCounters{head, cursor, -1, listed_cnt, listed_cursor, ctl + kCtlGrouped}, seg, A.dim_len, ctl + kCtlListed, list);
-  return check_launch(8);
+  if (int rc = check_launch(3)) return rc;
+  if (listed == 0) return B200_OK;
+  return launch_group<T>(pi, ps, px, po, A, head, cursor, ctl, listed_cnt, listed_cursor, list, seg, listed, status, st);
+}
+
+// ------------------------------------------------------------------ binned path
+// Matrices too tall for a strip of their columns to fit in shared memory, or off the strips'
+// 16-byte grid. self is viewed as [outer, rows, cols]; its columns are dealt into groups of at most 32, and the
+// rows of a group into bins of 2^shift rows whose sums fit in a warp's share of shared memory (kBinDests). Two launches:
+//   binned_sort: a CTA takes a chunk of the index -- rows of one column group -- and writes its
+//     contributions out grouped by bin, with a table of where each bin begins. The order is
+//     stable for every destination: a thread owns ONE column of a run of rows and takes its places
+//     in order from counters of its own run, and the runs follow one another; so nothing is sorted by
+//     position and a record is the destination and the value alone.
+//   binned_replay: a warp owns a bin. It walks the bin's records chunk after chunk, 32 to a step, and adds them to the
+//     sums in shared memory; two records of a step with one destination are found with a tag
+//     table, as in the strip kernels, and added in lane order, which is source order.
+// Every global access is in runs of a row or of a segment; what is random stays in shared memory, where the chain path
+// has its exchanges and look-ups in L2. fp16 150134 x 63, 75067 rows: 133 us in chains, 87 so (binned_sort 29, half of its
+// issue slots busy counting and placing; binned_replay 45: nine warps of 4096 sums fill an SM's shared memory, and each goes
+// at the speed of its chain of tag, look, sum; six more launches that begin and find nothing to do). fp32 4095 x 4095 556 -> 283,
+// 160000 x 400 3640 -> 1140, 888 x 4065 99 -> 58. Tried: a CTA to a bin, its records in chains in shared memory (123 us
+// for the replay, 18 instructions' worth of divergence to a destination); the records of 8 steps in registers
+// (80: a step unrolled eight times does not fit the instruction cache); 256 threads with runs of 32 rows in binned_sort (44).
+constexpr int kBinThreads = 512;
+constexpr int kBinItems = 16;  // rows of its column per thread of binned_sort, at most
+constexpr int kBinDests = 4096;
+constexpr int kBinAhead = 8;  // steps whose records are on the way while those before are added
+constexpr int kBinCountBytes = 40 * 1024;  // counters of binned_sort: two CTAs of it per SM
+
+struct BinnedArgs {
+  int64_t outer, rows, cols;  // self / out, contiguous
+  int64_t idx_outer, idx_rows, idx_cols;
+  int64_t idx_so, idx_sr, idx_sc, src_so, src_sr, src_sc;  // element strides of index / src
+  int c, groups, idx_groups;   // columns of a group; groups of self's columns, of the index's
+  int shift, bins;             // log2 of a bin's rows; bins of a group
+  int items, runs, chunk_rows, chunks;  // rows of a run (one thread's), runs of a chunk, rows of a chunk, chunks of a group
+  uint32_t c_magic;            // x / c == __umulhi(x, c_magic) for x < 2^16
+};
+
+template <typename T> struct BinRec { typedef uint32_t type; };
+template <> struct BinRec<float> { typedef uint2 type; };
+__device__ __forceinline__ uint32_t bin_rec(int dest, uint16_t bits) { return static_cast<uint32_t>(dest) | static_cast<uint32_t>(bits) << 16; }
+__device__ __forceinline__ void bin_make(uint32_t& r, int dest, __nv_bfloat16 v) { r = bin_rec(dest, __bfloat16_as_ushort(v)); }
+__device__ __forceinline__ void bin_make(uint32_t& r, int dest, __half v) { r = bin_rec(dest, __half_as_ushort(v)); }
+__device__ __forceinline__ void bin_make(uint2& r, int dest, float v) { r = make_uint2(static_cast<uint32_t>(dest), __float_as_uint(v)); }
+__device__ __forceinline__ int bin_dest(uint32_t r) { return static_cast<int>(r & 0xffffu); }
+__device__ __forceinline__ int bin_dest(uint2 r) { return static_cast<int>(r.x); }
+template <typename T> __device__ __forceinline__ float bin_value(typename BinRec<T>::type r);
+template <> __device__ __forceinline__ float bin_value<float>(uint2 r) { return __uint_as_float(r.y); }
+template <> __device__ __forceinline__ float bin_value<__nv_bfloat16>(uint32_t r) { return __uint_as_float(r & 0xffff0000u); }
+template <> __device__ __forceinline__ float bin_value<__half>(uint32_t r) { return __half2float(__ushort_as_half(static_cast<unsigned short>(r >> 16))); }
+
+// Exclusive prefix sums over the CTA's threads; `total` is the sum of all. `sums`: 16 words.
+__device__ __forceinline__ int bin_scan(int v, int* sums, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  __syncthreads();  // the sums of a call before
+  if (lane == 31) sums[warp] = inc;
+  __syncthreads();
+  int w = lane < kBinThreads / 32 ? sums[lane] : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += y;
+  }
+  total = __shfl_sync(0xffffffffu, w, 31);
+  const int before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+  return inc - v + (warp ? before : 0);
+}
+
+// Looks at a sample: where the destinations, or the bins, are crowded, one warp would walk most of the
+// records, and everything is grouped by destination instead, as on the chain path.
+__global__ void __launch_bounds__(kSample) binned_begin(const int64_t* __restrict__ index, const __grid_constant__ BinnedArgs A, const __grid_constant__ BucketArgs B, int* __restrict__ ctl) {
+  __shared__ int table[4 * kSample];
+  next_grid_may_start();
+  int dest[1];
+  const int s = sample_destinations<kSample>(index, B, dest);
+  const int same = equal_pairs<kSample>(dest, table);
+  if (dest[0] >= 0) {
+    const uint32_t d = static_cast<uint32_t>(dest[0]), cols = static_cast<uint32_t>(A.cols), rows = static_cast<uint32_t>(A.rows), row = d / cols, o = row / rows;
+    dest[0] = static_cast<int>((o * A.groups + (d - row * cols) / A.c) * A.bins + ((row - o * rows) >> A.shift));
+  }
+  const int near = equal_pairs<kSample>(dest, table);
+  if (threadIdx.x == 0) {
+    ctl[kCtlSlots] = 0;
+    ctl[kCtlListed] = 0;
+    ctl[kCtlGrouped] = crowded(same, s, static_cast<double>(A.idx_outer) * A.idx_cols * A.rows) || crowded(near, s, static_cast<double>(A.idx_outer) * A.idx_groups * A.bins) ? 1 : 0;
+  }
+}
+
+// rec: [outer][group][chunk][chunk_rows * c]; first: [outer][group][chunk][bins + 1], where each bin begins in its chunk
+template <typename T>
+__global__ void __launch_bounds__(kBinThreads, 2) binned_sort(const int64_t* __restrict__ index, const T* __restrict__ src, typename BinRec<T>::type* __restrict__ rec, uint16_t* __restrict__ first,
+                                                              const __grid_constant__ BinnedArgs A, const int* ctl, uint32_t* status) {
+  typedef typename BinRec<T>::type Rec;
+  extern __shared__ __align__(16) unsigned char bin_smem[];
+  __shared__ int sums[kBinThreads / 32];
+  const int tid = threadIdx.x;
+  const int words = (A.bins + 1) / 2;  // two 16-bit counters to a word
+  Rec* stage = reinterpret_cast<Rec*>(bin_smem);
+  uint32_t* count = reinterpret_cast<uint32_t*>(stage + A.chunk_rows * A.c);  // [runs][words]
+  const int chunk = static_cast<int>(blockIdx.x % static_cast<uint32_t>(A.chunks));
+  const int64_t og = blockIdx.x / static_cast<uint32_t>(A.chunks);
+  const int64_t o = og / A.idx_groups;
+  const int run = static_cast<int>(__umulhi(tid, A.c_magic)), col = tid - run * A.c;
+  const int64_t j = (og - o * A.idx_groups) * A.c + col;
+  const int64_t row0 = static_cast<int64_t>(chunk) * A.chunk_rows + run * A.items;
+  const int64_t left = A.idx_rows - row0;
+  const int mine = run < A.runs && j < A.idx_cols && left > 0 ? (left < A.items ? static_cast<int>(left) : A.items) : 0;
+  for (int i = tid; i < A.runs * words; i += kBinThreads) count[i] = 0;
+  __syncthreads();
+  const int64_t* pi = index + o * A.idx_so + row0 * A.idx_sr + j * A.idx_sc;
+  const T* ps = src + o * A.src_so + row0 * A.src_sr + j * A.src_sc;
+  uint32_t* counters = count + run * words;
+  constexpr uint32_t kNone = 0xffffffffu;
+  constexpr int kFlight = 16;  // index elements on the way
+  uint32_t key[kBinItems];
+  T v[kBinItems];
+  bool bad = false;
+#pragma unroll
+  for (int h = 0; h < kBinItems; h += kFlight) {
+    int64_t raw[kFlight];
+#pragma unroll
+    for (int u = 0; u < kFlight; ++u) {
+      raw[u] = -1;
+      if (h + u < mine) {
+        raw[u] = __ldcs(pi);
+        v[h + u] = __ldcs(ps);
+      }
+      pi += A.idx_sr;
+      ps += A.src_sr;
+    }
+#pragma unroll
+    for (int u = 0; u < kFlight; ++u) {
+      key[h + u] = kNone;
+      if (static_cast<uint64_t>(raw[u]) < static_cast<uint64_t>(A.rows)) {
+        key[h + u] = static_cast<uint32_t>(raw[u]);
+        const uint32_t bin = key[h + u] >> A.shift;
+        atomicAdd(&counters[bin >> 1], 1u << (16 * (bin & 1)));
+      } else if (h + u < mine) {
+        bad = true;
+      }
+    }
+  }
+  if (bad) flag_oob(status);
+  next_grid_may_start();
+  after_grids_before();  // (the index has been there all along)
+  if (ctl[kCtlGrouped]) return;
+  __syncthreads();
+  // counters -> the first place of the run's records of that bin
+  int total = 0;
+  uint16_t* f = first + static_cast<int64_t>(blockIdx.x) * (A.bins + 1);
+  for (int w0 = 0; w0 < words; w0 += kBinThreads) {
+    const int w = w0 + tid;
+    uint32_t sum = 0;
+    if (w < words)
+      for (int r = 0; r < A.runs; ++r) sum += count[r * words + w];
+    const int low = static_cast<int>(sum & 0xffffu), both = low + static_cast<int>(sum >> 16);
+    int all;
+    const int at = total + bin_scan(both, sums, all);
+    total += all;
+    if (w < words) {
+      uint32_t next = static_cast<uint32_t>(at) | static_cast<uint32_t>(at + low) << 16;
+      f[2 * w] = static_cast<uint16_t>(at);
+      if (2 * w + 1 <= A.bins) f[2 * w + 1] = static_cast<uint16_t>(at + low);
+      if (2 * w + 2 == A.bins) f[A.bins] = static_cast<uint16_t>(at + both);
+      for (int r = 0; r < A.runs; ++r) {
+        const uint32_t n = count[r * words + w];
+        count[r * words + w] = next;
+        next += n;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kBinItems; ++u)
+    if (key[u] != kNone) {
+      const uint32_t bin = key[u] >> A.shift, half = 16 * (bin & 1);
+      const uint32_t at = (atomicAdd(&counters[bin >> 1], 1u << half) >> half) & 0xffffu;
+      bin_make(stage[at], 4 * (static_cast<int>(key[u] & ((1u << A.shift) - 1u)) * A.c + col), v[u]);
+    }
+  __syncthreads();
+  Rec* to = rec + static_cast<int64_t>(blockIdx.x) * (A.chunk_rows * A.c);
+  for (int i = tid; i < total; i += kBinThreads) to[i] = stage[i];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, T* __restrict__ out, const typename BinRec<T>::type* __restrict__ rec, const uint16_t* __restrict__ first,
+                                                    const __grid_constant__ BinnedArgs A, const int* ctl, int* head, int64_t n_self) {
+  typedef typename BinRec<T>::type Rec;
+  constexpr uint32_t kAll = 0xffffffffu;
+  constexpr int kMove = 16;   // elements of self on the way per lane
+  extern __shared__ __align__(16) unsigned char bin_smem[];
+  __shared__ uint32_t piece[32];
+  __shared__ __align__(16) Rec ring[2][kBinAhead][32];
+  const int dests = A.c << A.shift, lane = threadIdx.x;
+  float* sum = reinterpret_cast<float*>(bin_smem);  // [dests + 32]: one to spare for each lane; behind them a byte of tag for each
+  const uint32_t sum_a = static_cast<uint32_t>(__cvta_generic_to_shared(bin_smem)), tag_a = sum_a + 4 * (dests + 32);
+  const int bin = static_cast<int>(blockIdx.x % static_cast<uint32_t>(A.bins));
+  const int64_t og = blockIdx.x / static_cast<uint32_t>(A.bins);
+  const int64_t o = og / A.groups, g = og - o * A.groups;
+  const int64_t row0 = static_cast<int64_t>(bin) << A.shift;
+  const int rows = static_cast<int>(A.rows - row0 < (1 << A.shift) ? A.rows - row0 : (1 << A.shift));
+  const int width = static_cast<int>(A.cols - g * A.c < A.c ? A.cols - g * A.c : A.c);
+  const int64_t base = (o * A.rows + row0) * A.cols + g * A.c;
+  // a group is 32 columns of a row, or whole rows (c == cols < 32): in memory, too, a lane's elements lie a constant step apart
+  const int used = rows * A.c;
+  const int64_t step = A.c == 32 ? A.cols : 32;
+  const int end = A.c < 32 || lane < width ? used : 0;
+  after_grids_before();
+  if (ctl[kCtlGrouped]) {  // the counters of the kernels that follow
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane; i < n_self; i += static_cast<int64_t>(gridDim.x) * 32) head[i] = -1;
+    return;
+  }
+  {
+    const T* p = self + base + lane;
+    for (int d0 = lane; d0 < end; d0 += 32 * kMove) {
+      T s[kMove];
+#pragma unroll
+      for (int u = 0; u < kMove; ++u) {
+        if (d0 + 32 * u < end) s[u] = *p;
+        p += step;
+      }
+#pragma unroll
+      for (int u = 0; u < kMove; ++u)
+        if (d0 + 32 * u < end) sum[d0 + 32 * u] = to_f32(s[u]);
+    }
+  }
+  const int chunks = g < A.idx_groups && o < A.idx_outer ? A.chunks : 0;
+  const int per_chunk = A.chunk_rows * A.c;
+  const int64_t chunk0 = (o * A.idx_groups + g) * A.chunks;
+  const uint16_t* f = first + (chunk0 + lane) * (A.bins + 1) + bin;
+  const int64_t f_step = 32LL * (A.bins + 1);
+  const Rec* from = rec + chunk0 * per_chunk;
+  // 32 chunks are a batch: a lane knows where its chunk's piece of this bin lies and which numbers its records have
+  int b = 0, e = 0, c_next = 0;            // the next batch's table and first chunk
+  int start = 0, total = 0, before = 0;    // number of the first record of the lane's piece; records of the batch; pieces that start before `pos`
+  int pos = 0;                             // records of the batch asked for
+  auto read_table = [&]() {
+    b = e = 0;
+    if (c_next + lane < chunks) { b = f[0]; e = f[1]; }
+    f += f_step;
+  };
+  auto open = [&]() {
+    int upto = e - b;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(kAll, upto, d);
+      if (lane >= d) upto += y;
+    }
+    total = __shfl_sync(kAll, upto, 31);
+    pos = before = 0;
+    start = upto - (e - b);
+    const uint32_t filled = __ballot_sync(kAll, e > b);
+    // where record number 0 would lie, were it this piece's; the pieces that have records stand side by side
+    if (e > b) piece[__popc(filled & ((1u << lane) - 1u))] = static_cast<uint32_t>(c_next + lane) * static_cast<uint32_t>(per_chunk) + static_cast<uint32_t>(b - start);
+    else start = 0x40000000;
+    __syncwarp();
+    c_next += 32;
+    read_table();
+  };
+  // asks for the next records, up to 32 * kBinAhead of a batch; how many there are
+  auto load = [&](int buf) {
+    while (pos >= total && c_next < chunks) open();
+    const int n = total - pos < 32 * kBinAhead ? total - pos : 32 * kBinAhead;
+#pragma unroll 1
+    for (int u = 0; 32 * u < n; ++u, pos += 32) {
+      const uint32_t t = static_cast<uint32_t>(start - pos);
+      const uint32_t starts = __reduce_or_sync(kAll, t < 32u ? 1u << t : 0u);
+      const int q = before + __popc(starts & ((2u << lane) - 1u)) - 1;
+      before += __popc(starts);
+      if (32 * u + lane < n) __pipeline_memcpy_async(&ring[buf][u][lane], from + (piece[q] + static_cast<uint32_t>(pos + lane)), sizeof(Rec));
+    }
+    __pipeline_commit();
+    __syncwarp();
+    return n;
+  };
+  auto add = [&](uint32_t off, float v) {  // off: 4 * destination
+    const uint32_t tag = tag_a + (off >> 2), at = sum_a + off;
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(tag), "r"(lane) : "memory");
+    __syncwarp();
+    uint32_t winner;
+    float old;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(winner) : "r"(tag) : "memory");
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(old) : "r"(at) : "memory");
+    const bool lost = winner != static_cast<uint32_t>(lane);
+    const uint32_t losers = __ballot_sync(kAll, lost);
+    if (losers == 0u) {
+      asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(old + v) : "memory");
+      __syncwarp();
+      return;
+    }
+    // the lanes of a clash are the losers and the lanes they name; all others add at once
+    uint32_t involved = losers | __reduce_or_sync(kAll, lost ? 1u << winner : 0u);
+    const int k = static_cast<int>(off >> 2);
+    if (__popc(involved) <= 8) {
+      if (!(involved >> lane & 1u)) sum[k] = old + v;
+      __syncwarp();
+      while (involved) {
+        if (lane == __ffs(involved) - 1) sum[k] += v;
+        involved &= involved - 1;
+        __syncwarp();
+      }
+    } else {
+      apply_in_rank_order(sum, k, v, rank_among_earlier<32>(k, lane));
+    }
+  };
+  __syncwarp();
+  if (chunks > 0) read_table();
+  int n = load(0);
+#pragma unroll 1
+  for (int buf = 0; n > 0; buf ^= 1) {
+    const int then = load(buf ^ 1);
+    __pipeline_wait_prior(1);
+#pragma unroll 1
+    for (int u = 0; 32 * u < n; ++u) {
+      uint32_t off = 4u * (dests + lane);
+      float v = 0.f;
+      if (32 * u + lane < n) {  // (a lane reads what it has copied itself)
+        const Rec r = ring[buf][u][lane];
+        off = static_cast<uint32_t>(bin_dest(r));
+        v = bin_value<T>(r);
+      }
+      add(off, v);
+    }
+    n = then;
+  }
+  __syncwarp();
+  T* p = out + base + lane;
+#pragma unroll 8
+  for (int d = lane; d < end; d += 32, p += step) *p = from_f32<T>(sum[d]);
+}
+
+// Fills in the geometry behind `src_sc`; false: not for this path (more bins than there is room to count in).
+static bool plan_binned(BinnedArgs& A) {
+  if (A.cols < 2 || A.rows >= 0x7fffffffLL || A.idx_rows >= 0x7fffffffLL) return false;
+  A.c = static_cast<int>(A.cols < 32 ? A.cols : 32);
+  A.groups = static_cast<int>((A.cols + A.c - 1) / A.c);
+  A.idx_groups = static_cast<int>((A.idx_cols + A.c - 1) / A.c);
+  A.c_magic = 0xffffffffu / static_cast<uint32_t>(A.c) + 1u;
+  A.runs = kBinThreads / A.c;
+  // bins: as large as a warp's share of shared memory, smaller where that leaves fewer than eight per SM
+  auto bins = [&](int sh) { return (A.rows + (1LL << sh) - 1) >> sh; };
+  A.shift = 0;
+  while ((A.c << (A.shift + 1)) <= kBinDests) ++A.shift;
+  while (A.shift > 0 && A.outer * A.groups * bins(A.shift) < 8LL * kNumSMs) --A.shift;
+  if (A.runs * ((bins(A.shift) + 1) / 2) * 4 > kBinCountBytes) return false;
+  A.bins = static_cast<int>(bins(A.shift));
+  // chunks: all a CTA can hold, less where that leaves fewer than two per SM
+  const int64_t columns = A.idx_outer * A.idx_groups;
+  A.items = static_cast<int>((A.idx_rows + A.runs - 1) / A.runs < kBinItems ? (A.idx_rows + A.runs - 1) / A.runs : kBinItems);
+  while (A.items > 1 && columns * ((A.idx_rows + A.items * A.runs - 1) / (A.items * A.runs)) < 2 * kNumSMs) --A.items;
+  A.chunk_rows = A.items * A.runs;
+  A.chunks = static_cast<int>((A.idx_rows + A.chunk_rows - 1) / A.chunk_rows);
+  return A.outer * A.groups * A.bins < 0x7fffffffLL && columns * A.chunks < 0x7ffffffeLL && static_cast<int64_t>(A.chunks) * A.chunk_rows * A.c < 0x7fffffffLL;
+}
+struct BinnedScratch {
+  int64_t first_bytes, rec_bytes, head_bytes, list_bytes, seg_bytes, total;
+};
+static BinnedScratch binned_scratch(const BinnedArgs& A, int es, int64_t n_self, int64_t n_idx) {
+  BinnedScratch s;
+  const int64_t chunks = A.idx_outer * A.idx_groups * A.chunks;
+  s.first_bytes = up256(2 * chunks * (A.bins + 1LL));
+  s.rec_bytes = up256(chunks * A.chunk_rows * A.c * (es == 4 ? 8 : 4));
+  s.head_bytes = up256(4 * n_self);
+  s.list_bytes = up256(4 * (n_idx / (kLightMax + 1) + 1));
+  s.seg_bytes = up256(8 * n_idx);
+  // the records, or what group_rest needs in their place
+  const int64_t grouped = 2 * s.head_bytes + s.list_bytes + s.seg_bytes;
+  s.total = 256 + (s.first_bytes + s.rec_bytes > grouped ? s.first_bytes + s.rec_bytes : grouped);
+  return s;
+}
+
+template <typename T>
+static int launch_binned(const void* self, const void* index, const void* src, void* out, const BinnedArgs& A, const BucketArgs& B, void* scratch, uint32_t* status, cudaStream_t st) {
+  typedef typename BinRec<T>::type Rec;
+  const BinnedScratch S = binned_scratch(A, static_cast<int>(sizeof(T)), B.n_self, B.n_idx);
+  int* ctl = static_cast<int*>(scratch);
+  char* base = static_cast<char*>(scratch) + 256;
+  uint16_t* first = reinterpret_cast<uint16_t*>(base);
+  Rec* rec = reinterpret_cast<Rec*>(base + S.first_bytes);
+  const size_t sort_smem = sizeof(Rec) * A.chunk_rows * A.c + 4 * static_cast<size_t>(A.runs) * ((A.bins + 1) / 2);
+  const size_t replay_smem = 5 * (static_cast<size_t>(A.c << A.shift) + 32);
+  cudaError_t e = cudaFuncSetAttribute(binned_sort<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 108 * 1024);
+  const int64_t sorts = A.idx_outer * A.idx_groups * A.chunks, replays = A.outer * A.groups * A.bins;
+  const int64_t* pi = static_cast<const int64_t*>(index);
+  const T* ps = static_cast<const T*>(src);
+  const T* px = static_cast<const T*>(self);
+  T* po = static_cast<T*>(out);
+  int* head = reinterpret_cast<int*>(base);
+  int* cursor = reinterpret_cast<int*>(base + S.head_bytes);
+  int* list = reinterpret_cast<int*>(base + 2 * S.head_bytes);
+  int2* seg = reinterpret_cast<int2*>(base + 2 * S.head_bytes + S.list_bytes);
+  binned_begin<<<1, kSample, 0, st>>>(pi, A, B, ctl);
+  if (e == cudaSuccess) e = launch_after(binned_sort<T>, sorts, kBinThreads, sort_smem, st, pi, ps, rec, first, A, ctl, status);
+  if (e == cudaSuccess) e = launch_after(binned_replay<T>, replays, 32, replay_smem, st, px, po, rec, first, A, ctl, head, B.n_self);
+  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+  if (int rc = check_launch(3)) return rc;
+  return launch_group<T>(pi, ps, px, po, B, head, cursor, ctl, nullptr, nullptr, list, seg, 0, status, st);
 }
 
 // ------------------------------------------------------------------ embedding_dense_backward
@@ -1605,13 +2043,26 @@ static int launch_rows(const void* self, const void* index, const void* src, voi
 
 namespace b200 {
 
-enum ScatterPath { kPathNone = 0, kPathStrip, kPathStripWide, kPathRows, kPathBucket, kPathChain, kPathLines };
+// Nanoseconds, as measured over 64 x 1024 ... 15000 x 1024, 33 x 100000 and 150134 x 63. A strip CTA takes 14.5 for a source row, whatever its
+// few columns are (twice that where the destination takes two windows), and 2400 to begin and end, and there are one or two of
+// them per SM; the binned path has more launches to pay for, and then time for each contribution and destination. fp32, as
+// many source rows as rows, strips against bins: 500 x 512 11.5 / 23 us, 2000 x 256 30 / 24, 200 x 4096 27 / 25, 4000 x 512 59 / 35,
+// 12000 x 512 312 / 131, 33 x 100000 236 / 94.
+static bool binned_beats_strip(const StripArgs& S, int64_t n_idx) {
+  const int64_t bytes = S.rows * kStripCols * 4, at_once = kNumSMs * (bytes <= kStripSmemTarget - 34 * 1024 ? 2 : 1);
+  const int64_t rounds = (S.outer * (S.cols / kStripCols) + at_once - 1) / at_once, windows = bytes <= kSmemBudget - 40 * 1024 ? 1 : 2;
+  const double strip = static_cast<double>(rounds) * (14.5 * static_cast<double>(S.idx_rows * windows) + 2400.0) + 2000.0;
+  return strip > 15000.0 + 0.011 * static_cast<double>(n_idx) + 0.003 * static_cast<double>(S.outer * S.rows * S.cols);
+}
+
+enum ScatterPath { kPathNone = 0, kPathStrip, kPathStripWide, kPathRows, kPathBinned, kPathBucket, kPathChain, kPathLines };
 
 struct ScatterPlan {
   ScatterPath path;
   int64_t n_self, n_idx, scratch_bytes;
   StripArgs strip;
   RowArgs rows;
+  BinnedArgs binned;
 };
 
 // Decides which kernel family serves a geometry (shared by the launcher and the scratch
@@ -1625,7 +2076,8 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
   P.path = kPathLines;
   if (P.n_self == 0 || P.n_idx == 0) { P.path = kPathNone; return P; }
   const bool small = P.n_idx <= (1 << 16);  // launch-bound either way
-  if (aligned16(self) && aligned16(out) && aligned16(index) && aligned16(src)) {
+  const bool aligned = aligned16(self) && aligned16(out) && aligned16(index) && aligned16(src);
+  {
     int64_t outer = 1, cols = 1, idx_outer = 1, idx_cols = 1;
     for (int d = 0; d < dim; ++d) { outer *= self_shape[d]; idx_outer *= index_shape[d]; }
     for (int d = dim + 1; d < ndim; ++d) { cols *= self_shape[d]; idx_cols *= index_shape[d]; }
@@ -1643,16 +2095,25 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
         const bool stride_ok = (src_strides[dim] * es) % 4 == 0 && (src_so * es) % 4 == 0;  // 4-byte value granules
         const int64_t strips = outer * (cols / kStripCols);
         const bool fits = rows * kStripCols * 4 <= 2 * (kSmemBudget - 64 * 1024);  // at most two destination windows
-        if (inner_ok && shape_ok && stride_ok && fits && (strips >= 32 || small)) {
+        P.binned = BinnedArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], index_strides[dt], src_so, src_strides[dim], src_strides[dt]};
+        const bool binned = P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && plan_binned(P.binned);
+        if (aligned && inner_ok && shape_ok && stride_ok && fits && (strips >= 32 || small)) {
           P.path = kPathStrip;
           P.strip = StripArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], src_so, src_strides[dim], 0, 0};
           // eight columns per CTA when the whole destination strip fits and every staged chunk is 16-byte aligned
           const bool wide_shape = cols % kWideCols == 0 && idx_cols % kWideCols == 0 && rows <= kWideMaxRows && idx_rows >= 256 && idx_rows < 0x7fffffffLL && outer * (cols / kWideCols) >= kNumSMs / 2;
           const bool wide_align = index_strides[dim] % 2 == 0 && idx_so % 2 == 0 && (src_strides[dim] * es) % 16 == 0 && (src_so * es) % 16 == 0;
           if (wide_shape && wide_align) P.path = kPathStripWide;
+          if (P.path == kPathStripWide || !binned || !binned_beats_strip(P.strip, P.n_idx)) return P;
+        }
+        // fp32, as many source rows as rows, lines or chains against bins: 16 x 333 13 / 15 us, 32 x 333 21 / 16, 64 x 63 35 / 15; 65 x 8191 30 / 35,
+        // 100 x 4095 27 / 29, 200 x 4095 39 / 35, 65 x 333 21 / 17, 200 x 63 20 / 15
+        if (binned && (idx_rows >= 128 || (idx_rows > 24 && cols <= 2048))) {
+          P.path = kPathBinned;
+          P.scratch_bytes = binned_scratch(P.binned, es, P.n_self, P.n_idx).total;
           return P;
         }
-      } else if (index_strides[dim] == 1 && src_strides[dim] == 1) {
+      } else if (aligned && index_strides[dim] == 1 && src_strides[dim] == 1) {
         const bool fits = rows * 2 * 4 <= kSmemBudget - 16 * 1024;
         if (fits && (outer >= 64 || small)) {
           P.path = kPathRows;
@@ -1728,7 +2189,7 @@ extern "C" int b200_scatter_add(const void* self, const void* index, const void*
       default: return launch_rows<__half>(self, index, src, out, P.rows, status, st);
     }
   }
-  if (P.path == kPathBucket || P.path == kPathChain) {
+  if (P.path == kPathBinned || P.path == kPathBucket || P.path == kPathChain) {
     if (!scratch || scratch_bytes < P.scratch_bytes) return B200_ESCRATCH;
     BucketArgs A;
     A.ndim = ndim;
@@ -1744,6 +2205,13 @@ extern "C" int b200_scatter_add(const void* self, const void* index, const void*
       st_out *= self_shape[d];
       A.idx_stride[d] = index_strides[d];
       A.src_stride[d] = src_strides[d];
+    }
+    if (P.path == kPathBinned) {
+      switch (dtype) {
+        case B200_F32: return launch_binned<float>(self, index, src, out, P.binned, A, scratch, status, st);
+        case B200_BF16: return launch_binned<__nv_bfloat16>(self, index, src, out, P.binned, A, scratch, status, st);
+        default: return launch_binned<__half>(self, index, src, out, P.binned, A, scratch, status, st);
+      }
     }
     const bool chain = P.path == kPathChain;
     switch (dtype) {

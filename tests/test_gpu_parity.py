@@ -629,6 +629,56 @@ def test_scatter_add_crowded_or_not_bit_exact(backend, dtype, spread):
         assert bits_equal(want.t().contiguous(), turned.cpu())
 
 
+# (self, dim, index, layout of index and src): a column group of one column, one of 31 and of two; bins cut short; more
+# contributions than a bin's ring and than destinations; an index smaller than self on every side; one row of indices for all
+# columns, indices and values read across their rows; the last one has no columns to deal out and hangs in chains
+BINNED = [
+    ((5003, 33), 0, (5003, 33), "rows"),
+    ((129, 31), 0, (700, 31), "rows"),
+    ((300, 2), 0, (3001, 2), "rows"),
+    ((20001, 40), 0, (20001, 40), "rows"),
+    ((600, 65), 0, (20000, 65), "rows"),
+    ((5, 701, 37), 1, (4, 650, 35), "rows"),
+    ((4100, 70), 0, (2050, 70), "expanded"),
+    ((4100, 45), 0, (4100, 45), "columns"),
+    ((70001,), 0, (70001,), "rows"),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("case", BINNED, ids=lambda c: f"{'x'.join(map(str, c[0]))}_{c[3]}")
+def test_scatter_add_in_bins_bit_exact(backend, dtype, case):
+    """Contributions sorted into bins of rows: the order of the additions into a destination, and so every bit, is that of
+    the sequential loop; an index out of range is reported and adds nothing; in place as well."""
+    impl = backend[torch.ops.aten.scatter_add.default]
+    shape, dim, ishape, layout = case
+    g = torch.Generator().manual_seed(11)
+    x, src = torch.randn(shape, generator=g).to(dtype), torch.randn(ishape, generator=g).to(dtype)
+    idx = torch.randint(0, shape[dim], ishape, generator=g)
+    if layout == "expanded":
+        idx = idx[:, :1].expand(ishape)
+    on_gpu = [x.to(DEV), idx.to(DEV), src.to(DEV)]
+    if layout == "columns":
+        on_gpu[1:] = [t.t().contiguous().t() for t in on_gpu[1:]]
+    if layout == "expanded":
+        on_gpu[1] = on_gpu[1][:, :1].expand(ishape)
+    want = oracle.scatter_add(x, dim, idx.contiguous(), src)
+    assert bits_equal(want, impl(on_gpu[0], dim, on_gpu[1], on_gpu[2]).cpu())
+    ops.check_device_status()
+    mine = on_gpu[0].clone()
+    backend[torch.ops.aten.scatter_add_.default](mine, dim, on_gpu[1], on_gpu[2])
+    assert bits_equal(want, mine.cpu())
+    bad = idx.clone().contiguous()
+    bad.view(-1)[[0, 1, -1]] = torch.tensor([shape[dim], -1, 1 << 40])
+    got = impl(on_gpu[0], dim, bad.to(DEV), on_gpu[2])
+    with pytest.raises(IndexError):
+        ops.check_device_status()
+    out = (bad < 0) | (bad >= shape[dim])
+    wide = torch.cat([x, torch.zeros([1 if d == dim else n for d, n in enumerate(shape)], dtype=dtype)], dim)
+    want = oracle.scatter_add(wide, dim, torch.where(out, shape[dim], bad), src).narrow(dim, 0, shape[dim]).contiguous()
+    assert bits_equal(want, got.cpu())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_scatter_add_with_an_empty_index_copies_self(backend, dtype):
     """No contributions at all (an index with a zero extent): the result is self, for every
