@@ -132,7 +132,7 @@ struct GemmTcParams {
   int tma_store;    // 1 = C goes out through TMA tile stores (N % 8 == 0, aligned), 0 = plain stores
   int col_fastest;  // tile order: 1 = column-block fastest (write-bound shapes), 0 = grouped row-block fastest
   int split_slabs;  // 0, or K slabs per plane of fp32 operands split into three bf16 planes (see gemm_f32_split_dispatch)
-  int range_slabs;  // with split_slabs: 0, or slabs per range of K; the ranges are what the kernel sees as batch entries
+  int range_slabs;  // fp32 results: 0, or slabs (per plane) per range of K; the ranges are what the kernel sees as batch entries
   const uint32_t* skip_if_set;  // when not NULL: the kernel returns at once if this device word is non-zero
   uint64_t wait_limit_ns;       // every mbarrier wait gives up after this long (kWaitLimitNs in ordinary calls)
   int withhold_first_slab;      // wait probe only: the producer never loads the first K slab of a CTA's first tile
@@ -225,11 +225,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // tensor map, Kp = 64 * split_slabs. One slab of the product needs the six plane pairs
   // whose product is not below fp32 resolution: (0,0) (0,1) (1,0) (0,2) (1,1) (2,0).
   // They are walked pair by pair over all slabs (see the producer).
-  const bool ranged = kPair && sizeof(TO) == 4 && p.range_slabs != 0;  // only fp32 results on pairs are cut into ranges
-  const int num_kb_all = p.split_slabs ? 6 * p.split_slabs : static_cast<int>((p.K + kBK - 1) / kBK);
+  const bool ranged = sizeof(TO) == 4 && p.range_slabs != 0;
+  const int k_slabs = static_cast<int>((p.K + kBK - 1) / kBK), planes = p.split_slabs ? 6 : 1, num_kb_all = planes * k_slabs;
   // a range of K has the slabs [b * range_slabs, (b + 1) * range_slabs), the last one what is left
   auto slabs_of = [&](int64_t b) {
-    const int left = p.split_slabs - static_cast<int>(b) * p.range_slabs;
+    const int left = k_slabs - static_cast<int>(b) * p.range_slabs;
     return left < p.range_slabs ? left : p.range_slabs;
   };
 
@@ -245,8 +245,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tile_coords(rem, mt, nt, mb, nb, p.col_fastest, p.group_m);
         // pair: this CTA's 128 rows of A and its half of the B slab's 256 rows
         const int m0 = mb * kTileM + static_cast<int>(cta_rank) * kBM, n0 = nb * kBN + static_cast<int>(cta_rank) * (kPair ? kBRows : 0);
-        const int tile_slabs = ranged ? slabs_of(b) : p.split_slabs, slab0 = ranged ? static_cast<int>(b) * p.range_slabs : 0;
-        const int num_kb = ranged ? 6 * tile_slabs : num_kb_all;
+        const int tile_slabs = ranged ? slabs_of(b) : k_slabs, slab0 = ranged ? static_cast<int>(b) * p.range_slabs : 0;
+        const int num_kb = planes * tile_slabs;
         const int entry = ranged ? 0 : static_cast<int>(b);  // the planes are one batch entry whatever range is walked
         int slab = 0, pair4 = 0;  // split operands: slab of the range, plane pair (times 4)
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -267,7 +267,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (kPair) tma_load_3d_pair(dst, map, fbar, c0, c1, c2);
             else tma_load_3d(dst, map, fbar, c0, c1, c2);
           };
-          int ka = kb * kBK, kbb = kb * kBK;
+          int ka = (slab0 + kb) * kBK, kbb = ka;
           if (sizeof(TO) == 4 && p.split_slabs) {
             // pairs (2,0) (1,1) (0,2) (1,0) (0,1) over all slabs first, then (0,0): the tensor
             // core truncates when it adds into the accumulator, by half a unit in the last
@@ -323,7 +323,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kBN);
-        const int num_kb = ranged ? 6 * slabs_of(t / (mt * nt)) : num_kb_all;
+        const int num_kb = ranged ? planes * slabs_of(t / (mt * nt)) : num_kb_all;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
           tc_fence_after();
@@ -391,6 +391,43 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const bool plain = p.alpha == 1.f && !p.has_bias;  // C = A x B: nothing to do but round
       const bool unit_scales = p.alpha == 1.f && p.beta == 1.f;
       const bool bias_vec = sizeof(TO) == sizeof(T) && p.has_bias && p.sbn == 1 && p.sbm % 8 == 0 && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
+      // a lane's 64 values of columns nb.. of its row: scaled, bias added in fp32, where they are (apart from
+      // the rounding, so that a product without either runs through none of this code)
+      auto scale = [&](uint32_t* rc, int64_t nb) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const int64_t n = nb + g * 8;
+          if (bias_vec && m < p.M && n + 8 <= p.N) {
+            // unit-stride bias (a row vector, or a matrix like C): eight values in one load
+            float bv[8];
+            widen<T>(ld_keep(bias + m * p.sbm + n), bv);  // TO is T on this path
+            if (unit_scales) {  // addmm as models call it: one add per value
+#pragma unroll
+              for (int e = 0; e < 8; ++e) rc[g * 8 + e] = __float_as_uint(__uint_as_float(rc[g * 8 + e]) + bv[e]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) rc[g * 8 + e] = __float_as_uint(fmaf(p.beta, bv[e], p.alpha * __uint_as_float(rc[g * 8 + e])));
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              float v = p.alpha * __uint_as_float(rc[g * 8 + e]);
+              if (p.has_bias && m < p.M && n + e < p.N) v = fmaf(p.beta, to_f32(bias[m * p.sbm + (n + e) * p.sbn]), v);
+              rc[g * 8 + e] = __float_as_uint(v);
+            }
+          }
+        }
+      };
+      // rounded once, into the 128-byte-swizzle layout of `mine`
+      auto park = [&](const uint32_t* rc, unsigned char* mine) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(rc[g * 8 + e]);
+          *reinterpret_cast<uint4*>(mine + lane * 128 + ((g ^ (lane & 7)) << 4)) = narrow<T>(v);
+        }
+      };
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
         tc_ld_wait();
@@ -406,8 +443,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             else mbar_arrive(tempty_bar(acc));
           }
         }
-        const uint32_t* rc = r[c & 1];
+        uint32_t* rc = r[c & 1];
         const int64_t nb = n0 + c * 64;
+        if constexpr (sizeof(TO) == 2) {
+          if (!plain) scale(rc, nb);
+        }
         if (p.tma_store) {
           // scale / bias in fp32, round once, park the lane's 64 outputs of its row in this
           // warp's 32 x 128-byte buffer in the 128-byte-swizzle layout (16-byte chunk index
@@ -417,67 +457,46 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           unsigned char* mine = epi_stage + (warp - 2) * kEpiStageBytes;
           if (lane == 0) tma_store_wait_read();  // the previous tile store has finished reading the buffer
           __syncwarp();
-#pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            const int64_t n = nb + g * 8;
-            float v[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(rc[g * 8 + e]);
-            if (!plain) {
-              if (bias_vec && m < p.M && n + 8 <= p.N) {
-                // unit-stride bias (a row vector, or a matrix like C): eight values in one load
-                float bv[8];
-                widen<T>(ld_keep(bias + m * p.sbm + n), bv);  // TO is T on this path
-                if (unit_scales) {  // addmm as models call it: one add per value
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) v[e] += bv[e];
-                } else {
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) v[e] = fmaf(p.beta, bv[e], p.alpha * v[e]);
-                }
-              } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  v[e] *= p.alpha;
-                  if (p.has_bias && m < p.M && n + e < p.N) v[e] = fmaf(p.beta, to_f32(bias[m * p.sbm + (n + e) * p.sbn]), v[e]);
-                }
-              }
-            }
-            *reinterpret_cast<uint4*>(mine + lane * 128 + ((g ^ (lane & 7)) << 4)) = narrow<T>(v);
-          }
+          park(rc, mine);
           fence_async_smem();
           __syncwarp();
           if (lane == 0 && nb < p.N && m0 + q * 32 < p.M) {
             tma_store_3d(&map_c, smem_u32(mine), static_cast<int>(nb), static_cast<int>(m0 + q * 32), static_cast<int>(b));
             tma_store_commit();
           }
-        } else if (sizeof(TO) == 2) {
+        } else if constexpr (sizeof(TO) == 2) {
           // 16-bit C whose rows are off the 16-byte grid (N not a multiple of 8): a lane owns a
           // row, so storing from registers would put every lane of a store in another row, one
           // 32-byte sector per 2-byte element. Park the chunk in the warp's buffer as above and
-          // write it out row by row, 64 contiguous bytes per store.
+          // write it out row by row, two elements to a lane; where a row starts between two 4-byte words
+          // a lane's pair is its second element and its neighbour's first, and the row's first element goes out alone.
+          // Element by element, with a row's address and the bias worked out for each, a tile took
+          // 12 us more than through the copy engine: bf16 4096 x 4098 x 512 75 -> 30 us (4096 wide 20), 2537 x 3709 x 920 61 -> 35.
           unsigned char* mine = epi_stage + (warp - 2) * kEpiStageBytes;
           __syncwarp();  // the previous chunk has been read out of the buffer
-#pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            const int64_t n = nb + g * 8;
-            float v[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              v[e] = p.alpha * __uint_as_float(rc[g * 8 + e]);
-              if (p.has_bias && m < p.M && n + e < p.N) v[e] = fmaf(p.beta, to_f32(bias[m * p.sbm + (n + e) * p.sbn]), v[e]);
-            }
-            *reinterpret_cast<uint4*>(mine + lane * 128 + ((g ^ (lane & 7)) << 4)) = narrow<T>(v);
-          }
+          park(rc, mine);
           __syncwarp();
-          const int64_t left = p.N - nb;
+          const int64_t left = p.N - nb, mr0 = m0 + q * 32;
           const int ncols = left < 64 ? static_cast<int>(left) : 64;  // <= 0: the chunk lies right of C
-          for (int rr = 0; rr < 32; ++rr) {
-            const int64_t mr = m0 + q * 32 + rr;
-            if (mr >= p.M) break;
-            TO* crow = C + (b * p.M + mr) * p.N + nb;
-            for (int cc = lane; cc < ncols; cc += 32)
-              crow[cc] = *reinterpret_cast<const TO*>(mine + rr * 128 + (((cc >> 3) ^ (rr & 7)) << 4) + (cc & 7) * 2);
+          const int nrows = p.M - mr0 < 32 ? static_cast<int>(p.M - mr0) : 32;
+          if (ncols > 0) {
+            unsigned short* crow = reinterpret_cast<unsigned short*>(C + (b * p.M + mr0) * p.N + nb);
+            const uint32_t mine_a = smem_u32(mine) + static_cast<uint32_t>(lane & 3) * 4;
+#pragma unroll 1
+            for (int r0 = 0; r0 < nrows; r0 += 8) {
+              uint32_t w[8];  // columns 2 lane, 2 lane + 1 of eight rows
+#pragma unroll
+              for (int u = 0; u < 8; ++u) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[u]) : "r"(mine_a + (r0 + u) * 128 + (((lane >> 2) ^ u) << 4)) : "memory");
+#pragma unroll
+              for (int u = 0; u < 8; ++u, crow += p.N) {
+                const uint32_t odd = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(crow) >> 1) & 1u;
+                const uint32_t after = __shfl_down_sync(0xffffffffu, w[u], 1), pair = __byte_perm(w[u], after, odd ? 0x5432 : 0x3210);
+                const int e0 = 2 * lane + static_cast<int>(odd), end = r0 + u < nrows ? ncols : 0;
+                if (e0 + 1 < end) *reinterpret_cast<uint32_t*>(crow + e0) = pair;
+                if (e0 + 1 == end) crow[e0] = static_cast<unsigned short>(pair);
+                if (odd && lane == 0 && end) crow[0] = static_cast<unsigned short>(w[u]);
+              }
+            }
           }
         } else if constexpr (!kRows) {
           // fp32 C, a lane to a row: 16 bytes at a time where the rows are on the grid. (Going through the
@@ -507,8 +526,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           // fp32 C off the grid (kRows): the same parking, 32 columns at a time, written out row by row, 128
           // contiguous bytes per store; the bias is looked up there, where a row and a column are all
           // that is live. Stores straight from the registers put every lane in another row, a
-          // sector per 4-byte element (1531 x 2050 x 1027 in fp32: 65.6 -> 59.6 us).
+          // sector per 4-byte element (1531 x 2050 x 1027 in fp32: 65.6 -> 59.6 us; eight rows on the way together 57.5).
           unsigned char* mine = epi_stage + (warp - 2) * kEpiStageBytes;
+          const int64_t mr0 = m0 + q * 32;
+          const int nrows = p.M - mr0 < 32 ? static_cast<int>(p.M - mr0) : 32;
+          const bool row_bias = p.has_bias && p.sbm == 0;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int64_t n = nb + h * 32 + lane;
@@ -521,14 +543,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               *reinterpret_cast<uint4*>(mine + lane * 128 + ((g ^ (lane & 7)) << 4)) = narrow<float>(v);
             }
             __syncwarp();
-            const int64_t mr0 = m0 + q * 32;
-            for (int rr = 0; rr < 32; ++rr) {
-              const int64_t mr = mr0 + rr;
-              if (mr >= p.M) break;
-              if (n < p.N) {
-                float v = *reinterpret_cast<const float*>(mine + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-                if (p.has_bias) v = fmaf(p.beta, to_f32(bias[mr * p.sbm + n * p.sbn]), v);
-                C[(b * p.M + mr) * p.N + n] = from_f32<TO>(v);
+            const float same = row_bias && n < p.N ? to_f32(bias[n * p.sbn]) : 0.f;  // a bias vector: one look for all rows
+            TO* c = C + (b * p.M + mr0) * p.N + n;
+            const uint32_t mine_a = smem_u32(mine) + static_cast<uint32_t>(lane & 3) * 4;
+#pragma unroll 1
+            for (int r0 = 0; r0 < nrows; r0 += 8) {
+              float v[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[u]) : "r"(mine_a + (r0 + u) * 128 + (((lane >> 2) ^ u) << 4)) : "memory");
+#pragma unroll
+              for (int u = 0; u < 8; ++u, c += p.N) {
+                if (n < p.N && r0 + u < nrows) {
+                  if (p.has_bias && !row_bias) v[u] = fmaf(p.beta, to_f32(bias[(mr0 + r0 + u) * p.sbm + n * p.sbn]), v[u]);
+                  *c = from_f32<TO>(row_bias ? fmaf(p.beta, same, v[u]) : v[u]);
+                }
               }
             }
           }
@@ -745,17 +773,17 @@ int gemm_tc_dispatch(const void* A, const void* B, const void* bias, void* C, in
 // ------------------------------------------------------------------ long contraction, few output tiles
 // A 16-bit product whose C is a handful of tiles leaves most SMs idle while one CTA per tile
 // walks all of K (5 x 4096 x 512: two CTAs, 64 K slabs each, 26 us). Here the contraction is
-// cut into S equal ranges that the kernel above sees as S batch entries -- A as [S][M][K/S],
-// B as [S][K/S][N], both only a different tensor map over the same memory -- and writes as
+// cut into S ranges of whole slabs that the kernel above sees as S batch entries and writes as
 // fp32 partial products [S][M][N] into caller scratch; a second kernel adds the S partials of
 // every element in the order 0 .. S-1, applies alpha, beta and the bias and rounds once. No
-// atomics: the result does not depend on scheduling.
+// atomics: the result does not depend on scheduling. The ranges need not be equal, so any K can be cut (in
+// equal ones on the 16-byte grid a K of 7221 could not: f16 17 x 152 x 7221 78 -> 35 us, 61 x 64 x 3966 35 -> 22, most of what is left moving the operands onto the 16-byte grid).
 struct SplitKPlan {
-  int splits;      // 1 = not worth it / not possible
-  int64_t kchunk;  // K / splits
+  int splits;       // 1 = not worth it
+  int range_slabs;  // K slabs per range; the last one has what is left
 };
 static SplitKPlan plan_splitk(int64_t batch, int64_t M, int64_t N, int64_t K) {
-  SplitKPlan r{1, K};
+  SplitKPlan r{1, 0};
   if (batch != 1) return r;
   const int bn = N <= 128 ? 128 : 256;
   const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn), slabs = (K + kBK - 1) / kBK;
@@ -764,11 +792,9 @@ static SplitKPlan plan_splitk(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int64_t s = kNumSMs / tiles;
   if (s > slabs / 4) s = slabs / 4;  // every range keeps at least four K slabs
   if (s > 32) s = 32;
-  for (; s >= 2; --s)
-    if (K % (8 * s) == 0) break;     // ranges start on the 16-byte grid of a K-major operand
   if (s < 2) return r;
-  r.splits = static_cast<int>(s);
-  r.kchunk = K / s;
+  r.range_slabs = static_cast<int>((slabs + s - 1) / s);
+  r.splits = static_cast<int>((slabs + r.range_slabs - 1) / r.range_slabs);
   return r;
 }
 
@@ -841,18 +867,17 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   if (pl.splits < 2) return B200_EINVAL;
   if (!scratch || scratch_bytes < gemm_tc_splitk_scratch_bytes(1, M, N, K)) return B200_ESCRATCH;
   float* part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~static_cast<uintptr_t>(255));
-  const int64_t S = pl.splits, Kc = pl.kchunk;
-  const int64_t sAb = Kc * sAk, sBb = Kc * sBk;  // range s of the contraction starts s * Kc further along K
-  const OperandLayout la = operand_layout(M, Kc, sAm, sAk, sAb, S, A);
-  const OperandLayout lb = operand_layout(N, Kc, sBn, sBk, sBb, S, B);
+  const int64_t S = pl.splits;
+  const OperandLayout la = operand_layout(M, K, sAm, sAk, 0, 1, A);
+  const OperandLayout lb = operand_layout(N, K, sBn, sBk, 0, 1, B);
   if (!la.ok || !lb.ok || !encode_fn()) return B200_EALIGN;
   const int bn = N <= 128 ? 128 : 256;
   alignas(64) CUtensorMap map_a, map_b;
-  if (!encode_operand(&map_a, A, dtype, la.mn_major, M, Kc, sAm, sAk, sAb, S, kBM)) return B200_EDRIVER;
-  if (!encode_operand(&map_b, B, dtype, lb.mn_major, N, Kc, sBn, sBk, sBb, S, bn)) return B200_EDRIVER;
+  if (!encode_operand(&map_a, A, dtype, la.mn_major, M, K, sAm, sAk, 0, 1, kBM)) return B200_EDRIVER;
+  if (!encode_operand(&map_b, B, dtype, lb.mn_major, N, K, sBn, sBk, 0, 1, bn)) return B200_EDRIVER;
   GemmTcParams p;
   p.tma_store = 0;
-  p.M = M; p.N = N; p.K = Kc; p.batch = S;
+  p.M = M; p.N = N; p.K = K; p.batch = S;
   p.sbm = 0; p.sbn = 0;
   p.alpha = 1.f;
   p.beta = 0.f;
@@ -862,17 +887,21 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   p.has_bias = 0;
   p.col_fastest = 1;
   p.split_slabs = 0;
-  p.range_slabs = 0;
+  p.range_slabs = pl.range_slabs;
   p.skip_if_set = nullptr;
   p.wait_limit_ns = kWaitLimitNs;
   p.withhold_first_slab = 0;
-  p.group_m = group_rows_for(Kc) / kBM;
+  p.group_m = group_rows_for(K) / kBM;
   const int64_t tiles = S * ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
   const int grid = static_cast<int>(tiles < kNumSMs ? tiles : kNumSMs);
   auto launch = [&](auto kernel) -> int { return launch_tc(kernel, false, grid, st, map_a, map_b, map_a, static_cast<const float*>(nullptr), part, p, status); };
   int rc;
-  if (dtype == B200_BF16) rc = bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float>);
-  else rc = bn == 128 ? launch(gemm_tcgen05_kernel<__half, 128, float>) : launch(gemm_tcgen05_kernel<__half, 256, float>);
+  auto launch_as = [&](auto as_rows) -> int {  // (rows of partial sums off the 16-byte grid: bf16 256 x 250 x 4096 27 -> 12 us)
+    constexpr bool kRows = decltype(as_rows)::value;
+    if (dtype == B200_BF16) return bn == 128 ? launch(gemm_tcgen05_kernel<__nv_bfloat16, 128, float, false, kRows>) : launch(gemm_tcgen05_kernel<__nv_bfloat16, 256, float, false, kRows>);
+    return bn == 128 ? launch(gemm_tcgen05_kernel<__half, 128, float, false, kRows>) : launch(gemm_tcgen05_kernel<__half, 256, float, false, kRows>);
+  };
+  rc = N >= 32 && N % 4 != 0 ? launch_as(std::true_type{}) : launch_as(std::false_type{});
   if (rc) return rc;
   const float al = static_cast<float>(alpha), be = static_cast<float>(beta);
   if (dtype == B200_BF16) launch_splitk_reduce<__nv_bfloat16>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st);

@@ -518,3 +518,41 @@ def test_fp32_products_cut_into_ranges_of_k(M, N, K):
     got = ops.mm_default(a, b)
     assert bool(torch.isinf(got[:, 7]).all()) and bool((torch.isfinite(got).sum(1) == N - 1).all())
     ops.check_device_status()
+
+
+def _within_rounding(got, a, b, extra=None):
+    """One rounding to the result's type (half a unit in the last of 8 or 11 places: 2^-8 of the value for bf16, 2^-11 for f16), and
+    in front of it K additions, each truncated at fp32 (2^-23 of the sum of magnitudes at most)."""
+    exact, mass = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    if extra is not None:
+        exact, mass = exact + extra.double(), mass + extra.double().abs()
+    half_ulp = 2.0**-8 if got.dtype == torch.bfloat16 else 2.0**-11
+    bound = exact.abs() * half_ulp * 1.01 + mass * (a.shape[-1] + 2) * 2.0**-23 + 2.0**-25  # (the last: subnormal f16)
+    assert bool(((got.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N", [129, 130, 132, 191, 250, 255, 257, 514, 770])
+def test_rows_of_c_between_two_words(dtype, N):
+    """16-bit results whose rows start anywhere: whole and partial chunks of 64 columns, row blocks cut short, batches (the
+    parity of a row's first element goes on through them), a bias vector on and off the 16-byte grid and a bias matrix."""
+    g = torch.Generator(device=DEV).manual_seed(31)
+    for batch, M, K in [(1, 33, 320), (1, 257, 320), (3, 130, 128), (2, 129, 520)]:
+        a, b = _rand((batch, M, K), dtype, g, K**-0.5), _rand((batch, N, K), dtype, g, 1.0).transpose(1, 2)
+        _within_rounding(ops.bmm_default(a, b), a, b)
+        row, col = _rand((N + 1,), dtype, g, 1.0), _rand((M, 1), dtype, g, 1.0)
+        for bias in (row[:N], row[1:], _rand((M, N), dtype, g, 1.0), col):
+            _within_rounding(ops.addmm_default(bias, a[0], b[0]), a[0], b[0], bias)
+    ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 152, 7221), (61, 64, 3966), (14, 888, 3342), (250, 250, 4096), (129, 255, 1537), (40, 129, 12345), (128, 1030, 2049)])
+def test_any_k_is_cut_into_ranges(M, N, K):
+    """Ranges of whole slabs, the last one shorter and its end off the slab grid; partial sums with rows off the 16-byte grid."""
+    g = torch.Generator(device=DEV).manual_seed(37)
+    for dtype in (torch.bfloat16, torch.float16):
+        a, w, bias = _rand((M, K), dtype, g, K**-0.5), _rand((N, K), dtype, g, 1.0), _rand((N,), dtype, g, 1.0)
+        _within_rounding(ops.addmm_default(bias, a, w.t()), a, w.t(), bias)
+        _within_rounding(ops.mm_default(a.t().contiguous().t(), w.t().contiguous()), a, w.t())
+        assert torch.equal(ops.mm_default(a, w.t()), ops.mm_default(a, w.t()))
+    ops.check_device_status()
