@@ -928,12 +928,16 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
 // kernel returns at once when the flag is up and the CUDA-core kernel, launched behind it
 // and gated the other way, computes that product in plain fp32.
 struct SplitArgs {
+  const float* x;
+  const float* end;              // behind the last element of x
+  __nv_bfloat16* out;
   int64_t batch, mn, k, kp;
   int64_t s_b, s_mn, s_k;        // source strides, elements
   int64_t o_b, o_row;            // output batch stride and row pitch, elements
   int mn_major;                  // output form
   uint32_t* any_flag;            // set when the operand holds an infinity or a NaN
 };
+__device__ __forceinline__ float4 ld_f4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
   if (!isfinite(x)) { a = __float2bfloat16_rn(x); b = c = __float2bfloat16_rn(0.f); return; }
   float x1 = __bfloat162float(__float2bfloat16_rn(x));
@@ -945,28 +949,58 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16&
   b = __float2bfloat16_rn(x2);
   c = __float2bfloat16_rn(r2);
 }
-__global__ void __launch_bounds__(256) split_f32_planes(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, SplitArgs A) {
-  // A thread produces 8 consecutive elements along the contiguous dimension of the output
-  // (k in the K-major form, mn in the MN-major form): two 16-byte loads when the source is
-  // contiguous and aligned there, three 16-byte stores.
+// Both operands in one launch: the first `blocks0` CTAs take the one, the others the other. A thread produces 8
+// consecutive elements along the contiguous dimension of the output (k in the K-major form, mn in the MN-major form) with
+// three 16-byte stores. Where the source is contiguous there it is read 16 bytes at a time: two loads, or, for
+// rows that start off the grid, three around the eight elements, which are then moved up by as many as
+// the row is off. (Element by element a warp's load touched 32 sectors: 1531 x 1027, both operands of
+// the product with 2050 x 1027, 17 us, FIG so.)
+__global__ void __launch_bounds__(256) split_f32_planes(const __grid_constant__ SplitArgs A0, const __grid_constant__ SplitArgs A1, unsigned blocks0) {
+  const bool second = blockIdx.x >= blocks0;
+  const SplitArgs& A = second ? A1 : A0;
+  const int64_t block = second ? blockIdx.x - blocks0 : blockIdx.x, nblocks = second ? gridDim.x - blocks0 : blocks0;
   const int64_t inner = A.mn_major ? A.mn : A.kp, outer = A.mn_major ? A.kp : A.mn;
   const int64_t groups = (inner + 7) / 8;  // kp is a multiple of 8; a ragged mn tail is a partial group
   const int64_t per_batch = groups * outer;
   const int64_t total = A.batch * per_batch;
   const int64_t s_in = A.mn_major ? A.s_mn : A.s_k, s_out = A.mn_major ? A.s_k : A.s_mn;  // source strides along inner / outer
   const int64_t lim_in = A.mn_major ? A.mn : A.k, lim_out = A.mn_major ? A.k : A.mn;      // where real data ends
-  const bool vec = s_in == 1 && s_out % 4 == 0 && A.s_b % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t b = i / per_batch, r = i - b * per_batch;
-    const int64_t o = r / groups, in0 = (r - o * groups) * 8;
+  for (int64_t i = block * 256 + threadIdx.x; i < total; i += nblocks * 256) {
+    int64_t b, o, g;
+    if (total <= 0x7fffffffLL) {
+      const uint32_t q = static_cast<uint32_t>(i) / static_cast<uint32_t>(groups), qb = A.batch == 1 ? 0u : q / static_cast<uint32_t>(outer);
+      g = static_cast<uint32_t>(i) - q * static_cast<uint32_t>(groups);
+      o = q - qb * static_cast<uint32_t>(outer);
+      b = qb;
+    } else {
+      b = i / per_batch;
+      const int64_t r = i - b * per_batch;
+      o = r / groups;
+      g = r - o * groups;
+    }
+    const int64_t in0 = g * 8;
     float v[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = 0.f;
     if (o < lim_out) {
-      const float* src = x + b * A.s_b + o * s_out + in0 * s_in;
-      if (vec && in0 + 8 <= lim_in) {
-        const float4 lo = __ldcs(reinterpret_cast<const float4*>(src)), hi = __ldcs(reinterpret_cast<const float4*>(src) + 1);
-        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+      const float* src = A.x + b * A.s_b + o * s_out + in0 * s_in;
+      const int off = static_cast<int>(reinterpret_cast<uintptr_t>(src) >> 2) & 3;
+      const float* p = src - off;
+      if (s_in == 1 && in0 + 8 <= lim_in && p >= A.x && p + 12 <= A.end) {
+        const float4 lo = ld_f4(p), mid = ld_f4(p + 4);
+        float4 hi = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (off) hi = ld_f4(p + 8);
+        float w[11] = {lo.x, lo.y, lo.z, lo.w, mid.x, mid.y, mid.z, mid.w, hi.x, hi.y, hi.z};
+        if (off & 1) {
+#pragma unroll
+          for (int e = 0; e < 10; ++e) w[e] = w[e + 1];
+        }
+        if (off & 2) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) w[e] = w[e + 2];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = w[e];
       } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e)
@@ -982,16 +1016,12 @@ __global__ void __launch_bounds__(256) split_f32_planes(const float* __restrict_
     }
     if (bad) *A.any_flag = 1u;
     // o_row is a multiple of 8 and so are in0 and kp: every store below is 16-byte aligned
-    __nv_bfloat16* ob = out + b * A.o_b;
-    if (A.mn_major) {
-      *reinterpret_cast<uint4*>(ob + o * A.o_row + in0) = *reinterpret_cast<const uint4*>(q0);
-      *reinterpret_cast<uint4*>(ob + (A.kp + o) * A.o_row + in0) = *reinterpret_cast<const uint4*>(q1);
-      *reinterpret_cast<uint4*>(ob + (2 * A.kp + o) * A.o_row + in0) = *reinterpret_cast<const uint4*>(q2);
-    } else {
-      *reinterpret_cast<uint4*>(ob + o * A.o_row + in0) = *reinterpret_cast<const uint4*>(q0);
-      *reinterpret_cast<uint4*>(ob + o * A.o_row + A.kp + in0) = *reinterpret_cast<const uint4*>(q1);
-      *reinterpret_cast<uint4*>(ob + o * A.o_row + 2 * A.kp + in0) = *reinterpret_cast<const uint4*>(q2);
-    }
+    __nv_bfloat16* ob = A.out + b * A.o_b;
+    const int64_t plane = A.mn_major ? A.kp * A.o_row : A.kp;
+    __nv_bfloat16* to = ob + o * A.o_row + in0;
+    *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(q0);
+    *reinterpret_cast<uint4*>(to + plane) = *reinterpret_cast<const uint4*>(q1);
+    *reinterpret_cast<uint4*>(to + 2 * plane) = *reinterpret_cast<const uint4*>(q2);
   }
 }
 
@@ -1046,11 +1076,13 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   const int64_t a_row = a_mn ? round_up(M, 8) : 3 * kp, a_rows = a_mn ? 3 * kp : M;
   const int64_t b_row = b_mn ? round_up(N, 8) : 3 * kp, b_rows = b_mn ? 3 * kp : N;
   __nv_bfloat16* pb = pa + batch * a_rows * a_row;  // a multiple of 8 elements: stays 16-byte aligned
-  const SplitArgs sa{batch, M, K, kp, sAb, sAm, sAk, a_rows * a_row, a_row, a_mn ? 1 : 0, any_flag};
-  const SplitArgs sb{batch, N, K, kp, sBb, sBn, sBk, b_rows * b_row, b_row, b_mn ? 1 : 0, any_flag};
+  const float* fa = static_cast<const float*>(A);
+  const float* fb = static_cast<const float*>(B);
+  const SplitArgs sa{fa, fa + (batch - 1) * sAb + (M - 1) * sAm + (K - 1) * sAk + 1, pa, batch, M, K, kp, sAb, sAm, sAk, a_rows * a_row, a_row, a_mn ? 1 : 0, any_flag};
+  const SplitArgs sb{fb, fb + (batch - 1) * sBb + (N - 1) * sBn + (K - 1) * sBk + 1, pb, batch, N, K, kp, sBb, sBn, sBk, b_rows * b_row, b_row, b_mn ? 1 : 0, any_flag};
   auto blocks = [](int64_t n) { const int64_t b = (n + 255) / 256; return static_cast<int>(b < 1 ? 1 : (b > kNumSMs * 32LL ? kNumSMs * 32LL : b)); };
-  split_f32_planes<<<blocks(batch * a_rows * a_row / 24), 256, 0, st>>>(static_cast<const float*>(A), pa, sa);
-  split_f32_planes<<<blocks(batch * b_rows * b_row / 24), 256, 0, st>>>(static_cast<const float*>(B), pb, sb);
+  const int blocks_a = blocks(batch * a_rows * a_row / 24), blocks_b = blocks(batch * b_rows * b_row / 24);
+  split_f32_planes<<<blocks_a + blocks_b, 256, 0, st>>>(sa, sb, static_cast<unsigned>(blocks_a));
   const cudaError_t se = cudaGetLastError();
   if (se != cudaSuccess) { set_last_cuda_error(se); return B200_ELAUNCH; }
 
@@ -1104,7 +1136,7 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   // the same product on the CUDA cores, run only when the split met an infinity or a NaN
   const int rs = gemm_simt_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, B200_F32, st, any_flag);
   if (rs) return rs;
-  return check_launch(ranges > 1 ? 4 : 3);
+  return check_launch(ranges > 1 ? 3 : 2);
 }
 
 }  // namespace b200
