@@ -62,7 +62,9 @@ constexpr int kGroupM = 16;                             // row-blocks per raster
 constexpr uint64_t kWaitLimitNs = 2000000000ull;        // every mbarrier wait gives up after 2 s
 constexpr int kEpiWarps = 8;
 constexpr int kEpiStageBytes = 32 * 128;                // per epilogue warp: 32 rows x 64 16-bit outputs, TMA-store staging
-constexpr size_t kGemmSmem = static_cast<size_t>(4) * (kABytes + 256 * kBK * 2) + kEpiWarps * kEpiStageBytes + 1024 /*align*/ + 256 /*barriers*/;  // same for both tile shapes (6 x 32 KB = 4 x 48 KB)
+constexpr int kRingBytes = 4 * (kABytes + 256 * kBK * 2);  // 4 x 48 KB = 6 x 32 KB
+constexpr int kMaxStages = 8;                             // of 24 KB
+constexpr size_t kGemmSmem = static_cast<size_t>(kRingBytes) + kEpiWarps * kEpiStageBytes + 1024 /*align*/ + 256 /*barriers*/;  // same for both tile shapes (6 x 32 KB = 4 x 48 KB)
 
 // ------------------------------------------------------------------ PTX wrappers (mbarrier and timer helpers: tma_common.cuh)
 // The same load issued by a CTA of a pair: the destination is this CTA's shared memory, the
@@ -89,6 +91,11 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
 }
 // pair forms: the barrier address is a shared::cluster address (own or peer CTA)
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster) { asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster) : "memory"); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   const uint32_t z = 0u;  // no output lane is disabled
   asm volatile(
@@ -137,6 +144,7 @@ struct GemmTcParams {
   uint64_t wait_limit_ns;       // every mbarrier wait gives up after this long (kWaitLimitNs in ordinary calls)
   int withhold_first_slab;      // wait probe only: the producer never loads the first K slab of a CTA's first tile
   int group_m;                  // row-blocks per rasterisation group (see tile_coords)
+  int bn;                       // pairs: columns of a tile, 256, 192 or 128 (see pair_tile_columns)
 };
 
 // Tile t of one batch entry -> (row-block, column-block): column-block fastest, or groups of
@@ -161,26 +169,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c, const TO* __restrict__ bias, TO* __restrict__ C, GemmTcParams p,
                     uint32_t* __restrict__ status) {
   using Cfg = TileCfg<kBN, kPair>;
-  constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes, kAccs = Cfg::kAccs, kBRows = Cfg::kBRows;
+  constexpr int kAccs = Cfg::kAccs;
   constexpr int kTileM = kPair ? 2 * kBM : kBM;  // rows of C one tile covers (both CTAs of a pair)
   static_assert(!kPair || kBN == 256, "CTA pairs work on 256 x 256 tiles");
   if (p.skip_if_set && *p.skip_if_set != 0u) return;  // every thread of every CTA reads the same word: a uniform exit before any barrier or TMEM set-up
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern repeats every 8 rows x 128 bytes
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  unsigned char* epi_stage = smem + kStages * kStageBytes;  // kEpiWarps x 4 KB, each 1024-byte aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes + kEpiWarps * kEpiStageBytes);
-  // barrier slots: [0,S) full, [S,2S) empty, [2S,2S+2) tmem_full, [2S+2,2S+4) tmem_empty
-  uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 2 * kAccs);
+  unsigned char* epi_stage = smem + kRingBytes;  // kEpiWarps x 4 KB, each 1024-byte aligned
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kRingBytes + kEpiWarps * kEpiStageBytes);
+  // barrier slots, S = kMaxStages: [0,S) full, [S,2S) empty, then one tmem_full and one tmem_empty per accumulator
+  uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 2 * kAccs);
   volatile uint32_t* abort_flag = tmem_base_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_u32(bars);
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
-  auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kStages + a); };
-  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kStages + kAccs + a); };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
+  auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + a); };
+  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + kAccs + a); };
+  // a pair's stages are as large as its tile is wide, and there are as many as fit
+  const int bn = kPair ? p.bn : kBN;
+  const int b_rows = kPair ? bn / 2 : Cfg::kBRows;  // of the B slab, in this CTA's shared memory: one box, or as many boxes of 64 as cover them
+  const uint32_t stage_bytes = kPair ? static_cast<uint32_t>(kABytes + (p.b_mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * kBK * 2) : static_cast<uint32_t>(Cfg::kStageBytes);
+  const int stages = kPair ? kRingBytes / static_cast<int>(stage_bytes) : Cfg::kStages;
 
   // pair: rank of this CTA in its 2-CTA cluster (0 = the CTA that issues the MMAs), and the
   // shared::cluster addresses of the even CTA's barriers that both CTAs signal
@@ -192,7 +205,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (p.tma_store) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_c)) : "memory");
   }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(full_bar(s), 1);   // pair: only the even CTA's is used (its producer arms it for both CTAs' bytes)
       mbar_init(empty_bar(s), 1);  // one tcgen05.commit per use (pair: the even CTA commits to both CTAs')
     }
@@ -218,7 +231,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
-  const int64_t mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + kBN - 1) / kBN;
+  const int64_t mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + bn - 1) / bn;
   const int64_t tiles = p.batch * mt * nt;
   const int64_t tile_first = kPair ? (blockIdx.x >> 1) : blockIdx.x, tile_step = kPair ? (gridDim.x >> 1) : gridDim.x;
   // Split operands: plane q of an operand occupies K coordinates [q * Kp, q * Kp + K) of its
@@ -243,26 +256,26 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int64_t b = t / (mt * nt), rem = t - b * (mt * nt);
         int mb, nb;
         tile_coords(rem, mt, nt, mb, nb, p.col_fastest, p.group_m);
-        // pair: this CTA's 128 rows of A and its half of the B slab's 256 rows
-        const int m0 = mb * kTileM + static_cast<int>(cta_rank) * kBM, n0 = nb * kBN + static_cast<int>(cta_rank) * (kPair ? kBRows : 0);
+        // pair: this CTA's 128 rows of A and its half of the B slab's rows
+        const int m0 = mb * kTileM + static_cast<int>(cta_rank) * kBM, n0 = nb * bn + static_cast<int>(cta_rank) * (kPair ? b_rows : 0);
         const int tile_slabs = ranged ? slabs_of(b) : k_slabs, slab0 = ranged ? static_cast<int>(b) * p.range_slabs : 0;
         const int num_kb = planes * tile_slabs;
         const int entry = ranged ? 0 : static_cast<int>(b);  // the planes are one batch entry whatever range is walked
         int slab = 0, pair4 = 0;  // split operands: slab of the range, plane pair (times 4)
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
-          const uint32_t a_dst = smem_base + stage * kStageBytes, b_dst = a_dst + kABytes;
+          const uint32_t a_dst = smem_base + stage * stage_bytes, b_dst = a_dst + kABytes;
           if (!kPair && p.withhold_first_slab && t == blockIdx.x && kb == 0) {
             // wait probe: this stage is never armed and never filled, so the MMA warp's wait on
             // it must run into its limit; the producer carries on until it needs the stage back
-            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            if (++stage == stages) { stage = 0; phase ^= 1u; }
             continue;
           }
           // pair: every copy of both CTAs completes on the even CTA's barrier, which its
           // producer arms for the bytes of both
           const uint32_t fbar = kPair ? map_to_cta(full_bar(stage), 0u) : full_bar(stage);
-          if (!kPair) mbar_expect_tx(full_bar(stage), kStageBytes);
-          else if (cta_rank == 0u) mbar_expect_tx(full_bar(stage), 2 * kStageBytes);
+          if (!kPair) mbar_expect_tx(full_bar(stage), stage_bytes);
+          else if (cta_rank == 0u) mbar_expect_tx(full_bar(stage), 2 * stage_bytes);
           auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2) {
             if (kPair) tma_load_3d_pair(dst, map, fbar, c0, c1, c2);
             else tma_load_3d(dst, map, fbar, c0, c1, c2);
@@ -284,20 +297,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int c = 0; c < kBM / 64; ++c) load(a_dst + c * 8192, &map_a, m0 + c * 64, ka, entry);  // box [64 k][64 m]
           }
           if (!p.b_mn_major) {
-            load(b_dst, &map_b, kbb, n0, entry);  // box [kBRows rows][64 k]
+            load(b_dst, &map_b, kbb, n0, entry);  // box [b_rows rows][64 k]
           } else {
 #pragma unroll
-            for (int c = 0; c < kBRows / 64; ++c) load(b_dst + c * 8192, &map_b, n0 + c * 64, kbb, entry);  // box [64 k][64 n]
+            for (int c = 0; c < Cfg::kBRows / 64; ++c)
+              if (!kPair || c * 64 < b_rows) load(b_dst + c * 8192, &map_b, n0 + c * 64, kbb, entry);  // box [64 k][64 n]
           }
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
       if (kPair && ok) {
         // tail: the even CTA's commits arrive on THIS CTA's empty barriers from afar; wait for
         // the ones still outstanding so that none lands after this CTA's shared memory is gone
-        for (int i = 0; i < kStages && ok; ++i) {
+        for (int i = 0; i < stages && ok; ++i) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.wait_limit_ns)) ok = false;
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) {
@@ -308,53 +322,68 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncwarp();  // lanes 1..31 rejoin lane 0 before the CTA-wide barrier below
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && cta_rank == 0u) {  // pair: the even CTA issues for both
+    if (cta_rank == 0u) {  // pair: the even CTA issues for both
       // instruction descriptor: fp32 accumulate, A/B format, majors, N >> 3, M >> 4
       const uint32_t fmt = p.is_bf16 ? 1u : 0u;
       const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(p.a_mn_major) << 15) | (static_cast<uint32_t>(p.b_mn_major) << 16) |
-                             (static_cast<uint32_t>(kBN >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
+                             (static_cast<uint32_t>(bn >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
       // per-UMMA (K = 16) advance of the start address and the two byte offsets per layout
       const uint32_t a_adv = p.a_mn_major ? 2048u : 32u, b_adv = p.b_mn_major ? 2048u : 32u;
       const uint32_t a_lbo = p.a_mn_major ? 8192u : 16u, b_lbo = p.b_mn_major ? 8192u : 16u;
+      const uint32_t empty0 = kPair ? map_to_cta(empty_bar(0), 0u) : 0u, empty1 = kPair ? map_to_cta(empty_bar(0), 1u) : 0u;
+      // The whole warp walks the slabs and one elected lane issues: descriptors and addresses are then the same in
+      // every lane, and the compiler works them out once per warp. With a single lane in the loop the issue took longer
+      // than the tensor cores need for a tile of 192 or 128 columns (4096^3 in tiles of 128: 132 -> 114 us).
+      auto warp_wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.wait_limit_ns)) != 0; };
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int64_t t = tile_first; t < tiles && ok; t += tile_step) {
-        if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+        if (!warp_wait(tempty_bar(acc), acc_phase ^ 1u)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kBN);
         const int num_kb = ranged ? planes * slabs_of(t / (mt * nt)) : num_kb_all;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+          if (!warp_wait(full_bar(stage), phase)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_base + stage * kStageBytes, b_addr = a_addr + kABytes;
+          const uint32_t a_addr = smem_base + stage * stage_bytes, b_addr = a_addr + kABytes;
+          uint64_t da[kBK / 16], db[kBK / 16];
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = smem_desc(a_addr + k * a_adv, a_lbo, 1024u);
-            const uint64_t db = smem_desc(b_addr + k * b_adv, b_lbo, 1024u);
-            if (kPair) tc_mma_f16_pair(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-            else tc_mma_f16(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+            da[k] = smem_desc(a_addr + k * a_adv, a_lbo, 1024u);
+            db[k] = smem_desc(b_addr + k * b_adv, b_lbo, 1024u);
           }
-          // the stage is free once these MMAs have read it (pair: in both CTAs)
-          if (kPair) {
-            tc_commit_pair(map_to_cta(empty_bar(stage), 0u));
-            tc_commit_pair(map_to_cta(empty_bar(stage), 1u));
-          } else {
-            tc_commit(empty_bar(stage));
+          const uint32_t e0 = kPair ? empty0 + 8u * stage : empty_bar(stage), e1 = empty1 + 8u * stage;
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) {
+              if (kPair) tc_mma_f16_pair(d_tmem, da[k], db[k], idesc, (kb | k) != 0 ? 1u : 0u);
+              else tc_mma_f16(d_tmem, da[k], db[k], idesc, (kb | k) != 0 ? 1u : 0u);
+            }
+            if (kPair) {
+              tc_commit_pair(e0);
+              tc_commit_pair(e1);
+            } else {
+              tc_commit(e0);
+            }
           }
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          __syncwarp();
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         // accumulator complete (pair: each CTA's epilogue waits on its own barrier)
-        if (kPair) {
-          tc_commit_pair(map_to_cta(tfull_bar(acc), 0u));
-          tc_commit_pair(map_to_cta(tfull_bar(acc), 1u));
-        } else {
-          tc_commit(tfull_bar(acc));
+        if (elect_one()) {
+          if (kPair) {
+            tc_commit_pair(map_to_cta(tfull_bar(acc), 0u));
+            tc_commit_pair(map_to_cta(tfull_bar(acc), 1u));
+          } else {
+            tc_commit(tfull_bar(acc));
+          }
         }
+        __syncwarp();
         if (++acc == kAccs) { acc = 0; acc_phase ^= 1u; }
       }
-      if (!ok) {
+      if (!ok && lane == 0) {
         *abort_flag = 1;
         if (status) atomicOr(status, B200_DEV_WAIT_TIMEOUT);
       }
@@ -374,7 +403,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int64_t b = t / (mt * nt), rem = t - b * (mt * nt);
       int mb, nb_blk;
       tile_coords(rem, mt, nt, mb, nb_blk, p.col_fastest, p.group_m);
-      const int64_t m0 = static_cast<int64_t>(mb) * kTileM + static_cast<int64_t>(cta_rank) * kBM, n0 = static_cast<int64_t>(nb_blk) * kBN + chalf * (kBN / 2);
+      const int64_t m0 = static_cast<int64_t>(mb) * kTileM + static_cast<int64_t>(cta_rank) * kBM, n0 = static_cast<int64_t>(nb_blk) * bn + chalf * (kBN / 2);
+      const int64_t tile_end = static_cast<int64_t>(nb_blk + 1) * bn, n_end = tile_end < p.N ? tile_end : p.N;  // (a chunk of 64 columns lies in the tile or behind it)
       int got = 0;
       if (lane == 0) got = mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.wait_limit_ns) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
@@ -460,7 +490,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           park(rc, mine);
           fence_async_smem();
           __syncwarp();
-          if (lane == 0 && nb < p.N && m0 + q * 32 < p.M) {
+          if (lane == 0 && nb < n_end && m0 + q * 32 < p.M) {
             tma_store_3d(&map_c, smem_u32(mine), static_cast<int>(nb), static_cast<int>(m0 + q * 32), static_cast<int>(b));
             tma_store_commit();
           }
@@ -476,7 +506,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           __syncwarp();  // the previous chunk has been read out of the buffer
           park(rc, mine);
           __syncwarp();
-          const int64_t left = p.N - nb, mr0 = m0 + q * 32;
+          const int64_t left = n_end - nb, mr0 = m0 + q * 32;
           const int ncols = left < 64 ? static_cast<int>(left) : 64;  // <= 0: the chunk lies right of C
           const int nrows = p.M - mr0 < 32 ? static_cast<int>(p.M - mr0) : 32;
           if (ncols > 0) {
@@ -501,7 +531,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         } else if constexpr (!kRows) {
           // fp32 C, a lane to a row: 16 bytes at a time where the rows are on the grid. (Going through the
           // buffer as below costs more than the wider stores give back: 8192 x 256 x 2048 91 us against 72.)
-          if (m < p.M && nb < p.N) {
+          if (m < p.M && nb < n_end) {
             TO* crow = C + (b * p.M + m) * p.N;
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
@@ -553,7 +583,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               for (int u = 0; u < 8; ++u) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[u]) : "r"(mine_a + (r0 + u) * 128 + (((lane >> 2) ^ u) << 4)) : "memory");
 #pragma unroll
               for (int u = 0; u < 8; ++u, c += p.N) {
-                if (n < p.N && r0 + u < nrows) {
+                if (n < n_end && r0 + u < nrows) {
                   if (p.has_bias && !row_bias) v[u] = fmaf(p.beta, to_f32(bias[(mr0 + r0 + u) * p.sbm + n * p.sbn]), v[u]);
                   *c = from_f32<TO>(row_bias ? fmaf(p.beta, same, v[u]) : v[u]);
                 }
@@ -690,6 +720,30 @@ static bool pair_launch_ok() {
   return on;
 }
 
+// Columns of a pair's tile: 256, or 192 or 128 where tiles of 256 are few rounds and leave pairs without one in the last. A
+// round of narrower tiles takes 0.83 or 0.69 of the time (with B along N, whose boxes are 64 columns wide, 192 columns
+// take as long as 256, and 128 0.73):
+// their rows of A are loaded and their slabs handed on all the same (4096^3 in tiles of 256, 192 and 128: 4, 5
+// and 7 rounds in 94, 97 and 114 us). Another width is taken where it saves a twentieth: bf16 2537 x 920 x 3712 24.7 -> 20.7
+// us, 1024^3 12.2 -> 10.5; fp32 1531 x 2050 x 1027 53.6 -> 48.7.
+static double tile_time(int bn, bool b_mn) { return bn == 256 ? 1.0 : bn == 192 ? (b_mn ? 1.0 : 0.83) : (b_mn ? 0.73 : 0.69); }
+static int64_t pair_tiles(int64_t M, int64_t N, int bn) { return ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + bn - 1) / bn); }
+static double pair_rounds(int64_t entries, int64_t M, int64_t N, int bn, bool b_mn) {
+  const int64_t slots = kNumSMs / 2;
+  return static_cast<double>((entries * pair_tiles(M, N, bn) + slots - 1) / slots) * tile_time(bn, b_mn);
+}
+static int pair_tile_columns(int64_t batch, int64_t M, int64_t N, bool b_mn) {
+  int best = 256;
+  double least = pair_rounds(batch, M, N, 256, b_mn);
+  if (least > 4.0) return best;
+  least *= 0.95;
+  for (int bn : {192, 128}) {
+    const double t = pair_rounds(batch, M, N, bn, b_mn);
+    if (t < least) { least = t; best = bn; }
+  }
+  return best;
+}
+
 int gemm_tc_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb,
                      int64_t sBk, int64_t sBn, int64_t sbm, int64_t sbn, double alpha, double beta, int dtype, uint32_t* status, cudaStream_t st, uint64_t wait_probe_limit_ns,
                      bool allow_pair) {
@@ -703,7 +757,9 @@ int gemm_tc_dispatch(const void* A, const void* B, const void* bias, void* C, in
   // (with four K slabs or fewer the kernel is bound by writing C and the pair is slower:
   // bmm 32 x 2048 x 128 x 2048 0.087 ms against 0.061 ms)
   const bool pair = allow_pair && M > kBM && N > 128 && (K + kBK - 1) / kBK > 4 && wait_probe_limit_ns == 0 && pair_launch_ok();
-  const int bn_box = (N <= 128 || pair) ? 128 : 256;  // rows of the B box: must match the tile shape chosen below
+  const bool narrow = N <= 128;
+  const int bn = pair ? pair_tile_columns(batch, M, N, lb.mn_major) : narrow ? 128 : 256;
+  const int bn_box = pair ? bn / 2 : bn;  // rows of the B box: a CTA of a pair loads half of them
   if (!encode_operand(&map_b, B, dtype, lb.mn_major, N, K, sBn, sBk, sBb, batch, bn_box)) return B200_EDRIVER;
   alignas(64) CUtensorMap map_c;
   const bool tma_store = (N % 8 == 0) && aligned16(C);
@@ -738,11 +794,10 @@ int gemm_tc_dispatch(const void* A, const void* B, const void* bias, void* C, in
   p.wait_limit_ns = wait_probe_limit_ns ? wait_probe_limit_ns : kWaitLimitNs;
   p.withhold_first_slab = wait_probe_limit_ns ? 1 : 0;
   p.group_m = group_rows_for(K) / (pair ? 2 * kBM : kBM);
+  p.bn = bn;
   // a narrow C takes the 128-wide tile. (Write-bound shapes with few K slabs were measured
   // slower on it: 256-byte row segments instead of 512-byte ones cost more in DRAM than the
   // deeper pipeline gains -- bmm 32x2048x128x2048: 0.162 ms vs 0.116 ms.)
-  const bool narrow = N <= 128;
-  const int bn = narrow ? 128 : 256;
   const int tile_m = pair ? 2 * kBM : kBM;
   const int64_t tiles = batch * ((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn);
   const int64_t slots = pair ? kNumSMs / 2 : kNumSMs;  // persistent: one CTA (or CTA pair) per SM (or TPC)
@@ -892,6 +947,7 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   p.wait_limit_ns = kWaitLimitNs;
   p.withhold_first_slab = 0;
   p.group_m = group_rows_for(K) / kBM;
+  p.bn = bn;
   const int64_t tiles = S * ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
   const int grid = static_cast<int>(tiles < kNumSMs ? tiles : kNumSMs);
   auto launch = [&](auto kernel) -> int { return launch_tc(kernel, false, grid, st, map_a, map_b, map_a, static_cast<const float*>(nullptr), part, p, status); };
@@ -953,8 +1009,8 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16&
 // consecutive elements along the contiguous dimension of the output (k in the K-major form, mn in the MN-major form) with
 // three 16-byte stores. Where the source is contiguous there it is read 16 bytes at a time: two loads, or, for
 // rows that start off the grid, three around the eight elements, which are then moved up by as many as
-// the row is off. (Element by element a warp's load touched 32 sectors: 1531 x 1027, both operands of
-// the product with 2050 x 1027, 17 us, FIG so.)
+// the row is off. (Element by element a warp's load touched 32 sectors: 1531 x 1027 and 2050 x 1027
+// together 12 -> 8 us.)
 __global__ void __launch_bounds__(256) split_f32_planes(const __grid_constant__ SplitArgs A0, const __grid_constant__ SplitArgs A1, unsigned blocks0) {
   const bool second = blockIdx.x >= blocks0;
   const SplitArgs& A = second ? A1 : A0;
@@ -1027,30 +1083,35 @@ __global__ void __launch_bounds__(256) split_f32_planes(const __grid_constant__ 
 
 static inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
-// Ranges of K for a product with fewer tiles than CTA pairs. What the product takes is the rounds of
-// tiles a pair walks times the slabs of a range (a slab, six plane pairs, takes about
-// 2.8 us), and writing and adding up the ranges' fp32 sums, 8 bytes per range and element of C at
+// Width of the tiles, and ranges of K for a product with fewer tiles than CTA pairs. What the product takes is the rounds of
+// tiles a pair walks times the time of a tile times the slabs of a range (a slab, six plane pairs of 256 columns, takes about
+// 2.4 us), and writing and adding up the ranges' fp32 sums, 8 bytes per range and element of C at
 // about 5 TB/s; the cut that makes the sum least is taken where it saves an eighth or more. fp32
 // 1531 x 1027 x 2050 (30 tiles on 74 pairs) 99 -> 66 us, 2050 x 1027 x 1531 (45 tiles) 81 -> 74 us.
 // Shorter chains of truncating additions make the result more exact, not less.
-static int plan_f32_ranges(int64_t batch, int64_t M, int64_t N, int64_t K) {
-  if (batch != 1 || M <= kBM || N <= 128 || !pair_launch_ok()) return 1;
-  const int64_t tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + 255) / 256), slots = kNumSMs / 2, slabs = (K + kBK - 1) / kBK;
-  if (tiles >= slots) return 1;
+struct F32Plan {
+  int ranges, bn;
+};
+static F32Plan plan_f32(int64_t batch, int64_t M, int64_t N, int64_t K, bool b_mn) {
+  if (M <= kBM || N <= 128 || !pair_launch_ok()) return F32Plan{1, N <= 128 ? 128 : 256};
+  const int64_t slabs = (K + kBK - 1) / kBK;
+  F32Plan best{1, pair_tile_columns(batch, M, N, b_mn)};
+  if (batch != 1 || pair_tiles(M, N, 256) >= kNumSMs / 2) return best;
   const double sums = static_cast<double>(M) * static_cast<double>(N) * 8 / 14e6;  // slabs' worth of time per range
-  double best = static_cast<double>(slabs);
-  int64_t ranges = 1;
-  for (int64_t s = 2; s <= 8 && slabs / s >= 4; ++s) {
-    const int64_t per = (slabs + s - 1) / s, n = (slabs + per - 1) / per;
-    const double cost = static_cast<double>((tiles * n + slots - 1) / slots * per) + sums * static_cast<double>(n);
-    if (cost < best) { best = cost; ranges = n; }
+  double least = pair_rounds(1, M, N, best.bn, b_mn) * static_cast<double>(slabs) * 0.875;
+  for (int bn : {256, 192, 128}) {
+    for (int64_t s = 2; s <= 8 && slabs / s >= 4; ++s) {
+      const int64_t per = (slabs + s - 1) / s, n = (slabs + per - 1) / per;
+      const double cost = pair_rounds(n, M, N, bn, b_mn) * static_cast<double>(per) + sums * static_cast<double>(n);
+      if (cost < least) { least = cost; best = F32Plan{static_cast<int>(n), bn}; }
+    }
   }
-  return best <= 0.875 * static_cast<double>(slabs) ? static_cast<int>(ranges) : 1;
+  return best;
 }
 
 int64_t gemm_f32_split_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   const int64_t kp = round_up(K, kBK);
-  const int ranges = plan_f32_ranges(batch, M, N, K);
+  const int along_k = plan_f32(batch, M, N, K, false).ranges, along_n = plan_f32(batch, M, N, K, true).ranges, ranges = along_k > along_n ? along_k : along_n;
   return batch * 3 * kp * (round_up(M, 8) + round_up(N, 8)) * 2 + 256 + 512 + (ranges > 1 ? ranges * M * N * 4 : 0);
 }
 
@@ -1088,10 +1149,11 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
 
   // the planes as [rows, 3 Kp] (K-major) or [3 Kp, rows] (MN-major) bf16 operands
   alignas(64) CUtensorMap map_a, map_b;
-  const int bn = N <= 128 ? 128 : 256;
   const bool pair = M > kBM && N > 128 && pair_launch_ok();  // the contraction is six planes deep: never write-bound
+  const F32Plan plan = plan_f32(batch, M, N, K, b_mn);
+  const int bn = plan.bn;
   if (!encode_operand(&map_a, pa, B200_BF16, a_mn, M, 3 * kp, a_mn ? 1 : a_row, a_mn ? a_row : 1, a_rows * a_row, batch, kBM)) return B200_EDRIVER;
-  if (!encode_operand(&map_b, pb, B200_BF16, b_mn, N, 3 * kp, b_mn ? 1 : b_row, b_mn ? b_row : 1, b_rows * b_row, batch, pair ? 128 : bn)) return B200_EDRIVER;
+  if (!encode_operand(&map_b, pb, B200_BF16, b_mn, N, 3 * kp, b_mn ? 1 : b_row, b_mn ? b_row : 1, b_rows * b_row, batch, pair ? bn / 2 : bn)) return B200_EDRIVER;
   GemmTcParams p;
   p.tma_store = 0;
   p.M = M; p.N = N; p.K = K; p.batch = batch;
@@ -1104,7 +1166,7 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   p.has_bias = (bias != nullptr && p.beta != 0.f) ? 1 : 0;
   p.split_slabs = static_cast<int>(kp / kBK);
   // fp32 partial products [ranges][M][N] behind the planes, added in the order of the ranges
-  const int ranges = plan_f32_ranges(batch, M, N, K);
+  const int ranges = plan.ranges;
   float* part = reinterpret_cast<float*>(pb + batch * b_rows * b_row);
   p.range_slabs = ranges > 1 ? (p.split_slabs + ranges - 1) / ranges : 0;
   if (ranges > 1) {
@@ -1117,6 +1179,7 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   p.withhold_first_slab = 0;
   p.col_fastest = 6 * p.split_slabs <= 4 ? 1 : 0;
   p.group_m = group_rows_for(3 * kp) / (pair ? 2 * kBM : kBM);
+  p.bn = bn;
   const int tile_m = pair ? 2 * kBM : kBM;
   const int64_t tiles = p.batch * ((M + tile_m - 1) / tile_m) * ((N + bn - 1) / bn);
   const int64_t slots = pair ? kNumSMs / 2 : kNumSMs;

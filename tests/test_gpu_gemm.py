@@ -556,3 +556,18 @@ def test_any_k_is_cut_into_ranges(M, N, K):
         _within_rounding(ops.mm_default(a.t().contiguous().t(), w.t().contiguous()), a, w.t())
         assert torch.equal(ops.mm_default(a, w.t()), ops.mm_default(a, w.t()))
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 129, 320), (1280, 1800, 640), (513, 385, 384), (1300, 960, 330), (2537, 920, 512), (300, 6700, 328), (4100, 193, 328)])
+def test_pair_tiles_of_every_width(M, N, K):
+    """Tiles of 256, 192 or 128 columns, whichever makes fewest rounds: the last one cut short in each of its chunks of 64
+    columns, B along K (any width) and along N, 16-bit and fp32 results."""
+    g = torch.Generator(device=DEV).manual_seed(41)
+    for dtype in (torch.bfloat16, torch.float16):
+        a, w, bias = _rand((M, K), dtype, g, K**-0.5), _rand((N, K), dtype, g, 1.0), _rand((N,), dtype, g, 1.0)
+        _within_rounding(ops.mm_default(a, w.t()), a, w.t())
+        _within_rounding(ops.addmm_default(bias, a, w.t().contiguous()), a, w.t(), bias)
+    a, w = torch.randn((M, K), generator=g, device=DEV) * K**-0.5, torch.randn((N, K), generator=g, device=DEV)
+    _check32(ops.mm_default(a, w.t()), a, w.t())
+    _check32(ops.mm_default(a, w.t().contiguous()), a, w.t())
+    ops.check_device_status()
