@@ -74,6 +74,17 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
                "r"(c1), "r"(c2)
                : "memory");
 }
+// 4-D forms: the 64-wide blocks of an MN-major operand in one copy
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(c0),
+               "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
+               "r"(c3)
+               : "memory");
+}
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) { return map_to_cta_addr(addr, rank); }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory"); }
 __device__ __forceinline__ void cluster_sync_all() { cluster_barrier(); }
@@ -133,7 +144,7 @@ struct GemmTcParams {
   int64_t M, N, K, batch;
   int64_t sbm, sbn;  // bias strides in elements (0 = broadcast)
   float alpha, beta;
-  int a_mn_major, b_mn_major;  // 0: K contiguous in global memory, 1: M (resp. N) contiguous
+  int a_mn_major, b_mn_major;  // 0: K contiguous in global memory, 1: M (resp. N) contiguous, 2: so and a multiple of 64 (see encode_operand)
   int is_bf16;
   int has_bias;
   int tma_store;    // 1 = C goes out through TMA tile stores (N % 8 == 0, aligned), 0 = plain stores
@@ -280,6 +291,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (kPair) tma_load_3d_pair(dst, map, fbar, c0, c1, c2);
             else tma_load_3d(dst, map, fbar, c0, c1, c2);
           };
+          auto load_blocks = [&](uint32_t dst, const CUtensorMap* map, int k, int block, int c2) {
+            if (kPair) tma_load_4d_pair(dst, map, fbar, 0, k, block, c2);
+            else tma_load_4d(dst, map, fbar, 0, k, block, c2);
+          };
           int ka = (slab0 + kb) * kBK, kbb = ka;
           if (sizeof(TO) == 4 && p.split_slabs) {
             // pairs (2,0) (1,1) (0,2) (1,0) (0,1) over all slabs first, then (0,0): the tensor
@@ -292,12 +307,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           }
           if (!p.a_mn_major) {
             load(a_dst, &map_a, ka, m0, entry);  // box [128 rows][64 k]
+          } else if (p.a_mn_major == 2) {
+            load_blocks(a_dst, &map_a, ka, m0 >> 6, entry);  // box [2][64 k][64 m]
           } else {
 #pragma unroll
             for (int c = 0; c < kBM / 64; ++c) load(a_dst + c * 8192, &map_a, m0 + c * 64, ka, entry);  // box [64 k][64 m]
           }
           if (!p.b_mn_major) {
             load(b_dst, &map_b, kbb, n0, entry);  // box [b_rows rows][64 k]
+          } else if (p.b_mn_major == 2) {
+            load_blocks(b_dst, &map_b, kbb, n0 >> 6, entry);  // box [b_rows / 64][64 k][64 n]
           } else {
 #pragma unroll
             for (int c = 0; c < Cfg::kBRows / 64; ++c)
@@ -325,7 +344,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (cta_rank == 0u) {  // pair: the even CTA issues for both
       // instruction descriptor: fp32 accumulate, A/B format, majors, N >> 3, M >> 4
       const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(p.a_mn_major) << 15) | (static_cast<uint32_t>(p.b_mn_major) << 16) |
+      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (p.a_mn_major ? 1u << 15 : 0u) | (p.b_mn_major ? 1u << 16 : 0u) |
                              (static_cast<uint32_t>(bn >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
       // per-UMMA (K = 16) advance of the start address and the two byte offsets per layout
       const uint32_t a_adv = p.a_mn_major ? 2048u : 32u, b_adv = p.b_mn_major ? 2048u : 32u;
@@ -651,17 +670,30 @@ bool gemm_tc_eligible(int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sA
   return encode_fn() != nullptr;
 }
 
+// An MN-major operand arrives as blocks of 64 columns. Where its columns are a multiple of 64 they are a dimension of
+// their own (the map ends where the operand does), and a tile's blocks, two or four copies otherwise, are one: a single thread issues them, and
+// with both operands MN-major that is what a slab waits for.
+static bool in_blocks(bool mn_major, int64_t mn, int tile_mn) { return mn_major && mn % 64 == 0 && tile_mn % 64 == 0; }
+static int mn_form(bool mn_major, int64_t mn, int tile_mn) { return mn_major ? (in_blocks(mn_major, mn, tile_mn) ? 2 : 1) : 0; }
 static bool encode_operand(CUtensorMap* map, const void* base, int dtype, bool mn_major, int64_t mn, int64_t k, int64_t s_mn, int64_t s_k, int64_t s_b, int64_t batch, int tile_mn) {
   const cuuint64_t inner = mn_major ? mn : k, outer = mn_major ? k : mn;
   int64_t outer_stride = mn_major ? s_k : s_mn;  // elements
   if (outer == 1 && outer_stride % 8 != 0) outer_stride = (static_cast<int64_t>(inner) + 7) / 8 * 8;  // never dereferenced beyond row 0
   int64_t batch_stride = batch > 1 ? s_b : outer_stride * static_cast<int64_t>(outer);
   if (batch_stride % 8 != 0 || batch_stride <= 0) batch_stride = (batch_stride / 8 + 1) * 8;
+  const CUtensorMapDataType dt = dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  if (in_blocks(mn_major, mn, tile_mn)) {  // [batch][mn / 64][k][64]: the blocks of a tile in one copy
+    cuuint64_t dims[4] = {64, outer, inner / 64, static_cast<cuuint64_t>(batch)};
+    cuuint64_t strides[3] = {static_cast<cuuint64_t>(outer_stride) * 2, 128, static_cast<cuuint64_t>(batch_stride) * 2};
+    cuuint32_t box[4] = {64, kBK, static_cast<cuuint32_t>(tile_mn / 64), 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    return encode_fn()(map, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  }
   cuuint64_t dims[3] = {inner, outer, static_cast<cuuint64_t>(batch)};
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(outer_stride) * 2, static_cast<cuuint64_t>(batch_stride) * 2};
   cuuint32_t box[3] = {64, static_cast<cuuint32_t>(mn_major ? kBK : tile_mn), 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapDataType dt = dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const CUresult r = encode_fn()(map, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
@@ -780,8 +812,8 @@ int gemm_tc_dispatch(const void* A, const void* B, const void* bias, void* C, in
   p.sbm = sbm; p.sbn = sbn;
   p.alpha = static_cast<float>(alpha);
   p.beta = static_cast<float>(beta);
-  p.a_mn_major = la.mn_major ? 1 : 0;
-  p.b_mn_major = lb.mn_major ? 1 : 0;
+  p.a_mn_major = mn_form(la.mn_major, M, kBM);
+  p.b_mn_major = mn_form(lb.mn_major, N, bn_box);
   p.is_bf16 = dtype == B200_BF16 ? 1 : 0;
   p.has_bias = (bias != nullptr && p.beta != 0.f) ? 1 : 0;
   // few K slabs per tile: the kernel is bound by writing C, so CTAs that run together should
@@ -936,8 +968,8 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   p.sbm = 0; p.sbn = 0;
   p.alpha = 1.f;
   p.beta = 0.f;
-  p.a_mn_major = la.mn_major ? 1 : 0;
-  p.b_mn_major = lb.mn_major ? 1 : 0;
+  p.a_mn_major = mn_form(la.mn_major, M, kBM);
+  p.b_mn_major = mn_form(lb.mn_major, N, bn);
   p.is_bf16 = dtype == B200_BF16 ? 1 : 0;
   p.has_bias = 0;
   p.col_fastest = 1;
@@ -1112,7 +1144,7 @@ static F32Plan plan_f32(int64_t batch, int64_t M, int64_t N, int64_t K, bool b_m
 int64_t gemm_f32_split_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   const int64_t kp = round_up(K, kBK);
   const int along_k = plan_f32(batch, M, N, K, false).ranges, along_n = plan_f32(batch, M, N, K, true).ranges, ranges = along_k > along_n ? along_k : along_n;
-  return batch * 3 * kp * (round_up(M, 8) + round_up(N, 8)) * 2 + 256 + 512 + (ranges > 1 ? ranges * M * N * 4 : 0);
+  return batch * 3 * kp * (round_up(M, 64) + round_up(N, 64)) * 2 + 256 + 512 + (ranges > 1 ? ranges * M * N * 4 : 0);
 }
 
 bool gemm_f32_split_eligible(int64_t batch, int64_t M, int64_t N, int64_t K) {
@@ -1134,8 +1166,10 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   if (me != cudaSuccess) { set_last_cuda_error(me); return B200_ELAUNCH; }
   auto* pa = reinterpret_cast<__nv_bfloat16*>(flags + flag_bytes);
   const bool a_mn = sAm == 1 && sAk != 1 && M > 1, b_mn = sBn == 1 && sBk != 1 && N > 1;  // keep the contiguous dimension of each source
-  const int64_t a_row = a_mn ? round_up(M, 8) : 3 * kp, a_rows = a_mn ? 3 * kp : M;
-  const int64_t b_row = b_mn ? round_up(N, 8) : 3 * kp, b_rows = b_mn ? 3 * kp : N;
+  // (MN-major planes have whole blocks of 64 columns, see encode_operand; what lies behind an operand's last column
+  // belongs to rows or columns that C does not have)
+  const int64_t a_row = a_mn ? round_up(M, 64) : 3 * kp, a_rows = a_mn ? 3 * kp : M;
+  const int64_t b_row = b_mn ? round_up(N, 64) : 3 * kp, b_rows = b_mn ? 3 * kp : N;
   __nv_bfloat16* pb = pa + batch * a_rows * a_row;  // a multiple of 8 elements: stays 16-byte aligned
   const float* fa = static_cast<const float*>(A);
   const float* fb = static_cast<const float*>(B);
@@ -1152,16 +1186,16 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   const bool pair = M > kBM && N > 128 && pair_launch_ok();  // the contraction is six planes deep: never write-bound
   const F32Plan plan = plan_f32(batch, M, N, K, b_mn);
   const int bn = plan.bn;
-  if (!encode_operand(&map_a, pa, B200_BF16, a_mn, M, 3 * kp, a_mn ? 1 : a_row, a_mn ? a_row : 1, a_rows * a_row, batch, kBM)) return B200_EDRIVER;
-  if (!encode_operand(&map_b, pb, B200_BF16, b_mn, N, 3 * kp, b_mn ? 1 : b_row, b_mn ? b_row : 1, b_rows * b_row, batch, pair ? bn / 2 : bn)) return B200_EDRIVER;
+  if (!encode_operand(&map_a, pa, B200_BF16, a_mn, a_mn ? a_row : M, 3 * kp, a_mn ? 1 : a_row, a_mn ? a_row : 1, a_rows * a_row, batch, kBM)) return B200_EDRIVER;
+  if (!encode_operand(&map_b, pb, B200_BF16, b_mn, b_mn ? b_row : N, 3 * kp, b_mn ? 1 : b_row, b_mn ? b_row : 1, b_rows * b_row, batch, pair ? bn / 2 : bn)) return B200_EDRIVER;
   GemmTcParams p;
   p.tma_store = 0;
   p.M = M; p.N = N; p.K = K; p.batch = batch;
   p.sbm = sbm; p.sbn = sbn;
   p.alpha = static_cast<float>(alpha);
   p.beta = static_cast<float>(beta);
-  p.a_mn_major = a_mn ? 1 : 0;
-  p.b_mn_major = b_mn ? 1 : 0;
+  p.a_mn_major = mn_form(a_mn, a_row, kBM);
+  p.b_mn_major = mn_form(b_mn, b_row, pair ? bn / 2 : bn);
   p.is_bf16 = 1;
   p.has_bias = (bias != nullptr && p.beta != 0.f) ? 1 : 0;
   p.split_slabs = static_cast<int>(kp / kBK);
