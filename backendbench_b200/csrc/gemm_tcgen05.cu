@@ -183,7 +183,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   constexpr int kAccs = Cfg::kAccs;
   constexpr int kTileM = kPair ? 2 * kBM : kBM;  // rows of C one tile covers (both CTAs of a pair)
   static_assert(!kPair || kBN == 256, "CTA pairs work on 256 x 256 tiles");
-  if (p.skip_if_set && *p.skip_if_set != 0u) return;  // every thread of every CTA reads the same word: a uniform exit before any barrier or TMEM set-up
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern repeats every 8 rows x 128 bytes
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -241,9 +240,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   if (kPair) cluster_sync_all();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  after_grids_before();  // what is above needs nothing that an earlier kernel writes
+  const bool skip = p.skip_if_set && *p.skip_if_set != 0u;  // the same word for every thread of every CTA
 
   const int64_t mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + bn - 1) / bn;
-  const int64_t tiles = p.batch * mt * nt;
+  const int64_t tiles = skip ? 0 : p.batch * mt * nt;
   const int64_t tile_first = kPair ? (blockIdx.x >> 1) : blockIdx.x, tile_step = kPair ? (gridDim.x >> 1) : gridDim.x;
   // Split operands: plane q of an operand occupies K coordinates [q * Kp, q * Kp + K) of its
   // tensor map, Kp = 64 * split_slabs. One slab of the product needs the six plane pairs
@@ -721,22 +722,20 @@ static int launch_tc(Kernel kernel, bool pair, int grid, cudaStream_t st, const 
                      const GemmTcParams& p, uint32_t* status) {
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem));
   if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
-  if (!pair) {
-    kernel<<<grid, kGemmThreads, kGemmSmem, st>>>(map_a, map_b, map_c, bias_t, c_t, p, status);
-    return B200_OK;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
   cfg.blockDim = dim3(kGemmThreads, 1, 1);
   cfg.dynamicSmemBytes = kGemmSmem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (see launch_after)
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pair ? 2 : 1;
   const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_c, bias_t, c_t, p, status);
   if (le != cudaSuccess) { set_last_cuda_error(le); return B200_ELAUNCH; }
   return B200_OK;
@@ -896,7 +895,8 @@ int64_t gemm_tc_splitk_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_
 // ranges at a time (20000 deep, 40 x 128 outputs: the call 12.7 us, 16 with eight in flight).
 template <typename T, int U, int B>
 __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ part, int splits, int64_t M, int64_t N, const T* __restrict__ bias, int64_t sbm, int64_t sbn, float alpha, float beta,
-                                                     T* __restrict__ C, const uint32_t* __restrict__ skip_if_set) {
+                                                     T* __restrict__ C, const uint32_t* skip_if_set) {
+  after_grids_before();
   if (skip_if_set && *skip_if_set != 0u) return;  // the partial products were not computed either
   const int64_t total = M * N;
   for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; i0 < total; i0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
@@ -936,16 +936,14 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
 }
 
 template <typename T>
-static void launch_splitk_reduce(const float* part, int splits, int64_t M, int64_t N, const void* bias, int64_t sbm, int64_t sbn, float alpha, float beta, void* C, const uint32_t* skip_if_set,
+static cudaError_t launch_splitk_reduce(const float* part, int splits, int64_t M, int64_t N, const void* bias, int64_t sbm, int64_t sbn, float alpha, float beta, void* C, const uint32_t* skip_if_set,
                                  cudaStream_t st) {
   const int64_t total = M * N, cap = kNumSMs * 8;
   const bool wide = total >= cap * 1024;
   int64_t blocks = wide ? (total + 1023) / 1024 : (total + 255) / 256;
   if (blocks > cap) blocks = cap;
-  auto go = [&](auto kernel) { kernel<<<static_cast<int>(blocks), 256, 0, st>>>(part, splits, M, N, static_cast<const T*>(bias), sbm, sbn, alpha, beta, static_cast<T*>(C), skip_if_set); };
-  if (wide) go(splitk_reduce<T, 4, 1>);
-  else if (total >= 1 << 16) go(splitk_reduce<T, 1, 1>);
-  else go(splitk_reduce<T, 1, 16>);
+  auto go = [&](auto kernel) { return launch_after(kernel, blocks, 256, 0, st, part, splits, M, N, static_cast<const T*>(bias), sbm, sbn, alpha, beta, static_cast<T*>(C), skip_if_set); };
+  return wide ? go(splitk_reduce<T, 4, 1>) : total >= 1 << 16 ? go(splitk_reduce<T, 1, 1>) : go(splitk_reduce<T, 1, 16>);
 }
 
 int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sAk, int64_t sBk, int64_t sBn, int64_t sbm,
@@ -992,8 +990,9 @@ int gemm_tc_splitk_dispatch(const void* A, const void* B, const void* bias, void
   rc = N >= 32 && N % 4 != 0 ? launch_as(std::true_type{}) : launch_as(std::false_type{});
   if (rc) return rc;
   const float al = static_cast<float>(alpha), be = static_cast<float>(beta);
-  if (dtype == B200_BF16) launch_splitk_reduce<__nv_bfloat16>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st);
-  else launch_splitk_reduce<__half>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st);
+  const cudaError_t re = dtype == B200_BF16 ? launch_splitk_reduce<__nv_bfloat16>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st)
+                                            : launch_splitk_reduce<__half>(part, static_cast<int>(S), M, N, bias, sbm, sbn, al, be, C, nullptr, st);
+  if (re != cudaSuccess) { set_last_cuda_error(re); return B200_ELAUNCH; }
   return check_launch(2);
 }
 
@@ -1044,6 +1043,7 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16&
 // the row is off. (Element by element a warp's load touched 32 sectors: 1531 x 1027 and 2050 x 1027
 // together 12 -> 8 us.)
 __global__ void __launch_bounds__(256) split_f32_planes(const __grid_constant__ SplitArgs A0, const __grid_constant__ SplitArgs A1, unsigned blocks0) {
+  next_grid_may_start();  // (the product's CTAs set themselves up meanwhile)
   const bool second = blockIdx.x >= blocks0;
   const SplitArgs& A = second ? A1 : A0;
   const int64_t block = second ? blockIdx.x - blocks0 : blockIdx.x, nblocks = second ? gridDim.x - blocks0 : blocks0;
@@ -1228,8 +1228,10 @@ int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void
   };
   const int rc = rows ? launch_as(std::true_type{}) : launch_as(std::false_type{});
   if (rc) return rc;
-  if (ranges > 1)
-    launch_splitk_reduce<float>(part, ranges, M, N, bias, sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), C, any_flag, st);
+  if (ranges > 1) {
+    const cudaError_t re = launch_splitk_reduce<float>(part, ranges, M, N, bias, sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), C, any_flag, st);
+    if (re != cudaSuccess) { set_last_cuda_error(re); return B200_ELAUNCH; }
+  }
   // the same product on the CUDA cores, run only when the split met an infinity or a NaN
   const int rs = gemm_simt_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, B200_F32, st, any_flag);
   if (rs) return rs;
