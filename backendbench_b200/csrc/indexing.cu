@@ -112,6 +112,104 @@ __global__ void __launch_bounds__(256) index_select_flat(const U* __restrict__ x
   }
 }
 
+// Rows off the 16-byte grid (126 bytes, say): a thread produces 16 bytes of the result, wherever they lie in it. They come
+// from one row, or from the end of one and the beginning of the next, and each part from the one or two aligned
+// 16-byte blocks around it, moved by as many bytes as source and result differ; only blocks that hold
+// a byte of the part are read. Element by element the kernel above is bound by its instructions: f16
+// 150134 x 63, 75067 rows 14.9 us, 9.0 so; 56 x 3527, 21648 rows 198 and 64. From 2^20 units on: with fewer, a thread's
+// chain of index, blocks and shifts takes longer than a thread for each unit (fp32 5000 x 130 3.6 us, 4.5 so).
+struct Block32 {
+  uint32_t w[8];
+};
+// bytes [sh, sh + 16) of two blocks, the words of which are in w[0..7]
+__device__ __forceinline__ uint4 bytes_from(Block32 b, uint32_t sh) {
+  if (sh & 4u) {
+#pragma unroll
+    for (int i = 0; i < 7; ++i) b.w[i] = b.w[i + 1];
+  }
+  if (sh & 8u) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) b.w[i] = b.w[i + 2];
+  }
+  const uint32_t bits = (sh & 3u) * 8;
+  return make_uint4(__funnelshift_r(b.w[0], b.w[1], bits), __funnelshift_r(b.w[1], b.w[2], bits), __funnelshift_r(b.w[2], b.w[3], bits), __funnelshift_r(b.w[3], b.w[4], bits));
+}
+// The 16 bytes at `at`, of which [lo, hi) count
+__device__ __forceinline__ uint4 bytes_at(const unsigned char* at, int lo, int hi) {
+  const uint32_t sh = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(at)) & 15u;
+  const uint4* block = reinterpret_cast<const uint4*>(at - sh);
+  uint4 a = make_uint4(0, 0, 0, 0), b = a;
+  if (static_cast<int>(sh) + lo < 16) a = __ldg(block);
+  if (static_cast<int>(sh) + hi > 16) b = __ldg(block + 1);
+  return bytes_from(Block32{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}}, sh);
+}
+constexpr int kRaggedUnroll = 2;
+constexpr int64_t kRaggedMinUnits = 1 << 20;
+__global__ void __launch_bounds__(256) select_rows_ragged(const unsigned char* __restrict__ x, const void* __restrict__ idx, unsigned char* __restrict__ out, int64_t outer, int64_t dim_size,
+                                                          int64_t row_bytes, int64_t n_idx, int idx_i32, uint32_t* status) {
+  const int64_t total = outer * n_idx * row_bytes, vecs = (total + 15) / 16, step = static_cast<int64_t>(gridDim.x) * 256;
+  const bool small = total <= 0x7fffffffLL;
+  // the row `q` of the result: where it lies in x, NULL: an index out of range
+  auto source = [&](int64_t q) -> const unsigned char* {
+    const int64_t o = outer == 1 ? 0 : q / n_idx, k = load_index(idx, q - o * n_idx, idx_i32);
+    if (k < 0 || k >= dim_size) {
+      flag_oob(status);
+      return nullptr;
+    }
+    return x + (o * dim_size + k) * row_bytes;
+  };
+  for (int64_t v0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; v0 < vecs; v0 += kRaggedUnroll * step) {
+    const unsigned char *one[kRaggedUnroll], *two[kRaggedUnroll];
+    int first[kRaggedUnroll];  // bytes of the vector that lie in the first row
+    uint4 r[kRaggedUnroll];
+#pragma unroll
+    for (int u = 0; u < kRaggedUnroll; ++u) {
+      const int64_t v = v0 + u * step;
+      one[u] = two[u] = nullptr;
+      first[u] = 16;
+      if (v < vecs) {
+        const int64_t p = v * 16, q = small ? static_cast<int64_t>(static_cast<uint32_t>(p) / static_cast<uint32_t>(row_bytes)) : p / row_bytes;
+        const int64_t in_row = p - q * row_bytes;
+        one[u] = source(q);
+        if (one[u]) one[u] += in_row;
+        if (row_bytes - in_row < 16) {
+          first[u] = static_cast<int>(row_bytes - in_row);
+          if (p + first[u] < total) two[u] = source(q + 1);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRaggedUnroll; ++u) {
+      r[u] = make_uint4(0, 0, 0, 0);
+      if (one[u]) r[u] = bytes_at(one[u], 0, first[u]);
+      if (first[u] < 16) {
+        uint4 s = make_uint4(0, 0, 0, 0);
+        if (two[u]) s = bytes_at(two[u] - first[u], first[u], 16);
+        // byte i is the first row's for i < first
+        auto merge = [&](uint32_t a, uint32_t b, int at) {
+          const int keep = first[u] - at;
+          const uint32_t mask = keep >= 4 ? 0xffffffffu : keep <= 0 ? 0u : (1u << (8 * keep)) - 1u;
+          return (a & mask) | (b & ~mask);
+        };
+        r[u] = make_uint4(merge(r[u].x, s.x, 0), merge(r[u].y, s.y, 4), merge(r[u].z, s.z, 8), merge(r[u].w, s.w, 12));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRaggedUnroll; ++u) {
+      const int64_t v = v0 + u * step, p = v * 16;
+      if (v >= vecs) break;
+      if (p + 16 <= total) {
+        __stcs(reinterpret_cast<uint4*>(out + p), r[u]);
+      } else {  // the result ends inside the last vector
+        const uint32_t w[4] = {r[u].x, r[u].y, r[u].z, r[u].w};
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (p + i < total) out[p + i] = static_cast<unsigned char>(w[i >> 2] >> (8 * (i & 3)));
+      }
+    }
+  }
+}
+
 struct GatherArgs {
   int ndim, dim;
   int64_t n;
@@ -239,6 +337,61 @@ __global__ void __launch_bounds__(256) gather_lastdim_vec(const U* __restrict__ 
       }
     }
     __stcs(reinterpret_cast<uint4*>(out + p), *reinterpret_cast<const uint4*>(v));
+  }
+}
+
+// 2-D, along either dim, with rows of any length: a thread produces 16 bytes of the contiguous result -- VE adjacent outputs,
+// which may go on in the next row -- with 16-byte index loads, one division and one store. (An element to a thread decodes
+// its coordinates with one division per dimension and moves two or four bytes per store: f16 150134 x 63, 75067
+// rows of indices, 27.3 us along the rows and 25.0 along the columns, 22.6 and 9.6 so; fp32 4095 x 4095 127 and 103, 79 and 51. With fewer
+// than 2^17 outputs the two are on a par.)
+constexpr int64_t kGather2dMin = 1 << 17;
+template <typename U, int DIM>
+__global__ void __launch_bounds__(256) gather_2d_vec(const U* __restrict__ self, const int64_t* __restrict__ index, U* __restrict__ out, uint32_t total, uint32_t cols, int64_t s_row, int64_t s_col,
+                                                     int64_t self_dim_size, uint32_t* status) {
+  constexpr int VE = 16 / static_cast<int>(sizeof(U));
+  const uint32_t groups = (total + VE - 1) / VE;
+  for (uint32_t q = blockIdx.x * 256 + threadIdx.x; q < groups; q += gridDim.x * 256) {
+    const uint32_t p = q * VE;
+    const bool whole = p + VE <= total;
+    int64_t k[VE];
+#pragma unroll
+    for (int h = 0; h < VE / 2; ++h) {
+      if (whole) {
+        const longlong2 t = __ldcs(reinterpret_cast<const longlong2*>(index + p) + h);
+        k[2 * h] = t.x;
+        k[2 * h + 1] = t.y;
+      } else {
+        k[2 * h] = p + 2 * h < total ? index[p + 2 * h] : 0;
+        k[2 * h + 1] = p + 2 * h + 1 < total ? index[p + 2 * h + 1] : 0;
+      }
+    }
+    const uint32_t row = p / cols;
+    uint32_t col = p - row * cols;
+    const U* at = self + (DIM == 0 ? col * s_col : row * s_row);  // of the coordinate that is kept
+    __align__(16) U v[VE];
+    bool bad = false;
+#pragma unroll
+    for (int e = 0; e < VE; ++e) {
+      const bool in = p + e < total, ok = k[e] >= 0 && k[e] < self_dim_size;
+      v[e] = in && ok ? at[k[e] * (DIM == 0 ? s_row : s_col)] : zero_of<U>();
+      bad |= in && !ok;
+      ++col;
+      if (DIM == 0) at += s_col;
+      if (col == cols) {
+        col = 0;
+        if (DIM == 0) at = self;
+        else at += s_row;
+      }
+    }
+    if (bad) flag_oob(status);
+    if (whole) {
+      __stcs(reinterpret_cast<uint4*>(out + p), *reinterpret_cast<const uint4*>(v));
+    } else {
+#pragma unroll
+      for (int e = 0; e < VE; ++e)
+        if (p + e < total) out[p + e] = v[e];
+    }
   }
 }
 
@@ -453,6 +606,13 @@ static int index_select_bytes(const void* x, const void* idx, void* out, int64_t
     }
     return check_launch();
   }
+  // (16-byte vectors of the result meet at most two rows)
+  const int64_t total = outer * n_idx * inner_bytes;
+  if (unit < 16 && inner_bytes >= 16 && aligned16(out) && total / unit >= kRaggedMinUnits) {
+    select_rows_ragged<<<capped_grid((total + 15) / 16, 256 * kRaggedUnroll, 16), 256, 0, st>>>(static_cast<const unsigned char*>(x), idx, static_cast<unsigned char*>(out), outer, dim_size, inner_bytes, n_idx, i32,
+                                                                                                status);
+    return check_launch();
+  }
   switch (unit) {
     case 16: launch_flat<uint4>(x, idx, out, outer, dim_size, units, n_idx, i32, status, st); break;
     case 8: launch_flat<uint64_t>(x, idx, out, outer, dim_size, units, n_idx, i32, status, st); break;
@@ -569,6 +729,17 @@ extern "C" int b200_gather(const void* self, const void* index, void* out, int n
       gather_lastdim_vec<uint32_t><<<g2, 256, 0, st>>>(static_cast<const uint32_t*>(self), static_cast<const int64_t*>(index), static_cast<uint32_t*>(out), index_shape[0], index_shape[1], self_strides[0], self_dim_size, status);
     else
       gather_lastdim_vec<uint16_t><<<g2, 256, 0, st>>>(static_cast<const uint16_t*>(self), static_cast<const int64_t*>(index), static_cast<uint16_t*>(out), index_shape[0], index_shape[1], self_strides[0], self_dim_size, status);
+    return check_launch();
+  }
+  if (ndim == 2 && (elem_size == 4 || elem_size == 2) && idx_contig && aligned16(index) && aligned16(out) && A.n >= kGather2dMin && A.n <= 0x7fffffffLL) {
+    const int g2 = capped_grid((A.n + ve - 1) / ve, 256, 32);
+    auto launch = [&](auto kernel, auto unit) {
+      typedef decltype(unit) U;
+      kernel<<<g2, 256, 0, st>>>(static_cast<const U*>(self), static_cast<const int64_t*>(index), static_cast<U*>(out), static_cast<uint32_t>(A.n), static_cast<uint32_t>(index_shape[1]), self_strides[0],
+                                 self_strides[1], self_dim_size, status);
+    };
+    if (elem_size == 4) dim == 0 ? launch(gather_2d_vec<uint32_t, 0>, uint32_t{}) : launch(gather_2d_vec<uint32_t, 1>, uint32_t{});
+    else dim == 0 ? launch(gather_2d_vec<uint16_t, 0>, uint16_t{}) : launch(gather_2d_vec<uint16_t, 1>, uint16_t{});
     return check_launch();
   }
   const bool along_rows = ndim == 0 || index_shape[ndim - 1] == 1 || index_strides[ndim - 1] == 1;

@@ -629,6 +629,50 @@ def test_scatter_add_crowded_or_not_bit_exact(backend, dtype, spread):
         assert bits_equal(want.t().contiguous(), turned.cpu())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int8])
+def test_rows_and_elements_off_the_16_byte_grid(backend, dtype):
+    """index_select and embedding of rows that start anywhere, 16 bytes of the result at a time: the shortest such rows, vectors
+    that meet two rows, a result that ends inside a vector, a table that begins between two blocks, slices of a middle dim;
+    gather of results whose rows end inside a vector, along either dim. An index out of range gives zeros and is reported."""
+    g = torch.Generator().manual_seed(3)
+    select, gather = backend[torch.ops.aten.index_select.default], backend[torch.ops.aten.gather.default]
+    es = torch.empty(0, dtype=dtype).element_size()
+    for rows, cols, n in [(5, 16 // es + 1, 70000), (70, 31 // es + 2, 60001), (3001, 63, 20011), (40, 3527, 601), (2, 100003, 23)]:
+        flat = torch.randint(-100, 100, (rows * cols + 1,), generator=g).to(dtype).to(DEV)
+        idx = torch.randint(0, rows, (n,), generator=g).to(DEV)
+        for x in (flat[:-1].view(rows, cols), flat[1:].view(rows, cols)):
+            assert torch.equal(select(x, 0, idx), x[idx])
+            mid = x.view(1, rows, cols).expand(3, rows, cols).contiguous() if rows * n * cols < 1 << 27 else None
+            if mid is not None and n < 30000:
+                assert torch.equal(select(mid, 1, idx), mid[:, idx])
+        if dtype != torch.int8:
+            assert torch.equal(backend[torch.ops.aten.embedding.default](flat[1:].view(rows, cols), idx.int()), flat[1:].view(rows, cols)[idx])
+        bad = idx.clone()
+        bad[[0, n // 2, n - 1]] = torch.tensor([rows, -1, 1 << 40], device=DEV)
+        got, want = select(x, 0, bad), x[idx].clone()
+        want[[0, n // 2, n - 1]] = 0
+        assert torch.equal(got, want)
+        with pytest.raises(IndexError):
+            ops.check_device_status()
+    if dtype == torch.int8:
+        return
+    for rows, cols, n in [(700, 301, 499), (131073, 3, 131073), (9, 20001, 9), (1000, 134, 1001)]:
+        flat = torch.randn(rows * cols + 1, generator=g).to(dtype).to(DEV)
+        for dim, shape in ((0, (n, cols)), (1, (min(n, rows), cols + 3))):
+            x = flat[1:].view(rows, cols)
+            if dim == 1 and cols == 20001:
+                x = flat[:-1].view(cols, rows).t()
+            idx = torch.randint(0, x.shape[dim], shape, generator=g).to(DEV)
+            assert torch.equal(gather(x, dim, idx), torch.gather(x, dim, idx))
+            ops.check_device_status()
+            idx[-1, -1], idx[0, 0] = -1, x.shape[dim]
+            want = torch.gather(x, dim, idx.clamp(0, x.shape[dim] - 1))
+            want[-1, -1], want[0, 0] = 0, 0
+            assert torch.equal(gather(x, dim, idx), want)
+            with pytest.raises(IndexError):
+                ops.check_device_status()
+
+
 # (self, dim, index, layout of index and src): a column group of one column, one of 31 and of two; bins cut short; more
 # contributions than a bin's ring and than destinations; an index smaller than self on every side; one row of indices for all
 # columns, indices and values read across their rows; the last one has no columns to deal out and hangs in chains
