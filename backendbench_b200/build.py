@@ -1,21 +1,25 @@
-"""Build libb200ops.so in-tree: `python -m backendbench_b200.build [--verbose] [--force]`.
+"""Build libb200ops.so and _b200host.so in-tree: `python -m backendbench_b200.build [--verbose] [--force]`.
 
-Runs the Makefile in csrc/ (nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo).
-nvcc cross-compiles without a GPU; the resulting shared object is what `_abi.lib()` loads.
+Runs the Makefile in csrc/ (nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo; the host
+module with the C++ compiler against torch's headers). nvcc cross-compiles without a GPU; the
+resulting shared objects are what `_abi.lib()` and `_native.module()` load.
 """
 
 from __future__ import annotations
 
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 from ._abi import CSRC_DIR, LIB_PATH
 
 
 def build(verbose: bool = False, force: bool = False, jobs: int = 0) -> str:
     jobs = jobs or min(os.cpu_count() or 4, 16)
-    cmd = ["make", "-C", CSRC_DIR, f"-j{jobs}"]
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cmd = ["make", "-C", CSRC_DIR, f"-j{jobs}", f"TORCH={torch_dir}", f"PYINC={sysconfig.get_paths()['include']}"]
     if force:
         cmd.append("-B")
     if verbose:

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from . import backward as _bw
 from . import ops as _ops
 
@@ -52,6 +53,9 @@ OPERATORS = {
 
 # aten spec name ("add.Tensor") -> name in the b200 namespace
 ATEN_TO_B200 = {str(a).split("aten.", 1)[-1]: name for name, (_, _, a) in OPERATORS.items()}
+
+# the host wrappers as they are: the native calls stand in for these, and step back while one of them is replaced
+_WRAPPERS = {name: getattr(module, attr) for name, (_, (module, attr), _) in OPERATORS.items()}
 
 _library = torch.library.Library("b200", "DEF")  # lives as long as the module
 
@@ -111,6 +115,17 @@ def entry(name: str):
             if i < len(args) and not isinstance(args[i], torch.Tensor):
                 return fn(*args, **kwargs)
         return op(*args, **kwargs)
+
+    native = _native.module()
+    if native is not None:
+        # plain calls without the dispatcher and the interpreter; everything else comes back to `run`
+        module, attr = OPERATORS[name][1]
+        general, direct, compiling = run, native.make(name, module, attr, _WRAPPERS[name], run), torch.compiler.is_compiling
+
+        def run(*args, **kwargs):
+            if compiling():  # a traced program sees the operator
+                return general(*args, **kwargs)
+            return direct(*args, **kwargs)
 
     run.__name__ = f"b200_{name}"
     return run

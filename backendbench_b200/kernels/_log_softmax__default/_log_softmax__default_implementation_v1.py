@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_log_softmax = _custom_ops.entry("log_softmax")  # torch.ops.b200.log_softmax
-
-
-def _log_softmax__default_kernel_impl(*args, **kwargs):
-    return _b200_log_softmax(*args, **kwargs)
+_log_softmax__default_kernel_impl = _b200_log_softmax

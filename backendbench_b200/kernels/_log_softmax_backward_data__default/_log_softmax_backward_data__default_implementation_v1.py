@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_log_softmax_backward = _custom_ops.entry("log_softmax_backward")  # torch.ops.b200.log_softmax_backward
-
-
-def _log_softmax_backward_data__default_kernel_impl(*args, **kwargs):
-    return _b200_log_softmax_backward(*args, **kwargs)
+_log_softmax_backward_data__default_kernel_impl = _b200_log_softmax_backward

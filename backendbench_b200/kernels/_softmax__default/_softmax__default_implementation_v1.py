@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_softmax = _custom_ops.entry("softmax")  # torch.ops.b200.softmax
-
-
-def _softmax__default_kernel_impl(*args, **kwargs):
-    return _b200_softmax(*args, **kwargs)
+_softmax__default_kernel_impl = _b200_softmax

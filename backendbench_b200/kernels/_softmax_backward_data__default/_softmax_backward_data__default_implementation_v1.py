@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_softmax_backward = _custom_ops.entry("softmax_backward")  # torch.ops.b200.softmax_backward
-
-
-def _softmax_backward_data__default_kernel_impl(*args, **kwargs):
-    return _b200_softmax_backward(*args, **kwargs)
+_softmax_backward_data__default_kernel_impl = _b200_softmax_backward

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_add = _custom_ops.entry("add")  # torch.ops.b200.add
-
-
-def add__Tensor_kernel_impl(*args, **kwargs):
-    return _b200_add(*args, **kwargs)
+add__Tensor_kernel_impl = _b200_add

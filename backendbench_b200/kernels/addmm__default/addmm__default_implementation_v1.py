@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_addmm = _custom_ops.entry("addmm")  # torch.ops.b200.addmm
-
-
-def addmm__default_kernel_impl(*args, **kwargs):
-    return _b200_addmm(*args, **kwargs)
+addmm__default_kernel_impl = _b200_addmm

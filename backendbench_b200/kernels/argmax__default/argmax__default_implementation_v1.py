@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_argmax = _custom_ops.entry("argmax")  # torch.ops.b200.argmax
-
-
-def argmax__default_kernel_impl(*args, **kwargs):
-    return _b200_argmax(*args, **kwargs)
+argmax__default_kernel_impl = _b200_argmax

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_bmm = _custom_ops.entry("bmm")  # torch.ops.b200.bmm
-
-
-def bmm__default_kernel_impl(*args, **kwargs):
-    return _b200_bmm(*args, **kwargs)
+bmm__default_kernel_impl = _b200_bmm

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_embedding = _custom_ops.entry("embedding")  # torch.ops.b200.embedding
-
-
-def embedding__default_kernel_impl(*args, **kwargs):
-    return _b200_embedding(*args, **kwargs)
+embedding__default_kernel_impl = _b200_embedding

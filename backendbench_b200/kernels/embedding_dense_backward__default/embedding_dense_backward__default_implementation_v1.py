@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_embedding_backward = _custom_ops.entry("embedding_backward")  # torch.ops.b200.embedding_backward
-
-
-def embedding_dense_backward__default_kernel_impl(*args, **kwargs):
-    return _b200_embedding_backward(*args, **kwargs)
+embedding_dense_backward__default_kernel_impl = _b200_embedding_backward

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_gather = _custom_ops.entry("gather")  # torch.ops.b200.gather
-
-
-def gather__default_kernel_impl(*args, **kwargs):
-    return _b200_gather(*args, **kwargs)
+gather__default_kernel_impl = _b200_gather

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_index_select = _custom_ops.entry("index_select")  # torch.ops.b200.index_select
-
-
-def index_select__default_kernel_impl(*args, **kwargs):
-    return _b200_index_select(*args, **kwargs)
+index_select__default_kernel_impl = _b200_index_select

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_mm = _custom_ops.entry("mm")  # torch.ops.b200.mm
-
-
-def mm__default_kernel_impl(*args, **kwargs):
-    return _b200_mm(*args, **kwargs)
+mm__default_kernel_impl = _b200_mm

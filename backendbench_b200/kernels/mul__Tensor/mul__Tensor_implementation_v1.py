@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_mul = _custom_ops.entry("mul")  # torch.ops.b200.mul
-
-
-def mul__Tensor_kernel_impl(*args, **kwargs):
-    return _b200_mul(*args, **kwargs)
+mul__Tensor_kernel_impl = _b200_mul

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_layer_norm = _custom_ops.entry("layer_norm")  # torch.ops.b200.layer_norm
-
-
-def native_layer_norm__default_kernel_impl(*args, **kwargs):
-    return _b200_layer_norm(*args, **kwargs)
+native_layer_norm__default_kernel_impl = _b200_layer_norm

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_layer_norm_backward = _custom_ops.entry("layer_norm_backward")  # torch.ops.b200.layer_norm_backward
-
-
-def native_layer_norm_backward__default_kernel_impl(*args, **kwargs):
-    return _b200_layer_norm_backward(*args, **kwargs)
+native_layer_norm_backward__default_kernel_impl = _b200_layer_norm_backward

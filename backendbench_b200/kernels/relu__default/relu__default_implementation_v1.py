@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_relu = _custom_ops.entry("relu")  # torch.ops.b200.relu
-
-
-def relu__default_kernel_impl(*args, **kwargs):
-    return _b200_relu(*args, **kwargs)
+relu__default_kernel_impl = _b200_relu

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_scatter_add = _custom_ops.entry("scatter_add")  # torch.ops.b200.scatter_add
-
-
-def scatter_add__default_kernel_impl(*args, **kwargs):
-    return _b200_scatter_add(*args, **kwargs)
+scatter_add__default_kernel_impl = _b200_scatter_add

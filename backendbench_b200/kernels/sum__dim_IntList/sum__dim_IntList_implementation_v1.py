@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_sum = _custom_ops.entry("sum")  # torch.ops.b200.sum
-
-
-def sum__dim_IntList_kernel_impl(*args, **kwargs):
-    return _b200_sum(*args, **kwargs)
+sum__dim_IntList_kernel_impl = _b200_sum

@@ -18,7 +18,4 @@ except ImportError:  # loaded by path from outside the repository root
 
 
 _b200_where = _custom_ops.entry("where")  # torch.ops.b200.where
-
-
-def where__self_kernel_impl(*args, **kwargs):
-    return _b200_where(*args, **kwargs)
+where__self_kernel_impl = _b200_where

@@ -19,7 +19,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import torch
 
-from . import _abi
+from . import _abi, _native
 from ._abi import check, i64_array, lib
 
 _DT = {
@@ -427,6 +427,9 @@ def _scratch(device: torch.device, nbytes: int) -> torch.Tensor:
     geometrically, reused; per stream, so that operators queued on different streams never
     share one)."""
     key = (device.index if device.index is not None else torch.cuda.current_device(), _stream_handle())
+    native = _native.module() if _allocator is None else None
+    if native is not None:  # one buffer for the calls that are served here and those that are served there
+        return native.scratch(key[0], key[1], nbytes)
     buf = _scratch_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = _new(max(nbytes, 1 << 20), torch.uint8, device)
