@@ -1024,6 +1024,221 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
   }
 }
 
+// ------------------------------------------------------------------ layer norm, rows off the 16-byte grid
+// A row is dealt out in chunks of E elements, the largest that every row starts on: one, two (16-bit rows
+// of even length), or a whole vector.
+template <typename T, int E> struct RowChunk;  // a chunk as it is loaded
+template <typename T> struct RowChunk<T, 1> {
+  T raw;
+  __device__ __forceinline__ void load(const T* p) { raw = __ldcs(p); }
+  __device__ __forceinline__ void widen_to(float* f) const { f[0] = to_f32(raw); }
+  static __device__ __forceinline__ void store(T* p, const float* f) { __stcs(p, from_f32<T>(f[0])); }
+};
+template <typename T> struct RowChunk<T, 2> {
+  uint32_t raw;
+  __device__ __forceinline__ void load(const T* p) { raw = __ldcs(reinterpret_cast<const uint32_t*>(p)); }
+  __device__ __forceinline__ void widen_to(float* f) const {
+    const T* e = reinterpret_cast<const T*>(&raw);
+    f[0] = to_f32(e[0]);
+    f[1] = to_f32(e[1]);
+  }
+  static __device__ __forceinline__ void store(T* p, const float* f) {
+    const T e[2] = {from_f32<T>(f[0]), from_f32<T>(f[1])};
+    __stcs(reinterpret_cast<uint32_t*>(p), *reinterpret_cast<const uint32_t*>(e));
+  }
+};
+template <typename T> struct RowVector {
+  uint4 raw;
+  __device__ __forceinline__ void load(const T* p) { raw = ld_stream(p); }
+  __device__ __forceinline__ void widen_to(float* f) const { widen<T>(raw, f); }
+  static __device__ __forceinline__ void store(T* p, const float* f) { st_stream(p, narrow<T>(f)); }
+};
+template <> struct RowChunk<float, 4> : RowVector<float> {};
+template <> struct RowChunk<__nv_bfloat16, 8> : RowVector<__nv_bfloat16> {};
+template <> struct RowChunk<__half, 8> : RowVector<__half> {};
+
+// Forward, a CTA to a row, which stays in registers as fp32. Three scalar passes over it (`layernorm_stream`)
+// took bf16 12544 x 2934 192 us, 56 so; fp32 8000 x 8191 356 and 138.
+template <typename T, typename TW, int E, int NPT>
+__global__ void __launch_bounds__(1024) layernorm_rows(const T* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ b, T* __restrict__ y, void* __restrict__ mean, void* __restrict__ rstd, int cols,
+                                                       float eps, int dt_stat) {
+  __shared__ float red[64];
+  const int64_t row = blockIdx.x;
+  const int t = threadIdx.x, tpr = blockDim.x, chunks = cols / E;
+  const T* xr = x + row * cols;
+  RowChunk<T, E> raw[NPT];
+  float f[NPT][E], s = 0.f;
+#pragma unroll
+  for (int u = 0; u < NPT; ++u)
+    if (t + u * tpr < chunks) raw[u].load(xr + (t + u * tpr) * E);
+#pragma unroll
+  for (int u = 0; u < NPT; ++u) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) f[u][e] = 0.f;
+    if (t + u * tpr < chunks) raw[u].widen_to(f[u]);
+#pragma unroll
+    for (int e = 0; e < E; ++e) s += f[u][e];
+  }
+  s = block_reduce_once(s, SumF{}, 0.f, red, 0);
+  float mu = s / static_cast<float>(cols);
+  if (!isfinite(mu)) mu = CUDART_NAN_F;  // same non-finite rule as the resident kernel
+  float q = 0.f;
+#pragma unroll
+  for (int u = 0; u < NPT; ++u)
+    if (t + u * tpr < chunks) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        f[u][e] -= mu;
+        q = fmaf(f[u][e], f[u][e], q);
+      }
+    }
+  q = block_reduce_once(q, SumF{}, 0.f, red, 1);
+  const float rs = rsqrtf(q / static_cast<float>(cols) + eps);
+  if (t == 0) {
+    store_from_f32(mean, row, dt_stat, mu);
+    store_from_f32(rstd, row, dt_stat, rs);
+  }
+#pragma unroll
+  for (int u = 0; u < NPT; ++u) {
+    const int c = (t + u * tpr) * E;
+    if (t + u * tpr < chunks) {
+      float o[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        o[e] = f[u][e] * rs;
+        if (w) o[e] *= to_f32(w[c + e]);
+        if (b) o[e] += to_f32(b[c + e]);
+      }
+      RowChunk<T, E>::store(y + row * cols + c, o);
+    }
+  }
+}
+
+// Backward, as layernorm_bwd_fused: persistent, the next row on its way, dw and db in registers across rows. A row is a
+// CTA's, or, up to 256 elements, a warp's: eight warps of a CTA then add up their shares of dw and db one
+// after the other before they go out, so that short rows fill an SM without many partial rows (a CTA of one warp each, eight to an SM: bf16 20000 x 256
+// 29.8 -> 14.3 us). Ragged rows, in three passes for dx and by columns for dw and db until now: bf16 12544 x 2934 510 -> 75, f16 29952 x 60
+// 240 -> 13.4, fp32 65536 x 33 449 -> 17.6.
+template <typename T, int E, int NPT, bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : 1024)
+layernorm_bwd_rows(const T* __restrict__ dy, const T* __restrict__ x, const void* __restrict__ w, const void* __restrict__ mean, const void* __restrict__ rstd, T* __restrict__ dx,
+                   float* __restrict__ part_w, float* __restrict__ part_b, int64_t rows, int cols, int dt_wb, int dt_stat) {
+  __shared__ float2 red[2][32];
+  __shared__ float share[WARP ? 2 * 32 * NPT * E : 1];
+  const int t = WARP ? threadIdx.x & 31 : threadIdx.x, tpr = WARP ? 32 : blockDim.x, chunks = cols / E;
+  const int64_t row0 = WARP ? static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5) : blockIdx.x, step = static_cast<int64_t>(gridDim.x) * (WARP ? 8 : 1);
+  const float inv_cols = 1.f / static_cast<float>(cols);
+  float wv[NPT][E], aw[NPT][E], ab[NPT][E];
+#pragma unroll
+  for (int u = 0; u < NPT; ++u) {
+    const int j = t + u * tpr;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      aw[u][e] = ab[u][e] = 0.f;
+      wv[u][e] = w && j < chunks ? load_as_f32(w, j * E + e, dt_wb) : 1.f;
+    }
+  }
+  RowChunk<T, E> ndy[NPT], nx[NPT];
+  float nmu = 0.f, nrs = 0.f;
+  auto request = [&](int64_t row) {
+    nmu = load_as_f32(mean, row, dt_stat);
+    nrs = load_as_f32(rstd, row, dt_stat);
+#pragma unroll
+    for (int u = 0; u < NPT; ++u) {
+      const int j = t + u * tpr;
+      if (j < chunks) {
+        ndy[u].load(dy + row * cols + j * E);
+        nx[u].load(x + row * cols + j * E);
+      }
+    }
+  };
+  if (row0 < rows) request(row0);
+  int phase = 0;
+  for (int64_t row = row0; row < rows; row += step, phase ^= 1) {
+    const float mu = nmu, rs = nrs;
+    float g[NPT][E], h[NPT][E], s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int u = 0; u < NPT; ++u) {
+      ndy[u].widen_to(g[u]);
+      nx[u].widen_to(h[u]);
+    }
+    if (row + step < rows) request(row + step);
+#pragma unroll
+    for (int u = 0; u < NPT; ++u)
+      if (t + u * tpr < chunks) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const float xhat = (h[u][e] - mu) * rs;
+          ab[u][e] += g[u][e];
+          aw[u][e] = fmaf(g[u][e], xhat, aw[u][e]);
+          const float gy = g[u][e] * wv[u][e];
+          s1 += gy;
+          s2 = fmaf(gy, xhat, s2);
+          g[u][e] = gy;
+          h[u][e] = xhat;
+        }
+      }
+    s1 = warp_reduce(s1, SumF{});
+    s2 = warp_reduce(s2, SumF{});
+    if constexpr (!WARP) {  // both sums behind one barrier; the row after next is the first to write these slots again
+      if ((t & 31) == 0) red[phase][t >> 5] = make_float2(s1, s2);
+      __syncthreads();
+      const float2 part = (t & 31) < (tpr >> 5) ? red[phase][t & 31] : make_float2(0.f, 0.f);
+      s1 = warp_reduce(part.x, SumF{});
+      s2 = warp_reduce(part.y, SumF{});
+    }
+    const float c1 = s1 * inv_cols, c2 = s2 * inv_cols;
+    if (dx) {
+#pragma unroll
+      for (int u = 0; u < NPT; ++u)
+        if (t + u * tpr < chunks) {
+          float o[E];
+#pragma unroll
+          for (int e = 0; e < E; ++e) o[e] = rs * (g[u][e] - c1 - h[u][e] * c2);
+          RowChunk<T, E>::store(dx + row * cols + (t + u * tpr) * E, o);
+        }
+    }
+  }
+  if (!part_w) return;
+  if constexpr (WARP) {
+    constexpr int kShare = 32 * NPT * E;
+    for (int k = 0; k < 8; ++k) {
+      if (static_cast<int>(threadIdx.x >> 5) == k) {
+#pragma unroll
+        for (int u = 0; u < NPT; ++u) {
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const int i = (u * E + e) * 32 + t;
+            share[i] = k ? share[i] + aw[u][e] : aw[u][e];
+            share[kShare + i] = k ? share[kShare + i] + ab[u][e] : ab[u][e];
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x >= 32) return;
+#pragma unroll
+    for (int u = 0; u < NPT; ++u) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        aw[u][e] = share[(u * E + e) * 32 + t];
+        ab[u][e] = share[kShare + (u * E + e) * 32 + t];
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < NPT; ++u) {
+    const int j = t + u * tpr;
+    if (j < chunks) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        part_w[static_cast<int64_t>(blockIdx.x) * cols + j * E + e] = aw[u][e];
+        part_b[static_cast<int64_t>(blockIdx.x) * cols + j * E + e] = ab[u][e];
+      }
+    }
+  }
+}
+
 // Any row length and alignment. dx: one CTA per row, scalar, three passes (the second and
 // third from cache). dw / db partials: one thread per column walking a chunk of rows
 // (coalesced across columns), one partial row per chunk.
@@ -1073,11 +1288,29 @@ __global__ void __launch_bounds__(1024) layernorm_bwd_finalize(const float* __re
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t c = static_cast<int64_t>(blockIdx.x) * 32 + tx;
   float aw = 0.f, ab = 0.f;
-  if (c < cols)
-    for (int64_t p = ty; p < parts; p += 32) {
-      aw += part_w[p * cols + c];
-      ab += part_b[p * cols + c];
+  after_grids_before();
+  if (c < cols && parts <= 32) {
+    if (ty < parts) {
+      aw = part_w[ty * cols + c];
+      ab = part_b[ty * cols + c];
     }
+  } else if (c < cols) {
+    constexpr int U = 8;  // partial rows on the way (one after the other 1184 of 112 columns took 14.5 us)
+    for (int64_t p0 = ty; p0 < parts; p0 += 32 * U) {
+      float w[U], b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t p = p0 + 32 * u;
+        w[u] = p < parts ? part_w[p * cols + c] : 0.f;
+        b[u] = p < parts ? part_b[p * cols + c] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        aw += w[u];
+        ab += b[u];
+      }
+    }
+  }
   sw[ty][tx] = aw;
   sb[ty][tx] = ab;
   __syncthreads();
@@ -2147,6 +2380,39 @@ extern "C" int b200_argmax(const void* x, int64_t* out, int64_t outer, int64_t d
   }
 }
 
+// Rows off the 16-byte grid, a CTA each: eight elements per thread, or as many as 128 threads leave
+constexpr int64_t kLnRowsMax = 8192;
+static int ln_rows_threads(int64_t cols, int e, int npt) { return static_cast<int>(((cols / e + npt - 1) / npt + 31) / 32 * 32); }
+// go(elements of a chunk, chunks of a thread): 8 elements per thread from 1024 columns on, 4 and 2 below
+template <typename T, typename Go>
+static void with_ln_chunks(bool pairs, int64_t cols, int64_t per_thread8, Go go) {
+  const int elems = cols > per_thread8 / 2 ? 8 : cols > per_thread8 / 4 ? 4 : 2;
+  if constexpr (sizeof(T) == 2) {
+    if (pairs) {
+      if (elems == 8) go(std::integral_constant<int, 2>{}, std::integral_constant<int, 4>{});
+      else if (elems == 4) go(std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
+      else go(std::integral_constant<int, 2>{}, std::integral_constant<int, 1>{});
+      return;
+    }
+  }
+  if (elems == 8) go(std::integral_constant<int, 1>{}, std::integral_constant<int, 8>{});
+  else if (elems == 4) go(std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{});
+  else go(std::integral_constant<int, 1>{}, std::integral_constant<int, 2>{});
+}
+static bool ln_pairs(int64_t cols, std::initializer_list<const void*> ps) {
+  uintptr_t m = static_cast<uintptr_t>(cols) * 2;
+  for (const void* p : ps) m |= reinterpret_cast<uintptr_t>(p);
+  return (m & 3u) == 0;
+}
+template <typename T, typename TW>
+static void layernorm_rows_launch(const void* x, const void* w, const void* b, void* y, void* mean, void* rstd, int64_t rows, int cols, float eps, int dt_stat, cudaStream_t st) {
+  with_ln_chunks<T>(ln_pairs(cols, {x, y}), cols, 1024, [&](auto e, auto npt) {
+    constexpr int E = decltype(e)::value, NPT = decltype(npt)::value;
+    layernorm_rows<T, TW, E, NPT><<<static_cast<unsigned>(rows), ln_rows_threads(cols, E, NPT), 0, st>>>(static_cast<const T*>(x), static_cast<const TW*>(w), static_cast<const TW*>(b), static_cast<T*>(y), mean,
+                                                                                                         rstd, cols, eps, dt_stat);
+  });
+}
+
 extern "C" int b200_layer_norm(const void* x, const void* w, const void* b, void* y, void* mean, void* rstd, int64_t rows, int64_t cols, double eps, int dt, int dt_wb, int dt_stat, void* stream) {
   if (rows < 0 || cols < 0) return B200_EINVAL;
   if (!is_float_dtype(dt) || !is_float_dtype(dt_stat) || ((w || b) && !is_float_dtype(dt_wb))) return B200_EDTYPE;
@@ -2162,13 +2428,36 @@ extern "C" int b200_layer_norm(const void* x, const void* w, const void* b, void
   const bool al = aligned16(x) && aligned16(y) && (!w || aligned16(w)) && (!b || aligned16(b));
   ResidentCfg c{false, false, 1, 128};
   if (cols > 0 && cols % ve == 0 && (dt_wb != B200_F32 || cols % 4 == 0) && al && wb_ok && cols < (1LL << 30)) c = resident_cfg(cols / ve, 32 / ve, ve == 4 ? 4 : 2);
-  if (!c.ok && cols > 0 && cols <= kRaggedMaxCols && rows >= 64) {
+  // ragged rows: a warp each where they are short and many, a CTA each elsewhere (bf16 20000 x 70 8.4 us against 12.7, 20000 x 301 26.4 / 18.4,
+  // 300 x 70 4.1 / 2.8)
+  if (!c.ok && cols > 0 && cols <= 256 && rows >= 4096) {
     const unsigned g = grid_for(rows, 4);
     const int ci = static_cast<int>(cols);
+    auto go = [&](auto npl) {
+      constexpr int NPL = decltype(npl)::value;
+      switch (dt) {
+        case B200_F32: layernorm_warp_ragged<float, NPL><<<g, 128, 0, st>>>(static_cast<const float*>(x), w, b, static_cast<float*>(y), mean, rstd, rows, ci, e, dt_wb, dt_stat); break;
+        case B200_BF16: layernorm_warp_ragged<__nv_bfloat16, NPL><<<g, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(x), w, b, static_cast<__nv_bfloat16*>(y), mean, rstd, rows, ci, e, dt_wb, dt_stat); break;
+        default: layernorm_warp_ragged<__half, NPL><<<g, 128, 0, st>>>(static_cast<const __half*>(x), w, b, static_cast<__half*>(y), mean, rstd, rows, ci, e, dt_wb, dt_stat); break;
+      }
+    };
+    if (cols <= 64) go(std::integral_constant<int, 2>{});
+    else if (cols <= 128) go(std::integral_constant<int, 4>{});
+    else go(std::integral_constant<int, 8>{});
+    return check_launch();
+  }
+  if (!c.ok && cols > 0 && cols <= kLnRowsMax && wb_ok) {
+    const bool f32 = (w || b) && dt_wb == B200_F32;
     switch (dt) {
-      case B200_F32: B200_DISPATCH_NPL(cols, (layernorm_warp_ragged<float, NPL><<<g, 128, 0, st>>>(static_cast<const float*>(x), w, b, static_cast<float*>(y), mean, rstd, rows, ci, e, dt_wb, dt_stat))) break;
-      case B200_BF16: B200_DISPATCH_NPL(cols, (layernorm_warp_ragged<__nv_bfloat16, NPL><<<g, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(x), w, b, static_cast<__nv_bfloat16*>(y), mean, rstd, rows, ci, e, dt_wb, dt_stat))) break;
-      default: B200_DISPATCH_NPL(cols, (layernorm_warp_ragged<__half, NPL><<<g, 128, 0, st>>>(static_cast<const __half*>(x), w, b, static_cast<__half*>(y), mean, rstd, rows, ci, e, dt_wb, dt_stat))) break;
+      case B200_F32: layernorm_rows_launch<float, float>(x, w, b, y, mean, rstd, rows, static_cast<int>(cols), e, dt_stat, st); break;
+      case B200_BF16:
+        if (f32) layernorm_rows_launch<__nv_bfloat16, float>(x, w, b, y, mean, rstd, rows, static_cast<int>(cols), e, dt_stat, st);
+        else layernorm_rows_launch<__nv_bfloat16, __nv_bfloat16>(x, w, b, y, mean, rstd, rows, static_cast<int>(cols), e, dt_stat, st);
+        break;
+      default:
+        if (f32) layernorm_rows_launch<__half, float>(x, w, b, y, mean, rstd, rows, static_cast<int>(cols), e, dt_stat, st);
+        else layernorm_rows_launch<__half, __half>(x, w, b, y, mean, rstd, rows, static_cast<int>(cols), e, dt_stat, st);
+        break;
     }
     return check_launch();
   }
@@ -2227,6 +2516,40 @@ static int layernorm_bwd_fused_per_sm(int threads, int vpt) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
+// Launches layernorm_bwd_rows; the number of partial rows.
+template <typename T, int E, int NPT, bool WARP>
+static int64_t layernorm_bwd_rows_go(const void* dy, const void* x, const void* w, const void* mean, const void* rstd, void* dx, float* pw, float* pb, int64_t rows, int cols, int dt_wb, int dt_stat,
+                                     int64_t parts_max, cudaStream_t st) {
+  auto kernel = layernorm_bwd_rows<T, E, NPT, WARP>;
+  const int threads = WARP ? 256 : ln_rows_threads(cols, E, NPT);
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+  int64_t grid = static_cast<int64_t>(per_sm > 8 ? 8 : per_sm) * kNumSMs;
+  const int64_t need = WARP ? (rows + 7) / 8 : rows;
+  if (grid > need) grid = need;
+  if (grid > parts_max) grid = parts_max;
+  kernel<<<static_cast<unsigned>(grid), threads, 0, st>>>(static_cast<const T*>(dy), static_cast<const T*>(x), w, mean, rstd, static_cast<T*>(dx), pw, pb, rows, cols, dt_wb, dt_stat);
+  return grid;
+}
+template <typename T>
+static int64_t layernorm_bwd_rows_launch(const void* dy, const void* x, const void* w, const void* mean, const void* rstd, void* dx, float* pw, float* pb, int64_t rows, int cols, int dt_wb, int dt_stat,
+                                         bool vectors, int64_t parts_max, cudaStream_t st) {
+  constexpr int VE = Vec<T>::N;
+  int64_t parts = 0;
+  auto go = [&](auto e, auto npt, auto warp) {
+    parts = layernorm_bwd_rows_go<T, decltype(e)::value, decltype(npt)::value, decltype(warp)::value>(dy, x, w, mean, rstd, dx, pw, pb, rows, cols, dt_wb, dt_stat, parts_max, st);
+  };
+  if (vectors) {  // at most 256 columns
+    if (cols <= 32 * VE) go(std::integral_constant<int, VE>{}, std::integral_constant<int, 1>{}, std::true_type{});
+    else if constexpr (VE == 4) go(std::integral_constant<int, VE>{}, std::integral_constant<int, 2>{}, std::true_type{});
+  } else if (cols <= 256) {
+    with_ln_chunks<T>(ln_pairs(cols, {dy, x, dx}), cols, 256, [&](auto e, auto npt) { go(e, npt, std::true_type{}); });
+  } else {
+    with_ln_chunks<T>(ln_pairs(cols, {dy, x, dx}), cols, 1024, [&](auto e, auto npt) { go(e, npt, std::false_type{}); });
+  }
+  return parts;
+}
+
 extern "C" int b200_layer_norm_backward(const void* dy, const void* x, const void* mean, const void* rstd, const void* w, void* dx, void* dw, void* db, int64_t rows, int64_t cols, int dt,
                                         int dt_wb, int dt_stat, void* scratch, int64_t scratch_bytes, void* stream) {
   if (rows < 0 || cols < 0) return B200_EINVAL;
@@ -2256,7 +2579,15 @@ extern "C" int b200_layer_norm_backward(const void* dy, const void* x, const voi
   // and db): one 16-byte vector of a 16-bit row, two of an fp32 row -- rows of up to 8192
   // elements; longer ones would spill
   const int target = ve == 4 ? 2 : 1;
-  if (cols % ve == 0 && (dt_wb != B200_F32 || !w || cols % 4 == 0) && al && wb_ok && cols / ve <= 1024 * target) {
+  const bool vectors = cols % ve == 0 && al;
+  if (vectors ? cols <= 256 && rows >= 64 : cols <= kLnRowsMax) {
+    const int ci = static_cast<int>(cols);
+    switch (dt) {
+      case B200_F32: parts = layernorm_bwd_rows_launch<float>(dy, x, w, mean, rstd, dx, pw, pb, rows, ci, dt_wb, dt_stat, vectors, parts_max, st); break;
+      case B200_BF16: parts = layernorm_bwd_rows_launch<__nv_bfloat16>(dy, x, w, mean, rstd, dx, pw, pb, rows, ci, dt_wb, dt_stat, vectors, parts_max, st); break;
+      default: parts = layernorm_bwd_rows_launch<__half>(dy, x, w, mean, rstd, dx, pw, pb, rows, ci, dt_wb, dt_stat, vectors, parts_max, st); break;
+    }
+  } else if (vectors && (dt_wb != B200_F32 || !w || cols % 4 == 0) && wb_ok && cols / ve <= 1024 * target) {
     const int64_t nvec = cols / ve;
     int threads = 32;
     while (threads < 1024 && threads * target < nvec) threads <<= 1;
@@ -2297,7 +2628,14 @@ extern "C" int b200_layer_norm_backward(const void* dy, const void* x, const voi
       layernorm_bwd_wb_lines<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(parts)), 256, 0, st>>>(dy, x, mean, rstd, pw, pb, rows, cols, rows_per, dt, dt_stat);
     }
   }
-  if (need_wb) layernorm_bwd_finalize<<<grid_for(cols, 32), 1024, 0, st>>>(pw, pb, dw, db, parts, cols, dt_wb);
+  if (need_wb) {
+    if (parts <= 32) {
+      layernorm_bwd_finalize<<<grid_for(cols, 32), 1024, 0, st>>>(pw, pb, dw, db, parts, cols, dt_wb);
+    } else {
+      const cudaError_t e = launch_after(layernorm_bwd_finalize, grid_for(cols, 32), 1024, 0, st, pw, pb, dw, db, parts, cols, dt_wb);
+      if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+    }
+  }
   return check_launch(need_wb ? 2 : 1);
 }
 

@@ -368,3 +368,37 @@ def test_autograd_through_registered_overrides():
     finally:
         bb.disable()
     torch.testing.assert_close(emb.weight.grad, want_w, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [1, 2, 9, 31, 33, 62, 63, 65, 66, 126, 127, 129, 250, 255, 256, 257, 258, 511, 513, 1023, 1026, 2047, 2934, 8190, 8191])
+def test_layer_norm_of_ragged_rows(backend, dtype, cols):
+    """Rows off the 16-byte grid, and short ones on it: whole rows in chunks of one or two elements or a vector, a warp or a CTA to a
+    row, rows that start between two words, more and fewer rows than there are warps. Each result is within its own
+    rounding (2^-24, 2^-8, 2^-11 of the value and a binade) plus a few fp32 roundings of the terms it is made of."""
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    unit = {torch.float32: 2.0**-23, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype]
+    forward, backward = backend[get_operator("native_layer_norm.default")], backend[get_operator("native_layer_norm_backward.default")]
+
+    def within(got, exact, scale):
+        assert bool(((got.double() - exact).abs() <= unit * exact.abs() + 2.0**-19 * scale + (2.0**-24 if dtype == torch.float16 else 0)).all())
+
+    for rows in (5, 700) + ((4099,) if cols < 300 else ()):
+        x, dy = (torch.randn(rows * cols + 1, device=DEV, generator=g).to(dtype)[k : k + rows * cols].view(rows, cols) for k in (1, 0))
+        for params in (dtype, torch.float32):
+            w, b = (torch.randn(cols, device=DEV, generator=g) * 0.3 + 1).to(params), torch.randn(cols, device=DEV, generator=g).to(params)
+            y, mean, rstd = forward(x, [cols], w, b, 1e-3)
+            X, W = x.double(), w.double()
+            mu = X.mean(1, keepdim=True)
+            rs = (X.sub(mu).square().mean(1, keepdim=True) + 1e-3).rsqrt()
+            assert bool(((mean.double() - mu).abs() <= 2.0**-20 * X.abs().mean(1, keepdim=True)).all()) and bool(((rstd.double() / rs - 1).abs() <= 2.0**-18).all())
+            within(y, (X - mu) * rs * W + b.double(), ((X - mu).abs() * rs + (X.abs().mean(1, keepdim=True)) * rs + 1) * (W.abs() + b.double().abs() + 1))
+            dx, dw, db = backward(dy, x, [cols], mean, rstd, w, b, [True, True, True])
+            D, M, R = dy.double(), mean.double(), rstd.double()
+            xh, gy = (X - M) * R, D * W
+            within(dx, R * (gy - gy.mean(1, keepdim=True) - xh * (gy * xh).mean(1, keepdim=True)), R * (gy.abs() + gy.abs().mean(1, keepdim=True) + xh.abs() * (gy * xh).abs().mean(1, keepdim=True) + 1))
+            within(dw, (D * xh).sum(0), (D * xh).abs().sum(0) + rows)
+            within(db, D.sum(0), D.abs().sum(0))
+            only = backward(dy, x, [cols], mean, rstd, w, b, [True, False, False])
+            assert torch.equal(only[0], dx) and only[1] is None and only[2] is None
+            assert all(torch.equal(p, q) for p, q in zip(backward(dy, x, [cols], mean, rstd, w, b, [False, True, True])[1:], (dw, db)))
