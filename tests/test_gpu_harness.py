@@ -245,3 +245,33 @@ def test_trace_replay_through_the_cli_on_the_gpu(tmp_path):
     assert r.exit_code == 0, r.output
     assert "correctness score (mean pass rate over all operators): 1.00" in r.output
     assert (out / "full_results.json").exists() and (out / "operator_summary.csv").exists()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16, torch.int64])
+@pytest.mark.parametrize("n", [1, 7, 2047, 2048, 2049, 2056, 4097, 32768, 32769, 65536, 65537, 100003])
+def test_the_record_is_whole_whoever_writes_it(dtype, n):
+    """One CTA, a cluster, or many CTAs behind a memset: mismatches are counted wherever they lie (each part of the tensor, its
+    last element, an operand off the 16-byte grid), the largest errors and the NaN flag found, and an old record leaves no trace."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    base = torch.randint(-50, 50, (n + 1,), generator=g, device=DEV).to(dtype)
+    rec = torch.empty(8, dtype=torch.int32, device=DEV)
+    for off in (0, 1):
+        x = base[off : n + off]
+        y = x.clone()
+        where = sorted({0, n // 9, n // 2, n - 1, max(n - 2, 0)})
+        for i in where:
+            y[i] = 100
+        want = int((x != y).sum())
+        for ref, res, bad in ((x, y, want), (y, x, want), (x, x, 0)):
+            rec.fill_(-1)
+            assert ev.compare_enqueue(ref, res, 0.0, 0.0, rec)
+            mism, mabs, mrel, nan_seen = ev.decode_record(rec.tolist())
+            d = (ref.double() - res.double()).abs()
+            assert mism == bad and mabs == float(d.max()) and not nan_seen and rec.tolist()[5:] == [0, 0, 0]
+            assert mrel == pytest.approx(float((d / (ref.double().abs() + 1e-10)).max()), rel=1e-5)
+        if dtype.is_floating_point:
+            y[n // 2] = float("nan")
+            rec.fill_(-1)
+            ev.compare_enqueue(x, y, 0.0, 0.0, rec)
+            mism, _, _, nan_seen = ev.decode_record(rec.tolist())
+            assert nan_seen and mism == want
