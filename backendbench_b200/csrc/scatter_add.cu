@@ -792,6 +792,7 @@ __device__ __forceinline__ void assign_segments_of(const int* __restrict__ cnt, 
 template <int ITEMS>
 __global__ void __launch_bounds__(256) assign_segments(const int* __restrict__ cnt, int* __restrict__ cursor, int64_t n, int* __restrict__ total, int light, int* __restrict__ heavy_count,
                                                        int* __restrict__ heavy_list) {
+  after_grids_before();
   assign_segments_of<ITEMS>(cnt, 0, cursor, n, total, light, heavy_count, heavy_list);
 }
 
@@ -1613,7 +1614,7 @@ static BinnedScratch binned_scratch(const BinnedArgs& A, int es, int64_t n_self,
   s.head_bytes = up256(4 * n_self);
   s.list_bytes = up256(4 * (n_idx / (kLightMax + 1) + 1));
   s.seg_bytes = up256(8 * n_idx);
-  // the records, or what group_rest needs in their place
+  // the records, or what the groups of launch_group need in their place
   const int64_t grouped = 2 * s.head_bytes + s.list_bytes + s.seg_bytes;
   s.total = 256 + (s.first_bytes + s.rec_bytes > grouped ? s.first_bytes + s.rec_bytes : grouped);
   return s;
@@ -1674,6 +1675,7 @@ __global__ void __launch_bounds__(256) emb_count(const void* __restrict__ idx, i
   }
 }
 __global__ void __launch_bounds__(256) emb_fill(const void* __restrict__ idx, int i32, int64_t n, int64_t V, int64_t padding_idx, int* __restrict__ cursor, int* __restrict__ seg_pos) {
+  after_grids_before();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t v = emb_index(idx, i, i32);
     if (v == padding_idx || v < 0 || v >= V) continue;
@@ -1691,6 +1693,7 @@ __global__ void __launch_bounds__(256) emb_sort(const int* __restrict__ cnt, con
   __shared__ int before[kEmbWindowWords];
   __shared__ int warp_sums[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  after_grids_before();
   const int nheavy = *heavy_count;
   for (int h = blockIdx.x; h < nheavy; h += gridDim.x) {
     const int64_t v = heavy_list[h];
@@ -1762,6 +1765,66 @@ __global__ void __launch_bounds__(256) emb_sort(const int* __restrict__ cnt, con
   }
 }
 
+// Few tokens and a short table: one CTA sorts (row, position) as one word and reads the segments off the sorted
+// words, in place of a memset and the four kernels above, whose launches are most of what they take (254 tokens on 43 rows
+// of 47 the call 18.8 us, 9.3 so). From some 2000 tokens on the one CTA takes longer.
+constexpr int kEmbSmallTokens = 1024, kEmbSmallRows = 1 << 15;
+__global__ void __launch_bounds__(kEmbSmallTokens / 2) emb_small(const void* __restrict__ idx, int i32, int n, int V, int64_t padding_idx, int* __restrict__ cnt, int* __restrict__ cursor, int* __restrict__ sorted,
+                                                  int* __restrict__ heavy_count, int* __restrict__ heavy_list, int slots, uint32_t* status) {
+  constexpr uint32_t kNone = 0xffffffffu;
+  constexpr int kPosBits = 10;
+  static_assert(kEmbSmallTokens == 1 << kPosBits, "a position in the low bits of a word");
+  __shared__ uint32_t key[kEmbSmallTokens];
+  __shared__ int heavy;
+  const int t = threadIdx.x;
+  if (t == 0) heavy = 0;
+  for (int i = t; i < slots; i += blockDim.x) {
+    uint32_t k = kNone;
+    if (i < n) {
+      const int64_t v = emb_index(idx, i, i32);
+      if (v == padding_idx) k = kNone;
+      else if (v < 0 || v >= V) flag_oob(status);
+      else k = static_cast<uint32_t>(v) << kPosBits | static_cast<uint32_t>(i);
+    }
+    key[i] = k;
+  }
+  for (int v = t; v < V; v += blockDim.x) cnt[v] = 0;
+  __syncthreads();
+  for (int size = 2; size <= slots; size <<= 1) {  // bitonic; `slots` is a power of two
+    for (int gap = size >> 1; gap > 0; gap >>= 1) {
+      for (int i = t; i < slots / 2; i += blockDim.x) {
+        const int a = 2 * i - (i & (gap - 1)), b = a + gap;
+        const uint32_t x = key[a], y = key[b];
+        if ((x > y) == ((a & size) == 0)) {
+          key[a] = y;
+          key[b] = x;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int i = t; i < n; i += blockDim.x) {
+    const uint32_t k = key[i];
+    if (k == kNone) continue;
+    sorted[i] = static_cast<int>(k & ((1u << kPosBits) - 1u));
+    const uint32_t v = k >> kPosBits;
+    if (i + 1 < n && key[i + 1] >> kPosBits == v) continue;
+    // the last of its row: the first one is found by bisection
+    int lo = 0, hi = i;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (key[mid] >> kPosBits < v) lo = mid + 1;
+      else hi = mid;
+    }
+    const int c = i + 1 - lo;
+    cnt[v] = c;  // (every counter was cleared before the barriers above)
+    cursor[v] = i + 1;
+    if (c > kEmbLight) heavy_list[atomicAdd(&heavy, 1)] = static_cast<int>(v);
+  }
+  __syncthreads();
+  if (t == 0) *heavy_count = heavy;
+}
+
 // WORD: the type of one load of the long rows (4 bytes where row length and bases allow it)
 template <typename T, typename WORD> __device__ __forceinline__ void emb_word_add(float* acc, WORD w) {
   if constexpr (sizeof(WORD) == sizeof(T)) {
@@ -1776,9 +1839,9 @@ template <typename T, typename WORD> __device__ __forceinline__ void emb_word_ad
 template <typename T, bool VEC, typename WORD>
 __global__ void __launch_bounds__(256, 4) emb_replay(const T* __restrict__ grad, T* __restrict__ out, const int* __restrict__ cnt, const int* __restrict__ cursor, const int* __restrict__ sorted,
                                                      int64_t V, int64_t D, const int* __restrict__ heavy_count, const int* __restrict__ heavy_list, int heavy_blocks, int tx_log2) {
+  after_grids_before();
   if (static_cast<int>(blockIdx.x) < heavy_blocks) {
     constexpr int PK = sizeof(WORD) / sizeof(T);
-    constexpr int kBatch = sizeof(WORD) == 4 ? 32 : 16;  // loads in flight (32 of the narrow kind would spill)
     const int lane = threadIdx.x & 31;
     const int64_t words = D / PK, chunks = (words + 31) / 32;
     const int64_t nunits = *heavy_count * chunks;
@@ -1789,21 +1852,27 @@ __global__ void __launch_bounds__(256, 4) emb_replay(const T* __restrict__ grad,
       const int64_t v = heavy_list[h];
       const int c = cnt[v];
       const int* seg = sorted + (cursor[v] - c);
-      const int64_t wc = w < words ? w : words - 1;  // lanes past the row read its last word and store nothing
+      const WORD* gl = gw + (w < words ? w : words - 1);  // lanes past the row read its last word and store nothing
       float acc[PK];
 #pragma unroll
       for (int q = 0; q < PK; ++q) acc[q] = 0.f;
+      // 32 rows at a time. A lane works out where one of the next 32 lies, and brings its line into L2 a batch ahead;
+      // the lanes hand these around. (With a product per load, and 16 at a time of 2-byte words: f16 21648 tokens on 56 rows of 3527
+      // 416 us the call, 180 so; bf16 32768 tokens on 16 rows of 4096 399, 278. Half a batch on its way while the other is added: 445.)
+      auto row_of = [&](int k) { return k + lane < c ? static_cast<int64_t>(seg[k + lane]) * words : 0; };
+      int64_t at = row_of(0), ahead = row_of(32);
       int k0 = 0;
-      int p = lane < c && lane < kBatch ? seg[lane] : 0;
-      for (; k0 + kBatch <= c; k0 += kBatch) {
-        WORD r[kBatch];
+      for (; k0 + 32 <= c; k0 += 32) {
+        WORD r[32];
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) r[k] = gw[static_cast<int64_t>(__shfl_sync(0xffffffffu, p, k)) * words + wc];
-        p = k0 + kBatch + lane < c && lane < kBatch ? seg[k0 + kBatch + lane] : 0;
+        for (int k = 0; k < 32; ++k) r[k] = gl[__shfl_sync(0xffffffffu, at, k)];
+        at = ahead;
+        ahead = row_of(k0 + 64);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(gw + (w - lane) + ahead));
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) emb_word_add<T, WORD>(acc, r[k]);
+        for (int k = 0; k < 32; ++k) emb_word_add<T, WORD>(acc, r[k]);
       }
-      for (int k = 0; k < c - k0; ++k) emb_word_add<T, WORD>(acc, gw[static_cast<int64_t>(__shfl_sync(0xffffffffu, p, k)) * words + wc]);
+      for (int k = 0; k < c - k0; ++k) emb_word_add<T, WORD>(acc, gl[__shfl_sync(0xffffffffu, at, k)]);
       if (w < words) {
         WORD o;
         T* e = reinterpret_cast<T*>(&o);
@@ -1813,6 +1882,36 @@ __global__ void __launch_bounds__(256, 4) emb_replay(const T* __restrict__ grad,
       }
     }
     return;
+  }
+  if constexpr (!VEC) {
+    if (tx_log2 < 0) {
+      // rows off the 16-byte grid, most of them without a contribution: 16 bytes of the table to a thread, which meet one row
+      // or two (fp32 39666 x 363, one token: element by element the call took 35 us, 20 so)
+      constexpr int VE = Vec<T>::N;
+      const int64_t total = V * D, step = static_cast<int64_t>(gridDim.x - heavy_blocks) * (256 * VE);
+      for (int64_t p = (static_cast<int64_t>(blockIdx.x - heavy_blocks) * 256 + threadIdx.x) * VE; p < total; p += step) {
+        const int64_t v = total <= 0x7fffffffLL ? static_cast<int64_t>(static_cast<uint32_t>(p) / static_cast<uint32_t>(D)) : p / D;
+        const int64_t u0 = p - v * D;
+        const bool crosses = u0 + VE > D && v + 1 < V;
+        const int c0 = cnt[v], c1 = crosses ? cnt[v + 1] : 0;
+        if ((c0 | c1) == 0 && p + VE <= total) {
+          st_stream(out + p, make_uint4(0, 0, 0, 0));
+          continue;
+        }
+        for (int e = 0; e < VE && p + e < total; ++e) {
+          const bool next = u0 + e >= D;
+          const int64_t row = next ? v + 1 : v, u = next ? u0 + e - D : u0 + e;
+          const int c = next ? c1 : c0;
+          if (c > kEmbLight) continue;  // a long row: not ours
+          const int* seg = sorted + (c ? cursor[row] - c : 0);
+          float acc = 0.f;
+#pragma unroll 4
+          for (int k = 0; k < c; ++k) acc += to_f32(grad[static_cast<int64_t>(seg[k]) * D + u]);
+          out[p + e] = from_f32<T>(acc);
+        }
+      }
+      return;
+    }
   }
   constexpr int VE = VEC ? Vec<T>::N : 1;
   const int64_t units = D / VE;
@@ -1886,16 +1985,25 @@ static int launch_embedding_backward(const void* grad, const void* idx, void* ou
   int* seg_pos = reinterpret_cast<int*>(base + S.cnt_bytes + S.cursor_bytes);
   int* sorted = reinterpret_cast<int*>(base + S.cnt_bytes + S.cursor_bytes + S.pos_bytes);
   int* heavy = reinterpret_cast<int*>(base + S.cnt_bytes + S.cursor_bytes + 2 * S.pos_bytes);
-  const cudaError_t e = cudaMemsetAsync(head, 0, static_cast<size_t>(S.cnt_bytes), st);
-  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
   auto grid = [](int64_t items, int per, int64_t cap) { const int64_t g = (items + per - 1) / per; return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g)); };
-  emb_count<<<grid(n, 256, 32 * kNumSMs), 256, 0, st>>>(idx, i32, n, V, padding_idx, cnt, status);
-  assign_segments<4><<<static_cast<unsigned>((V + 1023) / 1024), 256, 0, st>>>(cnt, cursor, V, head, kEmbLight, head + 1, heavy);
-  emb_fill<<<grid(n, 256, 32 * kNumSMs), 256, 0, st>>>(idx, i32, n, V, padding_idx, cursor, seg_pos);
-  // a CTA to 256 rows of the table or to one long row, of which a short table under many tokens has more (fp32, 32768
-  // tokens on 256 rows of 64: 88 us the call, 424 with the one CTA that the table alone asks for)
-  const int64_t long_rows = n / (kEmbLight + 1) < V ? n / (kEmbLight + 1) : V, row_groups = (V + 255) / 256;
-  emb_sort<<<grid(long_rows > row_groups ? long_rows : row_groups, 1, 2 * kNumSMs), 256, 0, st>>>(cnt, cursor, seg_pos, sorted, V, n, head + 1, heavy);
+  int launches = 2;
+  cudaError_t e = cudaSuccess;
+  if (n <= kEmbSmallTokens && V <= kEmbSmallRows) {
+    int slots = 32;
+    while (slots < n) slots <<= 1;
+    emb_small<<<1, slots / 2 < 64 ? 64 : slots / 2, 0, st>>>(idx, i32, static_cast<int>(n), static_cast<int>(V), padding_idx, cnt, cursor, sorted, head + 1, heavy, slots, status);
+  } else {
+    e = cudaMemsetAsync(head, 0, static_cast<size_t>(S.cnt_bytes), st);
+    if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+    emb_count<<<grid(n, 256, 32 * kNumSMs), 256, 0, st>>>(idx, i32, n, V, padding_idx, cnt, status);
+    e = launch_after(assign_segments<4>, (V + 1023) / 1024, 256, 0, st, cnt, cursor, V, head, kEmbLight, head + 1, heavy);
+    if (e == cudaSuccess) e = launch_after(emb_fill, grid(n, 256, 32 * kNumSMs), 256, 0, st, idx, i32, n, V, padding_idx, cursor, seg_pos);
+    // a CTA to 256 rows of the table or to one long row, of which a short table under many tokens has more (fp32, 32768
+    // tokens on 256 rows of 64: 88 us the call, 424 with the one CTA that the table alone asks for)
+    const int64_t long_rows = n / (kEmbLight + 1) < V ? n / (kEmbLight + 1) : V, row_groups = (V + 255) / 256;
+    if (e == cudaSuccess) e = launch_after(emb_sort, grid(long_rows > row_groups ? long_rows : row_groups, 1, 2 * kNumSMs), 256, 0, st, cnt, cursor, seg_pos, sorted, V, n, head + 1, heavy);
+    launches = 5;
+  }
   const T* g = static_cast<const T*>(grad);
   T* o = static_cast<T*>(out);
   const bool vec = (D * static_cast<int64_t>(sizeof(T))) % 16 == 0 && aligned16(grad) && aligned16(out);
@@ -1911,12 +2019,18 @@ static int launch_embedding_backward(const void* grad, const void* idx, void* ou
   }
   // a table so short that a list of long rows cannot exist gets no CTAs for it
   const int heavy_blocks = n > kEmbLight ? grid(n / (kEmbLight + 1) * ((D * static_cast<int64_t>(sizeof(T)) + 127) / 128), 8, kNumSMs) : 0;
-  const int light_blocks = grid(V, 256 >> tx_log2, 8 * kNumSMs);
-  auto launch = [&](auto kernel) { kernel<<<heavy_blocks + light_blocks, 256, 0, st>>>(g, o, cnt, cursor, sorted, V, D, head + 1, heavy, heavy_blocks, tx_log2); };
+  // (flat: 16 bytes of the table to a thread, see emb_replay)
+  const bool flat = !vec && n <= V && D * static_cast<int64_t>(sizeof(T)) >= 16 && aligned16(out);
+  const int light_blocks = flat ? grid(V * D, 256 * Vec<T>::N, 16 * kNumSMs) : grid(V, 256 >> tx_log2, 8 * kNumSMs);
+  if (flat) tx_log2 = -1;
+  auto launch = [&](auto kernel) {
+    if (e == cudaSuccess) e = launch_after(kernel, heavy_blocks + light_blocks, 256, 0, st, g, o, cnt, cursor, sorted, V, D, head + 1, heavy, heavy_blocks, tx_log2);
+  };
   if (vec) launch(emb_replay<T, true, uint32_t>);
   else if (words) launch(emb_replay<T, false, uint32_t>);
   else if constexpr (sizeof(T) == 2) launch(emb_replay<T, false, uint16_t>);
-  return check_launch(5);
+  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+  return check_launch(launches);
 }
 
 template <typename T>

@@ -244,6 +244,29 @@ def test_embedding_backward_at_the_edges_of_its_batches_and_windows(backend, dty
     assert bits_equal(oracle.embedding_backward(grad, idx, V, 7, False), got.cpu())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V,n,D", [(1, 1, 1), (2, 33, 4), (32768, 1024, 9), (32769, 1024, 9), (40000, 1025, 12), (9, 1024, 67), (5, 1025, 67), (3000, 65, 11), (70, 64, 4), (1030, 1000, 5)])
+def test_embedding_backward_of_few_tokens(backend, dtype, V, n, D):
+    """Both sides of the limits below which one CTA sorts the tokens, and tables off the 16-byte grid that are
+    written 16 bytes at a time (a word over two rows, long rows among them), padding and rows out of range, bit for bit."""
+    from conftest import bits_equal
+
+    g = torch.Generator().manual_seed(V + n)
+    idx = torch.randint(0, V, (n,), generator=g)
+    if n >= 64:
+        idx[torch.randperm(n, generator=g)[: n - 20]] = V - 1  # a long row; its neighbour is written by another thread
+    grad = torch.randn((n, D), generator=g).to(dtype)
+    pad = int(idx[-1]) if n == 33 else -1
+    got = backend[get_operator(EMB)](grad.to(DEV), idx.to(DEV), V, pad, False)
+    ops.check_device_status()
+    assert bits_equal(oracle.embedding_backward(grad, idx, V, pad, False), got.cpu())
+    if n >= 64:
+        idx[3] = V
+        backend[get_operator(EMB)](grad.to(DEV), idx.to(DEV), V, pad, False)
+        with pytest.raises(IndexError):
+            ops.check_device_status()
+
+
 @pytest.mark.parametrize("V,n,D", [(1, 5000, 9), (3, 40000, 64), (40, 3000, 192), (256, 20000, 63), (256, 20000, 200), (1000, 40000, 8)])
 def test_embedding_backward_of_short_tables_under_many_tokens(backend, V, n, D):
     """More rows of many contributions than groups of 256 table rows: they are sorted by CTAs of their own."""
