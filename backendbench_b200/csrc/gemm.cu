@@ -17,6 +17,7 @@ bool gemm_mma_small_preferred(const void* A, const void* B, int64_t batch, int64
                               int dtype);
 int gemm_mma_small_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb,
                             int64_t sBk, int64_t sBn, int64_t sbm, int64_t sbn, double alpha, double beta, int dtype, cudaStream_t st);
+bool gemm_deep_preferred(int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAk, int64_t sBn, int dtype);
 bool gemm_few_rows_preferred(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sAk, int64_t sBk, int64_t sBn, int dtype);
 bool gemm_few_rows_leaves_to_ranges(int64_t N, int64_t K);
 int gemm_few_rows_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sBn, int64_t sbm, int64_t sbn, double alpha,
@@ -30,10 +31,11 @@ bool gemm_f32_split_eligible(int64_t batch, int64_t M, int64_t N, int64_t K);
 int gemm_f32_split_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb,
                             int64_t sBk, int64_t sBn, int64_t sbm, int64_t sbn, double alpha, double beta, void* scratch, int64_t scratch_bytes, uint32_t* status, cudaStream_t st);
 
-// 1: small 16-bit products and those with few rows take the mma.sync kernels (the default); 0:
-// they go where they went without them (tcgen05 or CUDA cores) -- how the two are compared and the larger kernels tested
+// 1: small 16-bit products and those with few rows take the mma.sync kernels, those with few outputs and a long contraction
+// the kernel of gemm_deep.cu (the default); 0: they go where they went without them (tcgen05 or CUDA cores) -- how the two are compared and the larger kernels tested
 // on small shapes.
 static std::atomic<int> g_small_path{1};
+bool gemm_small_path_on() { return g_small_path.load(std::memory_order_relaxed) != 0; }
 
 __global__ void fill_bias_only(void* C, const void* bias, int64_t batch, int64_t M, int64_t N, int64_t sbm, int64_t sbn, float beta, int dt) {
   const int64_t total = batch * M * N;
@@ -66,9 +68,9 @@ extern "C" int b200_gemm(const void* A, const void* B, const void* bias, void* C
     return check_launch();
   }
   if (!A || !B) return B200_EINVAL;
-  if (g_small_path.load(std::memory_order_relaxed) && gemm_mma_small_preferred(A, B, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype))
+  if (gemm_small_path_on() && gemm_mma_small_preferred(A, B, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype))
     return gemm_mma_small_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, dtype, st);
-  if (g_small_path.load(std::memory_order_relaxed) && gemm_few_rows_preferred(A, B, batch, M, N, K, sAm, sAk, sBk, sBn, dtype))
+  if (gemm_small_path_on() && gemm_few_rows_preferred(A, B, batch, M, N, K, sAm, sAk, sBk, sBn, dtype))
     return gemm_few_rows_dispatch(A, B, bias, C, M, N, K, sAm, sBn, sbm, sbn, alpha, beta, dtype, st);
   if (gemm_tc_eligible(batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype, A, B, C))
     return gemm_tc_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, dtype, status, st);
@@ -84,7 +86,8 @@ extern "C" int b200_gemm_wait_probe(const void* A, const void* B, void* C, int64
 }
 
 extern "C" int64_t b200_gemm_f32_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
-  if (!gemm_f32_split_eligible(batch, M, N, K)) return 0;
+  // (few outputs: the CUDA cores, whatever the order of B)
+  if (!gemm_f32_split_eligible(batch, M, N, K) || gemm_deep_preferred(batch, M, N, K, 0, 0, B200_F32)) return 0;
   return gemm_f32_split_scratch_bytes(batch, M, N, K);
 }
 
@@ -101,7 +104,7 @@ extern "C" int b200_gemm_f32(const void* A, const void* B, const void* bias, voi
 extern "C" int64_t b200_gemm_splitk_scratch_bytes(const void* A, const void* B, const void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk,
                                                   int64_t sBb, int64_t sBk, int64_t sBn, int dtype) {
   if (batch != 1 || M < 1 || N < 1 || K < 1) return 0;
-  if (g_small_path.load(std::memory_order_relaxed) && gemm_few_rows_preferred(A, B, batch, M, N, K, sAm, sAk, sBk, sBn, dtype) && !gemm_few_rows_leaves_to_ranges(N, K)) return 0;
+  if (gemm_small_path_on() && gemm_few_rows_preferred(A, B, batch, M, N, K, sAm, sAk, sBk, sBn, dtype) && !gemm_few_rows_leaves_to_ranges(N, K)) return 0;
   if (!gemm_tc_eligible(batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype, A, B, C)) return 0;
   return gemm_tc_splitk_scratch_bytes(batch, M, N, K);
 }
@@ -119,5 +122,10 @@ extern "C" int b200_gemm_small_path(int enable) { return g_small_path.exchange(e
 
 extern "C" int b200_gemm_prefers_small(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb, int64_t sBk,
                                        int64_t sBn, int dtype) {
-  return (g_small_path.load(std::memory_order_relaxed) && gemm_mma_small_preferred(A, B, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype)) ? 1 : 0;
+  return (gemm_small_path_on() && gemm_mma_small_preferred(A, B, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype)) ? 1 : 0;
+}
+
+extern "C" int b200_gemm_takes_as_is(const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb, int64_t sBk,
+                                     int64_t sBn, int dtype) {
+  return b200_gemm_prefers_small(A, B, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, dtype) || gemm_deep_preferred(batch, M, N, K, sAk, sBn, dtype) ? 1 : 0;
 }

@@ -622,9 +622,16 @@ static int launch_simt(const void* A, const void* B, const void* bias, void* C, 
   return launch_simt_small<T, 64, 64>(A, B, bias, C, batch, g, st);
 }
 
+bool gemm_deep_preferred(int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAk, int64_t sBn, int dtype);
+int gemm_deep_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb,
+                       int64_t sBk, int64_t sBn, int64_t sbm, int64_t sbn, double alpha, double beta, int dtype, cudaStream_t st, const uint32_t* gate);
+
 int gemm_simt_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t sAb, int64_t sAm, int64_t sAk,
                        int64_t sBb, int64_t sBk, int64_t sBn, int64_t sbm, int64_t sbn, double alpha, double beta, int dtype, cudaStream_t st, const uint32_t* gate) {
   GemmArgs g{M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta), gate, 1, 0};
+  // (rows of A that a warp each streams past a narrow B stay where they are: 16 columns and many rows)
+  if (!(dtype == B200_F32 && skinny_warp_eligible<float>(A, batch, g)) && gemm_deep_preferred(batch, M, N, K, sAk, sBn, dtype))
+    return gemm_deep_dispatch(A, B, bias, C, batch, M, N, K, sAb, sAm, sAk, sBb, sBk, sBn, sbm, sbn, alpha, beta, dtype, st, gate);
   switch (dtype) {
     case B200_F32: return launch_simt<float>(A, B, bias, C, batch, g, st);
     case B200_BF16: return launch_simt<__nv_bfloat16>(A, B, bias, C, batch, g, st);

@@ -33,7 +33,7 @@ namespace {
   F(b200_relu) F(b200_add) F(b200_mul) F(b200_add_scalar) F(b200_mul_scalar) F(b200_where) F(b200_softmax) F(b200_softmax_backward) F(b200_reduce_scratch_bytes) F(b200_sum)           \
   F(b200_layer_norm) F(b200_layer_norm_backward_scratch_bytes) F(b200_layer_norm_backward) F(b200_argmax) F(b200_gather_rows) F(b200_index_select) F(b200_gather)                    \
   F(b200_scatter_add_scratch_bytes) F(b200_scatter_add) F(b200_embedding_backward_scratch_bytes) F(b200_embedding_backward) F(b200_copy_pitched) F(b200_gemm)                        \
-  F(b200_gemm_prefers_small) F(b200_gemm_f32_scratch_bytes) F(b200_gemm_f32) F(b200_gemm_splitk_scratch_bytes) F(b200_gemm_splitk) F(b200_allclose)
+  F(b200_gemm_takes_as_is) F(b200_gemm_f32_scratch_bytes) F(b200_gemm_f32) F(b200_gemm_splitk_scratch_bytes) F(b200_gemm_splitk) F(b200_allclose)
 struct Api {
 #define F(name) decltype(&::name) name;
   B200_ENTRIES(F)
@@ -653,7 +653,7 @@ PyObject* gemm(Operand a, Operand b, const Tensor& bias, int64_t batch, int64_t 
   if (!status) return nullptr;
   if (t != B200_F32 && (M * N * K * batch >= (1 << 24) || K >= 1024) && K >= 16) {
     bool ra = tma_ready(a, a.row, a.col, batch), rb = tma_ready(b, b.col, b.row, batch);
-    if (!(ra && rb) && api.b200_gemm_prefers_small(ptr(a.t), ptr(b.t), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, t)) ra = rb = true;
+    if (!(ra && rb) && api.b200_gemm_takes_as_is(ptr(a.t), ptr(b.t), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, t)) ra = rb = true;
     if (!ra) {
       if (a.row != 1 || a.col == 1) {
         if (!repitch(a, batch, M, K, a.row, a.col, a.row)) return nullptr;

@@ -730,10 +730,10 @@ def _gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor], batch:
     # the tensor cores to pay for the extra copy; otherwise the CUDA-core kernel takes them
     # (a long contraction with a small output is re-pitched too: the CUDA-core kernel would
     # walk all of K in one or two CTAs)
-    # (small products whose operands are on the 16-byte grid go to the mma.sync kernel as they are)
+    # (small products, and those with few outputs and a long contraction, go to kernels that take the operands as they are)
     if a.dtype != torch.float32 and (M * N * K * batch >= (1 << 24) or K >= 1024) and K >= 16:
         a_ready, b_ready = _tma_ready(a, sa[0], sa[1], sa[2], batch), _tma_ready(b, sb[0], sb[2], sb[1], batch)
-        if not (a_ready and b_ready) and lib().b200_gemm_prefers_small(a.data_ptr(), b.data_ptr(), batch, M, N, K, sa[0], sa[1], sa[2], sb[0], sb[1], sb[2], _dt(a.dtype)):
+        if not (a_ready and b_ready) and lib().b200_gemm_takes_as_is(a.data_ptr(), b.data_ptr(), batch, M, N, K, sa[0], sa[1], sa[2], sb[0], sb[1], sb[2], _dt(a.dtype)):
             a_ready = b_ready = True
         if not a_ready:
             if sa[1] != 1 or sa[2] == 1:  # keep A K-major unless it is M-major

@@ -296,16 +296,21 @@ int b200_gemm_f32(const void* A, const void* B, const void* bias, void* C, int64
 /* Small 16-bit products (at most 148 tiles of 64 x 64, K <= 256, at most 2^26 multiply-adds,
  * both operands with one unit stride and base / other strides on the 16-byte grid) are served
  * by a four-warp mma.sync kernel with cp.async staging instead of the tcgen05 kernel, whose
- * set-up alone takes about 5 us. b200_gemm_prefers_small tells a caller whether b200_gemm
- * will go that way.
+ * set-up alone takes about 5 us. Products with few outputs and a long contraction (fp32 ones, and
+ * 16-bit ones off the 16-byte grid) go to a CUDA-core kernel that cuts K once per warp.
+ * b200_gemm_prefers_small tells a caller whether b200_gemm goes the first of these ways,
+ * b200_gemm_takes_as_is whether operands off the grid are served best as they are, by either.
  * Products of at most 16 rows against weights along K (64 <= K <= 16384, on the 16-byte grid)
  * go to another mma.sync kernel that streams the weights once, unless they are so wide or so
  * deep and narrow that the tcgen05 kernel or its K-split is faster.
- * b200_gemm_small_path(0) switches both off process-wide (1 on again) and returns the
+ * b200_gemm_small_path(0) switches the three off process-wide (1 on again) and returns the
  * previous setting -- for comparisons and for testing the larger kernels on small shapes. */
 int b200_gemm_prefers_small(const void* A, const void* B, int64_t batch, int64_t M, int64_t N,
                             int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb, int64_t sBk,
                             int64_t sBn, int dtype);
+int b200_gemm_takes_as_is(const void* A, const void* B, int64_t batch, int64_t M, int64_t N,
+                          int64_t K, int64_t sAb, int64_t sAm, int64_t sAk, int64_t sBb, int64_t sBk,
+                          int64_t sBn, int dtype);
 int b200_gemm_small_path(int enable);
 
 /* A 16-bit product with a long contraction and a C of a few tiles (batch 1, at most a quarter

@@ -531,6 +531,37 @@ def _within_rounding(got, a, b, extra=None):
     assert bool(((got.double() - exact).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("b_along_k", [False, True])
+@pytest.mark.parametrize("batch,M,K,N", [(1, 1, 64, 1), (1, 4, 65, 33), (1, 5, 255, 64), (3, 8, 257, 65), (1, 9, 2049, 31), (1, 16, 511, 130), (2, 17, 513, 32), (1, 40, 1000, 97), (1, 41, 4097, 63), (2, 100, 7173, 70)])
+def test_few_outputs_and_a_long_contraction(dtype, b_along_k, batch, M, K, N, small_path):
+    """Rows and columns on both sides of a tile, K that leaves warps or whole CTAs of a cluster without a step or cuts
+    the last one, A along K and along M, strides on neither side, a bias, and NaN beside the operands that no lane may pick up."""
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+
+    def view(rows, cols, turned, step=1):  # a window into a buffer of NaN
+        buf = torch.full((batch, (cols if turned else rows) * step + 2, (rows if turned else cols) * step + 3), float("nan"), dtype=dtype, device=DEV)
+        v = buf[:, 1:-1:step, 1:-2:step] if step > 1 else buf[:, 1:-1, 1:-2]
+        v = v.transpose(1, 2) if turned else v
+        return v.copy_(_rand((batch, rows, cols), dtype, g, 1.0))
+
+    for a_turned, step in ((False, 1), (True, 1), (False, 2)):
+        a, b = view(M, K, a_turned), view(K, N, b_along_k, step)
+        bias = _rand((M, N), dtype, g, 1.0)
+        got = ops.bmm_default(a, b)
+        if dtype == torch.float32:
+            # one chain of K multiply-adds at most, each rounded to nearest (2^-24 of the sum of magnitudes so far); the bf16 planes
+            # of larger products truncate (2^-23) six of them
+            mass = a.double().abs() @ b.double().abs()
+            assert bool(((got.double() - a.double() @ b.double()).abs() <= mass * (K + 8) * 2.0**-23).all())
+            got = ops.addmm_default(bias, a[0], b[0], beta=0.5, alpha=2.0)
+            want = 0.5 * bias.double() + 2.0 * (a[0].double() @ b[0].double())
+            assert bool(((got.double() - want).abs() <= (2.0 * mass[0] + bias.double().abs()) * (K + 8) * 2.0**-23).all())
+        else:
+            _within_rounding(got, a, b)
+            _within_rounding(ops.addmm_default(bias, a[0], b[0]), a[0], b[0], bias)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("N", [129, 130, 132, 191, 250, 255, 257, 514, 770])
 def test_rows_of_c_between_two_words(dtype, N):
