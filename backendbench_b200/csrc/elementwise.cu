@@ -26,6 +26,8 @@ struct MulOp { __device__ __forceinline__ float operator()(float a, float b) con
 template <typename T, typename Op>
 __global__ void __launch_bounds__(kEwThreads) ew_unary_vec(const T* __restrict__ x, T* __restrict__ out, int64_t n, Op op) {
   constexpr int VE = Vec<T>::N;
+  next_grid_may_start();
+  after_grids_before();
   const int64_t nvec = n / VE;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * (kEwThreads * kUnroll) + threadIdx.x;
   Vec<T> v[kUnroll];
@@ -546,12 +548,14 @@ static int strided_grid(int64_t n) {
 template <typename Op>
 static int launch_unary_fast(const void* x, void* out, int64_t n, int dtype, Op op, cudaStream_t st) {
   const int per_block = kEwThreads * kUnroll;
+  cudaError_t e;
   switch (dtype) {
-    case B200_F32: ew_unary_vec<float, Op><<<grid_for(n / 4 + 1, per_block), kEwThreads, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(out), n, op); break;
-    case B200_BF16: ew_unary_vec<__nv_bfloat16, Op><<<grid_for(n / 8 + 1, per_block), kEwThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), n, op); break;
-    case B200_F16: ew_unary_vec<__half, Op><<<grid_for(n / 8 + 1, per_block), kEwThreads, 0, st>>>(static_cast<const __half*>(x), static_cast<__half*>(out), n, op); break;
+    case B200_F32: e = launch_after(ew_unary_vec<float, Op>, grid_for(n / 4 + 1, per_block), kEwThreads, 0, st, static_cast<const float*>(x), static_cast<float*>(out), n, op); break;
+    case B200_BF16: e = launch_after(ew_unary_vec<__nv_bfloat16, Op>, grid_for(n / 8 + 1, per_block), kEwThreads, 0, st, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), n, op); break;
+    case B200_F16: e = launch_after(ew_unary_vec<__half, Op>, grid_for(n / 8 + 1, per_block), kEwThreads, 0, st, static_cast<const __half*>(x), static_cast<__half*>(out), n, op); break;
     default: return B200_EDTYPE;
   }
+  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
   return check_launch();
 }
 

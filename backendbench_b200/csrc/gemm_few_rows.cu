@@ -4,15 +4,15 @@
 // CTAs, and a handful of stages in flight in each: 16 x 4096 x 11008 ran on 43 SMs (44 us,
 // 2.1 TB/s), 16 x 11008 x 4096 in 16 CTAs split over K with a second pass (29 us).
 //
-// Here a CTA owns 16 columns of C and its eight warps share K. A warp streams B from global
+// Here a CTA owns 8 to 40 columns of C and its eight warps share K. A warp streams B from global
 // memory straight into mma.sync operands, with no shared memory in between: in
 // mma.m16n8k16 lane (q, c) holds elements 2c, 2c + 1, 2c + 8, 2c + 9 of row q of B (and of rows
 // q, q + 8 of A). The order of the products in a sum over k is free, so the 32 k of
 // two such steps are dealt out as the 16-byte pieces 8c .. 8c + 7 of a row: one load
-// each. Four steps of both operands are in flight per lane; A comes from L2, where every CTA
+// each. Three or four steps of both operands are in flight per lane; A comes from L2, where every CTA
 // reads it. The warps' sums are added in warp order in fp32, then alpha, beta, the bias and
-// one rounding. bf16, 16 rows: K 4096 x N 11008 44 -> 22 us (4.1 TB/s), K 11008 x N 4096 29 -> 17.5 us
-// (5.1 TB/s; 256 CTAs, all resident, where the other has 2.3 rounds of them).
+// one rounding. bf16, 16 rows: K 4096 x N 11008 44 -> 16.6 us (5.4 TB/s), K 11008 x N 4096 29 -> 17.1 us
+// (5.3 TB/s; 256 CTAs, so the busiest SM has 32 columns where the mean is 27.7).
 #include <type_traits>
 
 #include "b200_common.cuh"
@@ -23,8 +23,8 @@ namespace {
 
 constexpr int kFewRows = 16;
 constexpr int kFewWarps = 8;
-constexpr int kFewFragments = 2;           // of eight columns each: 16 columns to a CTA, enough CTAs for two on every SM from N = 4736 on
-constexpr int kFewSteps = 4;              // 32-k steps in flight per lane
+constexpr int kFewMaxFragments = 5;       // of eight columns each, to a CTA: see few_fragments
+template <int NT> struct FewSteps { static constexpr int value = NT > 3 ? 3 : 4; };  // 32-k steps in flight per lane
 // Where the kernel is the faster one; bf16 with B out of HBM, us here / the tcgen05 kernel or its ranges of K.
 // The tcgen05 kernel has a CTA to 256 columns: up to 96 of them leave it SMs idle (N 20000, K 4096: 8 rows 33 /
 // 44, 16 rows 43.5 / 44). Beyond, this one wins by what it does not read twice, as long as the rows of A, which
@@ -56,9 +56,9 @@ __device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1
   }
 }
 
-template <typename T>
+template <typename T, int NT>
 __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ bias, T* __restrict__ C, FewRowsArgs p) {
-  constexpr int NT = kFewFragments, kCols = 8 * NT, kPitch = kCols + 1;
+  constexpr int kCols = 8 * NT, kPitch = kCols + 1, kFewSteps = FewSteps<NT>::value;
   __shared__ float red[kFewWarps][kFewRows][kPitch];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane >> 2, c = lane & 3;
   const int64_t n0 = static_cast<int64_t>(blockIdx.x) * kCols;
@@ -76,6 +76,17 @@ __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __re
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
   const int K = static_cast<int>(p.K);  // a multiple of 8: a piece is inside the row or outside it
+  // While the kernel before ends, the lines that the warp reads first are brought into L2 (which holds what that
+  // kernel writes all the same, should it be these).
+  next_grid_may_start();
+#pragma unroll
+  for (int u = 0; u < 2 * kFewSteps; ++u) {
+    const int k = (warp + (u / kFewSteps) * kFewWarps) * 32 * kFewSteps + 32 * (u % kFewSteps);
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+      if ((c & 1) == 0 && k + 8 * c < K && col[t]) asm volatile("prefetch.global.L2 [%0];" ::"l"(b[t] + k));
+  }
+  after_grids_before();
   for (int k0 = warp * 32 * kFewSteps; k0 < K; k0 += kFewWarps * 32 * kFewSteps) {
     uint4 ra[kFewSteps], rA[kFewSteps], rb[NT][kFewSteps];
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -136,17 +147,45 @@ bool gemm_few_rows_leaves_to_ranges(int64_t N, int64_t K) {
   return N < 2048 && (K > (N <= 1024 ? 11264 : 14336) || (K > 8448 && N >= 16 && N <= 512) || (K > 7168 && N > 64 && N <= 128));
 }
 
+// Fragments of eight columns to a CTA. What counts is that the CTAs, two to an SM, come out even, and best that all of
+// them run at once: 16 x 4096 against 11008 columns takes 21.7 us with two (688 CTAs, 2.3 rounds) and 16.6 with five (276), 8192 columns 25.9
+// with two (512), 30.8 with three, 22.4 with four (256). One CTA alone on an SM has too few loads in flight (4096 columns: 22.9 with four, 128
+// CTAs; 17.1 with two). Over many rounds the width matters by what a CTA reads of A and by what it keeps in flight: 32000 columns 59 / 47.5 /
+// 46.6 / 48.4 / 50.5 us with one to five. The figures below are those ratios.
+static int few_fragments(int64_t N) {
+  constexpr int kPer[kFewMaxFragments] = {127, 102, 100, 104, 108};
+  int best = 1;
+  double least = 0.;
+  for (int nt = 1; nt <= kFewMaxFragments; ++nt) {
+    const int64_t ctas = (N + 8 * nt - 1) / (8 * nt), slots = 2 * kNumSMs;
+    const double rounds = static_cast<double>(ctas) / slots, whole = static_cast<double>((ctas + slots - 1) / slots);
+    const double columns = nt * (ctas <= kNumSMs ? 1.16 : ctas <= slots ? 2. * 0.85 : rounds + whole);  // ("2 *" their mean)
+    if (nt == 1 || columns * kPer[nt - 1] < least) { least = columns * kPer[nt - 1]; best = nt; }
+  }
+  return best;
+}
+
 template <typename T>
-static void launch_few_rows(const void* A, const void* B, const void* bias, void* C, const FewRowsArgs& p, cudaStream_t st) {
-  gemm_few_rows<T><<<grid_for(p.N, 8 * kFewFragments), 32 * kFewWarps, 0, st>>>(static_cast<const T*>(A), static_cast<const T*>(B), static_cast<const T*>(bias), static_cast<T*>(C), p);
+static cudaError_t launch_few_rows(const void* A, const void* B, const void* bias, void* C, const FewRowsArgs& p, cudaStream_t st) {
+  const int nt = few_fragments(p.N);
+  auto launch = [&](auto kernel) {
+    return launch_after(kernel, (p.N + 8 * nt - 1) / (8 * nt), 32 * kFewWarps, 0, st, static_cast<const T*>(A), static_cast<const T*>(B), static_cast<const T*>(bias), static_cast<T*>(C), p);
+  };
+  switch (nt) {
+    case 1: return launch(gemm_few_rows<T, 1>);
+    case 2: return launch(gemm_few_rows<T, 2>);
+    case 3: return launch(gemm_few_rows<T, 3>);
+    case 4: return launch(gemm_few_rows<T, 4>);
+    default: return launch(gemm_few_rows<T, 5>);
+  }
 }
 
 int gemm_few_rows_dispatch(const void* A, const void* B, const void* bias, void* C, int64_t M, int64_t N, int64_t K, int64_t sAm, int64_t sBn, int64_t sbm, int64_t sbn, double alpha,
                            double beta, int dtype, cudaStream_t st) {
   const FewRowsArgs p{M, N, K, sAm, sBn, sbm, sbn, static_cast<float>(alpha), static_cast<float>(beta)};
   const void* bs = static_cast<float>(beta) != 0.f ? bias : nullptr;  // beta = 0 ignores the bias, NaN included
-  if (dtype == B200_BF16) launch_few_rows<__nv_bfloat16>(A, B, bs, C, p, st);
-  else launch_few_rows<__half>(A, B, bs, C, p, st);
+  const cudaError_t e = dtype == B200_BF16 ? launch_few_rows<__nv_bfloat16>(A, B, bs, C, p, st) : launch_few_rows<__half>(A, B, bs, C, p, st);
+  if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
   return check_launch();
 }
 

@@ -531,6 +531,20 @@ def _within_rounding(got, a, b, extra=None):
     assert bool(((got.double() - exact).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N", [1, 500, 4091, 6141, 8185, 11003, 11009])
+def test_few_rows_in_every_width_of_a_cta(dtype, N):
+    """One to five fragments of eight columns to a CTA, the last CTA cut short, K that ends within a step, within the first
+    round of the warps and beyond it, one row up to sixteen, with a bias and after a kernel that is still writing A."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    for M, K in [(1, 72), (9, 392), (16, 1032), (7, 2056)]:
+        x, w = _rand((M, K), dtype, g, K**-0.5), _rand((N, K), dtype, g, 1.0)
+        bias = _rand((N,), dtype, g, 1.0)
+        a = ops.relu(x)
+        _within_rounding(ops.mm_default(a, w.t()), a, w.t())
+        _within_rounding(ops.addmm_default(bias, a, w.t()), a, w.t(), bias)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 @pytest.mark.parametrize("b_along_k", [False, True])
 @pytest.mark.parametrize("batch,M,K,N", [(1, 1, 64, 1), (1, 4, 65, 33), (1, 5, 255, 64), (3, 8, 257, 65), (1, 9, 2049, 31), (1, 16, 511, 130), (2, 17, 513, 32), (1, 40, 1000, 97), (1, 41, 4097, 63), (2, 100, 7173, 70)])
