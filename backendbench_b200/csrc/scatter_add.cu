@@ -66,18 +66,13 @@ __device__ __forceinline__ void flag_oob(uint32_t* status) {
   if (status) atomicOr(status, B200_DEV_INDEX_OOB);
 }
 
-// Rank of this lane among the EARLIER in-order elements of its own group of GROUP adjacent
-// lanes that carry the same destination `k` (negative k = nothing to apply; made unique per
-// lane so it never matches). `pos` is the lane's position inside its group.
-template <int GROUP>
+// Rank of this lane among the EARLIER in-order elements of its own group of adjacent lanes that carry the same destination `k`
+// (negative k = nothing to apply; the rank is not used then). `pos` is the lane's position inside its group. (One match over the
+// warp: with a shuffle and a comparison per earlier lane, fp16 30000 x 300 onto 64 rows took 470 us, 308 so.)
 __device__ __forceinline__ int rank_among_earlier(int k, int pos) {
-  int rank = 0;
-#pragma unroll
-  for (int d = 1; d < GROUP; ++d) {
-    const int other = __shfl_up_sync(0xffffffffu, k, d);
-    rank += (pos >= d && other == k) ? 1 : 0;
-  }
-  return rank;
+  const int lane = threadIdx.x & 31;
+  const uint32_t same = __match_any_sync(0xffffffffu, k);
+  return __popc(same & (((1u << pos) - 1u) << (lane - pos)));
 }
 // Same-destination lanes add one rank after the other, so the in-order sequence is kept.
 __device__ __forceinline__ void apply_in_rank_order(float* col, int k, float v, int rank) {
@@ -107,7 +102,7 @@ __device__ __forceinline__ void ordered_step(float* col, unsigned char* tags, in
     if (k >= 0) col[k] += v;
     __syncwarp();
   } else {
-    apply_in_rank_order(col, k, v, rank_among_earlier<GROUP>(k, pos));
+    apply_in_rank_order(col, k, v, rank_among_earlier(k, pos));
   }
 }
 
@@ -512,7 +507,7 @@ scatter_add_strip_wide(const __grid_constant__ CUtensorMap map_idx, const __grid
                   __syncwarp();
                 }
               } else {
-                apply_in_rank_order(col, k[cur], v[cur], rank_among_earlier<32>(k[cur], lane));
+                apply_in_rank_order(col, k[cur], v[cur], rank_among_earlier(k[cur], lane));
               }
             }
           }
@@ -1261,7 +1256,8 @@ static int launch_chain(const void* self, const void* index, const void* src, vo
 // Every global access is in runs of a row or of a segment; what is random stays in shared memory, where the chain path
 // has its exchanges and look-ups in L2. fp16 150134 x 63, 75067 rows: 133 us in chains, 87 so (binned_sort 29, half of its
 // issue slots busy counting and placing; binned_replay 45: nine warps of 4096 sums fill an SM's shared memory, and each goes
-// at the speed of its chain of tag, look, sum; six more launches that begin and find nothing to do). fp32 4095 x 4095 556 -> 283,
+// at the speed of its chain of tag, look, sum; six more launches that begin and find nothing to do; 82 with the 4096 sums of a warp read 32 to
+// a lane behind the first table, 16 before). fp32 4095 x 4095 556 -> 283,
 // 160000 x 400 3640 -> 1140, 888 x 4065 99 -> 58. Tried: a CTA to a bin, its records in chains in shared memory (123 us
 // for the replay, 18 instructions' worth of divergence to a destination); the records of 8 steps in registers
 // (80: a step unrolled eight times does not fit the instruction cache); 256 threads with runs of 32 rows in binned_sort (44).
@@ -1438,7 +1434,7 @@ __global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, 
                                                     const __grid_constant__ BinnedArgs A, const int* ctl, int* head, int64_t n_self) {
   typedef typename BinRec<T>::type Rec;
   constexpr uint32_t kAll = 0xffffffffu;
-  constexpr int kMove = 16;   // elements of self on the way per lane
+  constexpr int kMove = 32;   // elements of self on the way per lane
   extern __shared__ __align__(16) unsigned char bin_smem[];
   __shared__ uint32_t piece[32];
   __shared__ __align__(16) Rec ring[2][kBinAhead][32];
@@ -1460,20 +1456,6 @@ __global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, 
   if (ctl[kCtlGrouped]) {  // the counters of the kernels that follow
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane; i < n_self; i += static_cast<int64_t>(gridDim.x) * 32) head[i] = -1;
     return;
-  }
-  {
-    const T* p = self + base + lane;
-    for (int d0 = lane; d0 < end; d0 += 32 * kMove) {
-      T s[kMove];
-#pragma unroll
-      for (int u = 0; u < kMove; ++u) {
-        if (d0 + 32 * u < end) s[u] = *p;
-        p += step;
-      }
-#pragma unroll
-      for (int u = 0; u < kMove; ++u)
-        if (d0 + 32 * u < end) sum[d0 + 32 * u] = to_f32(s[u]);
-    }
   }
   const int chunks = g < A.idx_groups && o < A.idx_outer ? A.chunks : 0;
   const int per_chunk = A.chunk_rows * A.c;
@@ -1551,11 +1533,25 @@ __global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, 
         __syncwarp();
       }
     } else {
-      apply_in_rank_order(sum, k, v, rank_among_earlier<32>(k, lane));
+      apply_in_rank_order(sum, k, v, rank_among_earlier(k, lane));
     }
   };
+  if (chunks > 0) read_table();  // (on its way while self is read)
+  {
+    const T* p = self + base + lane;
+    for (int d0 = lane; d0 < end; d0 += 32 * kMove) {
+      T s[kMove];
+#pragma unroll
+      for (int u = 0; u < kMove; ++u) {
+        if (d0 + 32 * u < end) s[u] = *p;
+        p += step;
+      }
+#pragma unroll
+      for (int u = 0; u < kMove; ++u)
+        if (d0 + 32 * u < end) sum[d0 + 32 * u] = to_f32(s[u]);
+    }
+  }
   __syncwarp();
-  if (chunks > 0) read_table();
   int n = load(0);
 #pragma unroll 1
   for (int buf = 0; n > 0; buf ^= 1) {
