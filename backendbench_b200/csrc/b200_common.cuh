@@ -179,6 +179,41 @@ template <typename T> __device__ __forceinline__ void vec_accumulate(float& s, c
     Mixed<T>::add2(s, raw.x); Mixed<T>::add2(s, raw.y); Mixed<T>::add2(s, raw.z); Mixed<T>::add2(s, raw.w);
   }
 }
+// Two fp32 values to a 64-bit register: sums and products of both in one instruction, each rounded as by itself.
+struct F2 {
+  unsigned long long v;
+  static __device__ __forceinline__ F2 of(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+  }
+};
+__device__ __forceinline__ void p_parts(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ F2 p_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 p_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 p_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// The same with an instruction to each value, where registers for aligned pairs cost more than they save.
+struct TwoF {
+  float lo, hi;
+  static __device__ __forceinline__ TwoF of(float lo, float hi) { return TwoF{lo, hi}; }
+};
+__device__ __forceinline__ void p_parts(TwoF a, float& lo, float& hi) { lo = a.lo; hi = a.hi; }
+__device__ __forceinline__ TwoF p_add(TwoF a, TwoF b) { return TwoF{a.lo + b.lo, a.hi + b.hi}; }
+__device__ __forceinline__ TwoF p_mul(TwoF a, TwoF b) { return TwoF{a.lo * b.lo, a.hi * b.hi}; }
+__device__ __forceinline__ TwoF p_fma(TwoF a, TwoF b, TwoF c) { return TwoF{fmaf(a.lo, b.lo, c.lo), fmaf(a.hi, b.hi, c.hi)}; }
+
 template <typename T> __device__ __forceinline__ void vec_minus(const uint4& raw, float c, float* d) {
   if constexpr (sizeof(T) == 4) {
     d[0] = __uint_as_float(raw.x) - c; d[1] = __uint_as_float(raw.y) - c; d[2] = __uint_as_float(raw.z) - c; d[3] = __uint_as_float(raw.w) - c;

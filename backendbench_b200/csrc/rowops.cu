@@ -900,27 +900,36 @@ layernorm_persistent(const T* __restrict__ x, const TW* __restrict__ w, const TW
 // CTAs, one row at a time per CTA; a thread owns the same columns of every row it sees, so it
 // carries its share of dw / db in registers across rows and writes one partial per CTA at
 // the end (dy and x are read once for all three results). A small second kernel adds the
-// per-CTA partials in order. fp32 arithmetic throughout. bf16 8192 x 4096: 53.7 -> 51.3 us (3.9 TB/s of
-// two reads and a write) with both sums behind one barrier and the row statistics fetched ahead; a
-// ring of four rows in shared memory (`cp.async`) in place of the one row in registers changed
-// nothing (52.4 us). Two CTAs of 512 threads run on an SM, 29 of its warps active on average, half of the
-// issue slots busy; the stalls are waits for a row's loads and for the shuffles and shared memory of its sums.
+// per-CTA partials in order. fp32 arithmetic throughout. bf16 8192 x 4096: 53.7 -> 51.3 us with both sums behind one barrier
+// and the row statistics fetched ahead; bound by its instructions (two CTAs of 512 threads on an SM, half of the issue
+// slots busy, and 20 % more instructions were 20 % more time), so two elements to an instruction (P, below), a shuffle per level for both sums,
+// and the partial sums stored 16 bytes at a time: 54 -> 44.6 us the call with its second kernel. Tried: a ring of four rows in shared
+// memory (`cp.async`) in place of the one row in registers (52.4 for 51.3); the row before finished behind the next row's sums,
+// so that nothing waits right after a barrier (64.9 for 54.3); two to eight rows to a CTA of 512 threads, fewer partial sums, behind
+// barriers of their own (30000 x 768 49.7 for 38.5).
 template <typename T, typename TW, int VPT, bool kAhead>
 __global__ void __launch_bounds__(1024)
 layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW* __restrict__ w, const void* __restrict__ mean, const void* __restrict__ rstd, T* __restrict__ dx,
                     float* __restrict__ part_w, float* __restrict__ part_b, int64_t rows, int cols, int dt_stat) {
-  constexpr int VE = Vec<T>::N;
-  __shared__ float2 red[2][32];
+  constexpr int VE = Vec<T>::N, VP = VE / 2;
+  typedef typename std::conditional<sizeof(T) == 2, F2, TwoF>::type P;  // (fp32 8192 x 4096, bound by memory: 74 us, 80 with F2)
+  __shared__ float red[2][2][32];  // [row parity][sum][warp]
   const int t = threadIdx.x, tpr = blockDim.x;
   const int nvec = cols / VE;
   const float inv_cols = 1.f / static_cast<float>(cols);
-  float wv[VPT][VE], aw[VPT][VE], ab[VPT][VE];
+  P wv[VPT][VP], aw[VPT][VP], ab[VPT][VP];  // (pairs: half the instructions of what bounds this)
 #pragma unroll
   for (int u = 0; u < VPT; ++u) {
     const int j = t + u * tpr;
+    float wf[VE];
 #pragma unroll
-    for (int e = 0; e < VE; ++e) { wv[u][e] = 1.f; aw[u][e] = 0.f; ab[u][e] = 0.f; }
-    if (w && j < nvec) load_weights<VE, TW>(w, j * VE, wv[u]);
+    for (int e = 0; e < VE; ++e) wf[e] = 1.f;
+    if (w && j < nvec) load_weights<VE, TW>(w, j * VE, wf);
+#pragma unroll
+    for (int e = 0; e < VP; ++e) {
+      wv[u][e] = P::of(wf[2 * e], wf[2 * e + 1]);
+      aw[u][e] = ab[u][e] = P::of(0.f, 0.f);
+    }
   }
   // the vectors of the next row are requested before this row is worked on: twice the bytes in flight per thread
   uint4 ndy[VPT], nx[VPT];
@@ -943,13 +952,18 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, phase ^= 1) {
     // (without kAhead: many small CTAs per SM hide these loads by themselves)
     const float mu = kAhead ? nmu : load_as_f32(mean, row, dt_stat), rs = kAhead ? nrs : load_as_f32(rstd, row, dt_stat);
-    float g[VPT][VE], h[VPT][VE];
-    float s1 = 0.f, s2 = 0.f;
+    const P rs2 = P::of(rs, rs);
+    P g[VPT][VP], h[VPT][VP];  // dy, then dy * w; x - mean, then xhat
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
-      widen<T>(ndy[u], g[u]);
-      if (sizeof(T) == 2) vec_minus<T>(nx[u], mu, h[u]);  // widened inside the subtraction
-      else widen<T>(nx[u], h[u]);
+      float gf[VE], hf[VE];
+      widen<T>(ndy[u], gf);
+      vec_minus<T>(nx[u], mu, hf);  // (16 bits: widened inside the subtraction)
+#pragma unroll
+      for (int e = 0; e < VP; ++e) {
+        g[u][e] = P::of(gf[2 * e], gf[2 * e + 1]);
+        h[u][e] = P::of(hf[2 * e], hf[2 * e + 1]);
+      }
     }
     const int64_t next = row + gridDim.x;
     if (next < rows) {
@@ -966,37 +980,47 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         }
       }
     }
+    P p1 = P::of(0.f, 0.f), p2 = p1;
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
-      const int j = t + u * tpr;
-      if (j < nvec) {
+      if (t + u * tpr < nvec) {
 #pragma unroll
-        for (int e = 0; e < VE; ++e) {
-          const float xhat = (sizeof(T) == 2 ? h[u][e] : h[u][e] - mu) * rs;
-          ab[u][e] += g[u][e];
-          aw[u][e] = fmaf(g[u][e], xhat, aw[u][e]);
-          const float gy = g[u][e] * wv[u][e];
-          s1 += gy;
-          s2 = fmaf(gy, xhat, s2);
-          g[u][e] = gy;
-          h[u][e] = xhat;
+        for (int e = 0; e < VP; ++e) {
+          h[u][e] = p_mul(h[u][e], rs2);
+          ab[u][e] = p_add(ab[u][e], g[u][e]);
+          aw[u][e] = p_fma(g[u][e], h[u][e], aw[u][e]);
+          g[u][e] = p_mul(g[u][e], wv[u][e]);
+          p1 = p_add(p1, g[u][e]);
+          p2 = p_fma(g[u][e], h[u][e], p2);
         }
       }
     }
+    float s1, s2, other;
+    p_parts(p1, s1, other);
+    s1 += other;
+    p_parts(p2, s2, other);
+    s2 += other;
     if constexpr (kAhead) {
-      // both sums behind one barrier; the row after next is the first to write these slots again
-      s1 = warp_reduce(s1, SumF{});
-      s2 = warp_reduce(s2, SumF{});
-      if ((t & 31) == 0) red[phase][t >> 5] = make_float2(s1, s2);
+      // both sums behind one barrier; the row after next is the first to write these slots again. The lower half
+      // of a warp goes on with the first sum, the upper with the second.
+      const int half = (t & 31) >> 4;
+      float s = (half ? s2 : s1) + __shfl_xor_sync(0xffffffffu, half ? s1 : s2, 16);
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      if ((t & 15) == 0) red[phase][half][t >> 5] = s;
       __syncthreads();
-      const float2 part = (t & 31) < (tpr >> 5) ? red[phase][t & 31] : make_float2(0.f, 0.f);
-      s1 = warp_reduce(part.x, SumF{});
-      s2 = warp_reduce(part.y, SumF{});
+      s = 0.f;
+      for (int k = t & 15; k < (tpr >> 5); k += 16) s += red[phase][half][k];
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      other = __shfl_xor_sync(0xffffffffu, s, 16);
+      s1 = half ? other : s;
+      s2 = half ? s : other;
     } else {  // (one after the other where the CTAs are small and many: fp32 65536 x 1024 144 us, 153 us behind one barrier)
-      s1 = block_reduce_once(s1, SumF{}, 0.f, &red[0][0].x, 0);
-      s2 = block_reduce_once(s2, SumF{}, 0.f, &red[0][0].x, 1);
+      s1 = block_reduce_once(s1, SumF{}, 0.f, &red[0][0][0], 0);
+      s2 = block_reduce_once(s2, SumF{}, 0.f, &red[0][0][0], 1);
     }
-    const float c1 = s1 * inv_cols, c2 = s2 * inv_cols;
+    const P m1 = P::of(-s1 * inv_cols, -s1 * inv_cols), m2 = P::of(-s2 * inv_cols, -s2 * inv_cols);
     if (dx) {
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
@@ -1004,21 +1028,40 @@ layernorm_bwd_fused(const T* __restrict__ dy, const T* __restrict__ x, const TW*
         if (j < nvec) {
           float o[VE];
 #pragma unroll
-          for (int e = 0; e < VE; ++e) o[e] = rs * (g[u][e] - c1 - h[u][e] * c2);
+          for (int e = 0; e < VP; ++e) p_parts(p_mul(rs2, p_fma(h[u][e], m2, p_add(g[u][e], m1))), o[2 * e], o[2 * e + 1]);
           st_stream(dx + row * cols + j * VE, narrow<T>(o));
         }
       }
     }
   }
   if (part_w) {
+    // (16 bytes at a time: a word at a time, 32 bytes apart over a warp, bf16 1000 x 4096 took 20.5 us, 13.1 so, 8192 x 4096 51 and 45. fp32
+    // sums would have to lie in registers in fours all through the loop, which spills: 8192 x 4096 73 us, 82)
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
       const int j = t + u * tpr;
       if (j < nvec) {
-        float* pw = part_w + static_cast<int64_t>(blockIdx.x) * cols + j * VE;
-        float* pb = part_b + static_cast<int64_t>(blockIdx.x) * cols + j * VE;
+        float pw[VE], pb[VE];
 #pragma unroll
-        for (int e = 0; e < VE; ++e) { pw[e] = aw[u][e]; pb[e] = ab[u][e]; }
+        for (int e = 0; e < VP; ++e) {
+          p_parts(aw[u][e], pw[2 * e], pw[2 * e + 1]);
+          p_parts(ab[u][e], pb[2 * e], pb[2 * e + 1]);
+        }
+        float* to_w = part_w + static_cast<int64_t>(blockIdx.x) * cols + j * VE;
+        float* to_b = part_b + static_cast<int64_t>(blockIdx.x) * cols + j * VE;
+        if constexpr (sizeof(T) == 2) {
+#pragma unroll
+          for (int e = 0; e < VE; e += 4) {
+            *reinterpret_cast<float4*>(to_w + e) = make_float4(pw[e], pw[e + 1], pw[e + 2], pw[e + 3]);
+            *reinterpret_cast<float4*>(to_b + e) = make_float4(pb[e], pb[e + 1], pb[e + 2], pb[e + 3]);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < VE; ++e) {
+            to_w[e] = pw[e];
+            to_b[e] = pb[e];
+          }
+        }
       }
     }
   }
@@ -1279,28 +1322,30 @@ __global__ void __launch_bounds__(256) layernorm_bwd_wb_lines(const void* __rest
   part_w[static_cast<int64_t>(blockIdx.y) * cols + c] = aw;
   part_b[static_cast<int64_t>(blockIdx.y) * cols + c] = ab;
 }
-// dw[c] = sum over the `parts` partial rows, same for db: a CTA takes 32 columns, its 32
-// warps take every 32nd partial row each (coalesced 128-byte reads), and the 32 slice sums
-// of a column are added in slice order -- a fixed order, so the result is reproducible.
+// dw[c] = sum over the `parts` partial rows, same for db: a CTA takes W columns, its 1024 / W rows of threads the partial
+// rows in turn; their sums are added in order. 32 columns (whole lines) where that makes enough CTAs, else 8, a sector:
+// bf16 2000 x 600, 1184 partial rows, 16.9 us the call with 32 columns to a CTA, 12.2 with 8.
+template <int W>
 __global__ void __launch_bounds__(1024) layernorm_bwd_finalize(const float* __restrict__ part_w, const float* __restrict__ part_b, void* __restrict__ dw, void* __restrict__ db, int64_t parts,
                                                                int64_t cols, int dt_wb) {
-  __shared__ float sw[32][33], sb[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t c = static_cast<int64_t>(blockIdx.x) * 32 + tx;
+  constexpr int R = 1024 / W;
+  __shared__ float sw[R][W + 1], sb[R][W + 1];
+  const int tx = threadIdx.x % W, ty = threadIdx.x / W;
+  const int64_t c = static_cast<int64_t>(blockIdx.x) * W + tx;
   float aw = 0.f, ab = 0.f;
   after_grids_before();
-  if (c < cols && parts <= 32) {
+  if (c < cols && parts <= R) {
     if (ty < parts) {
       aw = part_w[ty * cols + c];
       ab = part_b[ty * cols + c];
     }
   } else if (c < cols) {
     constexpr int U = 8;  // partial rows on the way (one after the other 1184 of 112 columns took 14.5 us)
-    for (int64_t p0 = ty; p0 < parts; p0 += 32 * U) {
+    for (int64_t p0 = ty; p0 < parts; p0 += R * U) {
       float w[U], b[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int64_t p = p0 + 32 * u;
+        const int64_t p = p0 + R * u;
         w[u] = p < parts ? part_w[p * cols + c] : 0.f;
         b[u] = p < parts ? part_b[p * cols + c] : 0.f;
       }
@@ -1314,6 +1359,19 @@ __global__ void __launch_bounds__(1024) layernorm_bwd_finalize(const float* __re
   sw[ty][tx] = aw;
   sb[ty][tx] = ab;
   __syncthreads();
+  // the first 32 rows of threads add up R / 32 sums each, the first row what these leave
+  if constexpr (R > 32) {
+    if (ty < 32) {
+#pragma unroll
+      for (int k = 1; k < R / 32; ++k) {
+        aw += sw[ty + 32 * k][tx];
+        ab += sb[ty + 32 * k][tx];
+      }
+      sw[ty][tx] = aw;
+      sb[ty][tx] = ab;
+    }
+    __syncthreads();
+  }
   if (ty == 0 && c < cols) {
     float tw = 0.f, tb = 0.f;
 #pragma unroll
@@ -2629,12 +2687,13 @@ extern "C" int b200_layer_norm_backward(const void* dy, const void* x, const voi
     }
   }
   if (need_wb) {
-    if (parts <= 32) {
-      layernorm_bwd_finalize<<<grid_for(cols, 32), 1024, 0, st>>>(pw, pb, dw, db, parts, cols, dt_wb);
-    } else {
-      const cudaError_t e = launch_after(layernorm_bwd_finalize, grid_for(cols, 32), 1024, 0, st, pw, pb, dw, db, parts, cols, dt_wb);
-      if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
-    }
+    auto finalize = [&](auto kernel, int w) -> cudaError_t {
+      if (parts > 32) return launch_after(kernel, grid_for(cols, w), 1024, 0, st, pw, pb, dw, db, parts, cols, dt_wb);
+      kernel<<<grid_for(cols, w), 1024, 0, st>>>(pw, pb, dw, db, parts, cols, dt_wb);
+      return cudaSuccess;
+    };
+    const cudaError_t e = parts > 32 && cols < 32 * (kNumSMs / 2) ? finalize(layernorm_bwd_finalize<8>, 8) : finalize(layernorm_bwd_finalize<32>, 32);
+    if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
   }
   return check_launch(need_wb ? 2 : 1);
 }
