@@ -70,8 +70,12 @@ __device__ __forceinline__ void warp_merge(CloseAcc& a) {
 // order like their bit patterns.
 // `direct`: the record is to start from zero and the launch is one CTA, or (kCloseCluster) one cluster,
 // whose CTAs leave their accumulators with the first: it simply writes the record (no memset node before the
-// kernel, no atomics).
+// kernel, no atomics). The first one's shared memory may be written only once that CTA is known to run: every CTA
+// arrives at the cluster's barrier as it starts and waits there before it stores, by when the others have long
+// arrived (their loads come in between).
 constexpr int kCloseCluster = 8;
+__device__ __forceinline__ void cluster_started_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_started_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 __device__ __forceinline__ void write_record(const CloseAcc& a, b200_close_record* rec) {
   rec->mismatches = a.bad;
   rec->max_abs = a.max_abs;
@@ -91,6 +95,7 @@ __device__ __forceinline__ void publish(CloseAcc a, b200_close_record* rec, int 
   }
   if (direct == kCloseCluster) {
     cg::cluster_group cluster = cg::this_cluster();
+    cluster_started_wait();
     if (threadIdx.x == 0) *cluster.map_shared_rank(&from[cluster.block_rank()], 0) = a;
     cluster.sync();
     if (cluster.block_rank() != 0 || warp != 0) return;
@@ -121,6 +126,7 @@ template <> struct kExpMask16<__half> { static constexpr uint32_t value = 0x7c00
 template <typename T>
 __global__ void __launch_bounds__(256, 4) allclose_kernel(const T* __restrict__ ref, const T* __restrict__ res, int64_t n, float rtol, float atol, b200_close_record* rec, int vec_ok, int direct) {
   constexpr int VE = Vec<T>::N;
+  if (direct == kCloseCluster) cluster_started_arrive();  // (publish waits)
   CloseAcc a{0ull, 0.f, 0.f, 0u};
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
