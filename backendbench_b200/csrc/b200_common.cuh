@@ -28,6 +28,10 @@ inline int check_launch(int launches = 1) {
 // A kernel that follows one of the same call: its CTAs may start before that one has ended (programmatic
 // dependent launch), which hides the launch, and begin with after_grids_before() or do first what does not depend on it. Every
 // kernel launched so calls after_grids_before(), whatever it then does: the next one relies on it for all that came earlier.
+// And while it lives the one before may still be writing: what that one writes is not read-only here, so it is neither `const
+// __restrict__` nor read with __ldg / __ldcs (ld_keep, ld_stream), which the compiler may move to before the wait, but with ordinary
+// loads, or those below from a pointer that has gone through waited(). What the first kernel of the call found complete (it is
+// launched the ordinary way) may be both.
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*kernel)(P...), int64_t grid, int block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg{};
@@ -44,6 +48,25 @@ inline cudaError_t launch_after(void (*kernel)(P...), int64_t grid, int block, s
 }
 // (device) what the grids before have written is there; the next grid's CTAs may start where there is room
 __device__ __forceinline__ void after_grids_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename T> __device__ __forceinline__ T* waited(T* p) {  // the address comes out behind the wait, and so do the loads from it
+  asm volatile("" : "+l"(p));
+  return p;
+}
+__device__ __forceinline__ uint4 ld_keep_after(const void* p) {
+  uint4 v;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_stream_after(const void* p) {
+  uint4 v;
+  asm("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_stream_after_f(const float* p) {
+  float v;
+  asm("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -24,17 +24,18 @@ struct MulConstOp { float c; __device__ __forceinline__ float operator()(float x
 struct MulOp { __device__ __forceinline__ float operator()(float a, float b) const { return a * b; } };
 
 template <typename T, typename Op>
-__global__ void __launch_bounds__(kEwThreads) ew_unary_vec(const T* __restrict__ x, T* __restrict__ out, int64_t n, Op op) {
+__global__ void __launch_bounds__(kEwThreads) ew_unary_vec(const T* x, T* __restrict__ out, int64_t n, Op op) {
   constexpr int VE = Vec<T>::N;
   next_grid_may_start();
   after_grids_before();
+  const T* xw = waited(x);
   const int64_t nvec = n / VE;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * (kEwThreads * kUnroll) + threadIdx.x;
   Vec<T> v[kUnroll];
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
     const int64_t i = base + u * kEwThreads;
-    if (i < nvec) v[u].raw = ld_stream(x + i * VE);
+    if (i < nvec) v[u].raw = ld_stream_after(xw + i * VE);
   }
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {

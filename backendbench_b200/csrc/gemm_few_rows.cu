@@ -57,7 +57,7 @@ __device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 template <typename T, int NT>
-__global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ bias, T* __restrict__ C, FewRowsArgs p) {
+__global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* A, const T* B, const T* bias, T* __restrict__ C, FewRowsArgs p) {
   constexpr int kCols = 8 * NT, kPitch = kCols + 1, kFewSteps = FewSteps<NT>::value;
   __shared__ float red[kFewWarps][kFewRows][kPitch];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane >> 2, c = lane & 3;
@@ -87,6 +87,10 @@ __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __re
       if ((c & 1) == 0 && k + 8 * c < K && col[t]) asm volatile("prefetch.global.L2 [%0];" ::"l"(b[t] + k));
   }
   after_grids_before();
+  a0 = waited(a0);
+  a1 = waited(a1);
+#pragma unroll
+  for (int t = 0; t < NT; ++t) b[t] = waited(b[t]);
   for (int k0 = warp * 32 * kFewSteps; k0 < K; k0 += kFewWarps * 32 * kFewSteps) {
     uint4 ra[kFewSteps], rA[kFewSteps], rb[NT][kFewSteps];
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -95,9 +99,9 @@ __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* __re
       const int k = k0 + 32 * u;
       const bool in = k + 8 * c < K;
 #pragma unroll
-      for (int t = 0; t < NT; ++t) rb[t][u] = in && col[t] ? ld_stream(b[t] + k) : zero;
-      ra[u] = in && row0 ? ld_keep(a0 + k) : zero;
-      rA[u] = in && row1 ? ld_keep(a1 + k) : zero;
+      for (int t = 0; t < NT; ++t) rb[t][u] = in && col[t] ? ld_stream_after(b[t] + k) : zero;
+      ra[u] = in && row0 ? ld_keep_after(a0 + k) : zero;
+      rA[u] = in && row1 ? ld_keep_after(a1 + k) : zero;
     }
 #pragma unroll
     for (int u = 0; u < kFewSteps; ++u) {

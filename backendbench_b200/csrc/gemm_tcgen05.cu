@@ -177,7 +177,7 @@ __device__ __forceinline__ void tile_coords(int64_t rem, int64_t mt, int64_t nt,
 // or float when the operands are the bf16 planes of split fp32 matrices.
 template <typename T, int kBN, typename TO, bool kPair = false, bool kRows = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c, const TO* __restrict__ bias, TO* __restrict__ C, GemmTcParams p,
+gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c, const TO* bias, TO* __restrict__ C, GemmTcParams p,
                     uint32_t* __restrict__ status) {
   using Cfg = TileCfg<kBN, kPair>;
   constexpr int kAccs = Cfg::kAccs;
@@ -241,6 +241,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
   after_grids_before();  // what is above needs nothing that an earlier kernel writes
+  const TO* bias_w = waited(bias);
   const bool skip = p.skip_if_set && *p.skip_if_set != 0u;  // the same word for every thread of every CTA
 
   const int64_t mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + bn - 1) / bn;
@@ -450,7 +451,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           if (bias_vec && m < p.M && n + 8 <= p.N) {
             // unit-stride bias (a row vector, or a matrix like C): eight values in one load
             float bv[8];
-            widen<T>(ld_keep(bias + m * p.sbm + n), bv);  // TO is T on this path
+            widen<T>(ld_keep_after(bias_w + m * p.sbm + n), bv);  // TO is T on this path
             if (unit_scales) {  // addmm as models call it: one add per value
 #pragma unroll
               for (int e = 0; e < 8; ++e) rc[g * 8 + e] = __float_as_uint(__uint_as_float(rc[g * 8 + e]) + bv[e]);
@@ -894,9 +895,10 @@ int64_t gemm_tc_splitk_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_
 // 12.3 -> 4.7 us), one below, where fewer and busier threads only wait longer, and of a small result B
 // ranges at a time (20000 deep, 40 x 128 outputs: the call 12.7 us, 16 with eight in flight).
 template <typename T, int U, int B>
-__global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ part, int splits, int64_t M, int64_t N, const T* __restrict__ bias, int64_t sbm, int64_t sbn, float alpha, float beta,
+__global__ void __launch_bounds__(256) splitk_reduce(const float* part, int splits, int64_t M, int64_t N, const T* bias, int64_t sbm, int64_t sbn, float alpha, float beta,
                                                      T* __restrict__ C, const uint32_t* skip_if_set) {
   after_grids_before();
+  const float* part_w = waited(part);
   if (skip_if_set && *skip_if_set != 0u) return;  // the partial products were not computed either
   const int64_t total = M * N;
   for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * (256 * U) + threadIdx.x; i0 < total; i0 += static_cast<int64_t>(gridDim.x) * (256 * U)) {
@@ -918,7 +920,7 @@ __global__ void __launch_bounds__(256) splitk_reduce(const float* __restrict__ p
       for (int s = 0; s < splits; ++s) {
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (i0 + u * 256 < total) sum[u] += __ldcs(part + s * total + i0 + u * 256);
+          if (i0 + u * 256 < total) sum[u] += ld_stream_after_f(part_w + s * total + i0 + u * 256);
       }
     }
 #pragma unroll

@@ -1326,7 +1326,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_wb_lines(const void* __rest
 // rows in turn; their sums are added in order. 32 columns (whole lines) where that makes enough CTAs, else 8, a sector:
 // bf16 2000 x 600, 1184 partial rows, 16.9 us the call with 32 columns to a CTA, 12.2 with 8.
 template <int W>
-__global__ void __launch_bounds__(1024) layernorm_bwd_finalize(const float* __restrict__ part_w, const float* __restrict__ part_b, void* __restrict__ dw, void* __restrict__ db, int64_t parts,
+__global__ void __launch_bounds__(1024) layernorm_bwd_finalize(const float* part_w, const float* part_b, void* __restrict__ dw, void* __restrict__ db, int64_t parts,
                                                                int64_t cols, int dt_wb) {
   constexpr int R = 1024 / W;
   __shared__ float sw[R][W + 1], sb[R][W + 1];

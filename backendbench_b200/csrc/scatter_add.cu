@@ -726,8 +726,8 @@ __global__ void __launch_bounds__(256) bucket_count(const int64_t* __restrict__ 
 // where a segment lies: one pass instead of an exclusive scan's three. Counters above `light`
 // are listed. The counters start at `zero`.
 template <int ITEMS>
-__device__ __forceinline__ void assign_segments_of(const int* __restrict__ cnt, int zero, int* __restrict__ cursor, int64_t n, int* __restrict__ total, int light, int* __restrict__ heavy_count,
-                                                   int* __restrict__ heavy_list) {
+__device__ __forceinline__ void assign_segments_of(const int* cnt, int zero, int* cursor, int64_t n, int* total, int light, int* heavy_count,
+                                                   int* heavy_list) {
   __shared__ int warp_sums[8];
   __shared__ int block_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -785,8 +785,8 @@ __device__ __forceinline__ void assign_segments_of(const int* __restrict__ cnt, 
   }
 }
 template <int ITEMS>
-__global__ void __launch_bounds__(256) assign_segments(const int* __restrict__ cnt, int* __restrict__ cursor, int64_t n, int* __restrict__ total, int light, int* __restrict__ heavy_count,
-                                                       int* __restrict__ heavy_list) {
+__global__ void __launch_bounds__(256) assign_segments(const int* cnt, int* cursor, int64_t n, int* total, int light, int* heavy_count,
+                                                       int* heavy_list) {
   after_grids_before();
   assign_segments_of<ITEMS>(cnt, 0, cursor, n, total, light, heavy_count, heavy_list);
 }
@@ -807,8 +807,8 @@ __global__ void __launch_bounds__(256) bucket_fill(const int64_t* __restrict__ i
 // One thread per destination: replay its segment in ascending source position. The counters start at
 // `zero`; nothing is done where `only_if` points to a zero.
 template <typename T>
-__global__ void __launch_bounds__(256) bucket_replay(const T* __restrict__ self, T* __restrict__ out, const int* __restrict__ cnt, int zero, const int* __restrict__ cursor,
-                                                     const int2* __restrict__ seg, int64_t n_self, const int* only_if) {
+__global__ void __launch_bounds__(256) bucket_replay(const T* __restrict__ self, T* __restrict__ out, const int* cnt, int zero, const int* cursor,
+                                                     const int2* seg, int64_t n_self, const int* only_if) {
   after_grids_before();
   if (only_if && *only_if == 0) return;
   for (int64_t d = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; d < n_self; d += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -848,7 +848,7 @@ struct HeavyCounters {
   const int* grouped;
 };
 template <typename T>
-__global__ void __launch_bounds__(256) bucket_replay_heavy(const T* __restrict__ self, T* __restrict__ out, HeavyCounters H, const int2* __restrict__ seg, int64_t dim_len,
+__global__ void __launch_bounds__(256) bucket_replay_heavy(const T* __restrict__ self, T* __restrict__ out, HeavyCounters H, const int2* seg, int64_t dim_len,
                                                            const int* heavy_count, const int* heavy_list) {
   __shared__ float slot_val[kHeavyWindow];
   __shared__ unsigned char slot_set[kHeavyWindow];
@@ -1139,7 +1139,7 @@ __global__ void __launch_bounds__(256) chain_replay(const T* __restrict__ self, 
 
 // The contributions of listed destinations, or all of them: counted (into the list's counters, or into
 // the heads, which stand at -1), given segments, filled in.
-__global__ void __launch_bounds__(256) chain_count(const int64_t* __restrict__ index, int* __restrict__ head, int* __restrict__ listed_cnt, const __grid_constant__ BucketArgs A,
+__global__ void __launch_bounds__(256) chain_count(const int64_t* __restrict__ index, int* head, int* listed_cnt, const __grid_constant__ BucketArgs A,
                                                    const int* ctl) {
   after_grids_before();
   const bool grouped = ctl[kCtlGrouped] != 0;
@@ -1156,8 +1156,8 @@ __global__ void __launch_bounds__(256) chain_count(const int64_t* __restrict__ i
     }
   }
 }
-__global__ void __launch_bounds__(256) chain_assign(const int* __restrict__ head, int* __restrict__ cursor, int64_t n_self, const int* __restrict__ listed_cnt, int* __restrict__ listed_cursor,
-                                                    int64_t listed, int* __restrict__ ctl, int* __restrict__ heavy_list) {
+__global__ void __launch_bounds__(256) chain_assign(const int* head, int* cursor, int64_t n_self, const int* listed_cnt, int* listed_cursor,
+                                                    int64_t listed, int* ctl, int* heavy_list) {
   constexpr int ITEMS = 16;
   after_grids_before();
   const bool grouped = ctl[kCtlGrouped] != 0;
@@ -1166,8 +1166,8 @@ __global__ void __launch_bounds__(256) chain_assign(const int* __restrict__ head
   else assign_segments_of<ITEMS>(listed_cnt, 0, listed_cursor, listed, ctl + kCtlSlots, 0x7fffffff, nullptr, nullptr);
 }
 template <typename T>
-__global__ void __launch_bounds__(256) chain_fill(const int64_t* __restrict__ index, const T* __restrict__ src, const int* __restrict__ head, int* __restrict__ cursor, int* __restrict__ listed_cursor,
-                                                  int2* __restrict__ seg, const __grid_constant__ BucketArgs A, const int* ctl, uint32_t* status) {
+__global__ void __launch_bounds__(256) chain_fill(const int64_t* __restrict__ index, const T* __restrict__ src, const int* head, int* cursor, int* listed_cursor,
+                                                  int2* seg, const __grid_constant__ BucketArgs A, const int* ctl, uint32_t* status) {
   after_grids_before();
   const bool grouped = ctl[kCtlGrouped] != 0;
   if (!grouped && ctl[kCtlListed] == 0) return;
@@ -1430,7 +1430,7 @@ __global__ void __launch_bounds__(kBinThreads, 2) binned_sort(const int64_t* __r
 }
 
 template <typename T>
-__global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, T* __restrict__ out, const typename BinRec<T>::type* __restrict__ rec, const uint16_t* __restrict__ first,
+__global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, T* __restrict__ out, const typename BinRec<T>::type* rec, const uint16_t* first,
                                                     const __grid_constant__ BinnedArgs A, const int* ctl, int* head, int64_t n_self) {
   typedef typename BinRec<T>::type Rec;
   constexpr uint32_t kAll = 0xffffffffu;
@@ -1670,7 +1670,7 @@ __global__ void __launch_bounds__(256) emb_count(const void* __restrict__ idx, i
     atomicAdd(&cnt[v], 1);
   }
 }
-__global__ void __launch_bounds__(256) emb_fill(const void* __restrict__ idx, int i32, int64_t n, int64_t V, int64_t padding_idx, int* __restrict__ cursor, int* __restrict__ seg_pos) {
+__global__ void __launch_bounds__(256) emb_fill(const void* __restrict__ idx, int i32, int64_t n, int64_t V, int64_t padding_idx, int* cursor, int* __restrict__ seg_pos) {
   after_grids_before();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t v = emb_index(idx, i, i32);
@@ -1683,8 +1683,8 @@ __global__ void __launch_bounds__(256) emb_fill(const void* __restrict__ idx, in
 // a segment are distinct). cursor[v] is the END of row v's segment by now. A CTA takes the
 // long ones: a bitmap of a window of positions, prefix sums of its words' bit counts, and
 // every position finds its own rank. A warp takes the others, ranked with shuffles.
-__global__ void __launch_bounds__(256) emb_sort(const int* __restrict__ cnt, const int* __restrict__ cursor, const int* __restrict__ seg_pos, int* __restrict__ sorted, int64_t V, int64_t n,
-                                                const int* __restrict__ heavy_count, const int* __restrict__ heavy_list) {
+__global__ void __launch_bounds__(256) emb_sort(const int* cnt, const int* cursor, const int* seg_pos, int* __restrict__ sorted, int64_t V, int64_t n,
+                                                const int* heavy_count, const int* heavy_list) {
   __shared__ uint32_t bitmap[kEmbWindowWords];
   __shared__ int before[kEmbWindowWords];
   __shared__ int warp_sums[8];
@@ -1833,8 +1833,8 @@ template <typename T, typename WORD> __device__ __forceinline__ void emb_word_ad
 }
 
 template <typename T, bool VEC, typename WORD>
-__global__ void __launch_bounds__(256, 4) emb_replay(const T* __restrict__ grad, T* __restrict__ out, const int* __restrict__ cnt, const int* __restrict__ cursor, const int* __restrict__ sorted,
-                                                     int64_t V, int64_t D, const int* __restrict__ heavy_count, const int* __restrict__ heavy_list, int heavy_blocks, int tx_log2) {
+__global__ void __launch_bounds__(256, 4) emb_replay(const T* __restrict__ grad, T* __restrict__ out, const int* cnt, const int* cursor, const int* sorted,
+                                                     int64_t V, int64_t D, const int* heavy_count, const int* heavy_list, int heavy_blocks, int tx_log2) {
   after_grids_before();
   if (static_cast<int>(blockIdx.x) < heavy_blocks) {
     constexpr int PK = sizeof(WORD) / sizeof(T);
