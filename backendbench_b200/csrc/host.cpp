@@ -172,28 +172,10 @@ Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like
 Tensor new_like(const Tensor& t) { return new_tensor(t.sizes(), t.scalar_type(), t); }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// One growing buffer per device and stream, as ops.py keeps them (it asks here when this module is loaded): the
-// 64 most recently sized are kept. Guarded by the interpreter lock.
-struct Scratch {
-  int64_t device;
-  void* stream;
-  Tensor buffer;
-};
-std::vector<Scratch>& scratch_pool() {
-  static auto* pool = new std::vector<Scratch>();  // never destroyed: no CUDA calls at exit
-  return *pool;
-}
-Tensor scratch_on(int64_t device, void* st, int64_t bytes) {
-  auto& pool = scratch_pool();
-  auto it = std::find_if(pool.begin(), pool.end(), [&](const Scratch& s) { return s.device == device && s.stream == st; });
-  if (it != pool.end() && it->buffer.numel() >= bytes) return it->buffer;
-  Tensor b = at::detail::empty_cuda({std::max<int64_t>(bytes, 1 << 20)}, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)), std::nullopt);
-  if (it != pool.end()) pool.erase(it);
-  pool.push_back(Scratch{device, st, b});
-  if (pool.size() > 64) pool.erase(pool.begin());
-  return b;
-}
-Tensor scratch(const Tensor& like, int64_t bytes) { return bytes > 0 ? scratch_on(like.get_device(), stream(), bytes) : Tensor(); }
+// Scratch is the call's own, from the caching allocator: a call is several launches that rely on what the ones before have left
+// there, and the interpreter lock is not held between them, so that a buffer kept per stream would be another thread's, too. It
+// goes back in stream order when the call's launches are queued, and belongs to the graph where they are captured.
+Tensor scratch(const Tensor& like, int64_t bytes) { return bytes > 0 ? new_tensor({bytes}, at::kByte, like) : Tensor(); }
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 // The device's status word (ops._status); nullptr with an exception set if that failed
@@ -552,7 +534,7 @@ PyObject* embedding_backward(ARGS) {
   uint32_t* status = status_word(*g);
   if (!status) return nullptr;
   const int64_t need = api.b200_embedding_backward_scratch_bytes(n, rows);
-  Tensor s = scratch_on(g->get_device(), stream(), need);
+  Tensor s = scratch(*g, need);
   if (!launched("b200_embedding_backward", [&, st = stream()] { return api.b200_embedding_backward(ptr(*g), ptr(*idx), ptr(out), n, rows, width, padding, dt(*g), index_dt(*idx), ptr(s), need, status, st); }))
     return nullptr;
   return wrap(std::move(out));
@@ -825,16 +807,6 @@ PyObject* make(PyObject*, PyObject* args) {
   return PyErr_Format(PyExc_KeyError, "%s", name);
 }
 
-// scratch(device index, stream, bytes)
-PyObject* scratch_py(PyObject*, PyObject* args) {
-  HANDLE_TH_ERRORS
-  long long device, bytes;
-  unsigned long long st;
-  if (!PyArg_ParseTuple(args, "LKL", &device, &st, &bytes)) return nullptr;
-  return wrap(scratch_on(device, reinterpret_cast<void*>(st), bytes));
-  END_HANDLE_TH_ERRORS
-}
-
 // compare(reference, result, atol, rtol, record): the pairs of tensors are queued into the device record. False: nothing
 // was done, the structures are not what this serves (tensors of one shape and floating dtype, contiguous, or a tuple of them).
 PyObject* compare(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -872,7 +844,6 @@ PyObject* compare(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 PyMethodDef kMethods[] = {{"setup", setup, METH_VARARGS, nullptr},
                           {"make", make, METH_VARARGS, nullptr},
-                          {"scratch", scratch_py, METH_VARARGS, nullptr},
                           {"compare", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compare)), METH_FASTCALL, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_b200host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -19,7 +19,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import torch
 
-from . import _abi, _native
+from . import _abi
 from ._abi import check, i64_array, lib
 
 _DT = {
@@ -416,28 +416,14 @@ def _log_softmax_default(self, dim, half_to_float) -> torch.Tensor:
     return _softmax_impl(self, dim, bool(half_to_float), True)
 
 
-_scratch_cache = {}
-
-
-_SCRATCH_MAX_STREAMS = 64
+_scratch_cache = {}  # holds nothing: scratch does not outlive its call
 
 
 def _scratch(device: torch.device, nbytes: int) -> torch.Tensor:
-    """A scratch buffer of at least `nbytes` for the current stream of `device` (grown
-    geometrically, reused; per stream, so that operators queued on different streams never
-    share one)."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream_handle())
-    native = _native.module() if _allocator is None else None
-    if native is not None:  # one buffer for the calls that are served here and those that are served there
-        return native.scratch(key[0], key[1], nbytes)
-    buf = _scratch_cache.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = _new(max(nbytes, 1 << 20), torch.uint8, device)
-        _scratch_cache.pop(key, None)
-        _scratch_cache[key] = buf
-        while len(_scratch_cache) > _SCRATCH_MAX_STREAMS:  # streams come and go: keep the most recently sized buffers only
-            _scratch_cache.pop(next(iter(_scratch_cache)))
-    return buf
+    """`nbytes` of scratch for one call, which keeps it until its launches are queued. (No buffer
+    per stream is kept: the launches of two threads' calls can interleave on a stream, ctypes
+    lets go of the interpreter lock, and each call relies on what its earlier kernels left there.)"""
+    return _new((nbytes,), torch.uint8, device)
 
 
 def _reduce_layout(self: torch.Tensor, dims: List[int]):

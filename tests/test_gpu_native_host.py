@@ -241,6 +241,41 @@ def test_streams_threads_capture_and_scratch(backend):
     assert bits_equal(ops.sum_dim_IntList(x, [0]), r)
 
 
+@pytest.mark.parametrize("native", [True, False])
+def test_threads_that_share_a_stream(backend, native):
+    """Operators of several launches and scratch between them, each thread with results of its own, all on one stream."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+
+    def one(k):
+        x = torch.randn(3000 + k, 33, generator=g, device=DEV)
+        i = torch.randint(0, 3000 + k, (3000, 33), generator=g, device=DEV)
+        t = torch.randint(0, 500 + k, (4000,), generator=g, device=DEV)
+        a, b = torch.randn(40, 3000 + 8 * k, generator=g, device=DEV).half(), torch.randn(3000 + 8 * k, 64, generator=g, device=DEV).half()
+        ones, m, s = torch.ones(33, device=DEV), x.mean(1, keepdim=True), 1 / x.std(1, keepdim=True)
+        return [("scatter_add.default", (x, 0, i, x[:3000].contiguous())), ("sum.dim_IntList", (x, [0])), ("embedding_dense_backward.default", (x[:3000], t[:3000], 500 + k, -1, False)),
+                ("mm.default", (a, b)), ("native_layer_norm_backward.default", (x, x, [33], m, s, ones, ones, [True, True, True]))]
+
+    work = [one(k) for k in range(6)]
+    call = {n: backend[get_operator(n)] if native else _wrapper(n) for n, _ in work[0]}
+    want = [[call[n](*args) for n, args in calls] for calls in work]
+    ops.check_device_status()
+    wrong = []
+
+    def run(k):
+        try:
+            for _ in range(30):
+                got = [call[n](*args) for n, args in work[k]]
+                wrong.extend((k, n) for (n, _), w, r in zip(work[k], want[k], got) if not _same(w, r))
+        except Exception as e:  # pragma: no cover
+            wrong.append(e)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(6)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    ops.check_device_status()
+    assert not wrong, wrong
+
+
 def test_comparisons_queued_natively_give_the_same_records(monkeypatch):
     g = torch.Generator(device=DEV).manual_seed(2)
     x = torch.randn(1000, 33, generator=g, device=DEV)

@@ -299,3 +299,14 @@ def test_enable_disable_on_cpu_key_with_watermark(tmp_path, capsys):
     bb.disable()
     assert torch.equal(torch.relu(x), torch.tensor([0.0, 0.0, 1.0]))
     bb.enable(kernel_dir=str(tmp_path / "nope"))  # missing directory: warning, no exception
+
+
+def test_each_call_has_scratch_of_its_own(monkeypatch):
+    """Two calls of one stream may be under way at once (threads): neither gets the other's buffer."""
+    from backendbench_b200 import _native, ops
+
+    monkeypatch.setattr(ops, "_stream_handle", lambda: 0)
+    monkeypatch.setattr(_native, "module", lambda: None)
+    device = torch.device("cpu", 0)
+    one, other = ops._scratch(device, 4096), ops._scratch(device, 4096)
+    assert one.numel() >= 4096 and one.data_ptr() != other.data_ptr()
