@@ -310,3 +310,19 @@ def test_each_call_has_scratch_of_its_own(monkeypatch):
     device = torch.device("cpu", 0)
     one, other = ops._scratch(device, 4096), ops._scratch(device, 4096)
     assert one.numel() >= 4096 and one.data_ptr() != other.data_ptr()
+
+
+def test_a_host_module_that_cannot_be_loaded_leaves_the_wrappers(monkeypatch, tmp_path):
+    """(built against another torch, say) One warning, and every call and every plugin works without it."""
+    from backendbench_b200 import _native, custom_ops
+
+    bad = tmp_path / "_b200host.so"
+    bad.write_bytes(b"not a module")
+    monkeypatch.setattr(_native, "PATH", str(bad))
+    monkeypatch.setattr(_native, "_module", None)
+    with pytest.warns(UserWarning, match="cannot be used"):
+        assert _native.module() is None
+    assert _native.module() is None
+    with pytest.raises(UnsupportedByB200):  # the wrapper's own answer to a CPU tensor
+        custom_ops.entry("relu")(torch.ones(2))
+    assert len(B200Backend().compiled_kernels) == len(os.listdir(KERNELS_DIR))
