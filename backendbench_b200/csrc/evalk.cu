@@ -230,8 +230,6 @@ extern "C" int b200_allclose(const void* ref, const void* res, int64_t n, int dt
   // and a launch (most of the sweep's cases are this small, and their cost is launches, not bytes): one CTA up to 2048
   // elements, a cluster of eight up to 65536. fp32, equal / different values: 32768 elements 6.2 / 15.2 us with
   // one CTA, 3.0 / 4.4 with a cluster; 65536 5.5 / 6.6 with a memset and 32 CTAs, 3.5 / 6.4; bf16 131072 6.1 / 6.7 and 3.8 / 8.3.
-  const int es = dtype_size(dtype);
-  if (es == 0) return B200_EDTYPE;
   const int direct = !reset || n == 0 ? 0 : n <= 2048 ? 1 : n <= 65536 && is_float_dtype(dtype) ? kCloseCluster : n <= 32768 ? 1 : 0;
   if (reset && !direct) {
     const cudaError_t e = cudaMemsetAsync(rec, 0, sizeof(b200_close_record), st);
@@ -239,6 +237,8 @@ extern "C" int b200_allclose(const void* ref, const void* res, int64_t n, int dt
   }
   if (n == 0) return B200_OK;
   if (!ref || !res) return B200_EINVAL;
+  const int es = dtype_size(dtype);
+  if (es == 0) return B200_EDTYPE;
   int64_t blocks = n <= 32768 ? 1 : (n + 256 * 8 - 1) / (256 * 8);
   const int64_t cap = static_cast<int64_t>(kNumSMs) * 8;  // one resident wave of 256-thread CTAs
   const int g = static_cast<int>(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));

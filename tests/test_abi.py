@@ -41,3 +41,11 @@ def test_argument_validation_needs_no_gpu():
     assert lib.b200_reduce_scratch_bytes(1, 1 << 26, 1) > 0
     assert lib.b200_reduce_scratch_bytes(8192, 4096, 1) == 0
     assert lib.b200_gemm(None, None, None, None, 1, 0, 5, 5, 0, 5, 1, 0, 5, 1, 0, 0, 1.0, 0.0, _abi.F32, None, None) == 0
+
+
+def test_nothing_to_compare_is_close_whatever_its_dtype():
+    lib = _abi.lib()
+    rec = ctypes.c_int64(0)  # (not written: the record is not to be reset)
+    for dtype in (_abi.F32, _abi.I64, _abi.F64, 99):
+        assert lib.b200_allclose(None, None, 0, dtype, 0.0, 0.0, ctypes.addressof(rec), 0, None) == 0
+    assert lib.b200_allclose(ctypes.addressof(rec), ctypes.addressof(rec), 1, 99, 0.0, 0.0, ctypes.addressof(rec), 0, None) == -2
