@@ -503,7 +503,11 @@ PyObject* layer_norm_backward(ARGS) {
 
 PyObject* embedding(ARGS) {
   Args a;
-  if (!a.parse(args, nargs, kwnames, {"weight", "indices", "padding_idx", "scale_grad_by_freq", "sparse"}, 2)) return nullptr;
+  int64_t padding;
+  bool freq, sparse;  // (these three count in the gradient alone)
+  if (!a.parse(args, nargs, kwnames, {"weight", "indices", "padding_idx", "scale_grad_by_freq", "sparse"}, 2) || (a[2] && !integer(a[2], padding)) || (a[3] && !boolean(a[3], freq)) ||
+      (a[4] && !boolean(a[4], sparse)))
+    return nullptr;
   const Tensor *w = tensor(a[0]), *idx = tensor(a[1]);
   if (!w || !idx || w->dim() < 1 || index_dt(*idx) < 0 || !w->is_contiguous() || !idx->is_contiguous() || !plain(*w, *idx)) return nullptr;
   at::DimVector shape(idx->sizes().begin(), idx->sizes().end());
@@ -571,7 +575,8 @@ bool index_fits(const Tensor& self, int64_t dim, const Tensor& index, const Tens
 PyObject* gather(ARGS) {
   Args a;
   int64_t dim, d;
-  if (nargs > 3 || !a.parse(args, nargs, kwnames, {"self", "dim", "index", "sparse_grad"}, 3) || !integer(a[1], dim)) return nullptr;
+  bool sparse;  // (counts in the gradient alone)
+  if (nargs > 3 || !a.parse(args, nargs, kwnames, {"self", "dim", "index", "sparse_grad"}, 3) || !integer(a[1], dim) || (a[3] && !boolean(a[3], sparse))) return nullptr;
   const Tensor *x = tensor(a[0]), *idx = tensor(a[2]);
   if (!x || !idx || !dimension(dim, x->dim(), d) || !index_fits(*x, d, *idx, Tensor()) || idx->numel() == 0 || !plain(*x, *idx)) return nullptr;
   uint32_t* status = status_word(*x);

@@ -154,6 +154,16 @@ def test_every_call_is_answered_as_the_wrapper_answers_it(backend):
     assert len(seen) == len(custom_ops.OPERATORS) and n > 1000
 
 
+def test_arguments_that_a_call_does_not_use_are_looked_at_all_the_same(backend):
+    """What the operator's schema refuses is refused by the native call, too."""
+    x, ix = torch.randn(9, 4, device=DEV), torch.zeros(9, 4, dtype=torch.int64, device=DEV)
+    embedding, gather = backend[get_operator("embedding.default")], backend[get_operator("gather.default")]
+    for call in (lambda: embedding(x, ix, "3"), lambda: embedding(x, ix, -1, "no"), lambda: embedding(x, ix, -1, False, ix), lambda: embedding(x, ix, padding_idx=None), lambda: gather(x, 0, ix, sparse_grad="no")):
+        with pytest.raises((RuntimeError, TypeError)):
+            call()
+    assert bits_equal(embedding(x, ix, 3, False, True), embedding(x, ix)) and bits_equal(gather(x, 0, ix, sparse_grad=True), gather(x, 0, ix))
+
+
 class _Seen(torch.Tensor):
     calls = 0
 
