@@ -606,9 +606,10 @@ static int index_select_bytes(const void* x, const void* idx, void* out, int64_t
     }
     return check_launch();
   }
-  // (16-byte vectors of the result meet at most two rows)
+  // (16-byte vectors of the result meet at most two rows. Rows on the 8-byte grid go a unit to a thread at every size: fp32 38 wide, 480810
+  // rows of the result, 37.0 us, 51.2 in ragged vectors, f16 164 wide, 127940 rows 17.9 and 27.1, fp32 4174 wide, 719 rows 5.8 and 7.1)
   const int64_t total = outer * n_idx * inner_bytes;
-  if (unit < 16 && inner_bytes >= 16 && aligned16(out) && total / unit >= kRaggedMinUnits) {
+  if (unit < 8 && inner_bytes >= 16 && aligned16(out) && total / unit >= kRaggedMinUnits) {
     select_rows_ragged<<<capped_grid((total + 15) / 16, 256 * kRaggedUnroll, 16), 256, 0, st>>>(static_cast<const unsigned char*>(x), idx, static_cast<unsigned char*>(out), outer, dim_size, inner_bytes, n_idx, i32,
                                                                                                 status);
     return check_launch();
