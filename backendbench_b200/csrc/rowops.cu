@@ -2487,8 +2487,9 @@ extern "C" int b200_layer_norm(const void* x, const void* w, const void* b, void
   ResidentCfg c{false, false, 1, 128};
   if (cols > 0 && cols % ve == 0 && (dt_wb != B200_F32 || cols % 4 == 0) && al && wb_ok && cols < (1LL << 30)) c = resident_cfg(cols / ve, 32 / ve, ve == 4 ? 4 : 2);
   // ragged rows: a warp each where they are short and many, a CTA each elsewhere (bf16 20000 x 70 8.4 us against 12.7, 20000 x 301 26.4 / 18.4,
-  // 300 x 70 4.1 / 2.8)
-  if (!c.ok && cols > 0 && cols <= 256 && rows >= 4096) {
+  // 300 x 70 4.1 / 2.8). The shorter they are, the fewer it takes: 2760 x 1 2.6 / 3.4, 3264 x 2 2.5 / 3.4, 2333 x 23 2.4 / 3.0, 952 x 4 2.2 / 2.5, 414 x 19 2.2 / 2.3;
+  // 1762 x 37 2.9 / 3.0, 652 x 44 2.8 / 2.6; 3632 x 95 3.9 / 4.1, 2392 x 71 3.8 / 3.3.
+  if (!c.ok && cols > 0 && cols <= 256 && rows >= (cols <= 32 ? 768 : cols <= 64 ? 2048 : 4096)) {
     const unsigned g = grid_for(rows, 4);
     const int ci = static_cast<int>(cols);
     auto go = [&](auto npl) {

@@ -982,3 +982,20 @@ def test_strip_gather_on_a_second_device_in_one_process(backend):
             got = gather(src, 0, idx)
             assert bits_equal(got, torch.gather(src, 0, idx)), dev
             ops.check_device_status(torch.device(dev))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(767, 31), (768, 31), (768, 33), (2047, 63), (2048, 63), (2048, 65), (4095, 67), (4096, 67), (3264, 1)])
+def test_layer_norm_of_short_ragged_rows_on_either_side_of_the_lines(backend, dtype, rows, cols):
+    """A warp or a CTA to a row: the same statistics and results. fp32 sums of at most 67 terms: 67 half units in the last place
+    of the statistics at most, 1e-5 of the result; 16-bit results are that, rounded once (2^-8 and 2^-11)."""
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    x = torch.randn(rows * cols + 1, generator=g, device=DEV).to(dtype)[1:].view(rows, cols)
+    w, b = torch.randn(cols, generator=g, device=DEV).to(dtype), torch.randn(cols, generator=g, device=DEV).to(dtype)
+    y, mean, rstd = backend[torch.ops.aten.native_layer_norm.default](x, [cols], w, b, 1e-5)
+    d = x.double()
+    mu = d.mean(1, keepdim=True)
+    rs = 1 / (((d - mu) ** 2).mean(1, keepdim=True) + 1e-5).sqrt()
+    tol = {torch.float32: 1e-5, torch.bfloat16: 2**-8, torch.float16: 2**-10}[dtype]
+    assert torch.allclose(mean.double(), mu, rtol=1e-5, atol=1e-5) and torch.allclose(rstd.double(), rs, rtol=1e-4)
+    assert torch.allclose(y.double(), (d - mu) * rs * w.double() + b.double(), rtol=tol, atol=4 * tol)
