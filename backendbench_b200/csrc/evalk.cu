@@ -63,17 +63,17 @@ __device__ __forceinline__ void warp_merge(CloseAcc& a) {
   }
 }
 
-// Merge the CTA's accumulators (256 threads) and fold them into the record with at most one
+// Merge the CTA's accumulators and fold them into the record with at most one
 // atomic per field per CTA, and only where the CTA's value can still change the record: every
 // atomic of every CTA goes to the same 32 bytes, so they queue up behind one another in L2
 // (one set per WARP cost more time than reading 128 MiB of operands). Non-negative floats
 // order like their bit patterns.
-// `direct`: the record is to start from zero and the launch is one CTA, or (kCloseCluster) one cluster,
+// `direct`: the record is to start from zero and the launch is one CTA, or (kCluster) one cluster,
 // whose CTAs leave their accumulators with the first: it simply writes the record (no memset node before the
 // kernel, no atomics). The first one's shared memory may be written only once that CTA is known to run: every CTA
 // arrives at the cluster's barrier as it starts and waits there before it stores, by when the others have long
 // arrived (their loads come in between).
-constexpr int kCloseCluster = 8;
+constexpr int kCloseCluster = 8, kClusterThreads = 1024;
 __device__ __forceinline__ void cluster_started_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cluster_started_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 __device__ __forceinline__ void write_record(const CloseAcc& a, b200_close_record* rec) {
@@ -83,17 +83,20 @@ __device__ __forceinline__ void write_record(const CloseAcc& a, b200_close_recor
   rec->nan_seen = a.nan_seen;
   rec->pad[0] = rec->pad[1] = rec->pad[2] = 0u;
 }
+template <bool kCluster>
 __device__ __forceinline__ void publish(CloseAcc a, b200_close_record* rec, int direct) {
-  __shared__ CloseAcc part[8], from[kCloseCluster];
+  constexpr int kWarps = kCluster ? kClusterThreads / 32 : 8;
+  __shared__ CloseAcc part[kWarps];
   warp_merge(a);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) part[warp] = a;
   __syncthreads();
   if (warp == 0) {
-    a = lane < 8 ? part[lane] : CloseAcc{0ull, 0.f, 0.f, 0u};
+    a = lane < static_cast<int>(blockDim.x >> 5) ? part[lane] : CloseAcc{0ull, 0.f, 0.f, 0u};
     warp_merge(a);
   }
-  if (direct == kCloseCluster) {
+  if constexpr (kCluster) {
+    __shared__ CloseAcc from[kCloseCluster];
     cg::cluster_group cluster = cg::this_cluster();
     cluster_started_wait();
     if (threadIdx.x == 0) *cluster.map_shared_rank(&from[cluster.block_rank()], 0) = a;
@@ -104,8 +107,7 @@ __device__ __forceinline__ void publish(CloseAcc a, b200_close_record* rec, int 
     if (lane == 0) write_record(a, rec);
     return;
   }
-  if (warp != 0) return;
-  if (lane != 0) return;
+  if (warp != 0 || lane != 0) return;
   if (direct) {
     write_record(a, rec);
     return;
@@ -123,10 +125,10 @@ template <typename T> struct kExpMask16 { static constexpr uint32_t value = 0u; 
 template <> struct kExpMask16<__nv_bfloat16> { static constexpr uint32_t value = 0x7f807f80u; };
 template <> struct kExpMask16<__half> { static constexpr uint32_t value = 0x7c007c00u; };
 
-template <typename T>
-__global__ void __launch_bounds__(256, 4) allclose_kernel(const T* __restrict__ ref, const T* __restrict__ res, int64_t n, float rtol, float atol, b200_close_record* rec, int vec_ok, int direct) {
+template <typename T, bool kCluster>
+__global__ void __launch_bounds__(kCluster ? kClusterThreads : 256, kCluster ? 1 : 4) allclose_kernel(const T* __restrict__ ref, const T* __restrict__ res, int64_t n, float rtol, float atol, b200_close_record* rec, int vec_ok, int direct) {
   constexpr int VE = Vec<T>::N;
-  if (direct == kCloseCluster) cluster_started_arrive();  // (publish waits)
+  if constexpr (kCluster) cluster_started_arrive();  // (publish waits)
   CloseAcc a{0ull, 0.f, 0.f, 0u};
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(256, 4) allclose_kernel(const T* __restrict__ 
     done = nvec * VE;
   }
   for (int64_t i = done + t0; i < n; i += stride) close_step(a, to_f32(ref[i]), to_f32(res[i]), rtol, atol);
-  publish(a, rec, direct);
+  publish<kCluster>(a, rec, direct);
 }
 
 // Integer / bool tensors: the same band as for floating point, |ref - res| <= atol + rtol * |res|,
@@ -193,7 +195,7 @@ __global__ void __launch_bounds__(256) allclose_int_kernel(const T* __restrict__
     a.max_abs = fmaxf(a.max_abs, diff);
     take_rel(a, diff, fabsf(fr) + 1e-10f);
   }
-  publish(a, rec, direct);
+  publish<false>(a, rec, direct);
 }
 
 __global__ void __launch_bounds__(256) l2_flush_kernel(uint4* __restrict__ p, int64_t nvec) {
@@ -203,9 +205,13 @@ __global__ void __launch_bounds__(256) l2_flush_kernel(uint4* __restrict__ p, in
 
 template <typename T>
 static int launch_allclose(const T* ref, const T* res, int64_t n, float rtol, float atol, b200_close_record* rec, int vec_ok, int direct, int grid, cudaStream_t st) {
+  if (direct != kCloseCluster) {
+    allclose_kernel<T, false><<<grid, 256, 0, st>>>(ref, res, n, rtol, atol, rec, vec_ok, direct);
+    return check_launch();
+  }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(direct == kCloseCluster ? kCloseCluster : grid));
-  cfg.blockDim = dim3(256);
+  cfg.gridDim = dim3(kCloseCluster);
+  cfg.blockDim = dim3(n <= 8192 ? 256 : kClusterThreads);
   cfg.stream = st;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -213,8 +219,8 @@ static int launch_allclose(const T* ref, const T* res, int64_t n, float rtol, fl
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = direct == kCloseCluster ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, allclose_kernel<T>, ref, res, n, rtol, atol, rec, vec_ok, direct);
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, allclose_kernel<T, true>, ref, res, n, rtol, atol, rec, vec_ok, direct);
   if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
   return check_launch();
 }

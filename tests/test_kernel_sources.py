@@ -26,7 +26,7 @@ def _body(text, name):
 def test_a_comparison_writes_its_neighbours_memory_only_when_that_runs():
     text = _source("evalk.cu")
     kernel, publish = _body(text, "allclose_kernel"), _body(text, "publish")
-    assert 0 <= kernel.find("cluster_started_arrive()") < kernel.find("ld_stream") < kernel.find("publish(")
+    assert 0 <= kernel.find("cluster_started_arrive()") < kernel.find("ld_stream") < kernel.find("publish<")
     assert 0 <= publish.find("cluster_started_wait()") < publish.find("map_shared_rank")
     assert "return" not in kernel[: kernel.find("cluster_started_arrive()")] and publish.find("return") > publish.find("cluster_started_wait()")
 
