@@ -211,7 +211,7 @@ static int launch_allclose(const T* ref, const T* res, int64_t n, float rtol, fl
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(kCloseCluster);
-  cfg.blockDim = dim3(n <= 8192 ? 256 : kClusterThreads);
+  cfg.blockDim = dim3(n <= kCloseCluster * 256 * Vec<T>::N ? 256 : kClusterThreads);  // (a vector to a thread)
   cfg.stream = st;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
