@@ -26,7 +26,7 @@ struct MulOp { __device__ __forceinline__ float operator()(float a, float b) con
 template <typename T, typename Op>
 __global__ void __launch_bounds__(kEwThreads) ew_unary_vec(const T* x, T* __restrict__ out, int64_t n, Op op) {
   constexpr int VE = Vec<T>::N;
-  next_grid_may_start();
+  if (gridDim.x <= kNumSMs) next_grid_may_start();  // (see launch_unary_fast)
   after_grids_before();
   const T* xw = waited(x);
   const int64_t nvec = n / VE;
@@ -549,6 +549,9 @@ static int strided_grid(int64_t n) {
 template <typename Op>
 static int launch_unary_fast(const void* x, void* out, int64_t n, int dtype, Op op, cudaStream_t st) {
   const int per_block = kEwThreads * kUnroll;
+  // (The next kernel may start at once where this one has a CTA to an SM at most. Its CTAs would take the place of loads in flight in a grid
+  // that fills more of the machine: relu in a row, bf16 1980668 elements 2.5 us, 1.6 so, 2932227 3.3 and 2.1, fp32 1072867 2.5 and 1.8, in the
+  // stream 2.7, 3.3, 2.7 and 1.8, 2.4, 1.9; beyond 4 million elements on a par.)
   cudaError_t e;
   switch (dtype) {
     case B200_F32: e = launch_after(ew_unary_vec<float, Op>, grid_for(n / 4 + 1, per_block), kEwThreads, 0, st, static_cast<const float*>(x), static_cast<float*>(out), n, op); break;
