@@ -107,6 +107,7 @@ __device__ __forceinline__ void ordered_step(float* col, unsigned char* tags, in
 }
 
 // ------------------------------------------------------------------ strip kernel (cols > 1)
+// Nothing is done where `only_if` points to a zero.
 struct StripArgs {
   int64_t outer, rows, cols;         // self / out: [outer, rows, cols] contiguous
   int64_t idx_outer, idx_rows, idx_cols;
@@ -117,8 +118,10 @@ struct StripArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(kStripThreads, 2)
-scatter_add_strip(const T* __restrict__ self, const int64_t* __restrict__ index, const T* __restrict__ src, T* __restrict__ out, StripArgs A, uint32_t* status) {
+scatter_add_strip(const T* __restrict__ self, const int64_t* __restrict__ index, const T* __restrict__ src, T* __restrict__ out, StripArgs A, const int* only_if, uint32_t* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  after_grids_before();
+  if (only_if && *only_if == 0) return;
   constexpr int kIdxTile = kTileRows * kStripCols * 8, kSrcTile = kTileRows * kStripCols * static_cast<int>(sizeof(T));
   unsigned char* ring = smem_raw;                                                                             // stages x (idx tile, src tile)
   unsigned char* tags = smem_raw + static_cast<size_t>(A.stages) * (kIdxTile + kSrcTile) + (threadIdx.x >> 5) * kTagSlots;  // one screening table per warp
@@ -1617,9 +1620,17 @@ static BinnedScratch binned_scratch(const BinnedArgs& A, int es, int64_t n_self,
 }
 
 template <typename T>
-static int launch_binned(const void* self, const void* index, const void* src, void* out, const BinnedArgs& A, const BucketArgs& B, void* scratch, uint32_t* status, cudaStream_t st) {
+static int launch_strip(const void* self, const void* index, const void* src, void* out, StripArgs A, uint32_t* status, cudaStream_t st, const int* only_if = nullptr);
+
+// `strip`: NULL, or the geometry for the strip kernel, which takes a crowded index then: its time does not depend on where the
+// index points. (f16 2672 x 332, all rows into five 108.9 us grouped by destination, 74.9 in strips behind the look at the
+// sample, 67.2 in strips alone; fp32 829 x 156, 23 of them, skewed 285, 118, 110; bins of an even index have one launch that finds
+// nothing to do behind them and not five.)
+template <typename T>
+static int launch_binned(const void* self, const void* index, const void* src, void* out, const BinnedArgs& A, const BucketArgs& B, const StripArgs* strip, void* scratch, uint32_t* status,
+                         cudaStream_t st) {
   typedef typename BinRec<T>::type Rec;
-  const BinnedScratch S = binned_scratch(A, static_cast<int>(sizeof(T)), B.n_self, B.n_idx);
+  const BinnedScratch S = binned_scratch(A, static_cast<int>(sizeof(T)), strip ? 0 : B.n_self, strip ? 0 : B.n_idx);
   int* ctl = static_cast<int*>(scratch);
   char* base = static_cast<char*>(scratch) + 256;
   uint16_t* first = reinterpret_cast<uint16_t*>(base);
@@ -1638,9 +1649,10 @@ static int launch_binned(const void* self, const void* index, const void* src, v
   int2* seg = reinterpret_cast<int2*>(base + 2 * S.head_bytes + S.list_bytes);
   binned_begin<<<1, kSample, 0, st>>>(pi, A, B, ctl);
   if (e == cudaSuccess) e = launch_after(binned_sort<T>, sorts, kBinThreads, sort_smem, st, pi, ps, rec, first, A, ctl, status);
-  if (e == cudaSuccess) e = launch_after(binned_replay<T>, replays, 32, replay_smem, st, px, po, rec, first, A, ctl, head, B.n_self);
+  if (e == cudaSuccess) e = launch_after(binned_replay<T>, replays, 32, replay_smem, st, px, po, rec, first, A, ctl, head, strip ? 0 : B.n_self);
   if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
   if (int rc = check_launch(3)) return rc;
+  if (strip) return launch_strip<T>(self, index, src, out, *strip, status, st, ctl + kCtlGrouped);
   return launch_group<T>(pi, ps, px, po, B, head, cursor, ctl, nullptr, nullptr, list, seg, 0, status, st);
 }
 
@@ -2030,7 +2042,7 @@ static int launch_embedding_backward(const void* grad, const void* idx, void* ou
 }
 
 template <typename T>
-static int launch_strip(const void* self, const void* index, const void* src, void* out, StripArgs A, uint32_t* status, cudaStream_t st) {
+static int launch_strip(const void* self, const void* index, const void* src, void* out, StripArgs A, uint32_t* status, cudaStream_t st, const int* only_if) {
   const int tile_bytes = kTileRows * kStripCols * (8 + static_cast<int>(sizeof(T)));
   const int tag_bytes = (kStripThreads / 32) * kTagSlots;
   // keep at least 4 stages of source tiles; the rest of the budget holds destination rows
@@ -2048,7 +2060,15 @@ static int launch_strip(const void* self, const void* index, const void* src, vo
   if (ae != cudaSuccess) { set_last_cuda_error(ae); return B200_ELAUNCH; }
   const int64_t items = A.outer * (A.cols / kStripCols);
   const int grid = static_cast<int>(items < 8LL * kNumSMs ? items : 8LL * kNumSMs);
-  scatter_add_strip<T><<<grid, kStripThreads, smem, st>>>(static_cast<const T*>(self), static_cast<const int64_t*>(index), static_cast<const T*>(src), static_cast<T*>(out), A, status);
+  const T *px = static_cast<const T*>(self), *ps = static_cast<const T*>(src);
+  const int64_t* pi = static_cast<const int64_t*>(index);
+  T* po = static_cast<T*>(out);
+  if (only_if) {
+    const cudaError_t e = launch_after(scatter_add_strip<T>, grid, kStripThreads, smem, st, px, pi, ps, po, A, only_if, status);
+    if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
+  } else {
+    scatter_add_strip<T><<<grid, kStripThreads, smem, st>>>(px, pi, ps, po, A, only_if, status);
+  }
   return check_launch();
 }
 
@@ -2170,6 +2190,7 @@ enum ScatterPath { kPathNone = 0, kPathStrip, kPathStripWide, kPathRows, kPathBi
 struct ScatterPlan {
   ScatterPath path;
   int64_t n_self, n_idx, scratch_bytes;
+  bool strips;  // bins, with strips for a crowded index
   StripArgs strip;
   RowArgs rows;
   BinnedArgs binned;
@@ -2206,7 +2227,9 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
         const int64_t strips = outer * (cols / kStripCols);
         const bool fits = rows * kStripCols * 4 <= 2 * (kSmemBudget - 64 * 1024);  // at most two destination windows
         P.binned = BinnedArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], index_strides[dt], src_so, src_strides[dim], src_strides[dt]};
-        const bool binned = P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && plan_binned(P.binned);
+        // fp32, as many source rows as rows, lines or chains against bins: 16 x 333 13 / 15 us, 32 x 333 21 / 16, 64 x 63 35 / 15; 65 x 8191 30 / 35,
+        // 100 x 4095 27 / 29, 200 x 4095 39 / 35, 65 x 333 21 / 17, 200 x 63 20 / 15
+        const bool bins_pay = (idx_rows >= 128 || (idx_rows > 24 && cols <= 2048)) && P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && plan_binned(P.binned);
         if (aligned && inner_ok && shape_ok && stride_ok && fits && (strips >= 32 || small)) {
           P.path = kPathStrip;
           P.strip = StripArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], src_so, src_strides[dim], 0, 0};
@@ -2214,13 +2237,12 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
           const bool wide_shape = cols % kWideCols == 0 && idx_cols % kWideCols == 0 && rows <= kWideMaxRows && idx_rows >= 256 && idx_rows < 0x7fffffffLL && outer * (cols / kWideCols) >= kNumSMs / 2;
           const bool wide_align = index_strides[dim] % 2 == 0 && idx_so % 2 == 0 && (src_strides[dim] * es) % 16 == 0 && (src_so * es) % 16 == 0;
           if (wide_shape && wide_align) P.path = kPathStripWide;
-          if (P.path == kPathStripWide || !binned || !binned_beats_strip(P.strip, P.n_idx)) return P;
+          if (P.path == kPathStripWide || !bins_pay || !binned_beats_strip(P.strip, P.n_idx)) return P;
+          P.strips = true;
         }
-        // fp32, as many source rows as rows, lines or chains against bins: 16 x 333 13 / 15 us, 32 x 333 21 / 16, 64 x 63 35 / 15; 65 x 8191 30 / 35,
-        // 100 x 4095 27 / 29, 200 x 4095 39 / 35, 65 x 333 21 / 17, 200 x 63 20 / 15
-        if (binned && (idx_rows >= 128 || (idx_rows > 24 && cols <= 2048))) {
+        if (bins_pay) {
           P.path = kPathBinned;
-          P.scratch_bytes = binned_scratch(P.binned, es, P.n_self, P.n_idx).total;
+          P.scratch_bytes = binned_scratch(P.binned, es, P.strips ? 0 : P.n_self, P.strips ? 0 : P.n_idx).total;
           return P;
         }
       } else if (aligned && index_strides[dim] == 1 && src_strides[dim] == 1) {
@@ -2318,9 +2340,9 @@ extern "C" int b200_scatter_add(const void* self, const void* index, const void*
     }
     if (P.path == kPathBinned) {
       switch (dtype) {
-        case B200_F32: return launch_binned<float>(self, index, src, out, P.binned, A, scratch, status, st);
-        case B200_BF16: return launch_binned<__nv_bfloat16>(self, index, src, out, P.binned, A, scratch, status, st);
-        default: return launch_binned<__half>(self, index, src, out, P.binned, A, scratch, status, st);
+        case B200_F32: return launch_binned<float>(self, index, src, out, P.binned, A, P.strips ? &P.strip : nullptr, scratch, status, st);
+        case B200_BF16: return launch_binned<__nv_bfloat16>(self, index, src, out, P.binned, A, P.strips ? &P.strip : nullptr, scratch, status, st);
+        default: return launch_binned<__half>(self, index, src, out, P.binned, A, P.strips ? &P.strip : nullptr, scratch, status, st);
       }
     }
     const bool chain = P.path == kPathChain;

@@ -49,3 +49,19 @@ def test_nothing_to_compare_is_close_whatever_its_dtype():
     for dtype in (_abi.F32, _abi.I64, _abi.F64, 99):
         assert lib.b200_allclose(None, None, 0, dtype, 0.0, 0.0, ctypes.addressof(rec), 0, None) == 0
     assert lib.b200_allclose(ctypes.addressof(rec), ctypes.addressof(rec), 1, 99, 0.0, 0.0, ctypes.addressof(rec), 0, None) == -2
+
+
+def _scatter_scratch(shape, ishape, dim, dtype, base=1 << 20):
+    """What scatter_add asks for, of contiguous tensors at (aligned) addresses that nobody looks behind."""
+    strides = [1]
+    for n in reversed(ishape[1:]):
+        strides.insert(0, strides[0] * n)
+    a = [_abi.i64_array(v) for v in (shape, ishape, strides, strides)]
+    return _abi.lib().b200_scatter_add_scratch_bytes(base, base, base, base, len(shape), *a, dim, dtype)
+
+
+def test_strips_go_on_where_bins_do_not_pay():
+    """65 to 127 rows of many columns on the strips' grid: bins would be the faster ones, were they open to them."""
+    for shape in ([100, 8192], [65, 40000], [127, 16384], [2, 100, 8192]):
+        assert _scatter_scratch(shape, shape, len(shape) - 2, _abi.F32) == 0, shape
+    assert _scatter_scratch([4000, 512], [4000, 512], 0, _abi.F32) > 0  # bins

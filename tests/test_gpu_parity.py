@@ -999,3 +999,17 @@ def test_layer_norm_of_short_ragged_rows_on_either_side_of_the_lines(backend, dt
     tol = {torch.float32: 1e-5, torch.bfloat16: 2**-8, torch.float16: 2**-10}[dtype]
     assert torch.allclose(mean.double(), mu, rtol=1e-5, atol=1e-5) and torch.allclose(rstd.double(), rs, rtol=1e-4)
     assert torch.allclose(y.double(), (d - mu) * rs * w.double() + b.double(), rtol=tol, atol=4 * tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,ishape", [((4000, 512), (4000, 512)), ((5208, 192), (5208, 192)), ((23, 829, 156), (23, 829, 156)), ((3001, 332), (1501, 328))])
+def test_scatter_add_onto_few_rows_of_a_matrix_on_the_strips_grid(backend, dtype, shape, ishape):
+    """An even index goes through bins, a crowded one (one row, five, skewed) through strips: the same bits as the sequential loop."""
+    g = torch.Generator().manual_seed(12)
+    dim = len(shape) - 2
+    x, src = torch.randn(shape, generator=g).to(dtype), torch.randn(ishape, generator=g).to(dtype)
+    even = torch.randint(0, shape[dim], ishape, generator=g)
+    for idx in (even, even * 0 + 7, even % 5, (torch.rand(ishape, generator=g).double() ** 8 * shape[dim]).long()):
+        got = backend[torch.ops.aten.scatter_add.default](x.to(DEV), dim, idx.to(DEV), src.to(DEV))
+        ops.check_device_status()
+        assert bits_equal(oracle.scatter_add(x, dim, idx, src), got.cpu())
