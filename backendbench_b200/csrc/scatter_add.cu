@@ -1043,7 +1043,7 @@ __global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ index, const T* __restrict__ src, int* __restrict__ head, int2* __restrict__ link, const int* __restrict__ ctl,
                                                   const __grid_constant__ BucketArgs A, uint32_t* status) {
-  if (ctl[kCtlGrouped]) return;
+  if (ctl && ctl[kCtlGrouped]) return;
   for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * kChainUnroll) + threadIdx.x; p0 < A.n_idx; p0 += static_cast<int64_t>(gridDim.x) * (256 * kChainUnroll)) {
     int64_t dest[kChainUnroll];
     T v[kChainUnroll];
@@ -1456,7 +1456,7 @@ __global__ void __launch_bounds__(32) binned_replay(const T* __restrict__ self, 
   const int64_t step = A.c == 32 ? A.cols : 32;
   const int end = A.c < 32 || lane < width ? used : 0;
   after_grids_before();
-  if (ctl[kCtlGrouped]) {  // the counters of the kernels that follow
+  if (ctl && ctl[kCtlGrouped]) {  // the counters of the kernels that follow
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane; i < n_self; i += static_cast<int64_t>(gridDim.x) * 32) head[i] = -1;
     return;
   }
@@ -1602,6 +1602,10 @@ static bool plan_binned(BinnedArgs& A) {
   A.chunks = static_cast<int>((A.idx_rows + A.chunk_rows - 1) / A.chunk_rows);
   return A.outer * A.groups * A.bins < 0x7fffffffLL && columns * A.chunks < 0x7ffffffeLL && static_cast<int64_t>(A.chunks) * A.chunk_rows * A.c < 0x7fffffffLL;
 }
+// With few source rows the worst that a crowded index can do is soon done: a warp that gets all records of its columns walks
+// idx_rows * c of them, 32 to a step, of which 32 / c at most have one destination. So nothing is looked at first and
+// nothing waits behind.
+constexpr int kBinUnseen = 128;
 struct BinnedScratch {
   int64_t first_bytes, rec_bytes, head_bytes, list_bytes, seg_bytes, total;
 };
@@ -1630,8 +1634,10 @@ template <typename T>
 static int launch_binned(const void* self, const void* index, const void* src, void* out, const BinnedArgs& A, const BucketArgs& B, const StripArgs* strip, void* scratch, uint32_t* status,
                          cudaStream_t st) {
   typedef typename BinRec<T>::type Rec;
-  const BinnedScratch S = binned_scratch(A, static_cast<int>(sizeof(T)), strip ? 0 : B.n_self, strip ? 0 : B.n_idx);
-  int* ctl = static_cast<int*>(scratch);
+  const bool unseen = A.idx_rows <= kBinUnseen;
+  const int64_t n_self = strip || unseen ? 0 : B.n_self;
+  const BinnedScratch S = binned_scratch(A, static_cast<int>(sizeof(T)), n_self, strip || unseen ? 0 : B.n_idx);
+  int* ctl = unseen ? nullptr : static_cast<int*>(scratch);
   char* base = static_cast<char*>(scratch) + 256;
   uint16_t* first = reinterpret_cast<uint16_t*>(base);
   Rec* rec = reinterpret_cast<Rec*>(base + S.first_bytes);
@@ -1647,11 +1653,16 @@ static int launch_binned(const void* self, const void* index, const void* src, v
   int* cursor = reinterpret_cast<int*>(base + S.head_bytes);
   int* list = reinterpret_cast<int*>(base + 2 * S.head_bytes);
   int2* seg = reinterpret_cast<int2*>(base + 2 * S.head_bytes + S.list_bytes);
-  binned_begin<<<1, kSample, 0, st>>>(pi, A, B, ctl);
-  if (e == cudaSuccess) e = launch_after(binned_sort<T>, sorts, kBinThreads, sort_smem, st, pi, ps, rec, first, A, ctl, status);
-  if (e == cudaSuccess) e = launch_after(binned_replay<T>, replays, 32, replay_smem, st, px, po, rec, first, A, ctl, head, strip ? 0 : B.n_self);
+  if (unseen) {  // (the call's first kernel is launched the ordinary way)
+    if (e == cudaSuccess) binned_sort<T><<<static_cast<unsigned>(sorts), kBinThreads, sort_smem, st>>>(pi, ps, rec, first, A, ctl, status);
+  } else {
+    binned_begin<<<1, kSample, 0, st>>>(pi, A, B, ctl);
+    if (e == cudaSuccess) e = launch_after(binned_sort<T>, sorts, kBinThreads, sort_smem, st, pi, ps, rec, first, A, ctl, status);
+  }
+  if (e == cudaSuccess) e = launch_after(binned_replay<T>, replays, 32, replay_smem, st, px, po, rec, first, A, ctl, head, n_self);
   if (e != cudaSuccess) { set_last_cuda_error(e); return B200_ELAUNCH; }
-  if (int rc = check_launch(3)) return rc;
+  if (int rc = check_launch(unseen ? 2 : 3)) return rc;
+  if (unseen) return B200_OK;
   if (strip) return launch_strip<T>(self, index, src, out, *strip, status, st, ctl + kCtlGrouped);
   return launch_group<T>(pi, ps, px, po, B, head, cursor, ctl, nullptr, nullptr, list, seg, 0, status, st);
 }
@@ -2229,7 +2240,7 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
         P.binned = BinnedArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], index_strides[dt], src_so, src_strides[dim], src_strides[dt]};
         // fp32, as many source rows as rows, lines or chains against bins: 16 x 333 13 / 15 us, 32 x 333 21 / 16, 64 x 63 35 / 15; 65 x 8191 30 / 35,
         // 100 x 4095 27 / 29, 200 x 4095 39 / 35, 65 x 333 21 / 17, 200 x 63 20 / 15
-        const bool bins_pay = (idx_rows >= 128 || (idx_rows > 24 && cols <= 2048)) && P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && plan_binned(P.binned);
+        const bool bins_pay = (idx_rows >= 128 || (idx_rows > 24 && outer * cols <= 2048)) && P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && plan_binned(P.binned);
         if (aligned && inner_ok && shape_ok && stride_ok && fits && (strips >= 32 || small)) {
           P.path = kPathStrip;
           P.strip = StripArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], src_so, src_strides[dim], 0, 0};
@@ -2242,7 +2253,8 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
         }
         if (bins_pay) {
           P.path = kPathBinned;
-          P.scratch_bytes = binned_scratch(P.binned, es, P.strips ? 0 : P.n_self, P.strips ? 0 : P.n_idx).total;
+          const bool alone = P.strips || idx_rows <= kBinUnseen;
+          P.scratch_bytes = binned_scratch(P.binned, es, alone ? 0 : P.n_self, alone ? 0 : P.n_idx).total;
           return P;
         }
       } else if (aligned && index_strides[dim] == 1 && src_strides[dim] == 1) {

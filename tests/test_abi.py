@@ -65,3 +65,10 @@ def test_strips_go_on_where_bins_do_not_pay():
     for shape in ([100, 8192], [65, 40000], [127, 16384], [2, 100, 8192]):
         assert _scatter_scratch(shape, shape, len(shape) - 2, _abi.F32) == 0, shape
     assert _scatter_scratch([4000, 512], [4000, 512], 0, _abi.F32) > 0  # bins
+
+
+def test_short_lines_side_by_side_stay_lines():
+    """25 to 64 source rows go through bins where there are few columns to walk them, however many dims these are dealt out over."""
+    bins, lines = lambda s: _scatter_scratch(s, s, len(s) - 2, _abi.F32) > 0, lambda s: _scatter_scratch(s, s, len(s) - 2, _abi.F32) == 0
+    assert bins([60, 333]) and bins([4, 60, 333]) and bins([1, 60, 2047])
+    assert lines([24, 333]) and lines([60, 2049]) and lines([267, 64, 23]) and lines([145, 42, 565])

@@ -1013,3 +1013,19 @@ def test_scatter_add_onto_few_rows_of_a_matrix_on_the_strips_grid(backend, dtype
         got = backend[torch.ops.aten.scatter_add.default](x.to(DEV), dim, idx.to(DEV), src.to(DEV))
         ops.check_device_status()
         assert bits_equal(oracle.scatter_add(x, dim, idx, src), got.cpu())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,rows", [((33, 3), 33), ((58, 74), 58), ((9, 48, 31), 48), ((395, 363), 39), ((60, 7), 128), ((700, 33), 129), ((16, 335), 32)])
+def test_scatter_add_of_few_source_rows_onto_few_rows(backend, dtype, shape, rows):
+    """Bins without a look at the index up to 128 source rows, whatever it points to: every record of a column onto one row, five, any."""
+    g = torch.Generator().manual_seed(13)
+    dim = len(shape) - 2
+    ishape = shape[:dim] + (rows,) + shape[dim + 1 :]
+    x, src = torch.randn(shape, generator=g).to(dtype), torch.randn(ishape, generator=g).to(dtype)
+    even = torch.randint(0, shape[dim], ishape, generator=g)
+    for idx in (even, even * 0 + 2, even % 5, (torch.rand(ishape, generator=g).double() ** 8 * shape[dim]).long()):
+        for d_idx in (idx.to(DEV), idx.transpose(-1, -2).contiguous().to(DEV).transpose(-1, -2)):
+            got = backend[torch.ops.aten.scatter_add.default](x.to(DEV), dim, d_idx, src.to(DEV))
+            ops.check_device_status()
+            assert bits_equal(oracle.scatter_add(x, dim, idx, src), got.cpu())
