@@ -1043,7 +1043,7 @@ __global__ void __launch_bounds__(kSample) chain_begin(const int64_t* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256) chain_link(const int64_t* __restrict__ index, const T* __restrict__ src, int* __restrict__ head, int2* __restrict__ link, const int* __restrict__ ctl,
                                                   const __grid_constant__ BucketArgs A, uint32_t* status) {
-  if (ctl && ctl[kCtlGrouped]) return;
+  if (ctl[kCtlGrouped]) return;
   for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * (256 * kChainUnroll) + threadIdx.x; p0 < A.n_idx; p0 += static_cast<int64_t>(gridDim.x) * (256 * kChainUnroll)) {
     int64_t dest[kChainUnroll];
     T v[kChainUnroll];
@@ -1393,7 +1393,7 @@ __global__ void __launch_bounds__(kBinThreads, 2) binned_sort(const int64_t* __r
   if (bad) flag_oob(status);
   next_grid_may_start();
   after_grids_before();  // (the index has been there all along)
-  if (ctl[kCtlGrouped]) return;
+  if (ctl && ctl[kCtlGrouped]) return;
   __syncthreads();
   // counters -> the first place of the run's records of that bin
   int total = 0;

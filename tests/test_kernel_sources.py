@@ -59,3 +59,12 @@ def test_what_the_grid_before_may_still_write_is_not_read_as_if_it_were_constant
         after = body[body.find("after_grids_before()") :]
         assert set(re.findall(r"\b(?:__ldg|__ldcs|ld_keep|ld_stream)\(\W*(\w+)", after)) <= READ_ONLY_ALL_ALONG, name
         assert ("_after(" in after or "_after_f(" in after) == ("waited(" in after), name
+
+
+def test_bins_without_a_control_block_do_not_look_into_one():
+    kernels = _kernels(_source("scatter_add.cu"))
+    for name in ("binned_sort", "binned_replay"):
+        body = kernels[name][1]
+        assert body.count("ctl[") == body.count("ctl && ctl[") == 1, name
+    for name in ("chain_link", "chain_replay", "chain_count", "chain_assign", "chain_fill"):
+        assert "ctl &&" not in kernels[name][1], name
