@@ -37,7 +37,8 @@ def _outcome(fn, args, kwargs):
 
 def _same(a, b):
     if isinstance(a, type) or isinstance(b, type):
-        return a is b or (isinstance(a, type) and isinstance(b, type) and issubclass(a, Exception) and issubclass(b, Exception))
+        # (an argument too many: Python's own refusal on the one side, the operator schema's on the other)
+        return a is b or {a, b} == {TypeError, RuntimeError}
     if isinstance(a, (tuple, list)):
         return len(a) == len(b) and all(_same(x, y) for x, y in zip(a, b))
     if a is None or b is None:
