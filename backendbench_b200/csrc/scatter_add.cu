@@ -2290,6 +2290,15 @@ extern "C" int64_t b200_scatter_add_scratch_bytes(const void* self, const void* 
   return plan_scatter(self, index, src, out, ndim, self_shape, index_shape, index_strides, src_strides, dim, dtype).scratch_bytes;
 }
 
+extern "C" int b200_scatter_add_path(const void* self, const void* index, const void* src, const void* out, int ndim, const int64_t* self_shape, const int64_t* index_shape,
+                                     const int64_t* index_strides, const int64_t* src_strides, int dim, int dtype) {
+  if (ndim < 1 || ndim > B200_MAX_DIMS || dim < 0 || dim >= ndim || !self_shape || !index_shape || !index_strides || !src_strides || !is_float_dtype(dtype)) return B200_EINVAL;
+  const ScatterPath p = plan_scatter(self, index, src, out, ndim, self_shape, index_shape, index_strides, src_strides, dim, dtype).path;
+  static_assert(kPathNone == B200_SCATTER_NONE && kPathStrip == B200_SCATTER_STRIP && kPathStripWide == B200_SCATTER_STRIP_WIDE && kPathRows == B200_SCATTER_ROWS &&
+                    kPathBinned == B200_SCATTER_BINS && kPathBucket == B200_SCATTER_BUCKETS && kPathChain == B200_SCATTER_CHAINS && kPathLines == B200_SCATTER_LINES, "the header's names");
+  return p;
+}
+
 extern "C" int b200_scatter_add(const void* self, const void* index, const void* src, void* out, int ndim, const int64_t* self_shape, const int64_t* index_shape,
                                 const int64_t* index_strides, const int64_t* src_strides, int dim, int dtype, void* scratch, int64_t scratch_bytes, uint32_t* status, void* stream) {
   if (ndim < 1 || ndim > B200_MAX_DIMS || dim < 0 || dim >= ndim || !self_shape || !index_shape || !index_strides || !src_strides) return B200_EINVAL;

@@ -222,11 +222,27 @@ int b200_gather(const void* self, const void* index, void* out, int ndim,
  * for each destination element -- the order of the sequential aten CPU kernel, so fp
  * results are bit-identical to it. self/out contiguous; index/src strided. bf16/f16
  * tensors accumulate in fp32 and round once (as aten CPU does). Wide matrices run on
- * shared-memory strip / row kernels without scratch; tall, narrow or strided geometries
- * chain or group the contributions by destination first and need scratch: counters and a
- * segment of 8 bytes per contribution, and where the scatter dimension is no longer than
- * self's also chain heads and links (8 n_self + 16.4 n_index bytes in all). Ask
- * b200_scatter_add_scratch_bytes with the same arguments and pass at least that much. */
+ * shared-memory strip / row kernels without scratch. Tall or ragged matrices sort the
+ * contributions into bins of rows whose sums stay in shared memory (scratch: a record of 4 or
+ * 8 bytes per contribution, or what grouping a crowded index takes). Other geometries chain or
+ * group the contributions by destination first (scratch: counters and a segment of 8 bytes
+ * per contribution, and where the scatter dimension is no longer than self's also chain heads
+ * and links, 8 n_self + 16.4 n_index bytes in all). Ask b200_scatter_add_scratch_bytes with the
+ * same arguments and pass at least that much. b200_scatter_add_path says which of these a call
+ * takes (negative: invalid arguments); nothing behind the addresses is looked at. */
+enum {
+  B200_SCATTER_NONE = 0,
+  B200_SCATTER_STRIP,
+  B200_SCATTER_STRIP_WIDE,
+  B200_SCATTER_ROWS,
+  B200_SCATTER_BINS,
+  B200_SCATTER_BUCKETS,
+  B200_SCATTER_CHAINS,
+  B200_SCATTER_LINES
+};
+int b200_scatter_add_path(const void* self, const void* index, const void* src, const void* out,
+                          int ndim, const int64_t* self_shape, const int64_t* index_shape,
+                          const int64_t* index_strides, const int64_t* src_strides, int dim, int dtype);
 int64_t b200_scatter_add_scratch_bytes(const void* self, const void* index, const void* src,
                                        const void* out, int ndim, const int64_t* self_shape,
                                        const int64_t* index_shape, const int64_t* index_strides,

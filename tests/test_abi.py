@@ -51,24 +51,44 @@ def test_nothing_to_compare_is_close_whatever_its_dtype():
     assert lib.b200_allclose(ctypes.addressof(rec), ctypes.addressof(rec), 1, 99, 0.0, 0.0, ctypes.addressof(rec), 0, None) == -2
 
 
-def _scatter_scratch(shape, ishape, dim, dtype, base=1 << 20):
-    """What scatter_add asks for, of contiguous tensors at (aligned) addresses that nobody looks behind."""
+STRIP, WIDE, ROWS, BINS, BUCKETS, CHAINS, LINES = range(1, 8)
+
+
+def _scatter_path(shape, ishape, dim, dtype, base=1 << 20, columns=False):
+    """Which kernels serve a scatter_add, and what scratch it asks for, of tensors at (aligned) addresses that nobody looks behind.
+    `columns`: index and src are laid out along their second-to-last dim."""
     strides = [1]
     for n in reversed(ishape[1:]):
         strides.insert(0, strides[0] * n)
+    if columns:
+        strides[-2:] = [1, ishape[-2]]
     a = [_abi.i64_array(v) for v in (shape, ishape, strides, strides)]
-    return _abi.lib().b200_scatter_add_scratch_bytes(base, base, base, base, len(shape), *a, dim, dtype)
+    args = (base, base, base, base, len(shape), *a, dim, dtype)
+    return _abi.lib().b200_scatter_add_path(*args), _abi.lib().b200_scatter_add_scratch_bytes(*args)
 
 
 def test_strips_go_on_where_bins_do_not_pay():
     """65 to 127 rows of many columns on the strips' grid: bins would be the faster ones, were they open to them."""
     for shape in ([100, 8192], [65, 40000], [127, 16384], [2, 100, 8192]):
-        assert _scatter_scratch(shape, shape, len(shape) - 2, _abi.F32) == 0, shape
-    assert _scatter_scratch([4000, 512], [4000, 512], 0, _abi.F32) > 0  # bins
+        assert _scatter_path(shape, shape, len(shape) - 2, _abi.F32) == (STRIP, 0), shape
+    assert _scatter_path([4000, 512], [4000, 512], 0, _abi.F32)[0] == BINS
+    assert _scatter_path([4096, 4096], [4096, 4096], 0, _abi.F32) == (WIDE, 0)
 
 
 def test_short_lines_side_by_side_stay_lines():
     """25 to 64 source rows go through bins where there are few columns to walk them, however many dims these are dealt out over."""
-    bins, lines = lambda s: _scatter_scratch(s, s, len(s) - 2, _abi.F32) > 0, lambda s: _scatter_scratch(s, s, len(s) - 2, _abi.F32) == 0
-    assert bins([60, 333]) and bins([4, 60, 333]) and bins([1, 60, 2047])
-    assert lines([24, 333]) and lines([60, 2049]) and lines([267, 64, 23]) and lines([145, 42, 565])
+    path = lambda s: _scatter_path(s, s, len(s) - 2, _abi.F32)[0]
+    assert path([60, 333]) == path([4, 60, 333]) == path([1, 60, 2047]) == BINS
+    assert path([24, 333]) == path([60, 2049]) == path([267, 64, 23]) == path([145, 42, 565]) == LINES
+
+
+def test_which_matrices_go_through_bins():
+    """The shapes of the bit-exact tests on a GPU, and those on either side of the rules."""
+    for dtype in (_abi.F32, _abi.BF16, _abi.F16):
+        for shape, ishape, dim in (((5003, 33), (5003, 33), 0), ((129, 31), (700, 31), 0), ((20001, 40), (20001, 40), 0), ((600, 65), (20000, 65), 0), ((5, 701, 37), (4, 650, 35), 1),
+                                   ((4100, 70), (2050, 70), 0), ((4100, 45), (4100, 45), 0), ((40, 2), (3001, 2), 0), ((150134, 63), (75067, 63), 0)):
+            assert _scatter_path(shape, ishape, dim, dtype)[0] == BINS, shape
+        assert _scatter_path((4100, 45), (4100, 45), 0, dtype, columns=True)[0] == BINS
+        assert _scatter_path((300, 2), (3001, 2), 0, dtype)[0] == BUCKETS  # more bins than there is room to count in
+        assert _scatter_path((200000, 63), (100000, 63), 0, dtype)[0] == CHAINS
+        assert _scatter_path((70001,), (70001,), 0, dtype)[0] in (ROWS, CHAINS)

@@ -673,13 +673,15 @@ def test_rows_and_elements_off_the_16_byte_grid(backend, dtype):
                 ops.check_device_status()
 
 
-# (self, dim, index, layout of index and src): a column group of one column, one of 31 and of two; bins cut short; more
+# (self, dim, index, layout of index and src): a column group of one column, one of 31 and of two (and one that is grouped by
+# destination, for want of room to count its bins); bins cut short; more
 # contributions than a bin's ring and than destinations; an index smaller than self on every side; one row of indices for all
 # columns, indices and values read across their rows; the last one has no columns to deal out and hangs in chains
 BINNED = [
     ((5003, 33), 0, (5003, 33), "rows"),
     ((129, 31), 0, (700, 31), "rows"),
     ((300, 2), 0, (3001, 2), "rows"),
+    ((40, 2), 0, (3001, 2), "rows"),
     ((20001, 40), 0, (20001, 40), "rows"),
     ((600, 65), 0, (20000, 65), "rows"),
     ((5, 701, 37), 1, (4, 650, 35), "rows"),
