@@ -77,14 +77,15 @@ __global__ void __launch_bounds__(32 * kFewWarps, 2) gemm_few_rows(const T* A, c
   for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
   const int K = static_cast<int>(p.K);  // a multiple of 8: a piece is inside the row or outside it
   // While the kernel before ends, the lines that the warp reads first are brought into L2 (which holds what that
-  // kernel writes all the same, should it be these).
+  // kernel writes all the same, should it be these). A CTA that comes after the first round has nothing to wait for: there it was
+  // the same lines asked for twice (bf16, 3 rows, K 3880 x N 18080 29.8 -> 27.7 us, 13 rows, K 1600 x N 44992 36.6 -> 34.8).
   next_grid_may_start();
 #pragma unroll
   for (int u = 0; u < 2 * kFewSteps; ++u) {
     const int k = (warp + (u / kFewSteps) * kFewWarps) * 32 * kFewSteps + 32 * (u % kFewSteps);
 #pragma unroll
     for (int t = 0; t < NT; ++t)
-      if ((c & 1) == 0 && k + 8 * c < K && col[t]) asm volatile("prefetch.global.L2 [%0];" ::"l"(b[t] + k));
+      if (blockIdx.x < 2 * kNumSMs && (c & 1) == 0 && k + 8 * c < K && col[t]) asm volatile("prefetch.global.L2 [%0];" ::"l"(b[t] + k));
   }
   after_grids_before();
   a0 = waited(a0);
