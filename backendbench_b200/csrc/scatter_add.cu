@@ -1627,9 +1627,9 @@ template <typename T>
 static int launch_strip(const void* self, const void* index, const void* src, void* out, StripArgs A, uint32_t* status, cudaStream_t st, const int* only_if = nullptr);
 
 // `strip`: NULL, or the geometry for the strip kernel, which takes a crowded index then: its time does not depend on where the
-// index points. (f16 2672 x 332, all rows into five 108.9 us grouped by destination, 74.9 in strips behind the look at the
-// sample, 67.2 in strips alone; fp32 829 x 156, 23 of them, skewed 285, 118, 110; bins of an even index have one launch that finds
-// nothing to do behind them and not five.)
+// index points. (f16 2672 x 332, all rows into five, 111.5 us grouped by destination, 72.1 in strips behind the look at the
+// sample, 67.6 in strips alone; fp32 829 x 156, 23 of them, skewed 285, 118, 110; bins of an even index have one launch that finds
+// nothing to do behind them and not five: the first shape 31.2 -> 24.4 us.)
 template <typename T>
 static int launch_binned(const void* self, const void* index, const void* src, void* out, const BinnedArgs& A, const BucketArgs& B, const StripArgs* strip, void* scratch, uint32_t* status,
                          cudaStream_t st) {
@@ -2184,16 +2184,16 @@ static int launch_rows(const void* self, const void* index, const void* src, voi
 
 namespace b200 {
 
-// Nanoseconds, as measured over 64 x 1024 ... 15000 x 1024, 33 x 100000 and 150134 x 63. A strip CTA takes 14.5 for a source row, whatever its
+// Nanoseconds, as measured over 64 x 1024 ... 15000 x 1024 and 150134 x 63. A strip CTA takes 14.5 for a source row, whatever its
 // few columns are (twice that where the destination takes two windows), and 2400 to begin and end, and there are one or two of
-// them per SM; the binned path has more launches to pay for, and then time for each contribution and destination. fp32, as
-// many source rows as rows, strips against bins: 500 x 512 11.5 / 23 us, 2000 x 256 30 / 24, 200 x 4096 27 / 25, 4000 x 512 59 / 35,
-// 12000 x 512 312 / 131, 33 x 100000 236 / 94.
+// them per SM; the binned path has more launches to pay for, and then time for each contribution and destination. Strips
+// against bins, in the stream, as many source rows as rows: fp32 2000 x 256 31.7 / 24.8 us, 4000 x 512 59.6 / 39.7, 12000 x 512 315 / 118, f16 969 x 252
+// 19.6 / 24.8, 2672 x 332 43.2 / 26.9; half as many: fp32 2446 x 168 24.7 / 25.5, bf16 1951 x 140 18.6 / 20.7.
 static bool binned_beats_strip(const StripArgs& S, int64_t n_idx) {
   const int64_t bytes = S.rows * kStripCols * 4, at_once = kNumSMs * (bytes <= kStripSmemTarget - 34 * 1024 ? 2 : 1);
   const int64_t rounds = (S.outer * (S.cols / kStripCols) + at_once - 1) / at_once, windows = bytes <= kSmemBudget - 40 * 1024 ? 1 : 2;
   const double strip = static_cast<double>(rounds) * (14.5 * static_cast<double>(S.idx_rows * windows) + 2400.0) + 2000.0;
-  return strip > 15000.0 + 0.011 * static_cast<double>(n_idx) + 0.003 * static_cast<double>(S.outer * S.rows * S.cols);
+  return strip > 20000.0 + 0.009 * static_cast<double>(n_idx) + 0.003 * static_cast<double>(S.outer * S.rows * S.cols);
 }
 
 enum ScatterPath { kPathNone = 0, kPathStrip, kPathStripWide, kPathRows, kPathBinned, kPathBucket, kPathChain, kPathLines };
@@ -2238,8 +2238,9 @@ static ScatterPlan plan_scatter(const void* self, const void* index, const void*
         const int64_t strips = outer * (cols / kStripCols);
         const bool fits = rows * kStripCols * 4 <= 2 * (kSmemBudget - 64 * 1024);  // at most two destination windows
         P.binned = BinnedArgs{outer, rows, cols, idx_outer, idx_rows, idx_cols, idx_so, index_strides[dim], index_strides[dt], src_so, src_strides[dim], src_strides[dt]};
-        // fp32, as many source rows as rows, lines or chains against bins: 16 x 333 13 / 15 us, 32 x 333 21 / 16, 64 x 63 35 / 15; 65 x 8191 30 / 35,
-        // 100 x 4095 27 / 29, 200 x 4095 39 / 35, 65 x 333 21 / 17, 200 x 63 20 / 15
+        // fp32, as many source rows as rows, lines or chains against bins: 32 x 333 21.2 / 7.1 us, 64 x 63 35.8 / 7.3, 65 x 333 21.5 / 7.5, 128 x 1023
+        // 23.1 / 11.4, 200 x 63 20.8 / 15.7, 200 x 4095 39.6 / 34.1; with the look at the index 65 x 8191 30 / 35 and 100 x 4095 27 / 29. Lines that there are
+        // many of: bf16 64 x 24, 267 of them, 20.3 / 29.5, f16 42 x 565, 145, 66 / 93.
         const bool bins_pay = (idx_rows >= 128 || (idx_rows > 24 && outer * cols <= 2048)) && P.n_self < 0x7fffffffLL && P.n_idx < 0x7fffffffLL && plan_binned(P.binned);
         if (aligned && inner_ok && shape_ok && stride_ok && fits && (strips >= 32 || small)) {
           P.path = kPathStrip;

@@ -71,7 +71,9 @@ def test_strips_go_on_where_bins_do_not_pay():
     """65 to 127 rows of many columns on the strips' grid: bins would be the faster ones, were they open to them."""
     for shape in ([100, 8192], [65, 40000], [127, 16384], [2, 100, 8192]):
         assert _scatter_path(shape, shape, len(shape) - 2, _abi.F32) == (STRIP, 0), shape
-    assert _scatter_path([4000, 512], [4000, 512], 0, _abi.F32)[0] == BINS
+    assert _scatter_path([4000, 512], [4000, 512], 0, _abi.F32)[0] == _scatter_path([2000, 256], [2000, 256], 0, _abi.F32)[0] == BINS
+    for shape, rows in (([969, 252], 969), ([1951, 140], 975), ([500, 512], 500)):
+        assert _scatter_path(shape, [rows, shape[1]], 0, _abi.F16) == (STRIP, 0), shape
     assert _scatter_path([4096, 4096], [4096, 4096], 0, _abi.F32) == (WIDE, 0)
 
 
