@@ -26,13 +26,14 @@ constexpr int kFewWarps = 8;
 constexpr int kFewMaxFragments = 5;       // of eight columns each, to a CTA: see few_fragments
 template <int NT> struct FewSteps { static constexpr int value = NT > 3 ? 3 : 4; };  // 32-k steps in flight per lane
 // Where the kernel is the faster one; bf16 with B out of HBM, us here / the tcgen05 kernel or its ranges of K.
-// The tcgen05 kernel has a CTA to 256 columns: up to 96 of them leave it SMs idle (N 20000, K 4096: 8 rows 33 /
-// 44, 16 rows 43.5 / 44). Beyond, this one wins by what it does not read twice, as long as the rows of A, which
-// every CTA reads from L2, are few (N 32000, K 4096: 8 rows 48 / 52, 16 rows 51 / 48; K 2048: 16 rows 28 / 31) and K
-// is long enough to pay for the many CTAs (N 32000, K 264: 10 / 9; N 128256, K 1024: 4 rows 52 / 65, 16 rows 58 / 52).
+// The tcgen05 kernel has a CTA to 256 columns: up to 96 of them leave it SMs idle (N 20000, K 4096: 8 rows 31.1 /
+// 43.5, 16 rows 33.2 / 37.2; N 24000: 16 rows 41.5 / 40.7). Beyond, this one wins by what it does not read twice, as long as the rows of A,
+// which every CTA reads from L2, are few (N 32000, K 4096: 8 rows 48.9 / 59.0, 16 rows 51.7 / 49.0; K 2048: 16 rows 28.4 / 32.6; between the two the line
+// could lie further out: K 3072, 12 rows 37.7 / 45.5) and K is long enough to pay for the many CTAs (N 32000: K 264 12.0 / 9.9, K 512 13.2 / 10.7, K 768
+// 14.6 / 14.2, K 1024 16.8 / 18.4; N 128256, K 1024: 4 rows 49.5 / 53.8, 16 rows 54.8 / 54.5).
 constexpr int64_t kFewMaxK = 16384;
 constexpr int64_t kFewMaxN = 96 * 256;  // with any number of rows
-constexpr int64_t kFewShortK = 256, kFewShortMaxN = 16384;  // (N 20000, K 64: 10-15 % slower here)
+constexpr int64_t kFewShortK = 256, kFewShortMaxN = 16384;  // (N 20000, K 64: 4 rows 5.3 / 5.1, 16 rows 5.7 / 5.1)
 static bool few_rows_pay(int64_t M, int64_t N, int64_t K) {
   if (N > kFewShortMaxN && K < kFewShortK) return false;
   return N <= kFewMaxN || (K >= (N > 65536 && M > 4 ? 2048 : 1024) && (M <= 8 || K <= 2048));
@@ -144,10 +145,11 @@ bool gemm_few_rows_preferred(const void* A, const void* B, int64_t batch, int64_
   return (M == 1 || (sAm % 8 == 0 && sAm >= 0)) && (N == 1 || (sBn % 8 == 0 && sBn >= 0));
 }
 
-// A CTA walks all of K. With few columns, so few CTAs, a long K is better cut into ranges, where the K-split
-// can take the product: 4 rows, N 512: K 8192 10.4 / 10.5, K 12288 14.7 / 10.3; N 128: K 8192 10.3 / 8.7; N 64: K
-// 8192 8.1 / 8.5, K 11008 11.0 / 9.0; N 1024: K 11008 12.1 / 13.5, K 16384 19.5 / 15.6; N 1536: K 12288 15.9 / 17.9, K 16384 19.7 /
-// 18.7; N 2048: K 16384 20.7 / 21.8; N 1: K 8192 6.1 / 8.0, K 11008 7.0 / 8.2.
+// A CTA walks all of K. With few columns, so few CTAs, a long K can be cut into ranges instead, where the K-split can take the
+// product. The line was drawn with 16 columns to every CTA; with as many as few_fragments gives, few rows do better here on
+// its far side, too, and only 16 rows are near it (here / ranges; 4 rows, N 512: K 8192 6.2 / 10.4, K 12288 8.4 / 11.6; N 128: K 8192 5.6 / 8.0; N 64: K
+// 11008 6.8 / 8.4; N 1024: K 11008 8.3 / 12.8, K 16384 11.6 / 14.5; N 1536: K 16384 12.8 / 16.6; N 2048: K 16384 14.1 / 19.1; 16 rows, N 128: K 8192 7.0 / 8.1; N 1536: K 12288
+// 14.2 / 15.0, K 16384 18.3 / 16.8).
 bool gemm_few_rows_leaves_to_ranges(int64_t N, int64_t K) {
   return N < 2048 && (K > (N <= 1024 ? 11264 : 14336) || (K > 8448 && N >= 16 && N <= 512) || (K > 7168 && N > 64 && N <= 128));
 }
