@@ -2,7 +2,7 @@
 // arguments, allocates the result and calls the C-ABI without the interpreter in between. What bounds a
 // small call is this work and not its kernel: add of 16 x 16 took 12 us of host time (dispatcher 2-3,
 // arguments and layout in Python 3, allocation 1.3, ctypes 3, the launch 2), 4.1 so; the evaluation sweep of 24 small
-// cases 847 us, 376.
+// cases 847 us, 327.
 //
 // Nothing here decides anything new. A call is served when its tensors are plain CUDA tensors of the
 // current device -- no subclass, no mode, no transform, no tracing, no gradient to record -- and its

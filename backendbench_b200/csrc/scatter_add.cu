@@ -14,13 +14,15 @@
 //     source rows at a time, lane = source row. Whether two lanes of a step hit the same
 //     destination is screened with a tiny per-warp tag table (each lane drops its id at a
 //     slot hashed from the destination and reads it back); only on a clash is the rank of
-//     every lane among EARLIER rows with the same destination computed with warp shuffles
-//     and the additions applied rank by rank -- source-row order is kept without
-//     __match_any_sync, whose throughput is ~250-500 cycles per call per SM.
+//     every lane among EARLIER rows with the same destination taken (one match over the
+//     warp) and the additions applied rank by rank: source-row order is kept.
 //   row kernel (cols == 1, i.e. the scatter dimension is the last one): a warp owns two
 //     rows of `outer`, their destination rows sit in shared memory, and the 16 lanes of a
-//     row read 16 consecutive source positions (coalesced) with the same rank-by-shuffle
-//     ordering.
+//     row read 16 consecutive source positions (coalesced) with the same screen and ranks.
+//   bins (matrices too tall for a strip, or off its grid): contributions are sorted by bins of
+//     destination rows, in source order, and a warp adds up a bin's in shared memory.
+//   chains and buckets (neither fits): contributions are chained or grouped by destination
+//     in global memory, and a thread adds up each destination's in order.
 //   Destinations that do not fit in shared memory are processed in windows (each window
 //     re-scans the sources); HBM traffic is the algorithmic minimum otherwise: self, index
 //     and src read once, out written once.
@@ -85,7 +87,7 @@ __device__ __forceinline__ void apply_in_rank_order(float* col, int k, float v, 
 
 // One in-order step of a warp: GROUP adjacent lanes hold consecutive in-order elements of
 // one independent unit (`unit` tells the groups of a warp apart), `col` is that unit's fp32
-// destination array in shared memory. A cheap screen makes the shuffle ranking rare: every
+// destination array in shared memory. A cheap screen makes the ranking rare: every
 // lane drops its lane id into a small per-warp table at a slot hashed from (destination,
 // unit) and reads it back. If all lanes read their own id, no two lanes share a slot, hence
 // no two lanes share a destination, and the additions are applied in one go. A clash (a

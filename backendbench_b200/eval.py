@@ -358,10 +358,9 @@ def cuda_bench_rotating(fns, reps=30, warmup=None, graph=False, replays=5):
     flush overhead); the last len(fns) results are kept alive so outputs rotate too.
 
     `graph=True`: the loop is captured once in a CUDA graph on a side stream (after warm-up
-    calls on that stream, which also size its scratch buffers) and the REPLAY is timed, median
-    of `replays`. Launched from Python, a call of this package costs the host about 20 us, more
-    than several of the kernels take (sum over 64 MiB: 14 us), so an eager loop measures the
-    interpreter; the replay measures the device."""
+    calls on that stream) and the REPLAY is timed, median of `replays`. Launched from Python, a
+    call of this package costs the host 4 us (about 20 through the wrappers alone), more than the
+    smaller kernels take, so an eager loop measures the host; the replay measures the device."""
     n = len(fns)
     ring = [None] * n
     if not graph:

@@ -2,9 +2,9 @@
 
 Loaded by a BackendBench DirectoryBackend (BackendBench/backends/directory.py:47-100):
 the folder name is the overload with "." spelt "__", the exported callable is
-`<folder>_kernel_impl`. The arithmetic runs in libb200ops.so through the C-ABI; this
-file forwards the aten arguments to the `b200::scatter_add` operator, whose CUDA kernel is the host
-wrapper of that C-ABI call.
+`<folder>_kernel_impl`. The arithmetic runs in libb200ops.so through the C-ABI,
+which a plain call reaches straight from native code, every other one (subclasses, modes,
+gradients, other devices) by way of the `b200::scatter_add` operator and its host wrapper.
 """
 
 import os

@@ -192,7 +192,7 @@ def prepare_cases(cases, backend, device):
 def sweep_enqueue(prepared, records, streams=None):
     """Queue one correctness pass (backend launch + fused compare per case); no read-back.
     With `streams`, case i goes to streams[i % len(streams)]: the cases are independent (own
-    inputs, own output, own verdict record, per-stream scratch), so their launch chains can
+    inputs, own output, own verdict record, own scratch), so their launch chains can
     run side by side -- most cases are too small to fill the GPU and their cost is the launch
     gap, not the kernel. The current stream forks to the side streams and joins them again,
     which under graph capture yields a graph with that many parallel branches."""
@@ -664,7 +664,7 @@ def run_b200(args):
     sampler = ClockSampler(local) if rank == 0 else None
     if sampler:
         sampler.start()
-    # Warm up eagerly (also sizes every scratch buffer), then capture the launch sequence of
+    # Warm up eagerly, then capture the launch sequence of
     # one pass -- ~1100 small kernels whose eager cost is host dispatch, not GPU time -- in a
     # CUDA graph; a timed step replays the graph and reads the verdict records back.
     eager_ms, _ = time_steps(lambda: sweep_pass(prepared, records), 1, max(args.warmup, 2))
@@ -674,7 +674,7 @@ def run_b200(args):
         if args.no_graph:
             return None, None
         try:
-            if streams:  # one eager multi-stream pass sizes the per-stream scratch buffers
+            if streams:  # one eager multi-stream pass first
                 sweep_enqueue(subset, recs, streams)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
