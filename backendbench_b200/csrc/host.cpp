@@ -19,6 +19,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/record_function.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
@@ -172,11 +173,60 @@ Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like
 Tensor new_like(const Tensor& t) { return new_tensor(t.sizes(), t.scalar_type(), t); }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// Scratch is the call's own, from the caching allocator: a call is several launches that rely on what the ones before have left
-// there, and the interpreter lock is not held between them, so that a buffer kept per stream would be another thread's, too. It
-// goes back in stream order when the call's launches are queued, and belongs to the graph where they are captured.
-Tensor scratch(const Tensor& like, int64_t bytes) { return bytes > 0 ? new_tensor({bytes}, at::kByte, like) : Tensor(); }
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+// Scratch is the call's own until its launches are queued: a call is several launches that rely on what the ones before have left
+// there, and the interpreter lock is not held between them, so that a buffer kept per stream would be another thread's, too.
+// It comes from the caching allocator and goes back in stream order; up to a megabyte from buffers of that size that earlier calls
+// on the stream have laid down, 64 of them at most (layer norm backward of 278 x 50 9.2 us a call with an allocation each, 8.6 so). What
+// is captured belongs to the graph. The pool is guarded by the interpreter lock; release() empties it.
+class Scratch {
+  struct Free {
+    c10::Device device;
+    void* stream;
+    Tensor buffer;
+  };
+  static constexpr int64_t kKept = 1 << 20;
+  static constexpr size_t kMost = 64;
+
+  Tensor buffer_;
+  void* stream_ = nullptr;  // where the buffer is laid down; NULL: nowhere
+  bool kept_ = false;
+
+ public:
+  static std::vector<Free>& pool() {
+    static auto* p = new std::vector<Free>();  // never destroyed: no CUDA calls at exit
+    return *p;
+  }
+  Scratch(const Tensor& like, int64_t bytes) {
+    if (bytes <= 0) return;
+    kept_ = bytes <= kKept && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+    if (kept_) {
+      stream_ = stream();
+      auto& p = pool();
+      for (auto it = p.rbegin(); it != p.rend(); ++it)
+        if (it->stream == stream_ && it->device == like.device()) {
+          buffer_ = std::move(it->buffer);
+          p.erase(std::next(it).base());
+          return;
+        }
+    }
+    buffer_ = new_tensor({kept_ ? kKept : bytes}, at::kByte, like);
+  }
+  ~Scratch() {
+    if (!kept_ || !buffer_.defined()) return;
+    auto& p = pool();
+    Tensor oldest;  // (given back when the pool is in order again)
+    if (p.size() >= kMost) {
+      oldest = std::move(p.front().buffer);
+      p.erase(p.begin());
+    }
+    p.push_back(Free{buffer_.device(), stream_, std::move(buffer_)});
+  }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  void* data() const { return ptr(buffer_); }
+};
 
 // The device's status word (ops._status); nullptr with an exception set if that failed
 uint32_t* status_word(const Tensor& t) {
@@ -412,8 +462,8 @@ PyObject* sum(ARGS) {
   if (out.numel() == 0) return wrap(std::move(out));
   const int64_t outer = product(x->sizes(), 0, first), len = product(x->sizes(), first, last + 1), inner = product(x->sizes(), last + 1, x->dim());
   const int64_t need = api.b200_reduce_scratch_bytes(outer, len, inner);
-  Tensor s = scratch(*x, need);
-  if (!launched("b200_sum", [&, st = stream()] { return api.b200_sum(ptr(*x), ptr(out), outer, len, inner, dt(*x), dt(*x), ptr(s), need, st); })) return nullptr;
+  Scratch s(*x, need);
+  if (!launched("b200_sum", [&, st = stream()] { return api.b200_sum(ptr(*x), ptr(out), outer, len, inner, dt(*x), dt(*x), s.data(), need, st); })) return nullptr;
   return wrap(std::move(out));
 }
 
@@ -432,8 +482,8 @@ PyObject* argmax(ARGS) {
   const int64_t outer = product(x->sizes(), 0, d), inner = product(x->sizes(), d + 1, x->dim());
   Tensor out = new_tensor(shape, at::kLong, *x);
   const int64_t need = api.b200_reduce_scratch_bytes(outer, x->size(d), inner);
-  Tensor s = scratch(*x, need);
-  if (!launched("b200_argmax", [&, st = stream()] { return api.b200_argmax(ptr(*x), static_cast<int64_t*>(ptr(out)), outer, x->size(d), inner, dt(*x), ptr(s), need, st); })) return nullptr;
+  Scratch s(*x, need);
+  if (!launched("b200_argmax", [&, st = stream()] { return api.b200_argmax(ptr(*x), static_cast<int64_t*>(ptr(out)), outer, x->size(d), inner, dt(*x), s.data(), need, st); })) return nullptr;
   return wrap(std::move(out));
 }
 
@@ -492,9 +542,9 @@ PyObject* layer_norm_backward(ARGS) {
   if (mask[1]) dw = new_tensor(shape, wb, *x);
   if (mask[2]) db = new_tensor(shape, wb, *x);
   const int64_t need = mask[1] || mask[2] ? api.b200_layer_norm_backward_scratch_bytes(rows, cols) : 0;
-  Tensor s = scratch(*x, need);
+  Scratch s(*x, need);
   if (!launched("b200_layer_norm_backward", [&, st = stream()] {
-        return api.b200_layer_norm_backward(ptr(*dy), ptr(*x), ptr(*mean), ptr(*rstd), ptr(*w), ptr(dx), ptr(dw), ptr(db), rows, cols, dt(*x), wb_dt, dt(*mean), ptr(s), need, st);
+        return api.b200_layer_norm_backward(ptr(*dy), ptr(*x), ptr(*mean), ptr(*rstd), ptr(*w), ptr(dx), ptr(dw), ptr(db), rows, cols, dt(*x), wb_dt, dt(*mean), s.data(), need, st);
       }))
     return nullptr;
   auto or_none = [](Tensor t) { return t.defined() ? wrap(std::move(t)) : Py_NewRef(Py_None); };
@@ -538,8 +588,8 @@ PyObject* embedding_backward(ARGS) {
   uint32_t* status = status_word(*g);
   if (!status) return nullptr;
   const int64_t need = api.b200_embedding_backward_scratch_bytes(n, rows);
-  Tensor s = scratch(*g, need);
-  if (!launched("b200_embedding_backward", [&, st = stream()] { return api.b200_embedding_backward(ptr(*g), ptr(*idx), ptr(out), n, rows, width, padding, dt(*g), index_dt(*idx), ptr(s), need, status, st); }))
+  Scratch s(*g, need);
+  if (!launched("b200_embedding_backward", [&, st = stream()] { return api.b200_embedding_backward(ptr(*g), ptr(*idx), ptr(out), n, rows, width, padding, dt(*g), index_dt(*idx), s.data(), need, status, st); }))
     return nullptr;
   return wrap(std::move(out));
 }
@@ -604,9 +654,9 @@ PyObject* scatter_add(ARGS) {
   const int nd = static_cast<int>(x->dim()), t = dt(*x);
   const int64_t *ss = x->sizes().data(), *is = idx->sizes().data(), *ist = idx->strides().data(), *rst = src->strides().data();
   const int64_t need = api.b200_scatter_add_scratch_bytes(ptr(*x), ptr(*idx), ptr(*src), ptr(out), nd, ss, is, ist, rst, static_cast<int>(d), t);
-  Tensor s = scratch(*x, need);
+  Scratch s(*x, need);
   if (!launched("b200_scatter_add",
-                [&, st = stream()] { return api.b200_scatter_add(ptr(*x), ptr(*idx), ptr(*src), ptr(out), nd, ss, is, ist, rst, static_cast<int>(d), t, ptr(s), need, status, st); }))
+                [&, st = stream()] { return api.b200_scatter_add(ptr(*x), ptr(*idx), ptr(*src), ptr(out), nd, ss, is, ist, rst, static_cast<int>(d), t, s.data(), need, status, st); }))
     return nullptr;
   return wrap(std::move(out));
 }
@@ -671,19 +721,19 @@ PyObject* gemm(Operand a, Operand b, const Tensor& bias, int64_t batch, int64_t 
   if (t == B200_F32 && macs >= f32_split_min_macs && K >= 32 && M > 64 && N > 64 && (tiles >= 8 || macs >= (1LL << 30))) {
     const int64_t need = api.b200_gemm_f32_scratch_bytes(batch, M, N, K);
     if (need > 0) {
-      Tensor s = scratch(a.t, need);
+      Scratch s(a.t, need);
       done = true;
       ok = launched("b200_gemm_f32", [&, st = stream()] {
-        return api.b200_gemm_f32(ptr(a.t), ptr(b.t), ptr(bias), ptr(out), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, sbm, sbn, alpha, beta, ptr(s), need, status, st);
+        return api.b200_gemm_f32(ptr(a.t), ptr(b.t), ptr(bias), ptr(out), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, sbm, sbn, alpha, beta, s.data(), need, status, st);
       });
     }
   } else if (t != B200_F32 && batch == 1 && K >= splitk_min_k && M * N <= splitk_max_outputs) {
     const int64_t need = api.b200_gemm_splitk_scratch_bytes(ptr(a.t), ptr(b.t), ptr(out), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, t);
     if (need > 0) {
-      Tensor s = scratch(a.t, need);
+      Scratch s(a.t, need);
       done = true;
       ok = launched("b200_gemm_splitk", [&, st = stream()] {
-        return api.b200_gemm_splitk(ptr(a.t), ptr(b.t), ptr(bias), ptr(out), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, sbm, sbn, alpha, beta, t, ptr(s), need, status, st);
+        return api.b200_gemm_splitk(ptr(a.t), ptr(b.t), ptr(bias), ptr(out), batch, M, N, K, a.batch, a.row, a.col, b.batch, b.row, b.col, sbm, sbn, alpha, beta, t, s.data(), need, status, st);
       });
     }
   }
@@ -812,6 +862,16 @@ PyObject* make(PyObject*, PyObject* args) {
   return PyErr_Format(PyExc_KeyError, "%s", name);
 }
 
+// release(): the scratch that no call is using goes back to the allocator
+PyObject* release(PyObject*, PyObject*) {
+  HANDLE_TH_ERRORS
+  auto free = std::move(Scratch::pool());
+  Scratch::pool().clear();
+  free.clear();
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
 // compare(reference, result, atol, rtol, record): the pairs of tensors are queued into the device record. False: nothing
 // was done, the structures are not what this serves (tensors of one shape and floating dtype, contiguous, or a tuple of them).
 PyObject* compare(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -849,6 +909,7 @@ PyObject* compare(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 PyMethodDef kMethods[] = {{"setup", setup, METH_VARARGS, nullptr},
                           {"make", make, METH_VARARGS, nullptr},
+                          {"release", release, METH_NOARGS, nullptr},
                           {"compare", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(compare)), METH_FASTCALL, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_b200host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

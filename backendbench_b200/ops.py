@@ -19,7 +19,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import torch
 
-from . import _abi
+from . import _abi, _native
 from ._abi import check, i64_array, lib
 
 _DT = {
@@ -416,14 +416,21 @@ def _log_softmax_default(self, dim, half_to_float) -> torch.Tensor:
     return _softmax_impl(self, dim, bool(half_to_float), True)
 
 
-_scratch_cache = {}  # holds nothing: scratch does not outlive its call
+_scratch_cache = {}  # holds nothing: the wrappers' scratch does not outlive its call
 
 
 def _scratch(device: torch.device, nbytes: int) -> torch.Tensor:
-    """`nbytes` of scratch for one call, which keeps it until its launches are queued. (No buffer
-    per stream is kept: the launches of two threads' calls can interleave on a stream, ctypes
-    lets go of the interpreter lock, and each call relies on what its earlier kernels left there.)"""
+    """`nbytes` of scratch for one call, which keeps it until its launches are queued. (No call shares
+    it: the launches of two threads' calls can interleave on a stream, ctypes lets go of the
+    interpreter lock, and each call relies on what its earlier kernels left there.)"""
     return _new((nbytes,), torch.uint8, device)
+
+
+def release_scratch() -> None:
+    """Give the small buffers that native calls keep between them (64 of a megabyte at most) back to the allocator."""
+    native = _native.module()
+    if native is not None:
+        native.release()
 
 
 def _reduce_layout(self: torch.Tensor, dims: List[int]):

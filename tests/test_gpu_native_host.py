@@ -285,6 +285,9 @@ def test_threads_that_share_a_stream(backend, native):
     [t.join() for t in threads]
     ops.check_device_status()
     assert not wrong, wrong
+    ops.release_scratch()
+    for calls, w in zip(work, want):
+        assert all(_same(x, call[n](*args)) for (n, args), x in zip(calls, w))
 
 
 def test_comparisons_queued_natively_give_the_same_records(monkeypatch):
