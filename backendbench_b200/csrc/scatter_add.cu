@@ -1001,7 +1001,8 @@ __device__ __forceinline__ int equal_pairs(const int (&key)[kSample / THREADS], 
   __syncthreads();
   return all;
 }
-__device__ __forceinline__ bool crowded(int pairs, int s, double places) { return pairs > 16.0 + 4.0 * (static_cast<double>(s) * s / (2.0 * places)); }
+// `times` as many pairs as an even index has on average
+__device__ __forceinline__ bool crowded(int pairs, int s, double places, double times = 4.0) { return pairs > 16.0 + times * (static_cast<double>(s) * s / (2.0 * places)); }
 // This thread's samples: their destinations, -1 where there is none.
 template <int THREADS>
 __device__ __forceinline__ int sample_destinations(const int64_t* __restrict__ index, const BucketArgs& A, int (&dest)[kSample / THREADS]) {
@@ -1320,7 +1321,7 @@ __device__ __forceinline__ int bin_scan(int v, int* sums, int& total) {
 
 // Looks at a sample: where the destinations, or the bins, are crowded, one warp would walk most of the
 // records, and everything is grouped by destination instead, as on the chain path.
-__global__ void __launch_bounds__(kSample) binned_begin(const int64_t* __restrict__ index, const __grid_constant__ BinnedArgs A, const __grid_constant__ BucketArgs B, int* __restrict__ ctl) {
+__global__ void __launch_bounds__(kSample) binned_begin(const int64_t* __restrict__ index, const __grid_constant__ BinnedArgs A, const __grid_constant__ BucketArgs B, int* __restrict__ ctl, double times) {
   __shared__ int table[4 * kSample];
   next_grid_may_start();
   int dest[1];
@@ -1334,7 +1335,7 @@ __global__ void __launch_bounds__(kSample) binned_begin(const int64_t* __restric
   if (threadIdx.x == 0) {
     ctl[kCtlSlots] = 0;
     ctl[kCtlListed] = 0;
-    ctl[kCtlGrouped] = crowded(same, s, static_cast<double>(A.idx_outer) * A.idx_cols * A.rows) || crowded(near, s, static_cast<double>(A.idx_outer) * A.idx_groups * A.bins) ? 1 : 0;
+    ctl[kCtlGrouped] = crowded(same, s, static_cast<double>(A.idx_outer) * A.idx_cols * A.rows, times) || crowded(near, s, static_cast<double>(A.idx_outer) * A.idx_groups * A.bins, times) ? 1 : 0;
   }
 }
 
@@ -1630,7 +1631,7 @@ static int launch_strip(const void* self, const void* index, const void* src, vo
 
 // `strip`: NULL, or the geometry for the strip kernel, which takes a crowded index then: its time does not depend on where the
 // index points. (f16 2672 x 332, all rows into five, 111.5 us grouped by destination, 72.1 in strips behind the look at the
-// sample, 67.6 in strips alone; fp32 829 x 156, 23 of them, skewed 285, 118, 110; bins of an even index have one launch that finds
+// sample, 67.6 in strips alone; fp32 181 x 8164, 362 skewed rows of it, 195 in bins that are not crowded enough for groups, 102, 95; fp32 829 x 156, 23 of them, skewed 285, 118, 110; bins of an even index have one launch that finds
 // nothing to do behind them and not five: the first shape 31.2 -> 24.4 us.)
 template <typename T>
 static int launch_binned(const void* self, const void* index, const void* src, void* out, const BinnedArgs& A, const BucketArgs& B, const StripArgs* strip, void* scratch, uint32_t* status,
@@ -1658,7 +1659,7 @@ static int launch_binned(const void* self, const void* index, const void* src, v
   if (unseen) {  // (the call's first kernel is launched the ordinary way)
     if (e == cudaSuccess) binned_sort<T><<<static_cast<unsigned>(sorts), kBinThreads, sort_smem, st>>>(pi, ps, rec, first, A, ctl, status);
   } else {
-    binned_begin<<<1, kSample, 0, st>>>(pi, A, B, ctl);
+    binned_begin<<<1, kSample, 0, st>>>(pi, A, B, ctl, strip ? 1.5 : 4.0);  // (strips cost little more than even bins, groups several times as much)
     if (e == cudaSuccess) e = launch_after(binned_sort<T>, sorts, kBinThreads, sort_smem, st, pi, ps, rec, first, A, ctl, status);
   }
   if (e == cudaSuccess) e = launch_after(binned_replay<T>, replays, 32, replay_smem, st, px, po, rec, first, A, ctl, head, n_self);

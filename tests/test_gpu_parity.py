@@ -1004,7 +1004,7 @@ def test_layer_norm_of_short_ragged_rows_on_either_side_of_the_lines(backend, dt
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("shape,ishape", [((4000, 512), (4000, 512)), ((5208, 192), (5208, 192)), ((23, 829, 156), (23, 829, 156)), ((3001, 332), (1501, 328))])
+@pytest.mark.parametrize("shape,ishape", [((4000, 512), (4000, 512)), ((5208, 192), (5208, 192)), ((23, 829, 156), (23, 829, 156)), ((3001, 332), (1501, 328)), ((181, 8164), (362, 8164))])
 def test_scatter_add_onto_few_rows_of_a_matrix_on_the_strips_grid(backend, dtype, shape, ishape):
     """An even index goes through bins, a crowded one (one row, five, skewed) through strips: the same bits as the sequential loop."""
     g = torch.Generator().manual_seed(12)
